@@ -20,6 +20,7 @@
 // memory; when memory binds (an allocation fails) S is halved down to 1, pure
 // uncomputation.
 #include <algorithm>
+#include <cmath>
 #include <complex>
 #include <cstring>
 #include <vector>
@@ -101,21 +102,189 @@ __global__ void __launch_bounds__(kAThreads) k_inner(const typename Elem<C64>::T
     block_sum2(ff2d(sr.h, sr.l), ff2d(si.h, si.l), out2);
 }
 
-// Dual-state tile sweep for the backward pass.
-//   kind 0 dense / 1 diagonal / 2 monomial: applied to both psi and lambda tiles;
-//   kind 3 gradient marker: acc[slot] += w * Im <lambda|G|psi> over the tile, G a
-//          Pauli string (xm on tile-local bits, zm on global bits, phase ph) or,
-//          when k == 1, the projector P1 on global bit gbit[0].
+// ---------------------------------------------------------------- backward sweep of both states
+// One sweep loads the same tile of psi and lambda, applies a run of daggered gates to both, and
+// accumulates the inner products of the run's parameterised gates on the way.  Items:
+//   kind 0 dense / 1 diagonal / 2 monomial: applied to both tiles;
+//   kind 3 marker: grad[slot] += w * Im <lambda|G|psi> over the tile, G a Pauli string that flips
+//          bits (xm on tile-local bits, zm on global bits, phase ph);
+//   kind 6 a 1-target dense gate whose marker (generator X or Y on the same bit) comes right before
+//          it: one pass over the pairs takes the inner product and applies the gate;
+//   kind 7 a diagonal phase: every diagonal gate and every diagonal-generator marker that the order
+//          of the run lets stand at this point.  Diagonal unitaries leave conj(lambda_i) psi_i as it
+//          is, so all these markers are sign sums of one vector v_i = Im conj(lambda_i) psi_i, formed
+//          once; the gates are folded on the host (FP64) into tables over up to 8 bits.
+// The markers of a phase: the 3 tile bits above the thread index are transformed in registers
+// (Walsh-Hadamard, 3 stages), the 8 x 512 partial sums go to shared memory, and each marker is then
+// one warp's signed sum of 512 of them, instead of a pass over both tiles with a block reduction
+// each (an ansatz layer has two diagonal parameters for every rotation).
+// What bounds it: FP32/INT issue.  512 threads: the complex128 tiles (128 KiB) allow one CTA per SM,
+// which at 256 threads left 8 warps to hide every latency.
 struct AdjGate {
-    TileGate g;
-    uint32_t xm_local;
-    int32_t ph;
+    TileGate g;          // kinds 0 and 6: npar = matrix class (0 complex, 1 real, 2 real diagonal and imaginary off-diagonal)
+    uint32_t xm_local;   // kind 7: first table
+    int32_t ph;          // kind 6: 0 generator X, 1 generator Y; kind 7: number of markers
     uint64_t zm;
+    int32_t slot;        // kind 7: first marker
+    int32_t n_tabs;      // kind 7: number of tables
+    double weight;
+};
+struct AdjTab {          // a folded diagonal: index bit q is tile bit pos[q], or global bit gbit[q] when pos[q] < 0
+    int32_t k, mat_off;
+    int8_t pos[8], gbit[8];
+};
+struct AdjMark {         // grad[slot] += weight * sum_i (-1)^popc(i & z) v_i; z split into tile and outer bits
+    uint64_t z_out;
+    uint32_t z_tile;
     int32_t slot;
-    int32_t projector;
     double weight;
 };
 
+constexpr int kSweepThreads = 512, kSweepLog = 9, kSweepPer = 4096 >> kSweepLog;   // values per thread of a 2^12 tile
+constexpr int kRotMax = 32;      // kind 6 / kind 3 sums kept per CTA before they are added to the result
+constexpr int kTabsPerPass = 4;
+
+// The two storages: complex128 tiles hold float-float values (float4: re hi, re lo, im hi, im lo) and
+// gates run in float-float; complex64 tiles hold float2 and gates run in FP32.  Inner products are
+// float-float sums of exact products in both.
+template <bool C64> struct Tile;
+template <> struct Tile<false> {
+    using S = float4;
+    using A = cff;
+    using G = double2;
+    static __device__ __forceinline__ A ld(const S& v) { return f4c(v); }
+    static __device__ __forceinline__ S st(const A& v) { return c4f(v); }
+    static __device__ __forceinline__ S from(const G& v) { return c4f(load_c128(v)); }
+    static __device__ __forceinline__ G to(const S& v) { return store_c128(f4c(v)); }
+    static __device__ __forceinline__ A mul(const float4& m, const A& x) { return cmul(f4c(m), x); }
+    static __device__ __forceinline__ A ipow(const A& x, int p) { return cmul_ipow(x, p); }
+    // a x + b y; CLS 1: a, b real; 2: a real, b imaginary (the dropped products are zeros)
+    template <int CLS>
+    static __device__ __forceinline__ A lin2(const float4& a, const A& x, const float4& b, const A& y) {
+        ffacc r, i;
+        if (CLS == 0) {
+            cmac_first(r, i, f4c(a), x);
+            cmac(r, i, f4c(b), y);
+        } else {
+            acc_first(r, a.x, a.y, x.rh, x.rl);
+            acc_first(i, a.x, a.y, x.ih, x.il);
+            if (CLS == 1) {
+                acc_add(r, b.x, b.y, y.rh, y.rl);
+                acc_add(i, b.x, b.y, y.ih, y.il);
+            } else {
+                acc_add(r, -b.z, -b.w, y.ih, y.il);
+                acc_add(i, b.z, b.w, y.rh, y.rl);
+            }
+        }
+        return cdone(r, i);
+    }
+    static __device__ __forceinline__ ff im_conj(const A& l, const A& x) {
+        ffacc m;
+        acc_first(m, l.rh, l.rl, x.ih, x.il);
+        acc_add(m, -l.ih, -l.il, x.rh, x.rl);
+        return acc_done(m);
+    }
+    static __device__ __forceinline__ ff re_conj(const A& l, const A& x) {
+        ffacc m;
+        acc_first(m, l.rh, l.rl, x.rh, x.rl);
+        acc_add(m, l.ih, l.il, x.ih, x.il);
+        return acc_done(m);
+    }
+};
+template <> struct Tile<true> {
+    using S = float2;
+    using A = float2;
+    using G = float2;
+    static __device__ __forceinline__ A ld(const S& v) { return v; }
+    static __device__ __forceinline__ S st(const A& v) { return v; }
+    static __device__ __forceinline__ S from(const G& v) { return v; }
+    static __device__ __forceinline__ G to(const S& v) { return v; }
+    static __device__ __forceinline__ A mul(const float4& m, const A& x) {
+        return make_float2(__fmaf_rn(m.x, x.x, -m.z * x.y), __fmaf_rn(m.x, x.y, m.z * x.x));
+    }
+    static __device__ __forceinline__ A ipow(const A& x, int p) {
+        switch (p & 3) {
+            case 0: return x;
+            case 1: return make_float2(-x.y, x.x);
+            case 2: return make_float2(-x.x, -x.y);
+            default: return make_float2(x.y, -x.x);
+        }
+    }
+    template <int CLS>
+    static __device__ __forceinline__ A lin2(const float4& a, const A& x, const float4& b, const A& y) {
+        if (CLS == 0) {
+            const float2 u = make_float2(__fmaf_rn(a.x, x.x, -a.z * x.y), __fmaf_rn(a.x, x.y, a.z * x.x));
+            return make_float2(__fmaf_rn(b.x, y.x, __fmaf_rn(-b.z, y.y, u.x)), __fmaf_rn(b.x, y.y, __fmaf_rn(b.z, y.x, u.y)));
+        }
+        if (CLS == 1) return make_float2(__fmaf_rn(b.x, y.x, a.x * x.x), __fmaf_rn(b.x, y.y, a.x * x.y));
+        return make_float2(__fmaf_rn(-b.z, y.y, a.x * x.x), __fmaf_rn(b.z, y.x, a.x * x.y));
+    }
+    static __device__ __forceinline__ ff im_conj(const A& l, const A& x) {
+        ffacc m;
+        acc_first(m, l.x, 0.f, x.y, 0.f);
+        acc_add(m, -l.y, 0.f, x.x, 0.f);
+        return acc_done(m);
+    }
+    static __device__ __forceinline__ ff re_conj(const A& l, const A& x) {
+        ffacc m;
+        acc_first(m, l.x, 0.f, x.x, 0.f);
+        acc_add(m, l.y, 0.f, x.y, 0.f);
+        return acc_done(m);
+    }
+};
+
+__device__ __forceinline__ int insert_zero(int x, int bit) { return ((x >> bit) << (bit + 1)) | (x & ((1 << bit) - 1)); }
+
+// float-float sum over a warp, by shuffles (an FP64 shuffle sum would cost 16 cycles of the SM's FP64
+// pipe per step and warp)
+__device__ __forceinline__ void warp_fsum(ffsum& a) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const float h = __shfl_xor_sync(0xffffffffu, a.h, o), l = __shfl_xor_sync(0xffffffffu, a.l, o);
+        fsum_add(a, h, l);
+    }
+}
+
+// A 1-target dense gate on both tiles.  ROT: 0 no marker, 1 generator X, 2 generator Y on the same bit;
+// the return value is then this thread's part of Im <lambda|G|psi> (before the gate).
+template <bool C64, int CLS, int ROT>
+__device__ __forceinline__ ffsum adj_1q(typename Tile<C64>::S* sa, typename Tile<C64>::S* sb, int T, const TileGate& g,
+                                        const float4* __restrict__ mats) {
+    using P = Tile<C64>;
+    const int t = g.tbit[0], b = 1 << t, ngroups = 1 << (T - 1);
+    const float4* m = mats + g.mat_off;
+    const float4 m00 = __ldg(m), m01 = __ldg(m + 1), m10 = __ldg(m + 2), m11 = __ldg(m + 3);
+    const int lcm = (int)g.lc_mask, lcv = (int)g.lc_val;
+    ffsum acc{0.f, 0.f};
+    for (int gr = threadIdx.x; gr < ngroups; gr += kSweepThreads) {
+        const int j0 = insert_zero(gr, t), j1 = j0 | b;
+        if (ROT == 0 && (j0 & lcm) != lcv) continue;
+        const auto x0 = P::ld(sa[j0]), x1 = P::ld(sa[j1]), y0 = P::ld(sb[j0]), y1 = P::ld(sb[j1]);
+        if (ROT == 1) {          // X: Im (conj(l0) x1 + conj(l1) x0)
+            const ff u = P::im_conj(y0, x1), v = P::im_conj(y1, x0);
+            fsum_add(acc, u.h, u.l);
+            fsum_add(acc, v.h, v.l);
+        } else if (ROT == 2) {   // Y: Im (-i conj(l0) x1 + i conj(l1) x0)
+            const ff u = P::re_conj(y0, x1), v = P::re_conj(y1, x0);
+            fsum_add(acc, -u.h, -u.l);
+            fsum_add(acc, v.h, v.l);
+        }
+        sa[j0] = P::st(P::template lin2<CLS>(m00, x0, m01, x1));
+        sa[j1] = CLS == 2 ? P::st(P::template lin2<CLS>(m11, x1, m10, x0)) : P::st(P::template lin2<CLS>(m10, x0, m11, x1));
+        sb[j0] = P::st(P::template lin2<CLS>(m00, y0, m01, y1));
+        sb[j1] = CLS == 2 ? P::st(P::template lin2<CLS>(m11, y1, m10, y0)) : P::st(P::template lin2<CLS>(m10, y0, m11, y1));
+    }
+    return acc;
+}
+template <bool C64, int ROT>
+__device__ __forceinline__ ffsum adj_1q_cls(typename Tile<C64>::S* sa, typename Tile<C64>::S* sb, int T, const TileGate& g,
+                                            const float4* __restrict__ mats) {
+    if (g.npar == 1) return adj_1q<C64, 1, ROT>(sa, sb, T, g, mats);
+    if (g.npar == 2) return adj_1q<C64, 2, ROT>(sa, sb, T, g, mats);
+    return adj_1q<C64, 0, ROT>(sa, sb, T, g, mats);
+}
+
+// 2- to 4-target dense gates, one tile at a time
 template <int K>
 __device__ void adj_dense(float4* sm, int T, const TileGate& g, const float4* __restrict__ mats) {
     constexpr int D = 1 << K;
@@ -124,11 +293,10 @@ __device__ void adj_dense(float4* sm, int T, const TileGate& g, const float4* __
     for (int a = 0; a < K; a++)
         for (int b = a + 1; b < K; b++)
             if (pos[b] < pos[a]) { int t = pos[a]; pos[a] = pos[b]; pos[b] = t; }
-    const int ngroups = 1 << (T - K);
     const float4* m = mats + g.mat_off;
-    for (int gr = threadIdx.x; gr < ngroups; gr += blockDim.x) {
+    for (int gr = threadIdx.x; gr < (1 << (T - K)); gr += blockDim.x) {
         int jb = gr;
-        for (int q = 0; q < K; q++) { int low = jb & ((1 << pos[q]) - 1); jb = ((jb >> pos[q]) << (pos[q] + 1)) | low; }
+        for (int q = 0; q < K; q++) jb = insert_zero(jb, pos[q]);
         if ((jb & (int)g.lc_mask) != (int)g.lc_val) continue;
         cff x[D];
         int idx[D];
@@ -149,239 +317,8 @@ __device__ void adj_dense(float4* sm, int T, const TileGate& g, const float4* __
         }
     }
 }
-
-__device__ void adj_apply(float4* sm, int T, int L, const TileGate& g, const float4* mats, const int32_t* perms,
-                          int64_t base, const int64_t* off_tab) {
-    const int nt = 1 << T, lowmask = (1 << L) - 1;
-    if (g.kind == 1) {
-        const float4* m = mats + g.mat_off;
-        for (int j = threadIdx.x; j < nt; j += blockDim.x) {
-            if ((j & (int)g.lc_mask) != (int)g.lc_val) continue;
-            int64_t gi = base | off_tab[j >> L] | (int64_t)(j & lowmask);
-            int di = 0;
-            for (int q = 0; q < g.k; q++) di |= (int)((gi >> g.gbit[q]) & 1) << q;
-            sm[j] = c4f(cmul(f4c(__ldg(m + di)), f4c(sm[j])));
-        }
-    } else if (g.kind == 0) {
-        switch (g.k) {
-            case 1: adj_dense<1>(sm, T, g, mats); break;
-            case 2: adj_dense<2>(sm, T, g, mats); break;
-            case 3: adj_dense<3>(sm, T, g, mats); break;
-            default: adj_dense<4>(sm, T, g, mats); break;
-        }
-    } else {
-        // monomial
-        const int D = 1 << g.k;
-        int pos[BS_TILE_MAXK];
-        for (int q = 0; q < g.k; q++) pos[q] = g.tbit[q];
-        for (int a = 0; a < g.k; a++)
-            for (int b = a + 1; b < g.k; b++)
-                if (pos[b] < pos[a]) { int t = pos[a]; pos[a] = pos[b]; pos[b] = t; }
-        const int32_t* p = perms + g.perm_off;
-        for (int gr = threadIdx.x; gr < (1 << (T - g.k)); gr += blockDim.x) {
-            int jb = gr;
-            for (int q = 0; q < g.k; q++) { int low = jb & ((1 << pos[q]) - 1); jb = ((jb >> pos[q]) << (pos[q] + 1)) | low; }
-            if ((jb & (int)g.lc_mask) != (int)g.lc_val) continue;
-            float4 x[16];
-            int idx[16];
-            for (int c = 0; c < D; c++) {
-                int j = jb;
-                for (int q = 0; q < g.k; q++) if ((c >> q) & 1) j |= 1 << g.tbit[q];
-                idx[c] = j;
-                x[c] = sm[j];
-            }
-            for (int c = 0; c < D; c++) sm[idx[__ldg(p + 2 * c)]] = c4f(cmul_ipow(f4c(x[c]), __ldg(p + 2 * c + 1)));
-        }
-    }
-}
-
-// The same gate on both tiles of the sweep (psi and lambda) in one pass: the index arithmetic and the
-// matrix reads are shared.  Dense gates on 1 or 2 targets and diagonal gates; others go through
-// adj_apply once per tile.
 template <int K>
-__device__ void adj_dense2(float4* sa, float4* sb, int T, const TileGate& g, const float4* __restrict__ mats) {
-    constexpr int D = 1 << K;
-    int pos[K];
-    for (int q = 0; q < K; q++) pos[q] = g.tbit[q];
-    for (int a = 0; a < K; a++)
-        for (int b = a + 1; b < K; b++)
-            if (pos[b] < pos[a]) { int t = pos[a]; pos[a] = pos[b]; pos[b] = t; }
-    const int ngroups = 1 << (T - K);
-    const float4* m = mats + g.mat_off;
-    for (int gr = threadIdx.x; gr < ngroups; gr += blockDim.x) {
-        int jb = gr;
-        for (int q = 0; q < K; q++) { int low = jb & ((1 << pos[q]) - 1); jb = ((jb >> pos[q]) << (pos[q] + 1)) | low; }
-        if ((jb & (int)g.lc_mask) != (int)g.lc_val) continue;
-        cff x[D], y[D];
-        int idx[D];
-#pragma unroll
-        for (int c = 0; c < D; c++) {
-            int j = jb;
-            for (int q = 0; q < K; q++) if ((c >> q) & 1) j |= 1 << g.tbit[q];
-            idx[c] = j;
-            x[c] = f4c(sa[j]);
-            y[c] = f4c(sb[j]);
-        }
-#pragma unroll
-        for (int r = 0; r < D; r++) {
-            ffacc ar, ai, br, bi;
-            const cff m0 = f4c(__ldg(m + r * D));
-            cmac_first(ar, ai, m0, x[0]);
-            cmac_first(br, bi, m0, y[0]);
-#pragma unroll
-            for (int c = 1; c < D; c++) {
-                const cff mc = f4c(__ldg(m + r * D + c));
-                cmac(ar, ai, mc, x[c]);
-                cmac(br, bi, mc, y[c]);
-            }
-            sa[idx[r]] = c4f(cdone(ar, ai));
-            sb[idx[r]] = c4f(cdone(br, bi));
-        }
-    }
-}
-
-__device__ void adj_apply2(float4* sa, float4* sb, int T, int L, const TileGate& g, const float4* mats,
-                           const int32_t* perms, int64_t base, const int64_t* off_tab) {
-    if (g.kind == 1) {
-        const int nt = 1 << T, lowmask = (1 << L) - 1;
-        const float4* m = mats + g.mat_off;
-        for (int j = threadIdx.x; j < nt; j += blockDim.x) {
-            if ((j & (int)g.lc_mask) != (int)g.lc_val) continue;
-            const int64_t gi = base | off_tab[j >> L] | (int64_t)(j & lowmask);
-            int di = 0;
-            for (int q = 0; q < g.k; q++) di |= (int)((gi >> g.gbit[q]) & 1) << q;
-            const cff dv = f4c(__ldg(m + di));
-            sa[j] = c4f(cmul(dv, f4c(sa[j])));
-            sb[j] = c4f(cmul(dv, f4c(sb[j])));
-        }
-    } else if (g.kind == 0 && g.k == 1) {
-        adj_dense2<1>(sa, sb, T, g, mats);
-    } else if (g.kind == 0 && g.k == 2) {
-        adj_dense2<2>(sa, sb, T, g, mats);
-    } else {
-        adj_apply(sa, T, L, g, mats, perms, base, off_tab);
-        adj_apply(sb, T, L, g, mats, perms, base, off_tab);
-    }
-}
-
-template <bool C64>
-__global__ void __launch_bounds__(kAThreads) k_adjoint_sweep(typename Elem<C64>::T* __restrict__ psi,
-                                                             typename Elem<C64>::T* __restrict__ lam, SweepDesc d,
-                                                             const AdjGate* __restrict__ ag,
-                                                             double* __restrict__ grad_acc, int64_t tile0) {
-    extern __shared__ float4 smem[];
-    const int T = d.T, L = d.L, H = T - L;
-    const int nt = 1 << T;
-    float4* sp = smem;
-    float4* sl = smem + nt;
-    int64_t* off_tab = reinterpret_cast<int64_t*>(smem + 2 * nt);
-    __shared__ int64_t s_base;
-    const int64_t tile = tile0 + (int64_t)blockIdx.x;
-    if (threadIdx.x == 0) {
-        int64_t base = 0;
-        int src = 0;
-        for (int bit = 0; bit < d.n_bits; bit++)
-            if (!((d.tile_mask >> bit) & 1ULL)) { base |= ((tile >> src) & 1LL) << bit; src++; }
-        s_base = base;
-    }
-    for (int i = threadIdx.x; i < (1 << H); i += blockDim.x) {
-        int64_t o = 0;
-        for (int j = 0; j < H; j++) if ((i >> j) & 1) o |= 1LL << d.hi_bits[j];
-        off_tab[i] = o;
-    }
-    __syncthreads();
-    const int64_t base = s_base;
-    const int lowmask = (1 << L) - 1;
-    // tile loads: four positions (eight loads) per thread in flight at a time (tiles <= 2^12)
-#pragma unroll
-    for (int r = 0; r < 4096 / kAThreads; r += 4) {
-        typename Elem<C64>::T xp[4], xl[4];
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const int j = (r + i) * kAThreads + (int)threadIdx.x;
-            if (j < nt) {
-                const int64_t gidx = base | off_tab[j >> L] | (int64_t)(j & lowmask);
-                xp[i] = psi[gidx];
-                xl[i] = lam[gidx];
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const int j = (r + i) * kAThreads + (int)threadIdx.x;
-            if (j < nt) {
-                sp[j] = c4f(Elem<C64>::load(xp[i]));
-                sl[j] = c4f(Elem<C64>::load(xl[i]));
-            }
-        }
-    }
-    __syncthreads();
-    for (int gi = 0; gi < d.n_gates; gi++) {
-        const AdjGate& a = ag[gi];   // fields read where used (a copy of the whole descriptor went to local memory)
-        if (a.g.kind == 3) {
-            // Im <lambda| G |psi> over the tile
-            ffsum acc{0.f, 0.f};
-            for (int j = threadIdx.x; j < nt; j += blockDim.x) {
-                int64_t gidx = base | off_tab[j >> L] | (int64_t)(j & lowmask);
-                cff l = f4c(sl[j]);
-                cff x;
-                if (a.projector) {
-                    if (!((gidx >> a.g.gbit[0]) & 1)) continue;
-                    x = f4c(sp[j]);
-                } else {
-                    x = f4c(sp[j ^ (int)a.xm_local]);
-                    int ph = a.ph + ((__popcll((unsigned long long)gidx & a.zm) & 1) ? 2 : 0);
-                    x = cmul_ipow(x, (4 - (ph & 3)) & 3);
-                }
-                // Im(conj(l) * x) = l.r x.i - l.i x.r
-                ffacc m;
-                acc_first(m, l.rh, l.rl, x.ih, x.il);
-                acc_add(m, -l.ih, -l.il, x.rh, x.rl);
-                ff v = acc_done(m);
-                fsum_add(acc, v.h, v.l);
-            }
-            double v = ff2d(acc.h, acc.l) * a.weight;
-            __shared__ double red[kAThreads / 32];
-            for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-            if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                double s = 0.0;
-                for (int w = 0; w < (int)(blockDim.x >> 5); w++) s += red[w];
-                atomicAdd(grad_acc + a.slot, s);
-            }
-            __syncthreads();
-            continue;
-        }
-        if ((base & (int64_t)a.g.gc_mask) != (int64_t)a.g.gc_val) continue;
-        adj_apply2(sp, sl, T, L, a.g, d.mats, d.perms, base, off_tab);
-        __syncthreads();
-    }
-    for (int j = threadIdx.x; j < nt; j += blockDim.x) {
-        int64_t gidx = base | off_tab[j >> L] | (int64_t)(j & lowmask);
-        psi[gidx] = Elem<C64>::store(f4c(sp[j]));
-        lam[gidx] = Elem<C64>::store(f4c(sl[j]));
-    }
-}
-
-// ---- complex64 states: the backward sweep's gates in FP32 on float2 tiles (the state's own
-// precision; half the shared memory and a sixth of the instructions of the float-float path), the
-// gradient inner products from the FP32 values with exact products and float-float sums.
-__device__ __forceinline__ float2 c32mul(float2 m, float2 x) {
-    return make_float2(__fmaf_rn(m.x, x.x, -m.y * x.y), __fmaf_rn(m.x, x.y, m.y * x.x));
-}
-__device__ __forceinline__ float2 c32ipow(float2 x, int p) {
-    switch (p & 3) {
-        case 0: return x;
-        case 1: return make_float2(-x.y, x.x);
-        case 2: return make_float2(-x.x, -x.y);
-        default: return make_float2(x.y, -x.x);
-    }
-}
-// matrix entry (float4 re hi, re lo, im hi, im lo) as the nearest complex64 value
-__device__ __forceinline__ float2 m32(float4 v) { return make_float2(v.x, v.z); }
-
-template <int K>
-__device__ void adj32_dense2(float2* sa, float2* sb, int T, const TileGate& g, const float4* __restrict__ mats) {
+__device__ void adj_dense(float2* sm, int T, const TileGate& g, const float4* __restrict__ mats) {
     constexpr int D = 1 << K;
     int pos[K];
     for (int q = 0; q < K; q++) pos[q] = g.tbit[q];
@@ -391,107 +328,100 @@ __device__ void adj32_dense2(float2* sa, float2* sb, int T, const TileGate& g, c
     const float4* m = mats + g.mat_off;
     for (int gr = threadIdx.x; gr < (1 << (T - K)); gr += blockDim.x) {
         int jb = gr;
-        for (int q = 0; q < K; q++) { int low = jb & ((1 << pos[q]) - 1); jb = ((jb >> pos[q]) << (pos[q] + 1)) | low; }
+        for (int q = 0; q < K; q++) jb = insert_zero(jb, pos[q]);
         if ((jb & (int)g.lc_mask) != (int)g.lc_val) continue;
-        float2 x[D], y[D];
+        float2 x[D];
         int idx[D];
 #pragma unroll
         for (int c = 0; c < D; c++) {
             int j = jb;
             for (int q = 0; q < K; q++) if ((c >> q) & 1) j |= 1 << g.tbit[q];
             idx[c] = j;
-            x[c] = sa[j];
-            y[c] = sb[j];
+            x[c] = sm[j];
         }
 #pragma unroll
         for (int r = 0; r < D; r++) {
-            float2 u = make_float2(0.f, 0.f), v = make_float2(0.f, 0.f);
+            float2 u = make_float2(0.f, 0.f);
 #pragma unroll
             for (int c = 0; c < D; c++) {
-                const float2 mc = m32(__ldg(m + r * D + c));
-                u.x = __fmaf_rn(mc.x, x[c].x, __fmaf_rn(-mc.y, x[c].y, u.x));
-                u.y = __fmaf_rn(mc.x, x[c].y, __fmaf_rn(mc.y, x[c].x, u.y));
-                v.x = __fmaf_rn(mc.x, y[c].x, __fmaf_rn(-mc.y, y[c].y, v.x));
-                v.y = __fmaf_rn(mc.x, y[c].y, __fmaf_rn(mc.y, y[c].x, v.y));
+                const float4 mc = __ldg(m + r * D + c);
+                u.x = __fmaf_rn(mc.x, x[c].x, __fmaf_rn(-mc.z, x[c].y, u.x));
+                u.y = __fmaf_rn(mc.x, x[c].y, __fmaf_rn(mc.z, x[c].x, u.y));
             }
-            sa[idx[r]] = u;
-            sb[idx[r]] = v;
+            sm[idx[r]] = u;
         }
     }
 }
-
-__device__ void adj32_apply2(float2* sa, float2* sb, int T, int L, const TileGate& g, const float4* mats,
-                             const int32_t* perms, int64_t base, const int64_t* off_tab) {
-    const int nt = 1 << T, lowmask = (1 << L) - 1;
-    if (g.kind == 1) {
-        const float4* m = mats + g.mat_off;
-        for (int j = threadIdx.x; j < nt; j += blockDim.x) {
-            if ((j & (int)g.lc_mask) != (int)g.lc_val) continue;
-            const int64_t gi = base | off_tab[j >> L] | (int64_t)(j & lowmask);
-            int di = 0;
-            for (int q = 0; q < g.k; q++) di |= (int)((gi >> g.gbit[q]) & 1) << q;
-            const float2 d = m32(__ldg(m + di));
-            sa[j] = c32mul(d, sa[j]);
-            sb[j] = c32mul(d, sb[j]);
+template <bool C64>
+__device__ void adj_monomial(typename Tile<C64>::S* sm, int T, const TileGate& g, const int32_t* __restrict__ perms) {
+    using P = Tile<C64>;
+    const int D = 1 << g.k;
+    int pos[BS_TILE_MAXK];
+    for (int q = 0; q < g.k; q++) pos[q] = g.tbit[q];
+    for (int a = 0; a < g.k; a++)
+        for (int b = a + 1; b < g.k; b++)
+            if (pos[b] < pos[a]) { int t = pos[a]; pos[a] = pos[b]; pos[b] = t; }
+    const int32_t* p = perms + g.perm_off;
+    for (int gr = threadIdx.x; gr < (1 << (T - g.k)); gr += blockDim.x) {
+        int jb = gr;
+        for (int q = 0; q < g.k; q++) jb = insert_zero(jb, pos[q]);
+        if ((jb & (int)g.lc_mask) != (int)g.lc_val) continue;
+        typename P::S x[16];
+        int idx[16];
+        for (int c = 0; c < D; c++) {
+            int j = jb;
+            for (int q = 0; q < g.k; q++) if ((c >> q) & 1) j |= 1 << g.tbit[q];
+            idx[c] = j;
+            x[c] = sm[j];
         }
-    } else if (g.kind == 0) {
-        switch (g.k) {
-            case 1: adj32_dense2<1>(sa, sb, T, g, mats); break;
-            case 2: adj32_dense2<2>(sa, sb, T, g, mats); break;
-            case 3: adj32_dense2<3>(sa, sb, T, g, mats); break;
-            default: adj32_dense2<4>(sa, sb, T, g, mats); break;
-        }
-    } else {
-        // monomial: column c goes to row perm[2c] with phase i^perm[2c+1]
-        const int D = 1 << g.k;
-        int pos[BS_TILE_MAXK];
-        for (int q = 0; q < g.k; q++) pos[q] = g.tbit[q];
-        for (int a = 0; a < g.k; a++)
-            for (int b = a + 1; b < g.k; b++)
-                if (pos[b] < pos[a]) { int t = pos[a]; pos[a] = pos[b]; pos[b] = t; }
-        const int32_t* p = perms + g.perm_off;
-        for (int gr = threadIdx.x; gr < (1 << (T - g.k)); gr += blockDim.x) {
-            int jb = gr;
-            for (int q = 0; q < g.k; q++) { int low = jb & ((1 << pos[q]) - 1); jb = ((jb >> pos[q]) << (pos[q] + 1)) | low; }
-            if ((jb & (int)g.lc_mask) != (int)g.lc_val) continue;
-            float2 x[16], y[16];
-            int idx[16];
-            for (int c = 0; c < D; c++) {
-                int j = jb;
-                for (int q = 0; q < g.k; q++) if ((c >> q) & 1) j |= 1 << g.tbit[q];
-                idx[c] = j;
-                x[c] = sa[j];
-                y[c] = sb[j];
-            }
-            for (int c = 0; c < D; c++) {
-                const int r = __ldg(p + 2 * c), ph = __ldg(p + 2 * c + 1);
-                sa[idx[r]] = c32ipow(x[c], ph);
-                sb[idx[r]] = c32ipow(y[c], ph);
-            }
-        }
+        for (int c = 0; c < D; c++) sm[idx[__ldg(p + 2 * c)]] = P::st(P::ipow(P::ld(x[c]), __ldg(p + 2 * c + 1)));
     }
 }
 
-__global__ void __launch_bounds__(kAThreads) k_adjoint_sweep_c64(float2* __restrict__ psi, float2* __restrict__ lam,
-                                                                 SweepDesc d, const AdjGate* __restrict__ ag,
-                                                                 double* __restrict__ grad_acc, int64_t tile0) {
-    extern __shared__ float4 smem4[];
+// index part of a folded diagonal's table from tile position j (bits outside the tile left out)
+__device__ __forceinline__ int tab_index(const AdjTab& t, int j) {
+    int di = 0;
+#pragma unroll
+    for (int q = 0; q < 8; q++)
+        if (q < t.k && t.pos[q] >= 0) di |= ((j >> t.pos[q]) & 1) << q;
+    return di;
+}
+__device__ __forceinline__ int tab_const(const AdjTab& t, int64_t base) {
+    int di = 0;
+#pragma unroll
+    for (int q = 0; q < 8; q++)
+        if (q < t.k && t.pos[q] < 0) di |= (int)((base >> t.gbit[q]) & 1) << q;
+    return di;
+}
+
+template <bool C64>
+__global__ void __launch_bounds__(kSweepThreads, C64 ? 2 : 1)
+    k_adjoint_sweep(typename Elem<C64>::T* __restrict__ psi, typename Elem<C64>::T* __restrict__ lam, SweepDesc d,
+                    const AdjGate* __restrict__ ag, const AdjTab* __restrict__ tabs, const AdjMark* __restrict__ marks,
+                    double* __restrict__ grad_acc, int64_t tile0) {
+    using P = Tile<C64>;
+    using S = typename P::S;
+    extern __shared__ float4 smem[];
     const int T = d.T, L = d.L, H = T - L;
     const int nt = 1 << T;
-    float2* sp = reinterpret_cast<float2*>(smem4);
-    float2* sl = sp + nt;
-    int64_t* off_tab = reinterpret_cast<int64_t*>(sl + nt);
+    S* sp = reinterpret_cast<S*>(smem);
+    S* sl = sp + nt;
+    float2* vt = reinterpret_cast<float2*>(sl + nt);                        // kSweepPer x kSweepThreads
+    int64_t* off_tab = reinterpret_cast<int64_t*>(vt + kSweepPer * kSweepThreads);
     __shared__ int64_t s_base;
-    __shared__ double red[kAThreads / 32];
+    __shared__ double red[kRotMax][kSweepThreads / 32];
+    __shared__ double red_w[kRotMax];
+    __shared__ int red_slot[kRotMax];
     const int64_t tile = tile0 + (int64_t)blockIdx.x;
-    if (threadIdx.x == 0) {
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (tid == 0) {
         int64_t base = 0;
         int src = 0;
         for (int bit = 0; bit < d.n_bits; bit++)
             if (!((d.tile_mask >> bit) & 1ULL)) { base |= ((tile >> src) & 1LL) << bit; src++; }
         s_base = base;
     }
-    for (int i = threadIdx.x; i < (1 << H); i += blockDim.x) {
+    for (int i = tid; i < (1 << H); i += kSweepThreads) {
         int64_t o = 0;
         for (int j = 0; j < H; j++) if ((i >> j) & 1) o |= 1LL << d.hi_bits[j];
         off_tab[i] = o;
@@ -499,55 +429,170 @@ __global__ void __launch_bounds__(kAThreads) k_adjoint_sweep_c64(float2* __restr
     __syncthreads();
     const int64_t base = s_base;
     const int lowmask = (1 << L) - 1;
-#pragma unroll 4
-    for (int j = threadIdx.x; j < nt; j += blockDim.x) {
-        const int64_t gidx = base | off_tab[j >> L] | (int64_t)(j & lowmask);
-        sp[j] = psi[gidx];
-        sl[j] = lam[gidx];
+    // tile loads: four positions (eight loads) per thread in flight at a time (tiles <= 2^12)
+#pragma unroll
+    for (int r = 0; r < kSweepPer; r += 4) {
+        typename Elem<C64>::T xp[4], xl[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int j = (r + i) * kSweepThreads + tid;
+            if (j < nt) {
+                const int64_t gidx = base | off_tab[j >> L] | (int64_t)(j & lowmask);
+                xp[i] = psi[gidx];
+                xl[i] = lam[gidx];
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int j = (r + i) * kSweepThreads + tid;
+            if (j < nt) {
+                sp[j] = P::from(xp[i]);
+                sl[j] = P::from(xl[i]);
+            }
+        }
     }
     __syncthreads();
+    int nred = 0;   // inner products waiting in red
+    // add the waiting inner products to the result (all threads; the caller's barrier is before it)
+    auto flush_red = [&]() {
+        if (tid < nred) {
+            double s = 0.0;
+            for (int w = 0; w < kSweepThreads / 32; w++) s += red[tid][w];
+            atomicAdd(grad_acc + red_slot[tid], s * red_w[tid]);
+        }
+        __syncthreads();
+        nred = 0;
+    };
+    auto keep_red = [&](ffsum acc, int slot, double w) {
+        warp_fsum(acc);
+        if (lane == 0) red[nred][warp] = ff2d(acc.h, acc.l);
+        if (tid == 0) { red_slot[nred] = slot; red_w[nred] = w; }
+        nred++;
+    };
     for (int gi = 0; gi < d.n_gates; gi++) {
-        const AdjGate& a = ag[gi];
-        if (a.g.kind == 3) {
-            // Im <lambda| G |psi> over the tile: exact FP32 products, float-float sums
-            ffsum acc{0.f, 0.f};
-            for (int j = threadIdx.x; j < nt; j += blockDim.x) {
-                const int64_t gidx = base | off_tab[j >> L] | (int64_t)(j & lowmask);
-                const float2 l = sl[j];
-                float2 x;
-                if (a.projector) {
-                    if (!((gidx >> a.g.gbit[0]) & 1)) continue;
-                    x = sp[j];
-                } else {
-                    const int ph = a.ph + ((__popcll((unsigned long long)gidx & a.zm) & 1) ? 2 : 0);
-                    x = c32ipow(sp[j ^ (int)a.xm_local], (4 - (ph & 3)) & 3);
+        const AdjGate& a = ag[gi];   // fields read where used (a copy of the whole descriptor went to local memory)
+        const int kind = a.g.kind;
+        if (kind == 7) {
+            const int nm = a.ph, ntab = a.n_tabs;
+            const AdjTab* tb = tabs + a.xm_local;
+            // The gates first, in a rolled loop (one unrolled loop over values and tables overflowed the
+            // instruction cache), then v: the gates do not change it.
+            for (int t0 = 0; t0 < ntab; t0 += kTabsPerPass) {
+                const int nk = min(kTabsPerPass, ntab - t0);
+                const float4* tm[kTabsPerPass];
+#pragma unroll
+                for (int u = 0; u < kTabsPerPass; u++)
+                    if (u < nk) tm[u] = d.mats + tb[t0 + u].mat_off + (tab_index(tb[t0 + u], tid) | tab_const(tb[t0 + u], base));
+#pragma unroll 1
+                for (int j = tid; j < nt; j += kSweepThreads) {
+                    auto x = P::ld(sp[j]), l = P::ld(sl[j]);
+#pragma unroll
+                    for (int u = 0; u < kTabsPerPass; u++)
+                        if (u < nk) {
+                            const float4 m = __ldg(tm[u] + tab_index(tb[t0 + u], j - tid));
+                            x = P::mul(m, x);
+                            l = P::mul(m, l);
+                        }
+                    sp[j] = P::st(x);
+                    sl[j] = P::st(l);
                 }
-                ffacc m;
-                acc_first(m, l.x, 0.f, x.y, 0.f);
-                acc_add(m, -l.y, 0.f, x.x, 0.f);
-                const ff v = acc_done(m);
-                fsum_add(acc, v.h, v.l);
             }
-            double v = ff2d(acc.h, acc.l) * a.weight;
-            for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-            if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                double t = 0.0;
-                for (int w = 0; w < (int)(blockDim.x >> 5); w++) t += red[w];
-                atomicAdd(grad_acc + a.slot, t);
+            if (nm) {
+                ffsum v[kSweepPer];
+#pragma unroll
+                for (int i = 0; i < kSweepPer; i++) {
+                    const int j = i * kSweepThreads + tid;
+                    v[i] = {0.f, 0.f};
+                    if (j < nt) {
+                        const ff f = P::im_conj(P::ld(sl[j]), P::ld(sp[j]));
+                        v[i] = {f.h, f.l};
+                    }
+                }
+                // Walsh-Hadamard over the tile bits above the thread index
+#pragma unroll
+                for (int o = 1; o < kSweepPer; o <<= 1)
+#pragma unroll
+                    for (int i = 0; i < kSweepPer; i++)
+                        if (!(i & o)) {
+                            ffsum s = v[i], t = v[i];
+                            fsum_add(s, v[i | o].h, v[i | o].l);
+                            fsum_add(t, -v[i | o].h, -v[i | o].l);
+                            v[i] = s;
+                            v[i | o] = t;
+                        }
+#pragma unroll
+                for (int i = 0; i < kSweepPer; i++) vt[i * kSweepThreads + tid] = make_float2(v[i].h, v[i].l);
+                __syncthreads();
+                for (int m = warp; m < nm; m += kSweepThreads / 32) {
+                    const AdjMark& k = marks[a.slot + m];
+                    const uint32_t z = k.z_tile;
+                    const float2* row = vt + (z >> kSweepLog) * kSweepThreads;
+                    const uint32_t neg0 = (uint32_t)__popcll((unsigned long long)base & k.z_out) + (uint32_t)__popc((uint32_t)lane & z);
+                    ffsum s{0.f, 0.f};
+#pragma unroll
+                    for (int u = 0; u < kSweepThreads / 32; u++) {
+                        const float2 w = row[32 * u + lane];
+                        const uint32_t sg = (neg0 + (uint32_t)__popc((uint32_t)(32 * u) & z)) << 31;
+                        fsum_add(s, __uint_as_float(__float_as_uint(w.x) ^ sg), __uint_as_float(__float_as_uint(w.y) ^ sg));
+                    }
+                    warp_fsum(s);
+                    if (lane == 0) atomicAdd(grad_acc + k.slot, ff2d(s.h, s.l) * k.weight);
+                }
             }
             __syncthreads();
             continue;
         }
+        if (kind == 3) {
+            // Im <lambda| G |psi> over the tile, G flipping bits
+            ffsum acc{0.f, 0.f};
+            for (int j = tid; j < nt; j += kSweepThreads) {
+                const int64_t gidx = base | off_tab[j >> L] | (int64_t)(j & lowmask);
+                const int ph = a.ph + ((__popcll((unsigned long long)gidx & a.zm) & 1) ? 2 : 0);
+                const ff v = P::im_conj(P::ld(sl[j]), P::ipow(P::ld(sp[j ^ (int)a.xm_local]), (4 - (ph & 3)) & 3));
+                fsum_add(acc, v.h, v.l);
+            }
+            keep_red(acc, a.slot, a.weight);
+            __syncthreads();
+            if (nred == kRotMax) flush_red();
+            continue;
+        }
+        if (kind == 6) {
+            const ffsum acc = a.ph ? adj_1q_cls<C64, 2>(sp, sl, T, a.g, d.mats) : adj_1q_cls<C64, 1>(sp, sl, T, a.g, d.mats);
+            keep_red(acc, a.slot, a.weight);
+            __syncthreads();
+            if (nred == kRotMax) flush_red();
+            continue;
+        }
         if ((base & (int64_t)a.g.gc_mask) != (int64_t)a.g.gc_val) continue;
-        adj32_apply2(sp, sl, T, L, a.g, d.mats, d.perms, base, off_tab);
+        if (kind == 1) {
+            const float4* m = d.mats + a.g.mat_off;
+            for (int j = tid; j < nt; j += kSweepThreads) {
+                if ((j & (int)a.g.lc_mask) != (int)a.g.lc_val) continue;
+                const int64_t gidx = base | off_tab[j >> L] | (int64_t)(j & lowmask);
+                int di = 0;
+                for (int q = 0; q < a.g.k; q++) di |= (int)((gidx >> a.g.gbit[q]) & 1) << q;
+                const float4 dv = __ldg(m + di);
+                sp[j] = P::st(P::mul(dv, P::ld(sp[j])));
+                sl[j] = P::st(P::mul(dv, P::ld(sl[j])));
+            }
+        } else if (kind == 0) {
+            switch (a.g.k) {
+                case 1: adj_1q_cls<C64, 0>(sp, sl, T, a.g, d.mats); break;
+                case 2: adj_dense<2>(sp, T, a.g, d.mats); adj_dense<2>(sl, T, a.g, d.mats); break;
+                case 3: adj_dense<3>(sp, T, a.g, d.mats); adj_dense<3>(sl, T, a.g, d.mats); break;
+                default: adj_dense<4>(sp, T, a.g, d.mats); adj_dense<4>(sl, T, a.g, d.mats); break;
+            }
+        } else {
+            adj_monomial<C64>(sp, T, a.g, d.perms);
+            adj_monomial<C64>(sl, T, a.g, d.perms);
+        }
         __syncthreads();
     }
-    for (int j = threadIdx.x; j < nt; j += blockDim.x) {
+    if (nred) flush_red();
+    for (int j = tid; j < nt; j += kSweepThreads) {
         const int64_t gidx = base | off_tab[j >> L] | (int64_t)(j & lowmask);
-        psi[gidx] = sp[j];
-        lam[gidx] = sl[j];
+        psi[gidx] = P::to(sp[j]);
+        lam[gidx] = P::to(sl[j]);
     }
 }
 
@@ -566,7 +611,86 @@ struct BwdItem {          // one element of the reversed gate list
     uint64_t xm = 0, zm = 0;   // endian masks of the generator
     int ph = 0;
     double weight = 1.0;
+    bool unitary_diag = false;    // kind 1 with entries of modulus 1
+
+    uint64_t touch() const {
+        uint64_t m = g.cmask | zm | xm;
+        for (int q = 0; q < g.k; q++) m |= 1ULL << g.ebit[q];
+        return m;
+    }
+    // leaves conj(lambda_i) psi_i alone and reads nothing else: commutes with its like on any bits
+    bool diag() const { return marker ? xm == 0 : unitary_diag; }
 };
+
+// Diagonal gates of one phase folded into tables over at most 8 bits each (they commute).
+constexpr int kTabBits = 8;
+struct FoldTab {
+    std::vector<int> eb;                      // endian bits, table index bit q <-> eb[q]
+    std::vector<std::complex<double>> d;
+};
+uint64_t tab_bits(const FoldTab& t) {
+    uint64_t m = 0;
+    for (int e : t.eb) m |= 1ULL << e;
+    return m;
+}
+// t <- t * h, over the union of their bits
+void fold_diag(FoldTab& t, const HostGate& h) {
+    uint64_t nb = tab_bits(t) | h.cmask;
+    for (int q = 0; q < h.k; q++) nb |= 1ULL << h.ebit[q];
+    std::vector<int> eb;
+    for (int e = 0; e < 64; e++) if ((nb >> e) & 1ULL) eb.push_back(e);
+    std::vector<std::complex<double>> d((size_t)1 << eb.size());
+    for (size_t x = 0; x < d.size(); x++) {
+        uint64_t g = 0;
+        for (size_t q = 0; q < eb.size(); q++) if ((x >> q) & 1) g |= 1ULL << eb[q];
+        std::complex<double> v(1.0, 0.0);
+        if (!t.d.empty()) {
+            size_t xi = 0;
+            for (size_t q = 0; q < t.eb.size(); q++) xi |= (size_t)((g >> t.eb[q]) & 1ULL) << q;
+            v = t.d[xi];
+        }
+        if ((g & h.cmask) == h.cval) {
+            int hi = 0;
+            for (int q = 0; q < h.k; q++) hi |= (int)((g >> h.ebit[q]) & 1ULL) << q;
+            v *= std::complex<double>(h.mat[2 * hi], h.mat[2 * hi + 1]);
+        }
+        d[x] = v;
+    }
+    t.eb = eb;
+    t.d = d;
+}
+// Fold a run of diagonal gates (each on at most kTabBits bits): each joins the table it widens least.
+void fold_diags(const std::vector<const HostGate*>& gates, std::vector<FoldTab>& tabs) {
+    for (const HostGate* h : gates) {
+        uint64_t hb = h->cmask;
+        for (int q = 0; q < h->k; q++) hb |= 1ULL << h->ebit[q];
+        int best = -1, added = 0;
+        for (size_t t = 0; t < tabs.size(); t++) {
+            const uint64_t tb = tab_bits(tabs[t]);
+            const int add = __builtin_popcountll(hb & ~tb);
+            if (__builtin_popcountll(tb | hb) <= kTabBits && (best < 0 || add < added)) { best = (int)t; added = add; }
+        }
+        if (best < 0) {
+            best = (int)tabs.size();
+            tabs.emplace_back();
+        }
+        fold_diag(tabs[(size_t)best], *h);
+    }
+}
+bool unit_modulus(const HostGate& h) {
+    for (int i = 0; i < (1 << h.k); i++) {
+        const double m = h.mat[2 * i] * h.mat[2 * i] + h.mat[2 * i + 1] * h.mat[2 * i + 1];
+        if (std::fabs(m - 1.0) > 4e-15) return false;
+    }
+    return true;
+}
+// matrix class of a 2x2 gate: 1 all real, 2 real diagonal and imaginary off-diagonal, else 0
+int class_2x2(const HostGate& h) {
+    if (h.mat[1] != 0.0 || h.mat[7] != 0.0) return 0;
+    if (h.mat[3] == 0.0 && h.mat[5] == 0.0) return 1;
+    if (h.mat[2] == 0.0 && h.mat[4] == 0.0) return 2;
+    return 0;
+}
 
 // U^dagger of a lowered gate (same targets and controls)
 HostGate dagger(const HostGate& h) {
@@ -745,13 +869,15 @@ extern "C" int bs_adjoint_gradient(bs_sim* s, const bs_op* ops, int64_t n_ops, c
         for (const HostGate& h : hg) {
             BwdItem it;
             it.g = dagger(h);
+            it.unitary_diag = it.g.kind == 1 && unit_modulus(it.g);
             items.push_back(it);
         }
     }
     while ((int)seg_item.size() < S) seg_item.push_back(items.size());
     seg_item.push_back(items.size());
     // plan sweeps segment by segment: markers need their flip bits in the tile, and they must not
-    // move past a gate sharing bits (they read the current psi and lambda)
+    // move past a gate sharing bits (they read the current psi and lambda); diagonal gates and
+    // diagonal-generator markers move past one another freely
     const int n_bits = n;
     const int T = std::min(BS_TILE_MAX_BITS, n_bits);
     const int L = std::min(BS_TILE_LOW_BITS, T);
@@ -764,11 +890,6 @@ extern "C" int bs_adjoint_gradient(bs_sim* s, const bs_op* ops, int64_t n_ops, c
         std::vector<char> done(G, 0);
         size_t remaining = G - seg_item[(size_t)r], first = seg_item[(size_t)r];
         bool seg_first = true;
-        auto touch = [&](const BwdItem& it) {
-            uint64_t m = it.g.cmask | it.zm | it.xm;
-            for (int q = 0; q < it.g.k; q++) m |= 1ULL << it.g.ebit[q];
-            return m;
-        };
         auto need = [&](const BwdItem& it) -> uint64_t {
             uint64_t m = 0;
             if (!it.marker && it.g.kind == 1) return m;
@@ -778,12 +899,13 @@ extern "C" int bs_adjoint_gradient(bs_sim* s, const bs_op* ops, int64_t n_ops, c
         };
         while (remaining) {
             std::vector<int> idx;
-            uint64_t chosen = 0, blocked = 0;
+            uint64_t chosen = 0, blocked = 0, blocked_diag = 0;   // bits of items left behind: any, diagonal
             int nch = 0;
             for (size_t i = first; i < G; i++) {
                 if (done[i]) continue;
-                uint64_t t = touch(items[i]);
-                if (t & blocked) { blocked |= t; continue; }
+                uint64_t t = items[i].touch();
+                const bool dg = items[i].diag();
+                if (t & (dg ? blocked : blocked | blocked_diag)) { (dg ? blocked_diag : blocked) |= t; continue; }
                 uint64_t nb = need(items[i]) & ~chosen;
                 int add = __builtin_popcountll(nb);
                 bool too_big = !items[i].marker && items[i].g.kind != 1 &&
@@ -815,8 +937,12 @@ extern "C" int bs_adjoint_gradient(bs_sim* s, const bs_op* ops, int64_t n_ops, c
             seg_first = false;
         }
     }
-    // pack device data
+    // pack device data.  The items of a sweep are taken in alternating phases that keep the order of
+    // items which share a bit and do not both stand on the diagonal: all diagonal items that nothing
+    // holds back (one kind 7), then all others that nothing holds back.
     std::vector<AdjGate> ag;
+    std::vector<AdjTab> tabs;
+    std::vector<AdjMark> marks;
     std::vector<float4> mats;
     std::vector<int32_t> perms;
     std::vector<int64_t> sweep_first;
@@ -826,25 +952,10 @@ extern "C" int bs_adjoint_gradient(bs_sim* s, const bs_op* ops, int64_t n_ops, c
         for (int b = 0; b < L; b++) local[b] = b;
         for (size_t i = 0; i < sweeps_hi[sw].size(); i++) local[sweeps_hi[sw][i]] = L + (int)i;
         sweep_first.push_back((int64_t)ag.size());
-        for (int ii : sweeps_items[sw]) {
-            const BwdItem& it = items[(size_t)ii];
+        auto emit_gate = [&](const HostGate& hg) {
             AdjGate a{};
-            a.g.kind = it.marker ? 3 : it.g.kind;
-            a.g.k = it.g.k;
-            if (it.marker) {
-                a.slot = it.slot;
-                a.projector = it.projector;
-                a.weight = it.weight;
-                a.zm = it.zm;
-                a.ph = it.ph;
-                uint32_t xl = 0;
-                for (int b = 0; b < n_bits; b++) if ((it.xm >> b) & 1ULL) xl |= 1u << local[b];
-                a.xm_local = xl;
-                if (it.projector) a.g.gbit[0] = it.g.ebit[0];
-                ag.push_back(a);
-                continue;
-            }
-            const HostGate& hg = it.g;
+            a.g.kind = hg.kind;
+            a.g.k = hg.k;
             uint64_t gcm = 0, gcv = 0;
             uint32_t lcm = 0, lcv = 0;
             for (int b = 0; b < n_bits; b++) {
@@ -863,7 +974,97 @@ extern "C" int bs_adjoint_gradient(bs_sim* s, const bs_op* ops, int64_t n_ops, c
             if (hg.kind == 0) for (int e = 0; e < (1 << (2 * hg.k)); e++) mats.push_back(to_cff(hg.mat[2 * e], hg.mat[2 * e + 1]));
             else if (hg.kind == 1) for (int e = 0; e < (1 << hg.k); e++) mats.push_back(to_cff(hg.mat[2 * e], hg.mat[2 * e + 1]));
             else perms.insert(perms.end(), hg.perm.begin(), hg.perm.end());
+            if (hg.kind == 0 && hg.k == 1) a.g.npar = class_2x2(hg);
             ag.push_back(a);
+        };
+        auto add_mark = [&](uint64_t zm, int slot, double w) {
+            AdjMark m{};
+            for (int b = 0; b < n_bits; b++) {
+                if (!((zm >> b) & 1ULL)) continue;
+                if (local[b] >= 0) m.z_tile |= 1u << local[b];
+                else m.z_out |= 1ULL << b;
+            }
+            m.slot = slot;
+            m.weight = w;
+            marks.push_back(m);
+        };
+        std::vector<int> left = sweeps_items[sw], rest;
+        while (!left.empty()) {
+            // diagonal phase: nothing but an earlier non-diagonal item on the same bits holds one back
+            std::vector<const HostGate*> folds;
+            AdjGate ph{};
+            ph.g.kind = 7;
+            ph.slot = (int32_t)marks.size();
+            uint64_t held = 0;
+            rest.clear();
+            std::vector<const HostGate*> wide;
+            for (int ii : left) {
+                const BwdItem& it = items[(size_t)ii];
+                const uint64_t t = it.touch();
+                if (!it.diag()) { held |= t; rest.push_back(ii); continue; }
+                if (t & held) { rest.push_back(ii); continue; }
+                if (!it.marker) {
+                    (__builtin_popcountll(t) <= kTabBits ? folds : wide).push_back(&it.g);
+                } else if (it.projector) {
+                    // P1 = (1 - Z) / 2
+                    add_mark(0, it.slot, 0.5 * it.weight);
+                    add_mark(1ULL << it.g.ebit[0], it.slot, -0.5 * it.weight);
+                } else {
+                    add_mark(it.zm, it.slot, it.weight);   // the phase (-i)^0: no Y in a generator that flips nothing
+                }
+            }
+            left.swap(rest);
+            ph.ph = (int32_t)marks.size() - ph.slot;
+            std::vector<FoldTab> ft;
+            fold_diags(folds, ft);
+            ph.xm_local = (uint32_t)tabs.size();
+            ph.n_tabs = (int32_t)ft.size();
+            for (const FoldTab& f : ft) {
+                AdjTab t{};
+                t.k = (int32_t)f.eb.size();
+                t.mat_off = (int32_t)mats.size();
+                for (size_t q = 0; q < f.eb.size(); q++) {
+                    t.gbit[q] = (int8_t)f.eb[q];
+                    t.pos[q] = (int8_t)local[f.eb[q]];
+                }
+                for (const std::complex<double>& v : f.d) mats.push_back(to_cff(v.real(), v.imag()));
+                tabs.push_back(t);
+            }
+            if (ph.ph || ph.n_tabs) ag.push_back(ph);
+            for (const HostGate* h : wide) emit_gate(*h);
+            // the others: anything earlier on the same bits holds one back
+            held = 0;
+            rest.clear();
+            for (size_t i = 0; i < left.size(); i++) {
+                const BwdItem& it = items[(size_t)left[i]];
+                const uint64_t t = it.touch();
+                if (it.diag() || (t & held)) { held |= t; rest.push_back(left[i]); continue; }
+                if (!it.marker) { emit_gate(it.g); continue; }
+                // a marker whose gate comes next, one dense target and a generator X or Y on it: one pass
+                if (i + 1 < left.size() && left[i + 1] == left[i] + 1) {
+                    const BwdItem& nx = items[(size_t)left[i + 1]];
+                    if (!nx.marker && nx.g.kind == 0 && nx.g.k == 1 && nx.g.cmask == 0 && it.xm == (1ULL << nx.g.ebit[0]) &&
+                        (it.zm == 0 || it.zm == it.xm)) {
+                        emit_gate(nx.g);
+                        AdjGate& a = ag.back();
+                        a.g.kind = 6;
+                        a.ph = it.zm ? 1 : 0;
+                        a.slot = it.slot;
+                        a.weight = it.weight;
+                        i++;
+                        continue;
+                    }
+                }
+                AdjGate a{};
+                a.g.kind = 3;
+                a.slot = it.slot;
+                a.weight = it.weight;
+                a.zm = it.zm;
+                a.ph = it.ph;
+                for (int b = 0; b < n_bits; b++) if ((it.xm >> b) & 1ULL) a.xm_local |= 1u << local[b];
+                ag.push_back(a);
+            }
+            left.swap(rest);
         }
     }
     sweep_first.push_back((int64_t)ag.size());
@@ -871,21 +1072,28 @@ extern "C" int bs_adjoint_gradient(bs_sim* s, const bs_op* ops, int64_t n_ops, c
     const int64_t b_ag = al((int64_t)ag.size() * (int64_t)sizeof(AdjGate));
     const int64_t b_m = al((int64_t)mats.size() * (int64_t)sizeof(float4));
     const int64_t b_p = al((int64_t)(perms.size() + 1) * 4);
-    rc = bs_ensure_plan(s, b_ag + b_m + b_p);
+    const int64_t b_t = al((int64_t)(tabs.size() + 1) * (int64_t)sizeof(AdjTab));
+    const int64_t b_k = al((int64_t)(marks.size() + 1) * (int64_t)sizeof(AdjMark));
+    rc = bs_ensure_plan(s, b_ag + b_m + b_p + b_t + b_k);
     if (rc) { cudaFreeAsync(lam, s->stream); free_ckpt(); return rc; }
-    std::vector<char> host((size_t)(b_ag + b_m + b_p), 0);
+    std::vector<char> host((size_t)(b_ag + b_m + b_p + b_t + b_k), 0);
     if (!ag.empty()) std::memcpy(host.data(), ag.data(), ag.size() * sizeof(AdjGate));
     if (!mats.empty()) std::memcpy(host.data() + b_ag, mats.data(), mats.size() * sizeof(float4));
     if (!perms.empty()) std::memcpy(host.data() + b_ag + b_m, perms.data(), perms.size() * 4);
+    if (!tabs.empty()) std::memcpy(host.data() + b_ag + b_m + b_p, tabs.data(), tabs.size() * sizeof(AdjTab));
+    if (!marks.empty()) std::memcpy(host.data() + b_ag + b_m + b_p + b_t, marks.data(), marks.size() * sizeof(AdjMark));
     cudaMemcpyAsync(s->plan_buf, host.data(), host.size(), cudaMemcpyHostToDevice, s->stream);
     const AdjGate* d_ag = (const AdjGate*)s->plan_buf;
     const float4* d_m = (const float4*)((char*)s->plan_buf + b_ag);
     const int32_t* d_p = (const int32_t*)((char*)s->plan_buf + b_ag + b_m);
+    const AdjTab* d_t = (const AdjTab*)((char*)s->plan_buf + b_ag + b_m + b_p);
+    const AdjMark* d_k = (const AdjMark*)((char*)s->plan_buf + b_ag + b_m + b_p + b_t);
     const int H = T - L;
-    const size_t smem = (size_t)2 * ((size_t)1 << T) * sizeof(float4) + ((size_t)1 << H) * sizeof(int64_t);
+    const size_t extra = (size_t)kSweepPer * kSweepThreads * sizeof(float2) + ((size_t)1 << H) * sizeof(int64_t);
+    const size_t smem = (size_t)2 * ((size_t)1 << T) * sizeof(float4) + extra;
+    const size_t smem64 = (size_t)2 * ((size_t)1 << T) * sizeof(float2) + extra;
     cudaFuncSetAttribute(k_adjoint_sweep<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    cudaFuncSetAttribute(k_adjoint_sweep_c64, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    const size_t smem64 = (size_t)2 * ((size_t)1 << T) * sizeof(float2) + ((size_t)1 << H) * sizeof(int64_t);
+    cudaFuncSetAttribute(k_adjoint_sweep<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     const int64_t ntiles = (int64_t)1 << (n_bits - T);
     for (size_t sw = 0; sw < sweeps_items.size(); sw++) {
         if (sweep_restore[sw] >= 0)
@@ -903,11 +1111,11 @@ extern "C" int bs_adjoint_gradient(bs_sim* s, const bs_op* ops, int64_t n_ops, c
         for (int64_t t0 = 0; t0 < ntiles; t0 += (1LL << 30)) {
             int64_t nb = std::min<int64_t>(ntiles - t0, 1LL << 30);
             if (c64)
-                k_adjoint_sweep_c64<<<(unsigned)nb, kAThreads, smem64, s->stream>>>((float2*)s->state, (float2*)lam, d,
-                                                                                    d_ag + sweep_first[sw], d_acc, t0);
+                k_adjoint_sweep<true><<<(unsigned)nb, kSweepThreads, smem64, s->stream>>>((float2*)s->state, (float2*)lam, d,
+                                                                                          d_ag + sweep_first[sw], d_t, d_k, d_acc, t0);
             else
-                k_adjoint_sweep<false><<<(unsigned)nb, kAThreads, smem, s->stream>>>((double2*)s->state, (double2*)lam, d,
-                                                                                      d_ag + sweep_first[sw], d_acc, t0);
+                k_adjoint_sweep<false><<<(unsigned)nb, kSweepThreads, smem, s->stream>>>((double2*)s->state, (double2*)lam, d,
+                                                                                         d_ag + sweep_first[sw], d_t, d_k, d_acc, t0);
         }
         s->stats.kernel_launches++;
         s->stats.sweeps++;

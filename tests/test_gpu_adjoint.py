@@ -142,3 +142,65 @@ def test_rrule_and_torch_autograd():
     out.backward()
     assert abs(out.item() - 3.0 * e) < 1e-12
     assert np.max(np.abs(theta.grad.numpy() - 3.0 * ps)) < 1e-10
+
+
+def _all_forms(n, layers, rng):
+    """Every item form of the backward sweep: X/Y rotations (gate and marker in one pass), diagonal
+    rotations and phases, two-qubit generators, fixed dense / monomial / diagonal gates with controls,
+    a diagonal gate on more bits than a folded table holds."""
+    ops = [bs.Instruction(bs.H(), [q]) for q in range(n)]
+    a = lambda: float(rng.uniform(-np.pi, np.pi))  # noqa: E731
+    for layer in range(layers):
+        for q in range(n):
+            ops.append(bs.Instruction([bs.Rx, bs.Ry, bs.Rz][(q + layer) % 3](a()), [q]))
+        for q in range(0, n - 1, 2):
+            ops.append(bs.Instruction([bs.ZZ, bs.XX, bs.YY][(q // 2 + layer) % 3](a()), [q, q + 1]))
+        for q in range(n):
+            ops.append(bs.Instruction(bs.PhaseShift(a()), [q]) if q % 2 else bs.Instruction(bs.Rz(a()), [q]))
+        if n > 1:
+            ops.append(bs.Instruction(bs.CNot(), [layer % n, (layer + 1) % n]))
+            ops.append(bs.Instruction(bs.CPhaseShift(0.3), [(layer + 1) % n, layer % n]))
+            ops.append(bs.Instruction(bs.Control(bs.H(), (1,)), [n - 1, 0]))
+        if n >= 10:
+            ops.append(bs.Instruction(bs.Control(bs.Z(), tuple([1] * 9)), list(range(10))))
+    return ops
+
+
+@pytest.mark.parametrize("n,layers", [(1, 3), (3, 2), (9, 2), (10, 1), (12, 1), (13, 1), (15, 1)])
+def test_backward_sweep_forms_match_parameter_shift(n, layers):
+    rng = np.random.default_rng(900 + n)
+    ops = _all_forms(n, layers, rng)
+    # the fixed controlled phases are not parameters; every differentiable gate is
+    h = hamiltonian(n, 6, rng)
+    sim = bs.StateVectorSimulator(n, 0)
+    e, g = adj.adjoint_gradient(sim, ops, h)
+    ps = adj.parameter_shift_gradient(sim, ops, h)
+    assert abs(e - adj.energy(sim, ops, h)) < 1e-12 * max(1.0, sum(abs(c) for c, _ in h))
+    assert np.max(np.abs(g - ps)) < 1e-10
+    e64, g64 = adj.adjoint_gradient(bs.StateVectorSimulator(n, 0, precision="c64"), ops, h)
+    assert np.max(np.abs(g64 - ps)) < 2e-5 * max(1.0, sum(abs(c) for c, _ in h))
+
+
+def test_more_rotations_in_a_sweep_than_the_sum_buffer_holds():
+    n, rng = 12, np.random.default_rng(77)   # one tile: every gate in one sweep, 60 rotation sums
+    ops = [bs.Instruction([bs.Rx, bs.Ry][layer % 2](float(rng.uniform(-3, 3))), [q]) for layer in range(5) for q in range(n)]
+    h = hamiltonian(n, 5, rng)
+    sim = bs.StateVectorSimulator(n, 0)
+    bs.set_tuning(sim, adj_segments=1)
+    _, g = adj.adjoint_gradient(sim, ops, h)
+    assert np.max(np.abs(g - adj.parameter_shift_gradient(sim, ops, h))) < 1e-10
+
+
+def test_diagonal_gate_that_is_not_unitary_keeps_its_place():
+    """A diagonal matrix with entries off the unit circle does not leave conj(lambda) psi alone: the
+    markers on its bits stay on their side of it, so the gradient equals the one with the same matrix
+    given as a dense gate with a tiny off-diagonal entry."""
+    rng = np.random.default_rng(5)
+    h = hamiltonian(4, 5, rng)
+    grads = []
+    for eps in (0.0, 1e-300):
+        m = np.array([[1.0, eps], [0.0, 0.7]], dtype=complex)
+        ops = [bs.Instruction(bs.H(), [q]) for q in range(4)] + [bs.Instruction(bs.Rz(0.4), [0]), bs.Instruction(bs.Ry(0.3), [1])]
+        ops += [bs.Instruction(bs.Unitary(m), [0]), bs.Instruction(bs.ZZ(0.9), [0, 2]), bs.Instruction(bs.Rx(-0.8), [0])]
+        grads.append(adj.adjoint_gradient(bs.StateVectorSimulator(4, 0), ops, h)[1])
+    assert np.max(np.abs(grads[0] - grads[1])) < 1e-12
