@@ -98,3 +98,52 @@ def test_c64_runs_on_qubit_pairs_fold_into_two_bit_gates():
     sim = bs.StateVectorSimulator(n, 0, precision="c64").evolve(ops)
     err = rel_err(sim.state_vector, oracle.OracleSV(n).evolve(ops).psi)
     assert err < 2e-5, err
+
+
+def _block_circuit(n, gates, rng, kinds):
+    """Gates of the register blocks' kinds on random qubits: one-target gates of every matrix class with
+    any controls, swaps, diagonals on and off the block, and (kind "wide") gates that keep their pass."""
+    ops, a = [], lambda: float(rng.uniform(-np.pi, np.pi))
+    for _ in range(gates):
+        q = [int(x) for x in rng.choice(n, min(n, 4), replace=False)]
+        k = kinds[int(rng.integers(len(kinds)))]
+        if k == "one":
+            g = [bs.H(), bs.X(), bs.Y(), bs.Rx(a()), bs.Ry(a()), bs.Rz(a()), bs.S(), bs.U(a(), a(), a()), bs.V()][int(rng.integers(9))]
+            ops.append(bs.Instruction(g, [q[0]]))
+        elif k == "ctrl":
+            g = [bs.X(), bs.Ry(a()), bs.U(a(), a(), a()), bs.Z()][int(rng.integers(4))]
+            nc = int(rng.integers(1, 3))   # the oracle has kernels for up to two controls
+            ops.append(bs.Instruction(bs.Control(g, tuple(int(b) for b in rng.integers(0, 2, nc))), q[:nc + 1]))
+        elif k == "diag":
+            g = [bs.CZ(), bs.ZZ(a()), bs.CPhaseShift(a()), bs.CPhaseShift01(a())][int(rng.integers(4))]
+            ops.append(bs.Instruction(g, q[:2]))
+        elif k == "swap":
+            ops.append(bs.Instruction(bs.Swap(), q[:2]))
+        else:
+            g = [bs.XX(a()), bs.ISwap(), bs.FermionicSWAP(a())][int(rng.integers(3))]
+            ops.append(bs.Instruction(g, q[:2]))
+    return ops
+
+
+@pytest.mark.parametrize("n,gates,kinds", [
+    (12, 60, ("one", "ctrl", "diag", "swap")),       # one tile, every bit in it
+    (13, 80, ("one", "ctrl", "diag", "swap")),       # one bit outside
+    (17, 120, ("one", "ctrl", "diag", "swap")),
+    (18, 90, ("one", "diag", "wide")),               # passes between blocks
+    (16, 60, ("diag",)),                             # no moved bit at all
+    (12, 400, ("one", "ctrl")),                      # more operations than are staged at a time
+    (11, 60, ("one", "ctrl", "diag")),               # below a full tile: no blocks
+])
+def test_register_blocks_match_the_oracle(n, gates, kinds):
+    rng = np.random.default_rng(7000 + n + gates)
+    ops = [bs.Instruction(bs.H(), [q]) for q in range(n)] + _block_circuit(n, gates, rng, kinds)
+    err = rel_err(bs.StateVectorSimulator(n, 0, precision="c64").evolve(ops).state_vector, oracle.OracleSV(n).evolve(ops).psi)
+    # an FP32 rounding of the matrix and of the state per gate, each at most 2^-24 of the norm
+    assert err < len(ops) * 2.0 ** -23, err
+
+
+def test_register_blocks_on_a_density_matrix():
+    n, rng = 7, np.random.default_rng(8)
+    ops = [bs.Instruction(bs.H(), [q]) for q in range(n)] + _block_circuit(n, 40, rng, ("one", "ctrl", "diag", "swap"))
+    err = rel_err(bs.DensityMatrixSimulator(n, 0, precision="c64").evolve(ops).density_matrix, oracle.OracleDM(n).evolve(ops).matrix)
+    assert err < 2 * len(ops) * 2.0 ** -23, err
