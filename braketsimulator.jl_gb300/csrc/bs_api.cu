@@ -138,6 +138,14 @@ int bs_ensure_plan(bs_sim* s, int64_t bytes) {
     return BS_OK;
 }
 
+int bs_ensure_counter(bs_sim* s) {
+    if (s->counter) return BS_OK;
+    if (s->capturing) return bs_fail(s, BS_ERR_STATE, "counter allocation during graph capture");
+    int rc = bs_cuda_check(s, cudaMalloc((void**)&s->counter, 256), "counter allocation");
+    if (rc) return rc;
+    return bs_cuda_check(s, cudaMemsetAsync(s->counter, 0, 256, s->stream), "counter reset");
+}
+
 namespace {
 
 __global__ void k_basis0(double2* psi) { psi[0] = make_double2(1.0, 0.0); }
@@ -239,6 +247,7 @@ int bs_destroy(bs_sim* s) {
     if (s->scratch) cudaFree(s->scratch);
     if (s->plan_buf) cudaFree(s->plan_buf);
     if (s->dev_flag) cudaFree(s->dev_flag);
+    if (s->counter) cudaFree(s->counter);
     if (s->alias_ap) cudaFree(s->alias_ap);
     if (s->alias_ix) cudaFree(s->alias_ix);
     if (s->ev0) cudaEventDestroy(s->ev0);

@@ -135,6 +135,7 @@ struct bs_sim {
     int64_t plan_bytes = 0;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     int* dev_flag = nullptr;      // device error flag of the tensor-core sweeps
+    unsigned* counter = nullptr;  // bs_ensure_counter
     bool flag_armed = false;
     std::vector<cudaEvent_t> tc_events;   // pool: an event pair around each tensor-core launch
     size_t tc_events_used = 0;            // pairs recorded since the last bs_collect_tc_time
@@ -171,6 +172,8 @@ int bs_cuda_check(bs_sim* s, cudaError_t e, const char* what);
 int bs_copy_out(bs_sim* s, void* host, const void* dev, size_t bytes, const char* what);
 int bs_ensure_scratch(bs_sim* s, int64_t bytes);
 int bs_ensure_plan(bs_sim* s, int64_t bytes);
+// The counter with which the last block of an expectation is found (zero between calls), allocated on first use.
+int bs_ensure_counter(bs_sim* s);
 // Pinned host region for one upload of `bytes`; call bs_stage_done after queuing the copy.
 char* bs_stage(bs_sim* s, size_t bytes);
 void bs_stage_done(bs_sim* s);

@@ -80,70 +80,129 @@ __device__ void block_sum_store(double v, double* partial, int64_t idx) {
     }
 }
 
-__device__ __forceinline__ void pauli_accumulate(ffsum* acc, const TermSet& ts, int64_t i, float wrh, float wrl,
-                                                 float wih, float wil) {
-    for (int t = 0; t < ts.nt; t++) {
-        bool neg = __popcll((unsigned long long)i & ts.zm[t]) & 1;
-        float vh, vl;
-        switch (ts.ph[t]) {            // Re((-i)^ph * w)
-            case 0: vh = wrh; vl = wrl; break;
-            case 1: vh = wih; vl = wil; break;
-            case 2: vh = -wrh; vl = -wrl; break;
-            default: vh = -wih; vl = -wil; break;
-        }
-        if (neg) { vh = -vh; vl = -vl; }
-        fsum_add(acc[t], vh, vl);
+// The sign and component of a term: Re((-i)^ph w) is +-Re w for even ph and +-Im w for odd, times the
+// parity of the index under the term's Z mask.
+template <int NT>
+__device__ __forceinline__ void pauli_accumulate(ffsum (&acc)[NT], const TermSet& ts, int64_t i, const ff& re, const ff& im) {
+#pragma unroll
+    for (int t = 0; t < NT; t++) {
+        if (NT > 1 && t >= ts.nt) break;
+        const uint32_t z = ((uint32_t)i & (uint32_t)ts.zm[t]) ^ ((uint32_t)(i >> 32) & (uint32_t)(ts.zm[t] >> 32));
+        const uint32_t sg = ((uint32_t)(ts.ph[t] >> 1) ^ (uint32_t)__popc(z)) << 31;
+        const ff v = (ts.ph[t] & 1) ? im : re;
+        fsum_add(acc[t], __uint_as_float(__float_as_uint(v.h) ^ sg), __uint_as_float(__float_as_uint(v.l) ^ sg));
     }
 }
 
-// SV Pauli terms sharing flip mask xm.  Pairs (i, i^xm) with the top bit of xm
-// clear contribute 2 Re(c(i) conj(psi_i) psi_{i^xm}); xm == 0 gives |psi_i|^2 * sign.
-template <bool C64>
-__global__ void __launch_bounds__(kRThreads) k_pauli_sv(const typename Elem<C64>::T* __restrict__ psi, int64_t n,
-                                                        uint64_t xm, TermSet ts, double* __restrict__ partial, int n_slots) {
-    ffsum acc[kMaxTermsPerPass];
-    for (int t = 0; t < kMaxTermsPerPass; t++) acc[t] = {0.f, 0.f};
-    const int64_t npairs = xm ? n / 2 : n;
-    int hb = xm ? 63 - __clzll((long long)xm) : 0;
-    for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < npairs; p += (int64_t)gridDim.x * blockDim.x) {
-        int64_t i = p;
-        if (xm) { int64_t low = p & ((1LL << hb) - 1); i = ((p >> hb) << (hb + 1)) | low; }
-        cff a = Elem<C64>::load(psi[i]);
-        float wrh, wrl, wih, wil;
-        if (xm) {
-            cff b = Elem<C64>::load(psi[i ^ (int64_t)xm]);
-            ffacc r, m;
-            acc_first(r, a.rh, a.rl, b.rh, b.rl);
-            acc_add(r, a.ih, a.il, b.ih, b.il);
-            acc_first(m, a.rh, a.rl, b.ih, b.il);
-            acc_add(m, -a.ih, -a.il, b.rh, b.rl);
-            ff rr = acc_done(r), mm = acc_done(m);
-            wrh = 2.f * rr.h; wrl = 2.f * rr.l; wih = 2.f * mm.h; wil = 2.f * mm.l;
-        } else {
-            ffacc r;
-            acc_first(r, a.rh, a.rl, a.rh, a.rl);
-            acc_add(r, a.ih, a.il, a.ih, a.il);
-            ff rr = acc_done(r);
-            wrh = rr.h; wrl = rr.l; wih = 0.f; wil = 0.f;
+// Last block of the call (its launches' blocks add up to last_total in *done): every partial is there,
+// so its warps form the results, one slot each at a time (FP64 sums with compensated leaves), and the
+// counter goes back to zero.  A launch fewer per call than a separate pass over the partials, which
+// took 2.5 to 5 us of device time.
+__device__ void finish_partials(double* partial, int nblocks, int n_slots, unsigned* done, unsigned last_total) {
+    __shared__ bool s_last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = atomicAdd(done, 1u) + 1u == last_total;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    double* out = partial + (int64_t)nblocks * n_slots;
+    const int lane = threadIdx.x & 31;
+    for (int slot = threadIdx.x >> 5; slot < n_slots; slot += kRThreads / 32) {
+        double s = 0.0, c = 0.0;
+        for (int b = lane; b < nblocks; b += 32) {
+            const double y = __ldcg(partial + (int64_t)b * n_slots + slot) - c;
+            const double t = s + y;
+            c = (t - s) - y;
+            s = t;
         }
-        pauli_accumulate(acc, ts, i, wrh, wrl, wih, wil);
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+        if (lane == 0) out[slot] = s;
     }
-    for (int t = 0; t < ts.nt; t++)
-        block_sum_store(ff2d(acc[t].h, acc[t].l), partial, (int64_t)blockIdx.x * n_slots + ts.slot[t]);
+    if (threadIdx.x == 0) *done = 0;
+}
+
+// SV Pauli terms sharing flip mask xm.  Pairs (i, i^xm) with the top bit of xm clear contribute
+// 2 Re(c(i) conj(psi_i) psi_{i^xm}); xm == 0 gives |psi_i|^2 * sign.  RE / IM: which part of the
+// product the launch's terms need.
+// What bounds it: HBM, once the arithmetic is down to the part needed (both parts and one pair in
+// flight per thread were ALU-bound at 3.2 TB/s) and eight amplitudes are in flight per thread.  26
+// qubits, one term: 337 -> 174 us with a flip mask (6.2 TB/s), 202 us without.
+// ONE: a single term (the usual expectation); several terms on one flip mask share the read.
+template <bool C64, bool FLIP, bool RE, bool IM, bool ONE>
+__global__ void __launch_bounds__(kRThreads, 4) k_pauli_sv(const typename Elem<C64>::T* __restrict__ psi, int64_t n, uint64_t xm,
+                                                           TermSet ts, double* __restrict__ partial, int n_slots,
+                                                           unsigned* __restrict__ done, unsigned last_total) {
+    constexpr int U = (FLIP ? 4 : 8) / (ONE ? 1 : 2);   // positions in flight
+    constexpr int NT = ONE ? 1 : kMaxTermsPerPass;
+    ffsum acc[NT];
+#pragma unroll
+    for (int t = 0; t < NT; t++) acc[t] = {0.f, 0.f};
+    const int64_t np = FLIP ? n / 2 : n, step = (int64_t)gridDim.x * blockDim.x;
+    const int64_t lowm = FLIP ? (1LL << (63 - __clzll((long long)xm))) - 1 : 0;
+    auto index = [&](int64_t p) { return FLIP ? ((p & ~lowm) << 1) | (p & lowm) : p; };
+    for (int64_t p0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p0 < np; p0 += U * step) {
+        typename Elem<C64>::T va[U], vb[FLIP ? U : 1];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int64_t p = p0 + u * step;
+            if (p < np) {
+                const int64_t i = index(p);
+                va[u] = psi[i];
+                if (FLIP) vb[u] = psi[i ^ (int64_t)xm];
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int64_t p = p0 + u * step;
+            if (p >= np) break;
+            const cff a = Elem<C64>::load(va[u]);
+            ff re{0.f, 0.f}, im{0.f, 0.f};
+            if (FLIP) {
+                const cff b = Elem<C64>::load(vb[u]);
+                if (RE) {
+                    ffacc r;
+                    acc_first(r, a.rh, a.rl, b.rh, b.rl);
+                    acc_add(r, a.ih, a.il, b.ih, b.il);
+                    re = {r.s, r.c};   // fsum_add takes the pair as it is
+                }
+                if (IM) {
+                    ffacc m;
+                    acc_first(m, a.rh, a.rl, b.ih, b.il);
+                    acc_add(m, -a.ih, -a.il, b.rh, b.rl);
+                    im = {m.s, m.c};
+                }
+            } else {
+                ffacc r;
+                acc_first(r, a.rh, a.rl, a.rh, a.rl);
+                acc_add(r, a.ih, a.il, a.ih, a.il);
+                re = {r.s, r.c};
+            }
+            pauli_accumulate<NT>(acc, ts, index(p), re, im);
+        }
+    }
+#pragma unroll
+    for (int t = 0; t < NT; t++) {
+        if (NT > 1 && t >= ts.nt) break;
+        block_sum_store((FLIP ? 2.0 : 1.0) * ff2d(acc[t].h, acc[t].l), partial, (int64_t)blockIdx.x * n_slots + ts.slot[t]);
+    }
+    finish_partials(partial, gridDim.x, n_slots, done, last_total);
 }
 
 // DM Pauli terms: E = sum_a Re(P[a, a^xm] S[a, a^xm]), S[r, c] at r + c*dim.
 template <bool C64>
 __global__ void __launch_bounds__(kRThreads) k_pauli_dm(const typename Elem<C64>::T* __restrict__ S, int64_t dim,
-                                                        uint64_t xm, TermSet ts, double* __restrict__ partial, int n_slots) {
+                                                        uint64_t xm, TermSet ts, double* __restrict__ partial, int n_slots,
+                                                        unsigned* __restrict__ done, unsigned last_total) {
     ffsum acc[kMaxTermsPerPass];
     for (int t = 0; t < kMaxTermsPerPass; t++) acc[t] = {0.f, 0.f};
     for (int64_t a = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; a < dim; a += (int64_t)gridDim.x * blockDim.x) {
-        cff v = Elem<C64>::load(S[a + (a ^ (int64_t)xm) * dim]);
-        pauli_accumulate(acc, ts, a, v.rh, v.rl, v.ih, v.il);
+        const cff v = Elem<C64>::load(S[a + (a ^ (int64_t)xm) * dim]);
+        pauli_accumulate<kMaxTermsPerPass>(acc, ts, a, {v.rh, v.rl}, {v.ih, v.il});
     }
     for (int t = 0; t < ts.nt; t++)
         block_sum_store(ff2d(acc[t].h, acc[t].l), partial, (int64_t)blockIdx.x * n_slots + ts.slot[t]);
+    finish_partials(partial, gridDim.x, n_slots, done, last_total);
 }
 
 __global__ void k_sum_partials(const double* __restrict__ partial, int nblocks, int n_slots, double* __restrict__ out) {
@@ -215,23 +274,68 @@ __global__ void __launch_bounds__(kRThreads) k_matrix_expect(const typename Elem
     block_sum_store(acc, partial, blockIdx.x);
 }
 
-// marginal probabilities: out[o] = sum of p_i over i whose target bits spell o
-// (output bit j <-> j-th smallest endian target bit)
+// marginal probabilities: out[o] = sum of p_i over i whose target bits spell o (output bit j <-> j-th
+// smallest endian target bit).  A block takes chunks of 2^cb consecutive indices; the low 8 bits of an
+// index are the thread's, and the chunk's other bits run with the target bits outermost, so a thread
+// adds up all indices of one output in float-float and touches the shared histogram once for them (an
+// FP64 shared-memory atomic per probability held the pass to 1.5 TB/s; 26 qubits, 8 targets: 0.69 ->
+// 0.32 ms).
+struct Marg {
+    int nbits, k, cb;
+    int bit[12];               // target endian bits, ascending
+    uint32_t tmask;            // target bits among the chunk's bits 8 .. cb
+};
+__device__ __forceinline__ uint32_t deposit(uint32_t v, uint32_t mask) {   // the bits of v into the places of mask
+    uint32_t out = 0;
+    for (; mask; mask &= mask - 1) {
+        if (v & 1u) out |= mask & (0u - mask);
+        v >>= 1;
+    }
+    return out;
+}
 template <bool C64>
-__global__ void __launch_bounds__(kRThreads) k_marginal(const typename Elem<C64>::T* __restrict__ st, int dm, int nbits_q,
-                                                        int k, const int* __restrict__ eb_sorted,
+__global__ void __launch_bounds__(kRThreads) k_marginal(const typename Elem<C64>::T* __restrict__ st, int dm, Marg d,
                                                         double* __restrict__ partial) {
     extern __shared__ double hist[];
-    const int D = 1 << k;
-    const int64_t dim = (int64_t)1 << nbits_q;
+    const int D = 1 << d.k;
+    const int64_t dim = (int64_t)1 << d.nbits;
     for (int o = threadIdx.x; o < D; o += blockDim.x) hist[o] = 0.0;
     __syncthreads();
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < dim; i += (int64_t)gridDim.x * blockDim.x) {
-        double p = dm ? (double)st[i * (dim + 1)].x : prob_of<C64>(st[i]);
-        int o = 0;
-        for (int q = 0; q < k; q++) o |= (int)((i >> eb_sorted[q]) & 1) << q;
-        atomicAdd(&hist[o], p);
-    }
+    const uint32_t rmask = (((1u << d.cb) - 1u) & ~255u) & ~d.tmask;   // traced bits of the chunk
+    const uint32_t nt = 1u << __popc(d.tmask), nr = 1u << __popc(rmask);
+    for (int64_t c = blockIdx.x; c == 0 || c < (dim >> d.cb); c += gridDim.x)
+        for (uint32_t t = 0; t < nt; t++) {
+            const int64_t i0 = (c << d.cb) | deposit(t, d.tmask) | threadIdx.x;
+            ffsum acc{0.f, 0.f};
+            uint32_t r = 0;          // runs over the submasks of rmask
+            for (uint32_t n = 0; n < nr; n += 8) {
+                typename Elem<C64>::T v[8];
+#pragma unroll
+                for (int u = 0; u < 8; u++) {
+                    const int64_t i = i0 | r;
+                    if (n + u < nr && (int64_t)threadIdx.x < dim) v[u] = st[dm ? i * (dim + 1) : i];
+                    r = (r - rmask) & rmask;
+                }
+#pragma unroll
+                for (int u = 0; u < 8; u++)
+                    if (n + u < nr && (int64_t)threadIdx.x < dim) {
+                        const cff a = Elem<C64>::load(v[u]);
+                        if (dm) {
+                            fsum_add(acc, a.rh, a.rl);
+                        } else {
+                            ffacc q;
+                            acc_first(q, a.rh, a.rl, a.rh, a.rl);
+                            acc_add(q, a.ih, a.il, a.ih, a.il);
+                            fsum_add(acc, q.s, q.c);
+                        }
+                    }
+            }
+            if ((int64_t)threadIdx.x < dim) {
+                int o = 0;
+                for (int q = 0; q < d.k; q++) o |= (int)((i0 >> d.bit[q]) & 1) << q;
+                atomicAdd(&hist[o], ff2d(acc.h, acc.l));
+            }
+        }
     __syncthreads();
     for (int o = threadIdx.x; o < D; o += blockDim.x) partial[(int64_t)blockIdx.x * D + o] = hist[o];
 }
@@ -297,12 +401,21 @@ int grid_for(int64_t work) {
 }
 
 template <bool C64>
-void launch_pauli(bs_sim* s, int nb, int64_t dim, uint64_t xm, const TermSet& set, double* partial, int n_terms) {
+void launch_pauli(bs_sim* s, int nb, int64_t dim, uint64_t xm, const TermSet& set, double* partial, int n_terms,
+                  unsigned* done, unsigned last_total) {
     using T = typename Elem<C64>::T;
-    if (s->kind == BS_KIND_SV)
-        k_pauli_sv<C64><<<nb, kRThreads, 0, s->stream>>>((const T*)s->state, dim, xm, set, partial, n_terms);
-    else
-        k_pauli_dm<C64><<<nb, kRThreads, 0, s->stream>>>((const T*)s->state, dim, xm, set, partial, n_terms);
+    const T* st = (const T*)s->state;
+    if (s->kind != BS_KIND_SV) {
+        k_pauli_dm<C64><<<nb, kRThreads, 0, s->stream>>>(st, dim, xm, set, partial, n_terms, done, last_total);
+        return;
+    }
+    int parts = 0;   // bit 0: a term needs the real part, bit 1: the imaginary part
+    for (int t = 0; t < set.nt; t++) parts |= 1 << (set.ph[t] & 1);
+    auto kern = k_pauli_sv<C64, true, true, true, false>;
+    if (set.nt == 1) kern = !xm ? k_pauli_sv<C64, false, true, false, true>
+                          : parts == 1 ? k_pauli_sv<C64, true, true, false, true> : k_pauli_sv<C64, true, false, true, true>;
+    else if (!xm) kern = k_pauli_sv<C64, false, true, false, false>;
+    kern<<<nb, kRThreads, 0, s->stream>>>(st, dim, xm, set, partial, n_terms, done, last_total);
 }
 
 }  // namespace
@@ -388,13 +501,17 @@ int bs_expectation_pauli(bs_sim* s, int n_terms, const uint64_t* xmask, const ui
         groups[xe].push_back(t);
     }
     const int64_t dim = (int64_t)1 << n;
-    const int nb = grid_for(dim);
+    // four CTAs of 256 per SM, each thread with eight amplitudes in flight
+    const int nb = (int)std::max<int64_t>(1, std::min<int64_t>((dim + 4 * kRThreads - 1) / (4 * kRThreads), 152 * 4));
     int rc = bs_ensure_scratch(s, ((int64_t)nb * n_terms + n_terms) * 8);
+    if (rc) return rc;
+    rc = bs_ensure_counter(s);
     if (rc) return rc;
     double* partial = (double*)s->scratch;
     double* res = partial + (int64_t)nb * n_terms;
-    rc = bs_cuda_check(s, cudaMemsetAsync(partial, 0, (size_t)nb * n_terms * 8, s->stream), "clear partials");
-    if (rc) return rc;
+    unsigned* done = s->counter;
+    unsigned launches = 0;
+    for (auto& kv : groups) launches += (unsigned)((kv.second.size() + kMaxTermsPerPass - 1) / kMaxTermsPerPass);
     for (auto& kv : groups) {
         const std::vector<int>& ts = kv.second;
         for (size_t c0 = 0; c0 < ts.size(); c0 += kMaxTermsPerPass) {
@@ -406,11 +523,12 @@ int bs_expectation_pauli(bs_sim* s, int n_terms, const uint64_t* xmask, const ui
                 set.ph[j] = ph[t];
                 set.slot[j] = t;
             }
-            if (s->precision == BS_PREC_C64) launch_pauli<true>(s, nb, dim, kv.first, set, partial, n_terms);
-            else launch_pauli<false>(s, nb, dim, kv.first, set, partial, n_terms);
+            if (s->precision == BS_PREC_C64) launch_pauli<true>(s, nb, dim, kv.first, set, partial, n_terms, done, launches * (unsigned)nb);
+            else launch_pauli<false>(s, nb, dim, kv.first, set, partial, n_terms, done, launches * (unsigned)nb);
         }
     }
-    k_sum_partials<<<n_terms, 256, 0, s->stream>>>(partial, nb, n_terms, res);
+    rc = bs_cuda_check(s, cudaGetLastError(), "expectation");
+    if (rc) return rc;
     if (s->capturing && coeffs) return bs_fail(s, BS_ERR_INVALID_ARG, "coefficients are applied after a captured graph runs");
     // during capture out is the graph owner's pinned buffer, filled on every replay
     rc = bs_copy_out(s, out, res, (size_t)n_terms * 8, "expectation");
@@ -474,19 +592,23 @@ int bs_marginal_probabilities(bs_sim* s, int k, const int* targets, double* host
     if (k > 12) return marginal_wide(s, k, eb, host_out);
     const int D = 1 << k;
     const int64_t dim = (int64_t)1 << s->n;
-    const int nb = grid_for(dim);
-    int rc = bs_ensure_plan(s, 256);
-    if (rc) return rc;
-    rc = bs_ensure_scratch(s, ((int64_t)nb * D + D) * 8);
-    if (rc) return rc;
-    rc = bs_cuda_check(s, cudaMemcpyAsync(s->plan_buf, eb.data(), sizeof(int) * (size_t)k, cudaMemcpyHostToDevice, s->stream), "marginal upload");
+    Marg d{};
+    d.nbits = s->n;
+    d.k = k;
+    for (int q = 0; q < k; q++) d.bit[q] = eb[(size_t)q];
+    // chunks of 2^8 to 2^14 indices, 1216 blocks where there are enough of them
+    d.cb = 8;
+    while (d.cb < 14 && (dim >> (d.cb + 1)) >= 152 * 8) d.cb++;
+    for (int q = 0; q < k; q++) if (eb[(size_t)q] >= 8 && eb[(size_t)q] < d.cb) d.tmask |= 1u << eb[(size_t)q];
+    const int nb = (int)std::max<int64_t>(1, std::min<int64_t>(dim >> d.cb, 152 * 8));
+    int rc = bs_ensure_scratch(s, ((int64_t)nb * D + D) * 8);
     if (rc) return rc;
     double* partial = (double*)s->scratch;
     const int dm = s->kind == BS_KIND_DM;
     if (s->precision == BS_PREC_C64)
-        k_marginal<true><<<nb, kRThreads, (size_t)D * 8, s->stream>>>((const float2*)s->state, dm, s->n, k, (const int*)s->plan_buf, partial);
+        k_marginal<true><<<nb, kRThreads, (size_t)D * 8, s->stream>>>((const float2*)s->state, dm, d, partial);
     else
-        k_marginal<false><<<nb, kRThreads, (size_t)D * 8, s->stream>>>((const double2*)s->state, dm, s->n, k, (const int*)s->plan_buf, partial);
+        k_marginal<false><<<nb, kRThreads, (size_t)D * 8, s->stream>>>((const double2*)s->state, dm, d, partial);
     k_sum_partials<<<D, 256, 0, s->stream>>>(partial, nb, D, partial + (int64_t)nb * D);
     return bs_copy_out(s, host_out, partial + (int64_t)nb * D, (size_t)D * 8, "marginal");
 }

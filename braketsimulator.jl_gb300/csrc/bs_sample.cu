@@ -30,6 +30,50 @@ __global__ void __launch_bounds__(128) k_block_sums(const double2* __restrict__ 
     block_chunk_sums(st, dm, dim, b, ch, cl, bsum + b, cinc + b * kCpb);
 }
 
+// The same for whole blocks of a state vector.  A warp loads its 32 chunks (one amplitude of each per
+// lane, eight loads in flight) and adds up all of them by one transposed reduction: at each step a lane
+// keeps half of its chunks and passes the other half on, 31 sums for 32 chunks where a butterfly per
+// chunk takes 160 (which held the pass to 2.4 TB/s).
+template <bool C64>
+__global__ void __launch_bounds__(128) k_block_sums_sv(const typename Elem<C64>::T* __restrict__ st, double* __restrict__ bsum,
+                                                       double* __restrict__ cinc) {
+    __shared__ float ch[kCpb], cl[kCpb];
+    const int64_t b = blockIdx.x;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const typename Elem<C64>::T* src = st + b * kBlk + warp * 32 * kChunk + lane;
+    ffsum v[32];
+#pragma unroll
+    for (int c0 = 0; c0 < 32; c0 += 8) {
+        typename Elem<C64>::T x[8];
+#pragma unroll
+        for (int c = 0; c < 8; c++) x[c] = src[(c0 + c) * kChunk];
+#pragma unroll
+        for (int c = 0; c < 8; c++) {
+            const cff a = Elem<C64>::load(x[c]);
+            ffacc r;
+            acc_first(r, a.rh, a.rl, a.rh, a.rl);
+            acc_add(r, a.ih, a.il, a.ih, a.il);
+            const ff p = acc_done(r);
+            v[c0 + c] = {p.h, p.l};
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const bool up_half = (lane & o) != 0;
+#pragma unroll
+        for (int c = 0; c < o; c++) {
+            const ffsum keep = up_half ? v[c + o] : v[c], pass = up_half ? v[c] : v[c + o];
+            const float h = __shfl_xor_sync(0xffffffffu, pass.h, o), l = __shfl_xor_sync(0xffffffffu, pass.l, o);
+            v[c] = keep;
+            fsum_add(v[c], h, l);
+        }
+    }
+    ch[warp * 32 + lane] = v[0].h;   // lane l holds chunk l of the warp
+    cl[warp * 32 + lane] = v[0].l;
+    __syncthreads();
+    scan_chunk_sums(ch, cl, bsum + b, cinc + b * kCpb);
+}
+
 // inclusive prefix of the block sums, one CTA of 1024 threads (nb is at most 2^22): a serial sum
 // over each thread's run of blocks, then a parallel scan of the 1024 run totals
 __global__ void __launch_bounds__(1024) k_scan_blocks(const double* __restrict__ bsum, int64_t nb, double* __restrict__ incl) {
@@ -37,7 +81,8 @@ __global__ void __launch_bounds__(1024) k_scan_blocks(const double* __restrict__
     const int64_t per = (nb + blockDim.x - 1) / blockDim.x;
     const int64_t b0 = threadIdx.x * per, b1 = std::min<int64_t>(nb, b0 + per);
     double s = 0.0;
-    for (int64_t b = b0; b < b1; b++) s += bsum[b];
+#pragma unroll 16
+    for (int64_t b = b0; b < b1; b++) s += bsum[b];   // unrolled for the loads: the additions stay in order
     part[threadIdx.x] = s;
     __syncthreads();
     for (int o = 1; o < (int)blockDim.x; o <<= 1) {
@@ -47,6 +92,7 @@ __global__ void __launch_bounds__(1024) k_scan_blocks(const double* __restrict__
         __syncthreads();
     }
     double run = threadIdx.x ? part[threadIdx.x - 1] : 0.0;
+#pragma unroll 16
     for (int64_t b = b0; b < b1; b++) { run += bsum[b]; incl[b] = run; }
 }
 
@@ -76,13 +122,13 @@ __global__ void k_sample_direct(const double2* __restrict__ st, int dm, int64_t 
 }
 
 
-// The same search by a whole warp: block by binary search over the block prefix sums, chunk by
-// binary search over the block's chunk prefix sums, then 32 probabilities per step with a warp
-// prefix sum and a ballot for the first running sum >= t.  The sums associate differently from a
-// left-to-right scan, so only exact boundary ties can land on a neighbouring index.
-__device__ int64_t cdf_find_warp(const double2* st, int dm, int64_t dim, const double* incl, const double* cinc,
-                                 int64_t nb, double t) {
-    const int lane = threadIdx.x & 31;
+// A shot's search down to its 32-probability chunk: block by binary search over the block prefix sums,
+// chunk by binary search over the block's chunk prefix sums.
+struct CdfPlace {
+    int64_t c, end;   // first index of the chunk, end of the block
+    double cw;        // running sum before the chunk
+};
+__device__ __forceinline__ CdfPlace cdf_place(int64_t dim, const double* incl, const double* cinc, int64_t nb, double t) {
     int64_t lo = 0, hi = nb - 1;
     while (lo < hi) {
         const int64_t mid = (lo + hi) >> 1;
@@ -95,9 +141,18 @@ __device__ int64_t cdf_find_warp(const double2* st, int dm, int64_t dim, const d
         const int mid = (clo + chi) >> 1;
         if (base + ci[mid] >= t) chi = mid; else clo = mid + 1;
     }
-    double cw = base + (clo == 0 ? 0.0 : ci[clo - 1]);
-    const int64_t end = std::min<int64_t>(dim, (lo + 1) * kBlk);
-    for (int64_t c = lo * kBlk + (int64_t)clo * kChunk; c < end; c += kChunk) {
+    CdfPlace p;
+    p.cw = base + (clo == 0 ? 0.0 : ci[clo - 1]);
+    p.end = std::min<int64_t>(dim, (lo + 1) * kBlk);
+    p.c = lo * kBlk + (int64_t)clo * kChunk;
+    return p;
+}
+// From there by a whole warp: 32 probabilities per step with a warp prefix sum and a ballot for the
+// first running sum >= t.  The sums associate differently from a left-to-right scan, so only exact
+// boundary ties can land on a neighbouring index.
+__device__ __forceinline__ int64_t cdf_scan_warp(const double2* st, int dm, int64_t dim, int64_t c0, int64_t end, double cw, double t) {
+    const int lane = threadIdx.x & 31;
+    for (int64_t c = c0; c < end; c += kChunk) {
         const int64_t i = c + lane;
         double p = (i < end) ? prob_at(st, dm, dim, i) : 0.0;
 #pragma unroll
@@ -111,16 +166,36 @@ __device__ int64_t cdf_find_warp(const double2* st, int dm, int64_t dim, const d
     }
     return end - 1;
 }
+__device__ int64_t cdf_find_warp(const double2* st, int dm, int64_t dim, const double* incl, const double* cinc,
+                                 int64_t nb, double t) {
+    const CdfPlace p = cdf_place(dim, incl, cinc, nb, t);
+    return cdf_scan_warp(st, dm, dim, p.c, p.end, p.cw, t);
+}
 
-// one shot per warp; uniforms from a counter-based splitmix64 stream
+// `per` shots per warp (1..32), uniforms from a counter-based splitmix64 stream.  Each lane searches for
+// a shot of its own down to the chunk (20 to 30 dependent loads, which bound the kernel at one shot per
+// warp: 1e5 shots at 26 qubits 0.25 -> 0.08 ms), then the warp scans the chunks one after the other.
 __global__ void k_sample_rng(const double2* __restrict__ st, int dm, int64_t dim, const double* __restrict__ incl,
-                             const double* __restrict__ cinc, int64_t nb, uint64_t seed, int64_t shots, int64_t* __restrict__ out) {
+                             const double* __restrict__ cinc, int64_t nb, uint64_t seed, int64_t shots, int per,
+                             int64_t* __restrict__ out) {
+    const int lane = threadIdx.x & 31;
     const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-    for (int64_t s = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; s < shots; s += warps) {
-        const uint64_t r = splitmix64(seed ^ splitmix64((uint64_t)s));
-        const double u = (double)(r >> 11) * 0x1.0p-53;
-        const int64_t v = cdf_find_warp(st, dm, dim, incl, cinc, nb, u * incl[nb - 1]);
-        if ((threadIdx.x & 31) == 0) out[s] = v;
+    for (int64_t s0 = ((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5) * per; s0 < shots; s0 += warps * per) {
+        const int cnt = (int)std::min<int64_t>(per, shots - s0);
+        CdfPlace p{0, 0, 0.0};
+        double t = 0.0;
+        if (lane < cnt) {
+            const uint64_t r = splitmix64(seed ^ splitmix64((uint64_t)(s0 + lane)));
+            t = (double)(r >> 11) * 0x1.0p-53 * incl[nb - 1];
+            p = cdf_place(dim, incl, cinc, nb, t);
+        }
+        int64_t mine = 0;
+        for (int k = 0; k < cnt; k++) {
+            const int64_t v = cdf_scan_warp(st, dm, dim, __shfl_sync(0xffffffffu, p.c, k), __shfl_sync(0xffffffffu, p.end, k),
+                                            __shfl_sync(0xffffffffu, p.cw, k), __shfl_sync(0xffffffffu, t, k));
+            if (lane == k) mine = v;
+        }
+        if (lane < cnt) out[s0 + lane] = mine;
     }
 }
 
@@ -204,7 +279,10 @@ int build_cdf(bs_sim* s, double** incl_out, double** cinc_out, int64_t* nb_out, 
     double* bsum = (double*)s->scratch;
     double* incl = bsum + nb;
     double* cinc = incl + nb;
-    k_block_sums<<<(unsigned)nb, 128, 0, s->stream>>>((const double2*)s->state, (s->kind == BS_KIND_DM ? 1 : 0) | (s->precision == BS_PREC_C64 ? 2 : 0), dim, bsum, cinc);
+    const int mode = (s->kind == BS_KIND_DM ? 1 : 0) | (s->precision == BS_PREC_C64 ? 2 : 0);
+    if (dim % kBlk || (mode & 1)) k_block_sums<<<(unsigned)nb, 128, 0, s->stream>>>((const double2*)s->state, mode, dim, bsum, cinc);
+    else if (mode & 2) k_block_sums_sv<true><<<(unsigned)nb, 128, 0, s->stream>>>((const float2*)s->state, bsum, cinc);
+    else k_block_sums_sv<false><<<(unsigned)nb, 128, 0, s->stream>>>((const double2*)s->state, bsum, cinc);
     k_scan_blocks<<<1, 1024, 0, s->stream>>>(bsum, nb, incl);
     *incl_out = incl;
     if (cinc_out) *cinc_out = cinc;
@@ -375,8 +453,10 @@ int bs_sample(bs_sim* s, uint64_t seed, int64_t shots, int64_t* out) {
         rc = build_cdf(s, &incl, &cinc, &nb, shots * 8, &buf);
         if (rc) return rc;
         dout = (int64_t*)buf;
-        k_sample_rng<<<grid(shots * 32, 128), 128, 0, s->stream>>>((const double2*)s->state, mode, dim, incl, cinc, nb,
-                                                                seed, shots, dout);
+        // as many shots per warp as still leave every SM 32 warps
+        const int per = (int)std::max<int64_t>(1, std::min<int64_t>(32, shots / (152 * 32)));
+        k_sample_rng<<<grid((shots + per - 1) / per * 32, 128), 128, 0, s->stream>>>((const double2*)s->state, mode, dim, incl,
+                                                                                   cinc, nb, seed, shots, per, dout);
     }
     rc = bs_cuda_check(s, cudaGetLastError(), "sample");
     if (rc) return rc;

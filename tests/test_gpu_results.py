@@ -444,3 +444,68 @@ def test_own_rng_samples_follow_the_inverse_cdf(kind, n):
     want = np.minimum(np.searchsorted(c, u * c[-1], side="left"), p.size - 1)
     got = sim.samples(seed=seed)
     assert np.mean(got == want) > 0.999
+
+
+def _dense_state(n, seed, **kw):
+    rng = np.random.default_rng(seed)
+    ops = [bs.Instruction(bs.U(*[float(a) for a in rng.uniform(-3, 3, 3)]), [q]) for q in range(n)]
+    ops += [bs.Instruction(bs.CZ(), [q, q + 1]) for q in range(n - 1)]
+    ops += [bs.Instruction(bs.U(*[float(a) for a in rng.uniform(-3, 3, 3)]), [q]) for q in range(n)]
+    return bs.StateVectorSimulator(n, 0, **kw).evolve(ops)
+
+
+@pytest.mark.parametrize("n", [1, 7, 8, 9, 12, 13, 20, 21])
+@pytest.mark.parametrize("precision", ["c128", "c64"])
+def test_readouts_at_the_kernels_edges(n, precision):
+    """Marginals (chunks of 2^8 indices and more, targets in the thread, chunk and block bits), Pauli sums
+    (one and several terms per flip mask, real and imaginary parts) and shots against the stored state."""
+    sim = _dense_state(n, 60 + n, precision=precision)
+    psi = sim.state_vector
+    p = (np.abs(psi) ** 2).reshape([2] * n)
+    rng = np.random.default_rng(n)
+    for k in sorted({1, min(3, n), min(8, n), min(12, n)}):
+        t = sorted(int(q) for q in rng.choice(n, k, replace=False))
+        ref = p.sum(axis=tuple(q for q in range(n) if q not in t)).ravel()
+        # FP64-grade sums of non-negative terms
+        assert np.max(np.abs(sim.marginal_probabilities(t) - ref)) < 1e-13
+    idx = np.arange(1 << n)
+    xm, zm = [], []
+    for f in (0, 1, (1 << n) - 1, 1 << (n - 1)):
+        for _ in range(11):                     # 11 terms on one flip mask: two passes
+            xm.append(f)
+            zm.append(int(rng.integers(1 << n)))
+    flips = []
+    for x, z in zip(xm, zm):
+        xe = sum(1 << (n - 1 - q) for q in range(n) if (x >> q) & 1)
+        ze = sum(1 << (n - 1 - q) for q in range(n) if (z >> q) & 1)
+        sign = 1.0 - 2.0 * (np.bitwise_count(idx & ze) & 1)
+        ny = bin(x & z).count("1")
+        flips.append(((-1j) ** ny * np.sum(sign * np.conj(psi) * psi[idx ^ xe])).real)
+
+    def call(sel):
+        from braketsimulator_gb300 import _abi
+        a = np.array([xm[i] for i in sel], dtype=np.uint64)
+        b = np.array([zm[i] for i in sel], dtype=np.uint64)
+        out = np.empty(len(sel))
+        sim._h.call("bs_expectation_pauli", len(sel), _abi.u64ptr(a), _abi.u64ptr(b), None, _abi.dptr(out))
+        return out
+
+    assert np.max(np.abs(call(range(len(xm))) - flips)) < 1e-12
+    for i in range(0, len(xm), 3):
+        assert abs(call([i])[0] - flips[i]) < 1e-12
+    # shots: the inverse CDF of the stored state at the generator's uniforms
+    shots = 5000
+    sim.shots = shots
+    got = sim.samples(seed=9)
+
+    def mix(x):
+        x = (x + 0x9e3779b97f4a7c15) & (2 ** 64 - 1)
+        x = ((x ^ (x >> 30)) * 0xbf58476d1ce4e5b9) & (2 ** 64 - 1)
+        x = ((x ^ (x >> 27)) * 0x94d049bb133111eb) & (2 ** 64 - 1)
+        return x ^ (x >> 31)
+
+    u = np.array([(mix(9 ^ mix(s)) >> 11) * 2.0 ** -53 for s in range(shots)])
+    cdf = np.cumsum(p.ravel())
+    want = np.searchsorted(cdf, u * cdf[-1])
+    # the host's running sum is off by about 1e-16 * sqrt(2^n): a shot that close to a boundary may differ
+    assert np.count_nonzero(got != want) <= 2
