@@ -684,14 +684,6 @@ bool unit_modulus(const HostGate& h) {
     }
     return true;
 }
-// matrix class of a 2x2 gate: 1 all real, 2 real diagonal and imaginary off-diagonal, else 0
-int class_2x2(const HostGate& h) {
-    if (h.mat[1] != 0.0 || h.mat[7] != 0.0) return 0;
-    if (h.mat[3] == 0.0 && h.mat[5] == 0.0) return 1;
-    if (h.mat[2] == 0.0 && h.mat[4] == 0.0) return 2;
-    return 0;
-}
-
 // U^dagger of a lowered gate (same targets and controls)
 HostGate dagger(const HostGate& h) {
     HostGate d = h;
@@ -974,7 +966,7 @@ extern "C" int bs_adjoint_gradient(bs_sim* s, const bs_op* ops, int64_t n_ops, c
             if (hg.kind == 0) for (int e = 0; e < (1 << (2 * hg.k)); e++) mats.push_back(to_cff(hg.mat[2 * e], hg.mat[2 * e + 1]));
             else if (hg.kind == 1) for (int e = 0; e < (1 << hg.k); e++) mats.push_back(to_cff(hg.mat[2 * e], hg.mat[2 * e + 1]));
             else perms.insert(perms.end(), hg.perm.begin(), hg.perm.end());
-            if (hg.kind == 0 && hg.k == 1) a.g.npar = class_2x2(hg);
+            if (hg.kind == 0 && hg.k == 1) a.g.npar = bs_class_2x2(hg);
             ag.push_back(a);
         };
         auto add_mark = [&](uint64_t zm, int slot, double w) {

@@ -11,7 +11,8 @@
 #define BS_TILE_MAXK 4           // dense targets per tile gate (16x16 superoperators for 2q noise)
 
 // One gate inside a tile sweep.
-//   kind 0: dense 2^k x 2^k on tile-local bits tbit[0..k-1] (matrix bit j <-> tbit[j])
+//   kind 0: dense 2^k x 2^k on tile-local bits tbit[0..k-1] (matrix bit j <-> tbit[j]); k = 1: npar is
+//           the matrix class (bs_class_2x2)
 //   kind 1: diagonal 2^k entries selected by global bits gbit[0..k-1]
 //   kind 2: monomial (one unit-modulus phase i^p per column) on tile-local bits
 //   kind 3: a run of CZ gates applied as one parity phase (npar, pshift, pmask)
@@ -191,8 +192,11 @@ int bs_lower_kraus_physical(bs_sim* s, const double* kraus, int nk, int k, const
                             unsigned flags, std::vector<HostGate>& out);
 // The gates are moved into the sweeps (the input is left with moved-from gates).
 void bs_plan_sweeps(std::vector<HostGate>& gates, int n_bits, int tile_bits, std::vector<Sweep>& out);
+// Matrix class of a 2x2 gate: 1 all real, 2 real diagonal and imaginary off-diagonal, else 0 (TileGate.npar).
+int bs_class_2x2(const HostGate& h);
 // Tuned values of a handle (its setting, else the environment, else the default)
 int bs_tile_bits(const bs_sim* s);
+int bs_sweep_tile_bits(const bs_sim* s);   // tile bits the sweeps use for the handle's size
 int bs_tile_threads(const bs_sim* s);
 bool bs_tc_enabled(const bs_sim* s);
 int bs_tc_min_bits(const bs_sim* s);

@@ -247,3 +247,21 @@ def test_bounded_wait_gives_up_and_the_handle_stays_usable():
     sim.evolve(ops)
     ref = oracle.OracleSV(8).evolve(ops).psi
     assert np.linalg.norm(sim.state_vector - ref) <= 1e-12 * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("n", [13, 16, 17, 18, 19])
+def test_small_tiles_and_matrix_classes(n):
+    """States with fewer than 2^12-amplitude tiles (13 to 18 qubits) and the first size without, under
+    matrices of every class (complex, real, real diagonal with imaginary off-diagonal), plain and controlled."""
+    rng = np.random.default_rng(400 + n)
+    a = lambda: float(rng.uniform(-np.pi, np.pi))  # noqa: E731
+    ops = []
+    for _ in range(3):
+        for q in range(n):
+            ops.append(bs.Instruction([bs.H(), bs.Rx(a()), bs.Ry(a()), bs.Rz(a()), bs.U(a(), a(), a()), bs.V()][int(rng.integers(6))], [q]))
+        for q in rng.permutation(n)[:6]:
+            r = int((q + 1 + rng.integers(n - 1)) % n)
+            g = [bs.CNot(), bs.CV(), bs.Control(bs.Ry(a()), (0,)), bs.XX(a()), bs.ZZ(a()), bs.Swap()][int(rng.integers(6))]
+            ops.append(bs.Instruction(g, [int(q), r]))
+    sim = bs.StateVectorSimulator(n, 0).evolve(ops)
+    assert rel_err(sim.state_vector, oracle.OracleSV(n).evolve(ops).psi) < 1e-12
