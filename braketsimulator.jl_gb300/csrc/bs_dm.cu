@@ -135,8 +135,8 @@ __global__ void k_kraus_ref_big(ST* __restrict__ S, int n, int k, const int* __r
 
 // A 1- or 2-target channel in the reference's update rule as a tile gate of a density-matrix sweep
 // (kind 5): ebit[0..k-1] are the row endian bits of the targets (matrix bit j <-> ebit[j], the
-// canonical order of bs_kraus_reference), ebit[k..2k-1] the column endian bits; mat holds the nk
-// Kraus matrices, row-major D x D complex each.
+// canonical order of bs_kraus_reference), ebit[k..2k-1] the column endian bits; mat holds the channel's
+// superoperator on a block, row-major, index row + D column.
 int bs_lower_kraus_reference(bs_sim* s, const double* kraus, int nk, int k, const int* targets, unsigned flags,
                              std::vector<HostGate>& out) {
     if (s->kind != BS_KIND_DM) return bs_fail(s, BS_ERR_STATE, "noise needs a density-matrix simulator");
@@ -158,8 +158,22 @@ int bs_lower_kraus_reference(bs_sim* s, const double* kraus, int nk, int k, cons
         g.ebit[j] = s->n - 1 - ct[(size_t)j];
         g.ebit[k + j] = g.ebit[j] + s->n;
     }
-    const int D = 1 << k;
-    g.mat.assign(kraus, kraus + (size_t)nk * D * D * 2);
+    // sum_q K_q B K_q^dagger: element (i, j) of the result takes K_q[i, l] conj(K_q[j, m]) of element (l, m)
+    const int D = 1 << k, DD = D * D;
+    g.mat.assign((size_t)2 * DD * DD, 0.0);
+    for (int q = 0; q < nk; q++) {
+        const double* K = kraus + (size_t)q * 2 * DD;
+        for (int i = 0; i < D; i++)
+            for (int j = 0; j < D; j++)
+                for (int l = 0; l < D; l++)
+                    for (int m = 0; m < D; m++) {
+                        const double ar = K[2 * (i * D + l)], ai = K[2 * (i * D + l) + 1];
+                        const double br = K[2 * (j * D + m)], bi = -K[2 * (j * D + m) + 1];
+                        double* e = g.mat.data() + 2 * ((size_t)(i + D * j) * DD + (size_t)(l + D * m));
+                        e[0] += ar * br - ai * bi;
+                        e[1] += ar * bi + ai * br;
+                    }
+    }
     out.push_back(std::move(g));
     return BS_OK;
 }

@@ -21,7 +21,8 @@
 //   kind 8: register block (complex64): tile bits gbit[0..4] are held in registers, perm_off: the 7 other
 //           tile bits in thread-index order, 4 bits each; the sweep's rops[mat_off .. mat_off + k) are applied
 //   kind 5: Kraus channel on k <= 2 targets in the reference's block-diagonal update rule
-//           (density matrix): tbit[0..2k-1] row then column target bits, pmask[0..1], npar = nk
+//           (density matrix): tbit[0..2k-1] row then column target bits, pmask[0..1], its superoperator
+//           at mat_off
 // Controls: (tile_index & lc_mask) == lc_val for in-tile controls,
 //           (global_base & gc_mask) == gc_val for controls outside the tile.
 struct TileGate {
@@ -80,7 +81,8 @@ struct SweepDesc {
 
 struct HostGate {                // a gate after lowering to the canonical convention
     int kind;                    // 0 dense, 1 diagonal, 2 monomial, 4 fused 5-bit unitary,
-                                 // 5 reference-rule Kraus channel (ebit: k row bits, then k column bits)
+                                 // 5 reference-rule Kraus channel (ebit: k row bits, then k column bits;
+                                 // mat: its superoperator on a block, index row + 2^k column)
     int k;
     int ebit[BS_MAX_TARGETS];    // endian bit of target j (matrix bit j)
     std::vector<double> mat;     // interleaved complex; dense 4^k*2, diag 2^k*2
@@ -131,6 +133,9 @@ struct bs_sim {
     int64_t* alias_ix = nullptr;
     int64_t alias_len = 0;
     bool alias_valid = false;
+    // adjoint gradients: checkpoints and lambda, kept between calls up to 1 GiB (bs_adjoint_gradient)
+    void* adj_work = nullptr;
+    size_t adj_work_bytes = 0;
     // plan upload buffer
     void* plan_buf = nullptr;
     int64_t plan_bytes = 0;

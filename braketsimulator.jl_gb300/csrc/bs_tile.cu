@@ -245,15 +245,14 @@ __device__ void tile_diag(float4* sm, int T, int L, const TileGate& g, const flo
 // all non-target bits (vec(S) index = row + column 2^n); other elements are left alone.  tbit[0..K-1]:
 // tile positions of the row target bits (matrix bit j <-> tbit[j]), tbit[K..2K-1]: of the column
 // target bits; pmask[0]: row-index mask of the non-target bits; pmask[1]: the non-target bits whose
-// row and column bits both lie outside the tile (so that part of the test is uniform in the CTA);
-// npar: number of Kraus matrices, row-major D x D each at mat_off.
-// With few registers (the tensor-core sweep's threads have none to spare, and the float-float
-// sweep's 2-target variant would otherwise need the 4-bit kernel): candidate blocks are tested and
-// the ones that pass the row/column test collected (all candidates tested in one pass), then one
-// thread per output element
-// of a collected block sums over the Kraus matrices reading the block from shared memory; all reads
-// of the collected blocks finish before any of their outputs is written.  s_act: 32 ints of shared
-// scratch.
+// row and column bits both lie outside the tile (so that part of the test is uniform in the CTA).
+// The channel comes as its superoperator on the block, a D^2 x D^2 matrix at mat_off (row and column
+// index r + D c), formed on the host in FP64: one product per pair of elements.  With the Kraus
+// matrices themselves a 2-target depolarizing channel was a chain of 16 x 4 x 5 complex products per
+// element, 60 k cycles in the few tiles that hold such blocks (13 qubits, 3 layers: 31.8 -> 27.4 ms).
+// Candidate blocks are tested and the ones that pass the row/column test collected (all candidates
+// tested in one pass), then one thread per output element of a collected block; all reads of the
+// collected blocks finish before any of their outputs is written.  s_act: 32 ints of shared scratch.
 template <int K, bool SW, typename OT>
 __device__ void tile_kraus_ref_lr(float4* sm, int T, int L, const TileGate& g, const float4* __restrict__ mats,
                                   int64_t base, OT off_tab, int osh, int n, int* s_act, int* s_cnt) {
@@ -304,21 +303,11 @@ __device__ void tile_kraus_ref_lr(float4* sm, int T, int L, const TileGate& g, c
                 }
                 return sx<SW>(j);
             };
-            ffacc ar{0.f, 0.f}, ai{0.f, 0.f};
-            bool first = true;
-            for (int q = 0; q < g.npar; q++) {
-                const float4* Kq = km + q * DD;
-                for (int c = 0; c < D; c++) {
-                    ffacc tr, ti;
-                    cmac_first(tr, ti, f4m(__ldg(Kq + i * D)), f4c(sm[at(0, c)]));
-                    for (int r = 1; r < D; r++) cmac(tr, ti, f4m(__ldg(Kq + i * D + r)), f4c(sm[at(r, c)]));
-                    const cff t = cdone(tr, ti);
-                    const float4 kj = __ldg(Kq + jj * D + c);
-                    const cff kc = {kj.x, kj.y, -kj.z, -kj.w};
-                    if (first) { cmac_first(ar, ai, kc, t); first = false; }
-                    else cmac(ar, ai, kc, t);
-                }
-            }
+            const float4* row = km + (i + D * jj) * DD;
+            ffacc ar, ai;
+            cmac_first(ar, ai, f4m(__ldg(row)), f4c(sm[at(0, 0)]));
+#pragma unroll 3
+            for (int f = 1; f < DD; f++) cmac(ar, ai, f4m(__ldg(row + f)), f4c(sm[at(f % D, f / D)]));
             outv = c4f(cdone(ar, ai));
             dst = at(i, jj);
         }
@@ -1444,7 +1433,7 @@ int bs_run_sweeps(bs_sim* s, const std::vector<Sweep>& sweeps) {
                 TileGate t{};
                 t.kind = 5;
                 t.k = hg.k;
-                const int nq = n_bits / 2, D = 1 << hg.k;
+                const int nq = n_bits / 2;
                 uint64_t rt = 0;
                 for (int q = 0; q < 2 * hg.k; q++) t.tbit[q] = local[hg.ebit[q]];
                 for (int q = 0; q < hg.k; q++) rt |= 1ULL << hg.ebit[q];
@@ -1454,7 +1443,6 @@ int bs_run_sweeps(bs_sim* s, const std::vector<Sweep>& sweeps) {
                     if (((nt >> b) & 1ULL) && local[b] < 0 && local[b + nq] < 0) unif |= 1ULL << b;
                 t.pmask[0] = nt;
                 t.pmask[1] = unif;
-                t.npar = (int32_t)(hg.mat.size() / (size_t)(2 * D * D));
                 t.mat_off = (int32_t)mats.size();
                 for (size_t e = 0; e + 1 < hg.mat.size(); e += 2) mats.push_back(to_cff(hg.mat[e], hg.mat[e + 1]));
                 tg.push_back(t);

@@ -103,3 +103,21 @@ def test_dm_config_shape(n):
         ref = oracle.OracleDM(n, physical=(mode == "physical")).evolve(ops)
         assert rel_err(sim.density_matrix, ref.matrix) < TOL
         assert rel_err(sim.probabilities(), ref.probabilities()) < TOL
+
+
+@pytest.mark.parametrize("n,nk", [(2, 1), (6, 3), (7, 16)])
+def test_reference_channels_as_superoperators(n, nk):
+    """Arbitrary Kraus sets (no unit trace, complex entries) on one and two targets in either order between
+    gates, in the reference's update rule, applied inside the sweeps."""
+    rng = np.random.default_rng(n + nk)
+    ops = []
+    for i in range(14):
+        a, b = (int(x) for x in rng.choice(n, 2, replace=False))
+        ops.append(bs.Instruction(bs.Ry(float(rng.uniform(-3, 3))), [a]))
+        ops.append(bs.Instruction(bs.CNot(), [a, b]))
+        d = 2 + 2 * (i % 2)
+        ks = [(rng.normal(size=(d, d)) + 1j * rng.normal(size=(d, d))) / np.sqrt(2 * d * nk) for _ in range(nk)]
+        ops.append(bs.Instruction(bs.Kraus(ks), [a] if d == 2 else [b, a]))
+    got = bs.DensityMatrixSimulator(n, 0).evolve(ops).density_matrix
+    ref = oracle.OracleDM(n).evolve(ops).matrix
+    assert np.linalg.norm(got - ref) <= 1e-12 * np.linalg.norm(ref)
