@@ -198,7 +198,15 @@ int alloc_state(bs_sim* s, int n) {
         if (s->state) cudaFree(s->state);
         s->state = nullptr;
         s->cap_bytes = 0;
-        int rc = bs_cuda_check(s, cudaMalloc(&s->state, (size_t)bytes), "state allocation");
+        cudaError_t e = cudaMalloc(&s->state, (size_t)bytes);
+        if (e != cudaSuccess && s->adj_work) {   // the kept workspace goes before a state does not fit
+            cudaGetLastError();
+            cudaFree(s->adj_work);
+            s->adj_work = nullptr;
+            s->adj_work_bytes = 0;
+            e = cudaMalloc(&s->state, (size_t)bytes);
+        }
+        int rc = bs_cuda_check(s, e, "state allocation");
         if (rc) return rc;
         s->cap_bytes = bytes;
     }
@@ -246,6 +254,7 @@ int bs_destroy(bs_sim* s) {
     if (s->state) cudaFree(s->state);
     if (s->scratch) cudaFree(s->scratch);
     if (s->plan_buf) cudaFree(s->plan_buf);
+    if (s->adj_work) cudaFree(s->adj_work);
     if (s->dev_flag) cudaFree(s->dev_flag);
     if (s->counter) cudaFree(s->counter);
     if (s->alias_ap) cudaFree(s->alias_ap);
