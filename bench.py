@@ -146,9 +146,9 @@ def peaks():
 
 
 # Tensor-core sweep (k_tile_sweep_tc): executed bf16 MMA work per fused gate per 2^12-amplitude tile
-# (26 digit pairs x 4 k-steps, each M=128 N=64 K=16), and the DRAM bytes per amplitude per launch that
+# (21 digit pairs x 4 k-steps, each M=128 N=64 K=16), and the DRAM bytes per amplitude per launch that
 # ncu measured for it on the 27-qubit dense circuit (2.1488e9 read + 2.0865e9 written per launch).
-TC_FLOP_PER_TILE_GATE = 104 * 2 * 128 * 64 * 16
+TC_FLOP_PER_TILE_GATE = 84 * 2 * 128 * 64 * 16
 TC_DRAM_BYTES_PER_AMP = (2.148804e9 + 2.086545e9) / 2 ** 27
 
 
@@ -938,7 +938,7 @@ def main():
                         "executed_bf16_TFLOPs": round(flop_per_launch / tc_launch_s / 1e12, 1),
                         "executed_frac_of_bf16_sustained": round(flop_per_launch / tc_launch_s / 1e12 / bf16, 3),
                         "algorithmic_TFLOPs": round(alg_flop_per_launch / tc_launch_s / 1e12, 2),
-                        "note": "executed = 26 bf16 digit-pair MMAs per complex128 product (exact split); "
+                        "note": "executed = 21 bf16 digit-pair MMAs per complex128 product (exact split); "
                                 "algorithmic = 256 flop per amplitude per fused 5-qubit unitary"}}
     else:
         per_launch_ms = dev_ms / max(1, sweeps)

@@ -8,17 +8,19 @@
 //
 // Exactness (Ozaki-style split): the tile is scaled by a power of two (from the
 // largest exponent over the tile) so that |x| < 2^8, and both x and U_real (on
-// the device, from the FP64 matrix) are split into six balanced 8-bit digits, digit j carried as bf16 d_j * 2^(-8j) with
-// |d_j| <= 128 (256 for the one digit that absorbs the float-float low word).
-// The 26 digit pairs with i + j <= 6 are accumulated in five rounds by digit
+// the device, from the FP64 matrix) are split into six balanced 9-bit digits, digit j carried as bf16 d_j * 2^(-9j) with
+// |d_j| <= 256, which 8 significant bits hold exactly.
+// The 21 digit pairs with i + j <= 5 are accumulated in five rounds by digit
 // weight: i+j = 0, 1, 2, 3 each alone (every product a multiple of the same
-// power of two and every partial sum below 2^24 of it, so these FP32 sums are
-// exact) and i+j = 4, 5, 6 together (rounding at 2^-56 of the result).  After
+// power of two and every partial sum at most 4 * 64 * 2^16 = 2^24 of it, so
+// these FP32 sums are exact) and i+j = 4, 5 together (rounding at 2^-59 of the
+// result).  8-bit digits left two of those 24 bits unused and took 26 pairs
+// for less precision (TODO).  After
 // each round the CUDA cores fold the FP32 accumulator into a running
 // float-float sum, while the tensor cores run other rounds in the other of two
 // accumulators; two threads issue, one per accumulator, so that neither chain
 // of issue, fold and re-issue waits for the other.  What remains is the 48-bit
-// truncation of both operands, ~2^-46 of the tile's largest value per fused gate.
+// float-float result, ~2^-47 of the tile's largest value per fused gate.
 //
 // TMEM (256 columns per CTA, so that two CTAs share an SM and one's MMAs
 // overlap the other's CUDA-core work):
@@ -157,23 +159,6 @@ __device__ __forceinline__ void commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 
-// Six digits of y = yh + yl (|y| < 2^7 after scaling): q[j] = d_j 2^(-8j), y ~ sum_j q[j].
-// Rounding to the digit grid uses the 1.5 * 2^(23-8j) shift, exact while |R| < 2^(22-8j).
-__device__ __forceinline__ void digits(float yh, float yl, float (&q)[6]) {
-    float R = yh;
-    q[0] = __fsub_rn(__fadd_rn(R, 12582912.0f), 12582912.0f);            // grid 1
-    R = __fsub_rn(R, q[0]);
-    q[1] = __fsub_rn(__fadd_rn(R, 49152.0f), 49152.0f);                  // grid 2^-8
-    R = __fsub_rn(R, q[1]);
-    q[2] = __fsub_rn(__fadd_rn(R, 192.0f), 192.0f);                      // grid 2^-16
-    R = __fadd_rn(__fsub_rn(R, q[2]), yl);                               // low word joins here
-    q[3] = __fsub_rn(__fadd_rn(R, 0.75f), 0.75f);                        // grid 2^-24
-    R = __fsub_rn(R, q[3]);
-    q[4] = __fsub_rn(__fadd_rn(R, 0.0029296875f), 0.0029296875f);        // grid 2^-32
-    R = __fsub_rn(R, q[4]);
-    q[5] = __fsub_rn(__fadd_rn(R, 1.1444091796875e-05f), 1.1444091796875e-05f);   // grid 2^-40
-}
-
 // error-free s + g (Knuth TwoSum): s <- rounded sum, returns the rounding error
 __device__ __forceinline__ float two_sum(float& s, float g) {
     const float t = __fadd_rn(s, g);
@@ -183,23 +168,26 @@ __device__ __forceinline__ float two_sum(float& s, float g) {
     return e;
 }
 
-// digits() on both halves
+// Six digits of y = yh + yl (|y| < 2^8 after scaling) on both halves: q[j] = d_j 2^(-9j), y ~ sum_j q[j].
+// Rounding to the digit grid adds and subtracts 1.5 * 2^(23-9j), exact while |R| < 2^(22-9j).  The low
+// word (up to 2^-17) overlaps digit 2, so it takes part in choosing digits 1 and 2 (left out, digit 2
+// reaches 258, which bf16 does not hold) and joins the remainder after them, where its last bits survive.
 __device__ __forceinline__ void digits2(f2 yh, f2 yl, f2 (&q)[6]) {
-    const f2 c0 = pk(12582912.0f, 12582912.0f), c1 = pk(49152.0f, 49152.0f), c2 = pk(192.0f, 192.0f),
-             c3 = pk(0.75f, 0.75f), c4 = pk(0.0029296875f, 0.0029296875f),
-             c5 = pk(1.1444091796875e-05f, 1.1444091796875e-05f);
+    const f2 c0 = pk(12582912.0f, 12582912.0f), c1 = pk(24576.0f, 24576.0f), c2 = pk(48.0f, 48.0f),
+             c3 = pk(0.09375f, 0.09375f), c4 = pk(0.00018310546875f, 0.00018310546875f),
+             c5 = pk(3.5762786865234375e-07f, 3.5762786865234375e-07f);
     f2 R = yh;
-    q[0] = sub2(add2(R, c0), c0);
+    q[0] = sub2(add2(R, c0), c0);            // grid 1
     R = sub2(R, q[0]);
-    q[1] = sub2(add2(R, c1), c1);
+    q[1] = sub2(add2(add2(R, yl), c1), c1);  // grid 2^-9
     R = sub2(R, q[1]);
-    q[2] = sub2(add2(R, c2), c2);
+    q[2] = sub2(add2(add2(R, yl), c2), c2);  // grid 2^-18
     R = add2(sub2(R, q[2]), yl);
-    q[3] = sub2(add2(R, c3), c3);
+    q[3] = sub2(add2(R, c3), c3);            // grid 2^-27
     R = sub2(R, q[3]);
-    q[4] = sub2(add2(R, c4), c4);
+    q[4] = sub2(add2(R, c4), c4);            // grid 2^-36
     R = sub2(R, q[4]);
-    q[5] = sub2(add2(R, c5), c5);
+    q[5] = sub2(add2(R, c5), c5);            // grid 2^-45
 }
 // two_sum() on both halves
 __device__ __forceinline__ f2 two_sum2(f2& s, f2 g) {
@@ -353,9 +341,9 @@ __device__ __forceinline__ void apply(float4* sm, const TileGate& g, const TileG
     uint32_t eall = s_wmax[0];
 #pragma unroll
     for (int w = 1; w < NT / 32; w++) eall = max(eall, s_wmax[w]);
-    const int ebc = max((int)(eall >> 23), max(6, 14 - g.tc_eu));
-    const float sc = __uint_as_float((uint32_t)(260 - ebc) << 23);                 // 2^(7 - E)
-    const float osc = __uint_as_float((uint32_t)(ebc - 13 + g.tc_eu) << 23);       // 2^(E + eu - 14)
+    const int ebc = max((int)(eall >> 23), max(7, 16 - g.tc_eu));
+    const float sc = __uint_as_float((uint32_t)(261 - ebc) << 23);                 // 2^(8 - E)
+    const float osc = __uint_as_float((uint32_t)(ebc - 15 + g.tc_eu) << 23);       // 2^(E + eu - 16)
     const uint32_t lane = (uint32_t)((warp & 3) * 32) << 16;
     const f2 sc2 = pk(sc, sc);
     // all of the thread's amplitudes loaded first (the loads overlap), then split and stored
@@ -384,7 +372,7 @@ __device__ __forceinline__ void apply(float4* sm, const TileGate& g, const TileG
     __syncthreads();
     fence_after();
     const uint64_t b0 = bdesc(su32(sB));
-    // Round 4 (weights 4..6, 64 MMAs) into D0 by thread 0: first the 20 MMAs that read state digits 4
+    // Round 4 (weights 4 and 5, 44 MMAs) into D0 by thread 0: first the 12 MMAs that read state digits 4
     // and 5, committed to barrier 5, so that D1, which takes their columns, is free once they have
     // completed; thread 128 then issues round 3 into D1 while thread 0 still issues round 4.  Two
     // issuers, each waiting only for the reads of its own accumulator: thread 0 runs D0 (rounds 4,
@@ -396,9 +384,9 @@ __device__ __forceinline__ void apply(float4* sm, const TileGate& g, const TileG
     if (tid == 0) {
         if (mbar_wait(st.bar, st.ph & 1u)) {
             fence_after();
-            issue_pairs<4, 6, 4, 5, true>(st.tmem, 0u, b0);
+            issue_pairs<4, 5, 4, 5, true>(st.tmem, 0u, b0);
             commit(st.bar + 40u);
-            issue_pairs<4, 6, 0, 3, false>(st.tmem, 0u, b0);
+            issue_pairs<4, 5, 0, 3, false>(st.tmem, 0u, b0);
             commit(st.bar + 8u);
         } else {
             ok = false;

@@ -580,10 +580,10 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_tile_sweep_tc(double2* __rest
 }
 
 // Digit slices of the fused matrices for the tensor-core sweep, one CTA per matrix variant.
-// mats: complex 32x32 row-major FP64 per variant; scale[v] = 2^(7 - eu) of the variant's gate.
+// mats: complex 32x32 row-major FP64 per variant; scale[v] = 2^(8 - eu) of the variant's gate.
 // Entry (n, k) of the real 64x64 embedding (n = 2t'+c' output re/im, k = 2t+c input re/im) is split
-// into six balanced digits d_i in [-128, 128] (u 2^(7-eu) = sum_i d_i 2^(-8i), each digit rounded to
-// nearest even), digit i stored as the bf16 of d_i 2^(-8i) at its place in the K-major no-swizzle
+// into six balanced digits d_i in [-256, 256] (u 2^(8-eu) = sum_i d_i 2^(-9i), each digit rounded to
+// nearest even), digit i stored as the bf16 of d_i 2^(-9i) at its place in the K-major no-swizzle
 // operand layout (per digit and k-step a 2 KiB block of 8x8 core matrices: row group n/8 at 256 B,
 // K half at 128 B, row n%8 at 16 B).
 __global__ void __launch_bounds__(256) k_tc_digits(const double* __restrict__ mats, const double* __restrict__ scale,
@@ -603,8 +603,8 @@ __global__ void __launch_bounds__(256) k_tc_digits(const double* __restrict__ ma
 #pragma unroll
         for (int i = 0; i < 6; i++) {
             const double d = rint(x);
-            x = (x - d) * 256.0;
-            const float f = __double2float_rn(d) * __int_as_float((127 - 8 * i) << 23);   // exact: |d| <= 128
+            x = (x - d) * 512.0;
+            const float f = __double2float_rn(d) * __int_as_float((127 - 9 * i) << 23);   // exact: |d| <= 256
             dst[(size_t)(i * 4 + s) * 1024 + pos] = (uint16_t)(__float_as_uint(f) >> 16);
         }
     }
@@ -1298,7 +1298,7 @@ int bs_run_sweeps(bs_sim* s, const std::vector<Sweep>& sweeps) {
     std::vector<int32_t> big_bits;
     std::vector<RegOp> rops;                 // operations of the register blocks (complex64)
     double reg_drift = 0;
-    std::vector<double> tc_mats, tc_scale;   // fused matrices (complex 32x32 per variant), 2^(7-eu) per variant
+    std::vector<double> tc_mats, tc_scale;   // fused matrices (complex 32x32 per variant), 2^(8-eu) per variant
     int64_t n_var = 0;
     const bool c64 = s->precision == BS_PREC_C64;
     // fused tensor-core sweeps from bs_tc_min_bits vector bits up (22 by default: measured wins at
@@ -1464,7 +1464,7 @@ int bs_run_sweeps(bs_sim* s, const std::vector<Sweep>& sweeps) {
                 if (!bs_tc_exponent(hg.mat.data(), nvar, eu))
                     return bs_fail(s, BS_ERR_INVALID_ARG, "fused gate matrix out of range");
                 tc_mats.insert(tc_mats.end(), hg.mat.begin(), hg.mat.begin() + (size_t)nvar * 2048);
-                for (int v = 0; v < nvar; v++) tc_scale.push_back(std::ldexp(1.0, 7 - eu));
+                for (int v = 0; v < nvar; v++) tc_scale.push_back(std::ldexp(1.0, 8 - eu));
                 n_var += nvar;
                 t.tc_eu = eu;
                 ln.tc_last = ln.n_gates;
