@@ -106,38 +106,69 @@ void apply_block(const HostGate& g, const int* pos, uint64_t uval, cd* U) {
     }
 }
 
-struct Block {
-    uint64_t bits = 0;               // tile bits touched
-    uint64_t ubits = 0;              // uniform (out-of-tile) bits the gates depend on
-    std::vector<int> idx;            // gate indices, in order
+// What the tensor-core fusion needs to know of a gate.
+struct FuseGate {
+    uint64_t bits = 0;    // tile bits it touches
+    uint64_t ub = 0;      // bits outside the tile it depends on (constant in a CTA)
+    uint64_t hard = 0;    // bits it moves amplitudes along
     double cost = 0;
+    bool fusable = false;
+    bool wide = false;    // 3 or more moved bits: no float-float path in the tensor-core sweep
 };
 
 }  // namespace
 
+// Greedy over the gates in order.  A block starts at the first gate left and grows bit by bit: of all
+// bit sets that add the bits of one more gate, the one whose block takes the most work (gates that
+// commute with everything they leave behind, out-of-tile bits at most kMaxUniform).  Blocks of one layer
+// of single-qubit gates therefore fill up with gates on other bits, and follow the light cone into the
+// next layers; fusing only blocks that share a bit left 18 single dense gates beside 30 fused unitaries
+// in the 28-qubit dense circuit, each of which costs 3/4 of a fused unitary (TODO).
 void bs_fuse_tc(const std::vector<HostGate>& in, const int* local, int T, double threshold, std::vector<HostGate>& out) {
     out.clear();
-    std::vector<Block> open;
-    auto emit = [&](Block& b) {
+    const size_t G = in.size();
+    std::vector<FuseGate> info(G);
+    for (size_t i = 0; i < G; i++) {
+        const HostGate& g = in[i];
+        FuseGate& f = info[i];
+        if (g.kind == 5) continue;
+        f.fusable = g.kind <= 2 && g.k <= 5;
+        for (int q = 0; q < g.k; q++) {
+            const int e = g.ebit[q];
+            if (g.kind != 1) f.hard |= 1ULL << e;
+            if (local[e] >= 0) f.bits |= 1ULL << e;
+            else if (g.kind == 1) f.ub |= 1ULL << e;
+            else f.fusable = false;
+        }
+        for (uint64_t r = g.cmask; r; r &= r - 1) {
+            const int e = __builtin_ctzll(r);
+            (local[e] >= 0 ? f.bits : f.ub) |= 1ULL << e;
+        }
+        if (__builtin_popcountll(f.bits) > 5 || __builtin_popcountll(f.ub) > kMaxUniform || f.bits == 0) f.fusable = false;
+        f.wide = g.kind != 1 && g.k >= 3;
+        // real and real/imaginary 2x2 matrices take half the products on the float-float path
+        f.cost = is_plain_cz(g) ? 0.1 : (g.kind == 0 && g.k == 1 && bs_class_2x2(g)) ? 0.6 : ff_cost(g);
+    }
+    auto emit = [&](uint64_t bits, uint64_t ubits, const std::vector<int>& idx, double cost) {
         int ndense = 0;
         bool wide = false;   // 3- and 4-target gates always fuse: the tensor-core sweep has no float-float path for them
-        for (int i : b.idx) {
+        for (int i : idx) {
             ndense += in[(size_t)i].kind == 0;
-            wide = wide || (in[(size_t)i].kind != 1 && in[(size_t)i].k >= 3);
+            wide = wide || info[(size_t)i].wide;
         }
-        if (!wide && (b.cost <= threshold || ndense == 0)) {
-            for (int i : b.idx) out.push_back(in[(size_t)i]);
+        if (!wide && (cost <= threshold || ndense == 0)) {
+            for (int i : idx) out.push_back(in[(size_t)i]);
             return;
         }
         // block bits ascending by tile position, padded to 5 with other tile bits (high ones first, so that
         // the low contiguous bits stay column bits of the GEMM where possible)
         std::vector<int> eb;
-        for (int e = 0; e < 64; e++) if ((b.bits >> e) & 1ULL) eb.push_back(e);
+        for (int e = 0; e < 64; e++) if ((bits >> e) & 1ULL) eb.push_back(e);
         std::vector<int> tile_e(T, -1);
         for (int e = 0; e < 64; e++) if (local[e] >= 0 && local[e] < T) tile_e[local[e]] = e;
         for (int p = T - 1; p >= 0 && (int)eb.size() < 5; p--) {
             int e = tile_e[p];
-            if (e >= 0 && !((b.bits >> e) & 1ULL)) eb.push_back(e);
+            if (e >= 0 && !((bits >> e) & 1ULL)) eb.push_back(e);
         }
         std::sort(eb.begin(), eb.end(), [&](int a, int c) { return local[a] < local[c]; });
         int pos[64];
@@ -147,7 +178,7 @@ void bs_fuse_tc(const std::vector<HostGate>& in, const int* local, int T, double
         f.kind = 4;
         f.k = 5;
         for (int q = 0; q < 5; q++) f.ebit[q] = eb[(size_t)q];
-        for (int e = 0; e < 64; e++) if ((b.ubits >> e) & 1ULL) f.ubits.push_back(e);
+        for (int e = 0; e < 64; e++) if ((ubits >> e) & 1ULL) f.ubits.push_back(e);
         const int nvar = 1 << f.ubits.size();
         f.mat.assign((size_t)nvar * 2 * 32 * 32, 0.0);
         for (int var = 0; var < nvar; var++) {
@@ -156,7 +187,7 @@ void bs_fuse_tc(const std::vector<HostGate>& in, const int* local, int T, double
             double* m = f.mat.data() + (size_t)var * 2048;
             std::vector<cd> U(32 * 32, cd(0, 0));
             for (int r = 0; r < 32; r++) U[(size_t)r * 33] = 1;
-            for (int i : b.idx) apply_block(in[(size_t)i], pos, uval, U.data());
+            for (int i : idx) apply_block(in[(size_t)i], pos, uval, U.data());
             for (int r = 0; r < 32 * 32; r++) {
                 m[2 * r] = U[(size_t)r].real();
                 m[2 * r + 1] = U[(size_t)r].imag();
@@ -164,110 +195,70 @@ void bs_fuse_tc(const std::vector<HostGate>& in, const int* local, int T, double
         }
         out.push_back(std::move(f));
     };
-    auto flush_if = [&](uint64_t bits) {
-        for (size_t j = 0; j < open.size();) {
-            if (open[j].bits & bits) {
-                emit(open[j]);
-                open.erase(open.begin() + (long)j);
-            } else {
-                j++;
+    std::vector<char> done(G, 0);
+    std::vector<int> left, take;
+    std::vector<uint64_t> tried;
+    for (size_t s0 = 0; s0 < G;) {
+        if (in[s0].kind == 5) { out.push_back(in[s0++]); continue; }   // commutes with nothing
+        size_t s1 = s0;
+        while (s1 < G && in[s1].kind != 5) s1++;
+        size_t first = s0;
+        while (true) {
+            while (first < s1 && done[first]) first++;
+            if (first == s1) break;
+            if (!info[first].fusable) {
+                out.push_back(in[first]);
+                done[first] = 1;
+                continue;
             }
-        }
-    };
-    for (size_t i = 0; i < in.size(); i++) {
-        const HostGate& g = in[i];
-        if (g.kind == 5) {
-            // a reference-rule channel commutes with nothing: every open block closes before it
-            for (Block& b : open) emit(b);
-            open.clear();
-            out.push_back(g);
-            continue;
-        }
-        // tile bits and uniform bits of the gate; dense and monomial targets must be in the tile
-        uint64_t bits = 0, ub = 0;
-        bool fusable = g.kind <= 2 && g.k <= 5;
-        for (int q = 0; q < g.k; q++) {
-            const int e = g.ebit[q];
-            if (local[e] >= 0) bits |= 1ULL << e;
-            else if (g.kind == 1) ub |= 1ULL << e;
-            else fusable = false;
-        }
-        for (int e = 0; e < 64; e++)
-            if ((g.cmask >> e) & 1ULL) {
-                if (local[e] >= 0) bits |= 1ULL << e;
-                else ub |= 1ULL << e;
-            }
-        if (__builtin_popcountll(bits) > 5 || __builtin_popcountll(ub) > kMaxUniform || bits == 0) fusable = false;
-        if (!fusable) {
-            // close every block sharing a bit with the gate, uniform bits included (the gate may act on them)
-            const uint64_t all = bits | ub | g.cmask;
-            uint64_t tgt = 0;
-            for (int q = 0; q < g.k; q++) tgt |= 1ULL << g.ebit[q];
-            for (size_t j = 0; j < open.size();) {
-                if ((open[j].bits | open[j].ubits) & (all | tgt)) {
-                    emit(open[j]);
-                    open.erase(open.begin() + (long)j);
-                } else {
-                    j++;
-                }
-            }
-            out.push_back(g);
-            continue;
-        }
-        const double gc = is_plain_cz(g) ? 0.1 : ff_cost(g);
-        uint64_t uni = bits, uu = ub;
-        for (const Block& b : open) if (b.bits & bits) { uni |= b.bits; uu |= b.ubits; }
-        if (__builtin_popcountll(uni) > 5 || __builtin_popcountll(uu) > kMaxUniform) {
-            // the gate links blocks that cannot all merge: keep the costliest block it fits into and close
-            // the others (their gates precede it and touch none of the kept block's tile bits)
-            int keep = -1;
-            for (size_t j = 0; j < open.size(); j++)
-                if ((open[j].bits & bits) && __builtin_popcountll(open[j].bits | bits) <= 5 &&
-                    __builtin_popcountll(open[j].ubits | ub) <= kMaxUniform &&
-                    (keep < 0 || open[j].cost > open[(size_t)keep].cost))
-                    keep = (int)j;
-            if (keep >= 0) {
-                const uint64_t kb = open[(size_t)keep].bits;
-                for (size_t j = 0; j < open.size();) {
-                    if ((open[j].bits & bits) && open[j].bits != kb) {
-                        emit(open[j]);
-                        open.erase(open.begin() + (long)j);
+            left.clear();   // the gates a block may draw from
+            for (size_t i = first; i < s1 && left.size() < 96; i++) if (!done[i]) left.push_back((int)i);
+            // the work a block on these bits takes, its gates into `take` when asked for
+            auto scan = [&](uint64_t bits, uint64_t* ubits, bool collect) {
+                uint64_t left_hard = 0, left_any = 0, u = 0;
+                double cost = 0;
+                for (int i : left) {
+                    const FuseGate& f = info[(size_t)i];
+                    const uint64_t all = f.bits | f.ub | f.hard;
+                    if (f.fusable && !(f.bits & ~bits) && !(f.hard & left_any) && !(all & left_hard) &&
+                        __builtin_popcountll(u | f.ub) <= kMaxUniform) {
+                        u |= f.ub;
+                        cost += f.cost;
+                        if (collect) take.push_back(i);
                     } else {
-                        j++;
+                        left_hard |= f.hard;
+                        left_any |= all;
+                        if (!(bits & ~left_hard)) break;   // every block bit is held back
                     }
                 }
-                for (const Block& b : open) if (b.bits == kb) { uni = kb | bits; uu = b.ubits | ub; }
-            }
-        }
-        if (__builtin_popcountll(uni) <= 5 && __builtin_popcountll(uu) <= kMaxUniform) {
-            Block nb;
-            nb.bits = uni;
-            nb.ubits = uu;
-            // merge the intersecting blocks (pairwise disjoint in tile bits, so their gates commute)
-            for (size_t j = 0; j < open.size();) {
-                if (open[j].bits & bits) {
-                    nb.idx.insert(nb.idx.end(), open[j].idx.begin(), open[j].idx.end());
-                    nb.cost += open[j].cost;
-                    open.erase(open.begin() + (long)j);
-                } else {
-                    j++;
+                if (ubits) *ubits = u;
+                return cost;
+            };
+            uint64_t bits = info[first].bits;
+            while (__builtin_popcountll(bits) < 5) {
+                tried.clear();
+                uint64_t best = 0;
+                double best_cost = -1;
+                for (int i : left) {
+                    const FuseGate& f = info[(size_t)i];
+                    const uint64_t nb = bits | f.bits;
+                    if (!f.fusable || nb == bits || __builtin_popcountll(nb) > 5) continue;
+                    if (std::find(tried.begin(), tried.end(), nb) != tried.end()) continue;
+                    tried.push_back(nb);
+                    const double c = scan(nb, nullptr, false) / (double)__builtin_popcountll(nb);   // work per bit
+                    if (c > best_cost + 1e-9) { best_cost = c; best = nb; }
                 }
+                if (!best) break;
+                bits = best;
             }
-            std::sort(nb.idx.begin(), nb.idx.end());
-            nb.idx.push_back((int)i);
-            nb.cost += gc;
-            open.push_back(std::move(nb));
-        } else {
-            flush_if(bits);
-            Block nb;
-            nb.bits = bits;
-            nb.ubits = ub;
-            nb.idx.push_back((int)i);
-            nb.cost = gc;
-            open.push_back(std::move(nb));
+            take.clear();
+            uint64_t ubits = 0;
+            const double cost = scan(bits, &ubits, true);
+            for (int i : take) done[(size_t)i] = 1;
+            emit(bits, ubits, take, cost);
         }
+        s0 = s1;
     }
-    for (Block& b : open) emit(b);
 }
 
 // Fusion for the sweeps that run on the CUDA cores (float-float and complex64 tile kernels): runs of
