@@ -37,10 +37,13 @@ def _generator(ix: Instruction):
     g = ix.operator
     if isinstance(g, PhaseShift):
         return 1, 0, 0
-    for cls, paulis in _GENERATORS.items():
-        if type(g) is cls:
-            return 0, *pauli_masks(dict(zip(ix.target, paulis)))
-    return None
+    paulis = _GENERATORS.get(type(g))
+    if paulis is None:
+        return None
+    m = 0
+    for q in ix.target[:len(paulis)]:
+        m |= 1 << q
+    return 0, (m if paulis[0] != "Z" else 0), (m if paulis[0] != "X" else 0)   # one Pauli on every target
 
 
 def parameterised(instructions) -> list:
@@ -56,10 +59,11 @@ def adjoint_gradient(sim: StateVectorSimulator, instructions: Sequence[Instructi
     param_index[i] = parameter slot of instruction i (-1: not a parameter); by default every
     differentiable gate gets its own slot in order.  Returns (energy, gradient array)."""
     instructions = list(instructions)
+    gens = [_generator(ix) for ix in instructions]
     if param_index is None:
         param_index, p = [], 0
-        for ix in instructions:
-            if _generator(ix) is not None:
+        for gen in gens:
+            if gen is not None:
                 param_index.append(p)
                 p += 1
             else:
@@ -73,16 +77,17 @@ def adjoint_gradient(sim: StateVectorSimulator, instructions: Sequence[Instructi
     gx = np.zeros(n_ops, dtype=np.uint64)
     gz = np.zeros(n_ops, dtype=np.uint64)
     scale = np.ones(n_params)
-    for i, ix in enumerate(instructions):
-        if pi[i] < 0:
+    for i, (ix, gen) in enumerate(zip(instructions, gens)):
+        slot = param_index[i]
+        if slot < 0:
             continue
-        gen = _generator(ix)
         if gen is None:
             raise ValueError(f"{ix.operator!r} has no supported generator")
         gk[i], gx[i], gz[i] = gen
-        scale[pi[i]] = ix.operator.pow_exponent
-    xm = np.array([pauli_masks(t)[0] for _, t in hamiltonian], dtype=np.uint64)
-    zm = np.array([pauli_masks(t)[1] for _, t in hamiltonian], dtype=np.uint64)
+        scale[slot] = ix.operator.pow_exponent
+    masks = [pauli_masks(t) for _, t in hamiltonian]
+    xm = np.array([x for x, _ in masks], dtype=np.uint64)
+    zm = np.array([z for _, z in masks], dtype=np.uint64)
     co = np.array([c for c, _ in hamiltonian], dtype=np.float64)
     energy = C.c_double()
     grad = np.zeros(max(1, n_params), dtype=np.float64)

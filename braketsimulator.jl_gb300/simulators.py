@@ -19,7 +19,8 @@ import numpy as np
 
 from . import _abi
 from .gates import Barrier, Control, Delay, Gate, Measure, Reset, Rx, Ry, Rz, Unitary, lower_gate
-from .noises import Noise, lower_noise
+from .noises import (AmplitudeDamping, BitFlip, Depolarizing, GeneralizedAmplitudeDamping, Noise, PauliChannel, PhaseDamping,
+                     PhaseFlip, TwoQubitDephasing, TwoQubitDepolarizing, lower_noise)
 from .observables import (H, HermitianObservable, I, Observable, StandardObservable, TensorProduct, X, Y, Z,
                           diagonalizing_gates)
 
@@ -76,19 +77,9 @@ def _ops_for(instructions, dm: bool, noise_mode: int):
         if isinstance(op, Noise):
             if not dm:
                 raise TypeError("noise channels need a DensityMatrixSimulator")
-            ln = lower_noise(op, t, noise_mode)
-            buf = np.concatenate([_abi.cplx_buffer(m) for m in ln.matrices])
+            o, buf = _noise_op(op, t, noise_mode)
             keep.append(buf)
-            o = _abi.BsOp()
-            o.kind = 1
-            o.flags = ln.flags
-            o.n_targets = len(ln.targets)
-            o.n_controls = 0
-            for j, q in enumerate(ln.targets):
-                o.targets[j] = q
-            o.n_matrices = len(ln.matrices)
-            o.matrix = _abi.dptr(buf)
-            ops.append(bytes(o))
+            ops.append(o)
             continue
         if not isinstance(op, Gate):
             raise TypeError(f"cannot apply {op!r}")
@@ -126,6 +117,44 @@ _ONE_TARGET_OPS: dict = {}   # target -> _one_target_op(target)
 # gate types whose lowering is cached by value (type, angles, pow_exponent, targets): every Gate
 # type but the matrix-carrying ones (Unitary, Control), added as they are first lowered
 _BY_VALUE = set()
+
+
+# Channels lowered by value: (type, parameters, targets' number, noise mode) -> (the bs_op struct without
+# its targets, Kraus buffer, which the engine only reads).  A circuit names a few channels on many
+# targets, and forming their matrices (16 Kronecker products for two-qubit depolarizing) was half of a
+# 12-qubit density-matrix evolution's wall time.
+_NOISE_CACHE: dict = {}
+_NOISE_CACHE_MAX = 1 << 12
+_NOISE_PARAMS = {BitFlip: ("probability",), PhaseFlip: ("probability",), Depolarizing: ("probability",),
+                 TwoQubitDepolarizing: ("probability",), TwoQubitDephasing: ("probability",), AmplitudeDamping: ("gamma",),
+                 PhaseDamping: ("gamma",), GeneralizedAmplitudeDamping: ("probability", "gamma"),
+                 PauliChannel: ("probX", "probY", "probZ")}
+
+
+def _noise_op(op: Noise, t: tuple, noise_mode: int):
+    """(bs_op struct bytes, Kraus buffer) of one channel on targets t."""
+    names = _NOISE_PARAMS.get(type(op))
+    key = hit = None
+    if names is not None:
+        key = (type(op), tuple(getattr(op, name) for name in names), len(t), noise_mode)
+        hit = _NOISE_CACHE.get(key)
+    if hit is None:
+        ln = lower_noise(op, t, noise_mode)
+        buf = np.concatenate([_abi.cplx_buffer(m) for m in ln.matrices])
+        o = _abi.BsOp()
+        o.kind = 1
+        o.flags = ln.flags
+        o.n_targets = len(ln.targets)
+        o.n_matrices = len(ln.matrices)
+        o.matrix = _abi.dptr(buf)
+        hit = (bytes(o), buf)
+        if key is not None:
+            if len(_NOISE_CACHE) >= _NOISE_CACHE_MAX:
+                _NOISE_CACHE.clear()
+            _NOISE_CACHE[key] = hit
+    b = bytearray(hit[0])
+    struct.pack_into(f"<{len(t)}i", b, _OFF_T0, *t)
+    return bytes(b), hit[1]
 
 
 def _rotation_values(op) -> tuple:

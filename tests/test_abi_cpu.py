@@ -184,3 +184,32 @@ def test_lowered_op_arrays_match_gate_by_gate_lowering():
             assert got[:off] == raw[:off] and got[off + 8:] == raw[off + 8:]
             nbytes = buf.size * 8
             assert C.string_at(arr[i].matrix, nbytes) == buf.tobytes()
+
+
+@pytest.mark.parametrize("op,targets", [
+    (bs.Depolarizing(0.1), (3,)), (bs.AmplitudeDamping(0.3), (0,)), (bs.PhaseDamping(0.2), (1,)), (bs.BitFlip(0.4), (2,)),
+    (bs.PhaseFlip(0.2), (1,)), (bs.PauliChannel(0.1, 0.2, 0.05), (2,)), (bs.GeneralizedAmplitudeDamping(0.2, 0.3), (4,)),
+    (bs.TwoQubitDephasing(0.1), (0, 2)), (bs.TwoQubitDepolarizing(0.02), (5, 1)),
+    (bs.Kraus([np.eye(4) * 0.6, np.diag([0.8, 0.8j, -0.8, 0.8])]), (2, 0))])
+@pytest.mark.parametrize("mode", [0, 16])
+def test_channels_lowered_by_value_equal_their_own_lowering(op, targets, mode):
+    import ctypes as C
+    from braketsimulator_gb300 import _abi, simulators
+    from braketsimulator_gb300.noises import lower_noise
+    for t in (targets, targets[::-1], tuple(q + 1 for q in targets)):    # kept under its value, other targets
+        got, buf = simulators._noise_op(op, t, mode)
+        ln = lower_noise(op, t, mode)
+        o = _abi.BsOp.from_buffer_copy(got)
+        assert (o.kind, o.flags, o.n_targets, o.n_controls, o.n_matrices) == (1, ln.flags, len(t), 0, len(ln.matrices))
+        assert list(o.targets)[:len(t)] == list(t) and not any(list(o.targets)[len(t):])
+        assert C.cast(o.matrix, C.c_void_p).value == buf.ctypes.data
+        assert buf.tobytes() == np.concatenate([_abi.cplx_buffer(m) for m in ln.matrices]).tobytes()
+
+
+def test_channels_on_the_wrong_number_of_targets_are_refused():
+    from braketsimulator_gb300 import simulators
+    simulators._noise_op(bs.Depolarizing(0.1), (0,), 0)
+    with pytest.raises(ValueError):
+        simulators._noise_op(bs.Depolarizing(0.1), (0, 1), 0)
+    with pytest.raises(ValueError):
+        simulators._noise_op(bs.TwoQubitDepolarizing(0.1), (1,), 0)
