@@ -159,15 +159,6 @@ __device__ __forceinline__ void commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 
-// error-free s + g (Knuth TwoSum): s <- rounded sum, returns the rounding error
-__device__ __forceinline__ float two_sum(float& s, float g) {
-    const float t = __fadd_rn(s, g);
-    const float bb = __fsub_rn(t, s);
-    const float e = __fadd_rn(__fsub_rn(s, __fsub_rn(t, bb)), __fsub_rn(g, bb));
-    s = t;
-    return e;
-}
-
 // Six digits of y = yh + yl (|y| < 2^8 after scaling) on both halves: q[j] = d_j 2^(-9j), y ~ sum_j q[j].
 // Rounding to the digit grid adds and subtracts 1.5 * 2^(23-9j), exact while |R| < 2^(22-9j).  The low
 // word (up to 2^-17) overlaps digit 2, so it takes part in choosing digits 1 and 2 (left out, digit 2
@@ -189,11 +180,12 @@ __device__ __forceinline__ void digits2(f2 yh, f2 yl, f2 (&q)[6]) {
     R = sub2(R, q[4]);
     q[5] = sub2(add2(R, c5), c5);            // grid 2^-45
 }
-// two_sum() on both halves
-__device__ __forceinline__ f2 two_sum2(f2& s, f2 g) {
+// error-free s + g on both halves where g is a multiple of ulp(s) (Dekker's FastTwoSum, which that
+// suffices for): s <- rounded sum, returns the rounding error.  Here g is a round's sum, a multiple of
+// 2^(-9w), and s the smaller rounds' sum, below 2^24 2^(-9(w+1)) + ..., so its ulp is at most 2^(-9w).
+__device__ __forceinline__ f2 fast_two_sum2(f2& s, f2 g) {
     const f2 t = add2(s, g);
-    const f2 bb = sub2(t, s);
-    const f2 e = add2(sub2(s, sub2(t, bb)), sub2(g, bb));
+    const f2 e = sub2(s, sub2(t, g));
     s = t;
     return e;
 }
@@ -260,7 +252,7 @@ __device__ __forceinline__ void issue_round(uint32_t tmem, uint32_t dcol, uint64
 }
 
 // Fold of one round's accumulator columns (this thread's NA amplitudes, re and im packed) into the
-// float-float sums: MODE 0: E = D, 1: E += D, 2: S = D, 3: E += TwoSum(S, D) error with S updated.
+// float-float sums: MODE 0: E = D, 1: E += D, 2: S = D, 3: E += FastTwoSum(S, D) error with S updated.
 template <int MODE, int NA>
 __device__ __forceinline__ void fold(uint32_t taddr, f2 (&S)[NA], f2 (&E)[NA]) {
 #pragma unroll
@@ -278,7 +270,7 @@ __device__ __forceinline__ void fold(uint32_t taddr, f2 (&S)[NA], f2 (&E)[NA]) {
                 if (MODE == 0) E[o] = gv;
                 else if (MODE == 1) E[o] = add2(E[o], gv);
                 else if (MODE == 2) S[o] = gv;
-                else E[o] = add2(E[o], two_sum2(S[o], gv));
+                else E[o] = add2(E[o], fast_two_sum2(S[o], gv));
             }
     }
 }
@@ -301,28 +293,34 @@ __device__ __forceinline__ bool wait_bar1(const State& st, int k) {
 
 // Applies fused gate g to the (swizzled) 2^12 tile sm of float4 (re hi, im hi, re lo, im lo).
 // Called by all NT threads of the CTA (NT/128 threads per tile column, 32*128/NT amplitudes each),
-// which then synchronise.  base: the CTA's global base index (selects the matrix variant).  s_tsw:
-// 32 ints of shared scratch; s_wmax: NT/32 per-warp maxima of the high words' exponent fields.
+// which then synchronise.  base: the CTA's global base index (selects the matrix variant).  s_wmax: NT/32 per-warp maxima of the high words' exponent fields.
 // gnext: the tile's next fused gate, whose digit slices are copied ahead as soon as this gate's
 // MMAs have completed (null: none, or it copies its own); s_nsrc: shared scratch for their source.
-// The swizzle is linear over XOR, so the position of column m's amplitude t is
-// sw(column bits) ^ sw(target bits of t); both come from the gate's host-made table (tab: 56
-// uint16, sw of the column bits of m & 15 and of m >> 4, then sw of the target bits of t).
+// The position of column m's amplitude t is sw(column bits) ^ sw(target bits of t); both come from the
+// gate's host-made table (tab: 56 uint16, sw of the column bits of m & 15 and of m >> 4, then sw of the
+// target bits of t).
 // On a wait that gives up, sets *fail and *err and leaves the tile partly updated.
 template <int NT>
 __device__ __forceinline__ void apply(float4* sm, const TileGate& g, const TileGate* gnext,
                                       const uint16_t* __restrict__ pool, const uint16_t* __restrict__ tab,
                                       uint16_t* sB, State& st, int64_t base,
-                                      uint32_t* s_wmax, bool emax_ok, int* s_tsw, const uint16_t** s_nsrc, int* s_fail,
+                                      uint32_t* s_wmax, bool emax_ok, const uint16_t** s_nsrc, int* s_fail,
                                       int* err) {
     constexpr int HP = NT / 128;   // threads per column
     constexpr int NA = 32 / HP;    // amplitudes per thread
     const int tid = threadIdx.x, warp = tid >> 5, lane_id = tid & 31, m = tid & 127, h = tid >> 7;
     // the previous readers of sB (the MMAs of the previous fused gate) have completed
     if (!st.pref && tid == 0) copy_slices(su32(sB), slice_src(g, pool, base), st.bar);
-    if (tid < 32) s_tsw[tid] = tab[24 + tid];
-    const int spm = tab[m & 15] ^ tab[16 + (m >> 4)];
-    const int* tsw = s_tsw + NA * h;
+    // byte offsets in the tile: amplitude a of the thread is at the XOR of its column, its half and the
+    // masks of the bits of a (the swizzle is linear over XOR)
+    const uint32_t spm = 16u * (uint32_t)(tab[m & 15] ^ tab[16 + (m >> 4)] ^ (HP > 1 ? tab[24 + NA * h] : 0));
+    const uint32_t ms[4] = {16u * tab[25], 16u * tab[26], 16u * tab[28], 16u * tab[32]};
+    auto at = [&](int a) -> float4& {
+        uint32_t o = spm;
+#pragma unroll
+        for (int q = 0; q < 4; q++) if ((a >> q) & 1) o ^= ms[q];
+        return *reinterpret_cast<float4*>(reinterpret_cast<char*>(sm) + o);
+    };
     // Tile scale: the largest exponent of the high words over the tile, per warp in s_wmax.  It was
     // left there by the previous fused gate's write-back or the tile load unless a gate that may
     // change magnitudes ran since (emax_ok false); then it is taken here in one pass.
@@ -349,7 +347,7 @@ __device__ __forceinline__ void apply(float4* sm, const TileGate& g, const TileG
     // all of the thread's amplitudes loaded first (the loads overlap), then split and stored
     float4 vv[NA];
 #pragma unroll
-    for (int a = 0; a < NA; a++) vv[a] = sm[spm ^ tsw[a]];
+    for (int a = 0; a < NA; a++) vv[a] = at(a);
 #pragma unroll
     for (int c = 0; c < NA / 4; c++) {   // four amplitudes, then one 4-column TMEM store per digit slice
         uint32_t w[6][4];
@@ -379,7 +377,7 @@ __device__ __forceinline__ void apply(float4* sm, const TileGate& g, const TileG
     // 1), thread 128 runs D1 (rounds 3, 2) and round 0 into D2, the columns of state digits 2 and 3,
     // which are free once rounds 4, 3 and 2 have completed.  Every warp folds the rounds in the order
     // 4, 3, 2, 1, 0 (smallest digit weights first), E collecting rounds 4 and 3 in FP32 and S rounds
-    // 2, 1, 0 with their TwoSum errors into E.
+    // 2, 1, 0 with the errors of their sums into E.
     bool ok = true;
     if (tid == 0) {
         if (mbar_wait(st.bar, st.ph & 1u)) {
@@ -453,7 +451,7 @@ __device__ __forceinline__ void apply(float4* sm, const TileGate& g, const TileG
         const f2 hs = add2(S[a], E[a]);
         const f2 ls = sub2(E[a], sub2(hs, S[a]));
         const float2 hh = up(mul2(hs, osc2)), ll = up(mul2(ls, osc2));
-        sm[spm ^ tsw[a]] = make_float4(hh.x, hh.y, ll.x, ll.y);
+        at(a) = make_float4(hh.x, hh.y, ll.x, ll.y);
         mx = fmaxf(mx, fmaxf(fabsf(hh.x), fabsf(hh.y)));
     }
     // the next fused gate's tile scale (read after the caller's barrier)

@@ -399,8 +399,8 @@ __global__ void __launch_bounds__(NT) k_tile_sweep(double2* __restrict__ psi, Sw
 
 // Sweep with fused 5-bit unitaries on the tensor cores (gate kind 4), T = 12, L = 5.
 // Dynamic shared memory: 48 KiB matrix digit slices | 64 KiB tile (static: split offset tables, the
-// per-warp exponents, kind-5 scratch), so that two CTAs fit on an SM; each holds 256 of the SM's 512 TMEM columns (from its first to its last
-// fused gate), so one CTA's MMAs overlap the other's CUDA-core work.  The tile is stored with the
+// per-warp exponents, kind-5 scratch), so that two CTAs fit on an SM; each holds 256 of the SM's 512
+// TMEM columns, so one CTA's MMAs overlap the other's CUDA-core work.  The tile is stored with the
 // bank swizzle tc::sw.
 #ifndef BS_TC_THREADS
 #define BS_TC_THREADS 256
@@ -416,31 +416,28 @@ struct HiOff {
     __device__ __forceinline__ uint32_t operator[](int i) const { return a[i & 7] | b[i >> 3]; }
 };
 
+// Persistent: two CTAs per SM take tiles in turn, so that barriers, offset tables and TMEM are set up once.
+// Without any gate a sweep of 28 qubits takes 1.8 ms (2.4 with a CTA per tile; HBM allows 1.26), with the
+// gates of the 12-qubit density matrix 7.3 ms instead of 7.7.  The next tile's loads issued before this
+// one's stores (64 registers of them) were slower, 62 against 59 ms at 28 qubits.
 __global__ void __launch_bounds__(kTcThreads, 2) k_tile_sweep_tc(double2* __restrict__ psi, SweepDesc d, int64_t tile0,
-                                                                 int tc_last) {
+                                                                 int64_t tile_end) {
     // 128-byte alignment: each 128-byte core matrix of the matrix operand sits in one shared-memory line
     extern __shared__ __align__(128) unsigned char dsm[];
     uint16_t* sB = reinterpret_cast<uint16_t*>(dsm);
     float4* smem = reinterpret_cast<float4*>(dsm + 49152);
     __shared__ __align__(8) uint64_t bars[7];   // digit copy, MMAs into D0 / D1, D0 / D1 read, D1 free, D2
     __shared__ uint32_t s_tmem;
-    __shared__ int64_t s_base;
     __shared__ int s_fail;
-    __shared__ int s_tsw[32];
     __shared__ uint32_t s_offa[8], s_offb[16];
     __shared__ uint32_t s_wmax[kTcThreads / 32];   // per-warp largest high-word exponent field
     __shared__ int s_act[32], s_cnt;                 // kind 5: blocks passing the row/column test
     __shared__ int s_tcq[16], s_ntc;                 // the tile's first 16 fused gates, in order
     __shared__ const uint16_t* s_nsrc;
     const HiOff off32{s_offa, s_offb};
-    constexpr int T = 12, L = 5, H = 7, nt = 1 << T, lowmask = (1 << L) - 1;
-    const int64_t tile = tile0 + (int64_t)blockIdx.x;
+    constexpr int T = 12, L = 5, H = 7, nt = 1 << T, lowmask = (1 << L) - 1, NL = nt / kTcThreads;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
-        int64_t base = 0;
-        int src = 0;
-        for (int bit = 0; bit < d.n_bits; bit++)
-            if (!((d.tile_mask >> bit) & 1ULL)) { base |= ((tile >> src) & 1LL) << bit; src++; }
-        s_base = base;
         s_fail = 0;
         tc::mbar_init(tc::su32(&bars[0]));
         tc::mbar_init(tc::su32(&bars[1]));
@@ -457,23 +454,35 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_tile_sweep_tc(double2* __rest
         if (threadIdx.x < 8) s_offa[threadIdx.x] = (uint32_t)(o >> L);
         else s_offb[threadIdx.x - 8] = (uint32_t)(o >> L);
     }
+    if (warp == 0) tc::tmem_alloc(tc::su32(&s_tmem));
+    // lane i holds the place of the tile number's bit i in the vector index: the i-th bit outside the tile
+    int out_bit = 63;
+    for (int bit = 0, src = 0; bit < d.n_bits; bit++)
+        if (!((d.tile_mask >> bit) & 1ULL)) { if (src == lane) out_bit = bit; src++; }
+    auto base_of = [&](int64_t tile) {
+        const uint64_t v = (out_bit < 63 && ((tile >> lane) & 1)) ? 1ULL << out_bit : 0ULL;
+        const uint32_t lo = __reduce_or_sync(0xffffffffu, (uint32_t)v), hi = __reduce_or_sync(0xffffffffu, (uint32_t)(v >> 32));
+        return (int64_t)(((uint64_t)hi << 32) | lo);
+    };
+    tc::fence_before();
     __syncthreads();
-    const int64_t base = s_base;
-    const int warp = threadIdx.x >> 5;
-    // tile load: each thread's 16 loads are issued together (coalesced 512 B rows), then converted to
-    // float-float at the swizzled positions
-    {
-        constexpr int NL = nt / kTcThreads;
-        double2 x[NL];
+    tc::fence_after();
+    tc::State st{s_tmem, tc::su32(&bars[0]), 0u, false};
+    double2 x[NL];   // the next tile's amplitudes, coalesced 512 B rows, all loads issued together
+    auto load = [&](int64_t b) {
 #pragma unroll
         for (int i = 0; i < NL; i++) {
             const int j = i * kTcThreads + (int)threadIdx.x;
-            x[i] = __ldcs(psi + (base | ((int64_t)off32[j >> L] << L) | (int64_t)(j & lowmask)));
+            x[i] = __ldcs(psi + (b | ((int64_t)off32[j >> L] << L) | (int64_t)(j & lowmask)));
         }
+    };
+    int64_t tile = tile0 + (int64_t)blockIdx.x;
+    int64_t base = base_of(tile);
+    load(base);
+    for (;;) {
         if (warp == kTcThreads / 32 - 1) {
             // while the loads are in flight: the fused gates this tile runs (those whose controls its
             // base satisfies), and the copy of the first one's digit slices
-            const int lane = threadIdx.x & 31;
             int cnt = 0, first = -1;
             for (int c0 = 0; c0 < d.n_gates; c0 += 32) {
                 const int gi = c0 + lane;
@@ -495,88 +504,82 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_tile_sweep_tc(double2* __rest
                 if (first >= 0) tc::copy_slices(tc::su32(sB), tc::slice_src(d.gates[first], d.tc_pool, base), tc::su32(&bars[0]));
             }
         }
-        uint32_t eb = 0;
+        // float-float at the swizzled positions
+        {
+            uint32_t eb = 0;
 #pragma unroll
-        for (int i = 0; i < NL; i++) {
-            const float4 v = c4f(load_c128(x[i]));
-            smem[tc::sw(i * kTcThreads + (int)threadIdx.x)] = v;
-            eb = max(eb, max(__float_as_uint(v.x) & 0x7F800000u, __float_as_uint(v.y) & 0x7F800000u));
+            for (int i = 0; i < NL; i++) {
+                const float4 v = c4f(load_c128(x[i]));
+                smem[tc::sw(i * kTcThreads + (int)threadIdx.x)] = v;
+                eb = max(eb, max(__float_as_uint(v.x) & 0x7F800000u, __float_as_uint(v.y) & 0x7F800000u));
+            }
+            eb = __reduce_max_sync(0xffffffffu, eb);
+            if (lane == 0) s_wmax[warp] = eb;
         }
-        eb = __reduce_max_sync(0xffffffffu, eb);
-        if ((threadIdx.x & 31) == 0) s_wmax[threadIdx.x >> 5] = eb;
-    }
-    __syncthreads();
-    tc::State st{0u, tc::su32(&bars[0]), 0u, s_ntc > 0};
-    int q = 0;   // fused gates run so far
-    bool have = false;
-    bool emax_ok = true;   // s_wmax holds the tile's largest exponent (no magnitude-changing gate since)
-    for (int gi = 0; gi < d.n_gates; gi++) {
-        const TileGate& g = d.gates[gi];
-        if ((base & (int64_t)g.gc_mask) != (int64_t)g.gc_val) continue;
-        const int kind = g.kind, k = g.k;
-        if (kind == 0 || kind == 1 || kind == 5) emax_ok = false;   // these may change magnitudes
-        if (kind == 4) {
-            if (s_fail) continue;
-            if (!have) {
-                if (warp == 0) tc::tmem_alloc(tc::su32(&s_tmem));
-                tc::fence_before();
-                __syncthreads();
-                tc::fence_after();
-                st.tmem = s_tmem;
-                have = true;
-            }
-            const TileGate* gn = q + 1 < s_ntc ? d.gates + s_tcq[q + 1] : nullptr;
-            tc::apply<kTcThreads>(smem, g, gn, d.tc_pool, reinterpret_cast<const uint16_t*>(d.perms + g.perm_off), sB,
-                                  st, base, s_wmax, emax_ok, s_tsw, &s_nsrc, &s_fail,
-                                  d.err);
-            q++;
-            emax_ok = true;
-            if (gi == tc_last) {
-                __syncthreads();
-                if (warp == 0) tc::tmem_dealloc(st.tmem);
-                have = false;
-            }
-        } else if (kind == 3) {
-            for (int j = threadIdx.x; j < nt; j += blockDim.x) {
-                const int64_t gg = base | ((int64_t)off32[j >> L] << L) | (int64_t)(j & lowmask);
-                if (parity_odd(g, gg)) {
-                    const int js = tc::sw(j);
-                    float4 v = smem[js];
-                    smem[js] = make_float4(-v.x, -v.y, -v.z, -v.w);
+        __syncthreads();
+        st.pref = s_ntc > 0;
+        int q = 0;             // fused gates run so far
+        bool emax_ok = true;   // s_wmax holds the tile's largest exponent (no magnitude-changing gate since)
+        for (int gi = 0; gi < d.n_gates; gi++) {
+            const TileGate& g = d.gates[gi];
+            if ((base & (int64_t)g.gc_mask) != (int64_t)g.gc_val) continue;
+            const int kind = g.kind, k = g.k;
+            if (kind == 0 || kind == 1 || kind == 5) emax_ok = false;   // these may change magnitudes
+            if (kind == 4) {
+                if (s_fail) continue;
+                const TileGate* gn = q + 1 < s_ntc ? d.gates + s_tcq[q + 1] : nullptr;
+                tc::apply<kTcThreads>(smem, g, gn, d.tc_pool, reinterpret_cast<const uint16_t*>(d.perms + g.perm_off), sB,
+                                      st, base, s_wmax, emax_ok, &s_nsrc, &s_fail,
+                                      d.err);
+                q++;
+                emax_ok = true;
+            } else if (kind == 3) {
+                for (int j = threadIdx.x; j < nt; j += blockDim.x) {
+                    const int64_t gg = base | ((int64_t)off32[j >> L] << L) | (int64_t)(j & lowmask);
+                    if (parity_odd(g, gg)) {
+                        const int js = tc::sw(j);
+                        float4 v = smem[js];
+                        smem[js] = make_float4(-v.x, -v.y, -v.z, -v.w);
+                    }
                 }
+            } else if (kind == 1) {
+                tile_diag<HiOff, true>(smem, T, L, g, d.mats, base, off32, L);
+            } else if (kind == 5) {
+                if (k == 1) tile_kraus_ref_lr<1, true, HiOff>(smem, T, L, g, d.mats, base, off32, L, d.n_bits / 2, s_act, &s_cnt);
+                else tile_kraus_ref_lr<2, true, HiOff>(smem, T, L, g, d.mats, base, off32, L, d.n_bits / 2, s_act, &s_cnt);
+            } else if (kind == 0) {   // the planner routes sweeps with unfused 3- or 4-target gates elsewhere
+                if (k == 1) tile_dense<1, true>(smem, T, g, d.mats);
+                else tile_dense<2, true>(smem, T, g, d.mats);
+            } else {
+                if (k == 1) tile_monomial<1, true>(smem, T, g, d.perms);
+                else tile_monomial<2, true>(smem, T, g, d.perms);
             }
-        } else if (kind == 1) {
-            tile_diag<HiOff, true>(smem, T, L, g, d.mats, base, off32, L);
-        } else if (kind == 5) {
-            if (k == 1) tile_kraus_ref_lr<1, true, HiOff>(smem, T, L, g, d.mats, base, off32, L, d.n_bits / 2, s_act, &s_cnt);
-            else tile_kraus_ref_lr<2, true, HiOff>(smem, T, L, g, d.mats, base, off32, L, d.n_bits / 2, s_act, &s_cnt);
-
-        } else if (kind == 0) {   // the planner routes sweeps with unfused 3- or 4-target gates elsewhere
-            if (k == 1) tile_dense<1, true>(smem, T, g, d.mats);
-            else tile_dense<2, true>(smem, T, g, d.mats);
-        } else {
-            if (k == 1) tile_monomial<1, true>(smem, T, g, d.perms);
-            else tile_monomial<2, true>(smem, T, g, d.perms);
+            __syncthreads();
         }
-        __syncthreads();
-    }
-    if (have) {
-        // a wait gave up: give the copies and MMAs in flight a bounded time to land before releasing TMEM
-        if (threadIdx.x == 0 && s_fail) {
-            tc::mbar_wait(st.bar, st.ph & 1u);
-            tc::mbar_wait(st.bar + 8u, (st.ph >> 1) & 1u);
-            tc::mbar_wait(st.bar + 16u, (st.ph >> 2) & 1u);
-            tc::mbar_wait(st.bar + 48u, (st.ph >> 6) & 1u);
-        }
-        __syncthreads();
-        if (warp == 0) tc::tmem_dealloc(st.tmem);
-    }
-    // tile store: streaming stores, nothing waits for them
+        const int64_t here = base;
+        tile += gridDim.x;
+        const bool more = tile < tile_end && !s_fail;   // uniform: s_fail is written before a barrier of the loop above
+        // tile store: streaming stores, nothing waits for them
 #pragma unroll 4
-    for (int i = 0; i < nt / kTcThreads; i++) {
-        const int j = i * kTcThreads + (int)threadIdx.x;
-        __stcs(psi + (base | ((int64_t)off32[j >> L] << L) | (int64_t)(j & lowmask)), store_c128(f4c(smem[tc::sw(j)])));
+        for (int i = 0; i < NL; i++) {
+            const int j = i * kTcThreads + (int)threadIdx.x;
+            __stcs(psi + (here | ((int64_t)off32[j >> L] << L) | (int64_t)(j & lowmask)), store_c128(f4c(smem[tc::sw(j)])));
+        }
+        if (!more) break;
+        base = base_of(tile);
+        load(base);
+        __syncthreads();   // every thread has read the tile (and s_ntc) before the next one is written
     }
+    // a wait gave up: give the copies and MMAs in flight a bounded time to land before releasing TMEM
+    if (threadIdx.x == 0 && s_fail) {
+        tc::mbar_wait(st.bar, st.ph & 1u);
+        tc::mbar_wait(st.bar + 8u, (st.ph >> 1) & 1u);
+        tc::mbar_wait(st.bar + 16u, (st.ph >> 2) & 1u);
+        tc::mbar_wait(st.bar + 48u, (st.ph >> 6) & 1u);
+    }
+    tc::fence_before();
+    __syncthreads();
+    if (warp == 0) tc::tmem_dealloc(st.tmem);
 }
 
 // Digit slices of the fused matrices for the tensor-core sweep, one CTA per matrix variant.
@@ -1288,7 +1291,6 @@ int bs_run_sweeps(bs_sim* s, const std::vector<Sweep>& sweeps) {
     std::vector<int32_t> perms;
     struct Launch {
         int64_t gate0; int n_gates; std::vector<int> hi; bool big; int big_gate; int kmax = 1;
-        int tc_last = -1;          // index (within the sweep) of the last fused tensor-core gate, -1 if none
         int n_tc = 0;
         bool blk = false;          // has register blocks, with operations rop0 .. rop0 + n_rops
         size_t rop0 = 0;
@@ -1467,7 +1469,6 @@ int bs_run_sweeps(bs_sim* s, const std::vector<Sweep>& sweeps) {
                 for (int v = 0; v < nvar; v++) tc_scale.push_back(std::ldexp(1.0, 8 - eu));
                 n_var += nvar;
                 t.tc_eu = eu;
-                ln.tc_last = ln.n_gates;
                 ln.n_tc++;
                 tg.push_back(t);
                 ln.n_gates++;
@@ -1675,10 +1676,10 @@ int bs_run_sweeps(bs_sim* s, const std::vector<Sweep>& sweeps) {
         d.err = s->dev_flag;
         for (int64_t t0 = 0; t0 < ntiles; t0 += (1LL << 30)) {
             int64_t nb = std::min<int64_t>(ntiles - t0, 1LL << 30);
-            if (ln.tc_last >= 0 && s->capturing) {
-                k_tile_sweep_tc<<<(unsigned)nb, kTcThreads, kTcSmem, s->stream>>>(psi, d, t0, ln.tc_last);
+            if (ln.n_tc > 0 && s->capturing) {
+                k_tile_sweep_tc<<<(unsigned)std::min<int64_t>(nb, 2 * 152), kTcThreads, kTcSmem, s->stream>>>(psi, d, t0, t0 + nb);
                 s->stats.tc_launches++;
-            } else if (ln.tc_last >= 0) {
+            } else if (ln.n_tc > 0) {
                 const size_t pe = 2 * s->tc_events_used;
                 while (s->tc_events.size() < pe + 2) {
                     cudaEvent_t e;
@@ -1687,7 +1688,7 @@ int bs_run_sweeps(bs_sim* s, const std::vector<Sweep>& sweeps) {
                     s->tc_events.push_back(e);
                 }
                 cudaEventRecord(s->tc_events[pe], s->stream);
-                k_tile_sweep_tc<<<(unsigned)nb, kTcThreads, kTcSmem, s->stream>>>(psi, d, t0, ln.tc_last);
+                k_tile_sweep_tc<<<(unsigned)std::min<int64_t>(nb, 2 * 152), kTcThreads, kTcSmem, s->stream>>>(psi, d, t0, t0 + nb);
                 cudaEventRecord(s->tc_events[pe + 1], s->stream);
                 s->tc_events_used++;
                 s->stats.tc_launches++;
