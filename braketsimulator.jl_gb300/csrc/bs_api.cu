@@ -578,7 +578,7 @@ int bs_run_small(bs_sim* s, const bs_op* ops, int64_t n_ops, int64_t shots, uint
     std::vector<char> key;
     bool keyed = n_ops >= 0 && (n_ops == 0 || ops);
     if (keyed) {
-        const int head[2] = {s->n, bs_tile_bits(s)};
+        const int head[2] = {s->n, bs_sweep_tile_bits(s)};
         key.insert(key.end(), (const char*)head, (const char*)head + sizeof(head));
         size_t mat_bytes = 0;
         for (int64_t i = 0; i < n_ops && keyed; i++) {

@@ -110,7 +110,16 @@ struct BsTuning {
 
 // The packed plan of one small-circuit run (bs_run_small): the whole state is one tile, so the plan is
 // the gate table, its matrices and permutations, and the largest dense or monomial target count.
+// States above 2^10 run in a cluster of CTAs that hold 2^9 amplitudes each, sweep by sweep: `sweeps` then
+// lists the sweeps (else it is empty).
+constexpr int kSmallTileBits = 9;
+struct SmallSweep {
+    int32_t g0, ng;             // its gates
+    int8_t hi[4];               // tile bits 5..8: endian bits
+    int8_t out[4];              // the endian bits outside the tile, ascending: the CTA's rank
+};
 struct SmallPlan {
+    std::vector<SmallSweep> sweeps;
     std::vector<TileGate> tg;
     std::vector<float4> mats;
     std::vector<int32_t> perms;

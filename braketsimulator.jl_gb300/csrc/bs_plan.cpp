@@ -190,16 +190,16 @@ int bs_tile_bits(const bs_sim* s) {
     return (b >= 10 && b <= BS_TILE_MAX_BITS) ? b : BS_TILE_MAX_BITS;
 }
 
-// Complex128 vectors of 13 to 18 bits take smaller tiles where nothing sets the tile bits (and no
-// tensor-core sweeps, which have tiles of 2^12, are asked for): 128 tiles at 17 and 18 bits, 8 to 64 of
-// 2^10 below, for 152 SMs.  A gate's pass over a tile takes its time per amplitude, which outweighs the
+// Complex128 vectors of 11 to 18 bits take smaller tiles where nothing sets the tile bits (and no
+// tensor-core sweeps, which have tiles of 2^12, are asked for): 128 tiles at 16 to 18 bits, 4 to 64 of
+// 2^9 below, for 152 SMs.  A gate's pass over a tile takes its time per amplitude, which outweighs the
 // launches of the extra sweeps: 17 qubits, 8 ansatz layers, 15 sweeps of 32 tiles (2^12) 0.90 ms, 22 of
 // 128 (2^10) 0.33 ms, with 16 warps a tile and half the products of the real rotations.
 int bs_sweep_tile_bits(const bs_sim* s) {
     const int n = bs_vec_bits(s), b = bs_tile_bits(s);
     if (s->tune.tile_bits >= 0 || getenv("BS_TILE_BITS") || s->precision != BS_PREC_C128) return b;
-    if (n <= BS_TILE_MAX_BITS || n >= 19 || (bs_tc_enabled(s) && n >= bs_tc_min_bits(s))) return b;
-    return std::max(10, n - 7);
+    if (n <= 10 || n >= 19 || (bs_tc_enabled(s) && n >= bs_tc_min_bits(s))) return b;
+    return std::max(kSmallTileBits, n - 7);
 }
 
 int bs_tile_threads(const bs_sim* s) {

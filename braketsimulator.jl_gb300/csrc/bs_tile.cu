@@ -10,6 +10,7 @@
 // src/dm_simulator.jl:130-140 is two tile gates (column bits U, row bits conj U).
 #include <algorithm>
 #include <atomic>
+#include <cooperative_groups.h>
 #include <cmath>
 #include <complex>
 #include <cstring>
@@ -1797,6 +1798,89 @@ __device__ __forceinline__ void small_run_done(volatile int64_t* done, int64_t t
     if (threadIdx.x == 0) *done = ticket;
 }
 
+// The shots sh0, sh0 + step, ... as bs_sample draws them for a state of one CDF block (k_sample_small):
+// the same chunk sums and chunk prefix sums, the same in-chunk running sums (a warp's shuffle scan, kept
+// here per element), the same uniforms and comparisons, so the same indices; one thread per shot.
+// sprob: the nt probabilities; scan: room for two arrays of whole chunks.
+struct SmallCdf {
+    float ch[kCpb], cl[kCpb];
+    double cinc[kCpb], total;
+    long long ckey[kCpb];
+};
+__device__ __forceinline__ void small_shots(const double* sprob, int nt, double* scan, SmallCdf& c, int64_t sh0, int64_t step,
+                                            int64_t shots, uint64_t seed, int64_t* __restrict__ samples) {
+    const int nc32 = (nt + kChunk - 1) / kChunk * kChunk;
+    block_chunk_sums_p(sprob, nt, 0, c.ch, c.cl, &c.total, c.cinc);
+    // per element: the largest value, as an integer key, of (chunk base + running sum) over the chunk
+    // up to it, so that a binary search finds the first element whose own value reaches the target
+    long long* fkey = reinterpret_cast<long long*>(scan + nc32);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    for (int q = warp; q * kChunk < nt; q += nw) {
+        const int i = q * kChunk + lane;
+        double p = (i < nt) ? sprob[i] : 0.0;
+        const double cb = q == 0 ? 0.0 : c.cinc[q - 1];   // 0.0 + cb is cb: the sums are non-negative
+        if (__ballot_sync(0xffffffffu, p != 0.0) == 0u) {
+            // a chunk of zeros: every running sum is 0, every compared value the chunk base
+            scan[i] = 0.0;
+            fkey[i] = __double_as_longlong(cb);
+            continue;
+        }
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const double v = __shfl_up_sync(0xffffffffu, p, o);
+            if (lane >= o) p += v;
+        }
+        scan[i] = p;
+        long long key = __double_as_longlong(cb + p);
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const long long v = __shfl_up_sync(0xffffffffu, key, o);
+            if (lane >= o) key = max(key, v);
+        }
+        fkey[i] = key;
+    }
+    for (int q = threadIdx.x; q < kCpb; q += blockDim.x) c.ckey[q] = __double_as_longlong(0.0 + c.cinc[q]);
+    __syncthreads();
+    // Every value compared below is a sum of probabilities, so non-negative: its order is the order of
+    // its bit pattern as an integer, which keeps the comparisons off the FP64 pipe (2 per clock per SM).
+    const double total = 0.0 + c.total;
+    // u * total with u = (r >> 11) 2^-53: the scaling by 2^-53 is exact on either factor, so
+    // (r >> 11) * (total 2^-53) rounds the same real product once, as the samplers' u * total does
+    const double tscale = total * 0x1.0p-53;
+    for (int64_t sh = sh0; sh < shots; sh += step) {
+        const uint64_t r = splitmix64(seed ^ splitmix64((uint64_t)sh));
+        const double t = (double)(r >> 11) * tscale;
+        const long long tb = __double_as_longlong(t);
+        int clo = 0, chi = kCpb - 1;
+        while (clo < chi) {
+            const int mid = (clo + chi) >> 1;
+            if (c.ckey[mid] >= tb) chi = mid; else clo = mid + 1;
+        }
+        const int c0 = clo * kChunk;
+        int lo = 0, hi = kChunk;   // first element of the chunk whose value reaches the target
+        while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if (fkey[c0 + mid] >= tb) hi = mid; else lo = mid + 1;
+        }
+        int64_t out = nt - 1;
+        bool found = lo < kChunk && c0 + lo < nt;
+        if (found) out = c0 + lo;
+        if (!found && c0 < nt) {
+            // the chunk's own running sum fell short of its prefix sum by rounding: go on as the
+            // one-block sampler does, with the running sum carried from chunk to chunk
+            double cw = (0.0 + (clo == 0 ? 0.0 : c.cinc[clo - 1])) + scan[c0 + kChunk - 1];
+            for (int q = c0 + kChunk; q < nt && !found; q += kChunk) {
+                for (int l = 0; l < kChunk; l++) {
+                    const int i = q + l;
+                    if (i < nt && cw + scan[i] >= t) { out = i; found = true; break; }
+                }
+                cw += scan[q + kChunk - 1];
+            }
+        }
+        samples[sh] = out;
+    }
+}
+
 // STAGED: the matrices and permutations are copied into shared memory first (one round trip to the
 // plan, which may live in host-mapped memory) instead of being read from the plan at every gate.
 template <int KMAX, bool STAGED>
@@ -1808,9 +1892,6 @@ __global__ void __launch_bounds__(512) k_small_run(double2* __restrict__ psi, in
                                                    int64_t* times) {
     if (times && threadIdx.x == 0) times[0] = globaltimer_ns();
     extern __shared__ float4 smem[];
-    __shared__ float s_ch[kCpb], s_cl[kCpb];
-    __shared__ double s_cinc[kCpb], s_total;
-    __shared__ long long s_ckey[kCpb];
     __shared__ TileGate s_gates[kGateChunk];
     const int nt = 1 << n, nc32 = (nt + kChunk - 1) / kChunk * kChunk;
     // the probabilities, after the tile (or after the sampler's two arrays, which replace the tile),
@@ -1863,80 +1944,128 @@ __global__ void __launch_bounds__(512) k_small_run(double2* __restrict__ psi, in
         small_run_done(done, ticket, times);
         return;
     }
-    // The shots, as bs_sample draws them for a state of one CDF block (k_sample_small): the same
-    // chunk sums and chunk prefix sums, the same in-chunk running sums (a warp's shuffle scan, kept
-    // here per element), the same uniforms and comparisons, so the same indices; one thread per shot.
-    block_chunk_sums_p(sprob, nt, 0, s_ch, s_cl, &s_total, s_cinc);
-    double* scan = reinterpret_cast<double*>(smem);   // the tile is no longer needed
-    // per element: the largest value, as an integer key, of (chunk base + running sum) over the chunk
-    // up to it, so that a binary search finds the first element whose own value reaches the target
-    long long* fkey = reinterpret_cast<long long*>(scan + nc32);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    for (int c = warp; c * kChunk < nt; c += nw) {
-        const int i = c * kChunk + lane;
-        double p = (i < nt) ? sprob[i] : 0.0;
-        const double cb = c == 0 ? 0.0 : s_cinc[c - 1];   // 0.0 + cb is cb: the sums are non-negative
-        if (__ballot_sync(0xffffffffu, p != 0.0) == 0u) {
-            // a chunk of zeros: every running sum is 0, every compared value the chunk base
-            scan[i] = 0.0;
-            fkey[i] = __double_as_longlong(cb);
-            continue;
-        }
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const double v = __shfl_up_sync(0xffffffffu, p, o);
-            if (lane >= o) p += v;
-        }
-        scan[i] = p;
-        long long key = __double_as_longlong(cb + p);
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const long long v = __shfl_up_sync(0xffffffffu, key, o);
-            if (lane >= o) key = max(key, v);
-        }
-        fkey[i] = key;
-    }
-    for (int c = threadIdx.x; c < kCpb; c += blockDim.x) s_ckey[c] = __double_as_longlong(0.0 + s_cinc[c]);
-    __syncthreads();
-    // Every value compared below is a sum of probabilities, so non-negative: its order is the order of
-    // its bit pattern as an integer, which keeps the comparisons off the FP64 pipe (2 per clock per SM).
-    const double total = 0.0 + s_total;
-    // u * total with u = (r >> 11) 2^-53: the scaling by 2^-53 is exact on either factor, so
-    // (r >> 11) * (total 2^-53) rounds the same real product once, as the samplers' u * total does
-    const double tscale = total * 0x1.0p-53;
-    for (int64_t sh = threadIdx.x; sh < shots; sh += blockDim.x) {
-        const uint64_t r = splitmix64(seed ^ splitmix64((uint64_t)sh));
-        const double t = (double)(r >> 11) * tscale;
-        const long long tb = __double_as_longlong(t);
-        int clo = 0, chi = kCpb - 1;
-        while (clo < chi) {
-            const int mid = (clo + chi) >> 1;
-            if (s_ckey[mid] >= tb) chi = mid; else clo = mid + 1;
-        }
-        const int c0 = clo * kChunk;
-        int lo = 0, hi = kChunk;   // first element of the chunk whose value reaches the target
-        while (lo < hi) {
-            const int mid = (lo + hi) >> 1;
-            if (fkey[c0 + mid] >= tb) hi = mid; else lo = mid + 1;
-        }
-        int64_t out = nt - 1;
-        bool found = lo < kChunk && c0 + lo < nt;
-        if (found) out = c0 + lo;
-        if (!found && c0 < nt) {
-            // the chunk's own running sum fell short of its prefix sum by rounding: go on as the
-            // one-block sampler does, with the running sum carried from chunk to chunk
-            double cw = (0.0 + (clo == 0 ? 0.0 : s_cinc[clo - 1])) + scan[c0 + kChunk - 1];
-            for (int c = c0 + kChunk; c < nt && !found; c += kChunk) {
-                for (int l = 0; l < kChunk; l++) {
-                    const int i = c + l;
-                    if (i < nt && cw + scan[i] >= t) { out = i; found = true; break; }
-                }
-                cw += scan[c + kChunk - 1];
-            }
-        }
-        samples[sh] = out;
-    }
+    __shared__ SmallCdf s_cdf;
+    small_shots(sprob, nt, reinterpret_cast<double*>(smem) /* the tile is no longer needed */, s_cdf, threadIdx.x, blockDim.x, shots,
+                seed, samples);
     small_run_done(done, ticket, times);
+}
+
+// The same for states of 2^11 and 2^12: a cluster of 4 or 8 CTAs holds 2^9 amplitudes each, so that the
+// gates' float-float arithmetic, which bounds the one-CTA kernel (1.6 us a gate at 12 qubits), runs on
+// as many SMs.  The plan is the sweeps bs_evolve would run for tiles of 2^9; between sweeps every CTA
+// gathers its next tile from the others' shared memory (two tiles by turns, one cluster barrier a
+// sweep).  At the end every CTA gets all probabilities and draws its share of the shots.
+template <int KMAX, bool STAGED>
+__global__ void __launch_bounds__(256) k_small_cluster(double2* __restrict__ psi, int n, const SmallSweep* __restrict__ sweeps,
+                                                       int ns, const TileGate* __restrict__ gates, int ng,
+                                                       const float4* __restrict__ mats, int n_mats,
+                                                       const int32_t* __restrict__ perms, int n_perms,
+                                                       double* __restrict__ probs, int64_t shots, uint64_t seed,
+                                                       int64_t* __restrict__ samples, volatile int64_t* done, int64_t ticket,
+                                                       int64_t* times) {
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    constexpr int T = kSmallTileBits, L = 5, nt = 1 << T;
+    const int rank = (int)cluster.block_rank(), ranks = (int)cluster.num_blocks(), rb = n - T, dim = 1 << n;
+    const int tid = threadIdx.x;
+    if (times && rank == 0 && tid == 0) times[0] = globaltimer_ns();
+    extern __shared__ float4 smem[];
+    __shared__ int64_t s_off[1 << (T - L)];
+    __shared__ SmallCdf s_cdf;
+    float4* tile0 = smem;                                         // two tiles, taken by turns
+    double* sprob = reinterpret_cast<double*>(smem + 2 * nt);     // all probabilities
+    double* scan = sprob + dim;                                   // two arrays for the sampler
+    float4* ms = reinterpret_cast<float4*>(scan + 2 * dim);
+    TileGate* gs = reinterpret_cast<TileGate*>(ms + (STAGED ? n_mats : 0));
+    int32_t* ps = reinterpret_cast<int32_t*>(gs + (STAGED ? ng : 0));
+    SmallSweep* ss = reinterpret_cast<SmallSweep*>(ps + (STAGED ? (n_perms + 3) / 4 * 4 : 0));
+    if (STAGED) {
+        // the plan may live in host-mapped memory: one round trip for all of it
+        for (int j = tid; j < n_mats; j += blockDim.x) ms[j] = mats[j];
+        stage_words(gs, gates, ng * (int)(sizeof(TileGate) / 4));
+        for (int j = tid; j < n_perms; j += blockDim.x) ps[j] = perms[j];
+        stage_words(ss, sweeps, ns * (int)(sizeof(SmallSweep) / 4));
+    }
+    const float4* m_op = STAGED ? ms : mats;
+    const int32_t* p_op = STAGED ? ps : perms;
+    const TileGate* g_op = STAGED ? gs : gates;
+    const SmallSweep* w_op = STAGED ? ss : sweeps;
+    cluster.sync();   // every CTA runs before another touches its shared memory; also orders the staging
+    int64_t base = 0;
+    for (int w = 0; w < ns; w++) {
+        const SmallSweep sw = w_op[w];
+        float4* cur = tile0 + (w & 1) * nt;
+        base = 0;
+        for (int q = 0; q < rb; q++) base |= (int64_t)((rank >> q) & 1) << sw.out[q];
+        if (tid < (1 << (T - L))) {
+            int64_t o = 0;
+            for (int q = 0; q < T - L; q++) o |= (int64_t)((tid >> q) & 1) << sw.hi[q];
+            s_off[tid] = o;
+        }
+        if (w == 0) {
+            for (int j = tid; j < nt; j += blockDim.x)
+                cur[j] = make_float4(j == 0 && base == 0 ? 1.f : 0.f, 0.f, 0.f, 0.f);
+            __syncthreads();
+        } else {
+            const SmallSweep pv = w_op[w - 1];
+            cluster.sync();   // the previous sweep is done everywhere; also orders s_off
+            for (int j = tid; j < nt; j += blockDim.x) {
+                const int64_t g = base | s_off[j >> L];
+                int pj = j & ((1 << L) - 1), pr = 0;
+                for (int q = 0; q < T - L; q++) pj |= (int)((g >> pv.hi[q]) & 1) << (L + q);
+                for (int q = 0; q < rb; q++) pr |= (int)((g >> pv.out[q]) & 1) << q;
+                // through complex128, as a sweep's store and the next one's load: the same values
+                cur[j] = c4f(load_c128(store_c128(f4c(cluster.map_shared_rank(tile0 + ((w - 1) & 1) * nt, pr)[pj]))));
+            }
+            __syncthreads();
+        }
+        for (int gi = sw.g0; gi < sw.g0 + sw.ng; gi++) {
+            const TileGate& g = g_op[gi];
+            if ((base & (int64_t)g.gc_mask) != (int64_t)g.gc_val) continue;   // uniform in the CTA
+            const int kind = g.kind, k = g.k;
+            if (kind == 0) {
+                if (k == 1) tile_dense<1, false, STAGED>(cur, T, g, m_op);
+                else if (k == 2) tile_dense<2, false, STAGED>(cur, T, g, m_op);
+                else if (KMAX == 4 && k == 3) tile_dense<3, false, STAGED>(cur, T, g, m_op);
+                else if (KMAX == 4) tile_dense<4, false, STAGED>(cur, T, g, m_op);
+            } else if (kind == 1) {
+                tile_diag<const int64_t*, false, STAGED>(cur, T, L, g, m_op, base, s_off, 0);
+            } else {
+                if (k == 1) tile_monomial<1, false, STAGED>(cur, T, g, p_op);
+                else if (k == 2) tile_monomial<2, false, STAGED>(cur, T, g, p_op);
+                else if (KMAX == 4 && k == 3) tile_monomial<3, false, STAGED>(cur, T, g, p_op);
+                else if (KMAX == 4) tile_monomial<4, false, STAGED>(cur, T, g, p_op);
+            }
+            __syncthreads();
+        }
+    }
+    // the state and its probabilities, these to every CTA
+    const float4* cur = tile0 + ((ns - 1) & 1) * nt;
+    for (int j = tid; j < nt; j += blockDim.x) {
+        const int64_t i = base | s_off[j >> L] | (int64_t)(j & ((1 << L) - 1));
+        const double2 v = store_c128(f4c(cur[j]));
+        psi[i] = v;
+        const cff x = load_c128(v);
+        ffacc a;
+        acc_first(a, x.rh, x.rl, x.rh, x.rl);
+        acc_add(a, x.ih, x.il, x.ih, x.il);
+        const ff r = acc_done(a);
+        const double pj = ff2d(r.h, r.l);   // prob_at's value for this amplitude
+        probs[i] = pj;
+        if (shots > 0)
+            for (int r2 = 0; r2 < ranks; r2++) cluster.map_shared_rank(sprob, r2)[i] = pj;
+    }
+    cluster.sync();   // no CTA's shared memory is touched by another from here on
+    if (shots > 0)
+        small_shots(sprob, dim, scan, s_cdf, (int64_t)rank * blockDim.x + tid, (int64_t)ranks * blockDim.x, shots, seed, samples);
+    if (!done) return;
+    __threadfence_system();
+    cluster.sync();   // every CTA's results are visible to the host
+    if (rank == 0 && tid == 0) {
+        if (times) times[1] = globaltimer_ns();
+        __threadfence_system();
+        *done = ticket;
+    }
 }
 
 }  // namespace
@@ -1944,15 +2073,33 @@ __global__ void __launch_bounds__(512) k_small_run(double2* __restrict__ psi, in
 int bs_small_pack(const bs_sim* s, const std::vector<Sweep>& sweeps, SmallPlan& out) {
     const int n = s->n;
     if (s->kind != BS_KIND_SV || s->precision != BS_PREC_C128 || n > 12) return BS_ERR_UNSUPPORTED;
+    const int T = std::min(bs_sweep_tile_bits(s), n), L = BS_TILE_LOW_BITS;
+    const bool cluster = T == kSmallTileBits && n > T;   // else the whole state is the tile, whatever the sweeps
     std::vector<TileGate>& tg = out.tg;
     std::vector<float4>& mats = out.mats;
     std::vector<int32_t>& perms = out.perms;
+    out.sweeps.clear();
     tg.clear();
     mats.clear();
     perms.clear();
     int kmax = 1;
     std::vector<HostGate> merged;
     for (const Sweep& sw : sweeps) {
+        int local[64];           // tile position of an endian bit: its own, or (cluster) as in the sweep
+        for (int b = 0; b < 64; b++) local[b] = cluster ? -1 : b;
+        if (cluster) {
+            if ((int)sw.hi_bits.size() != T - L) return BS_ERR_UNSUPPORTED;   // a gate no tile holds
+            SmallSweep w{};
+            for (int b = 0; b < L; b++) local[b] = b;
+            for (int q = 0; q < T - L; q++) {
+                local[sw.hi_bits[(size_t)q]] = L + q;
+                w.hi[q] = (int8_t)sw.hi_bits[(size_t)q];
+            }
+            int r = 0;
+            for (int b = L; b < n; b++) if (local[b] < 0) w.out[r++] = (int8_t)b;
+            w.g0 = (int32_t)tg.size();
+            out.sweeps.push_back(w);
+        }
         merge_diagonals(sw.gates, merged);
         for (const HostGate& hg : merged) {
             if (hg.kind != 0 && hg.kind != 1 && hg.kind != 2) return BS_ERR_UNSUPPORTED;
@@ -1960,11 +2107,16 @@ int bs_small_pack(const bs_sim* s, const std::vector<Sweep>& sweeps, SmallPlan& 
             TileGate t{};
             t.kind = hg.kind;
             t.k = hg.k;
-            t.lc_mask = (uint32_t)hg.cmask;   // every bit is in the tile, at its own position
-            t.lc_val = (uint32_t)hg.cval;
+            for (int b = 0; b < n; b++) {
+                if (!((hg.cmask >> b) & 1ULL)) continue;
+                const uint64_t v = (hg.cval >> b) & 1ULL;
+                if (local[b] >= 0) { t.lc_mask |= 1u << local[b]; t.lc_val |= (uint32_t)v << local[b]; }
+                else { t.gc_mask |= 1ULL << b; t.gc_val |= v << b; }
+            }
             for (int q = 0; q < hg.k; q++) {
                 t.gbit[q] = hg.ebit[q];
-                if (q < BS_TILE_MAXK) t.tbit[q] = hg.ebit[q];
+                if (q < BS_TILE_MAXK) t.tbit[q] = local[hg.ebit[q]];
+                if (hg.kind != 1 && local[hg.ebit[q]] < 0) return BS_ERR_UNSUPPORTED;
             }
             t.mat_off = (int32_t)mats.size();
             t.perm_off = (int32_t)perms.size();
@@ -1980,6 +2132,13 @@ int bs_small_pack(const bs_sim* s, const std::vector<Sweep>& sweeps, SmallPlan& 
             }
             tg.push_back(t);
         }
+        if (cluster) out.sweeps.back().ng = (int32_t)tg.size() - out.sweeps.back().g0;
+    }
+    if (cluster && out.sweeps.empty()) {   // no gate: |0...0> still has to be written
+        SmallSweep w{};
+        for (int q = 0; q < T - L; q++) w.hi[q] = (int8_t)(L + q);
+        for (int b = T, r = 0; b < n; b++) w.out[r++] = (int8_t)b;
+        out.sweeps.push_back(w);
     }
     out.kmax = kmax;
     return BS_OK;
@@ -1996,17 +2155,21 @@ int bs_small_launch(bs_sim* s, const SmallPlan& plan, double* dprobs, int64_t sh
     const int64_t b_tg = al((int64_t)(tg.size() + 1) * (int64_t)sizeof(TileGate));
     const int64_t b_m = al((int64_t)(mats.size() + 1) * (int64_t)sizeof(float4));
     const int64_t b_p = al((int64_t)(perms.size() + 1) * (int64_t)sizeof(int32_t));
-    const int64_t b_all = b_tg + b_m + b_p;
+    const int64_t b_w = al((int64_t)(plan.sweeps.size() + 1) * (int64_t)sizeof(SmallSweep));
+    const int64_t b_all = b_tg + b_m + b_p + b_w;
     char* dev;
     int rc;
+    auto write = [&](char* host) {
+        if (!tg.empty()) std::memcpy(host, tg.data(), tg.size() * sizeof(TileGate));
+        if (!mats.empty()) std::memcpy(host + b_tg, mats.data(), mats.size() * sizeof(float4));
+        if (!perms.empty()) std::memcpy(host + b_tg + b_m, perms.data(), perms.size() * sizeof(int32_t));
+        if (!plan.sweeps.empty()) std::memcpy(host + b_tg + b_m + b_p, plan.sweeps.data(), plan.sweeps.size() * sizeof(SmallSweep));
+    };
     if (io && b_all <= (int64_t)io->plan_cap) {
         // the plan goes straight into host-mapped memory, which the kernel reads (the previous run on
         // this thread has completed, so nothing reads it any more); the launch orders these writes
         // before the kernel's reads
-        char* host = io->hplan;
-        if (!tg.empty()) std::memcpy(host, tg.data(), tg.size() * sizeof(TileGate));
-        if (!mats.empty()) std::memcpy(host + b_tg, mats.data(), mats.size() * sizeof(float4));
-        if (!perms.empty()) std::memcpy(host + b_tg + b_m, perms.data(), perms.size() * sizeof(int32_t));
+        write(io->hplan);
         std::atomic_thread_fence(std::memory_order_release);
         dev = io->dplan;
     } else {
@@ -2014,13 +2177,52 @@ int bs_small_launch(bs_sim* s, const SmallPlan& plan, double* dprobs, int64_t sh
         if (rc) return rc;
         char* host = bs_stage(s, (size_t)b_all);
         if (!host) return bs_fail(s, BS_ERR_ALLOC, "pinned staging allocation");
-        if (!tg.empty()) std::memcpy(host, tg.data(), tg.size() * sizeof(TileGate));
-        if (!mats.empty()) std::memcpy(host + b_tg, mats.data(), mats.size() * sizeof(float4));
-        if (!perms.empty()) std::memcpy(host + b_tg + b_m, perms.data(), perms.size() * sizeof(int32_t));
+        write(host);
         dev = (char*)s->plan_buf;
         rc = bs_cuda_check(s, cudaMemcpyAsync(dev, host, (size_t)b_all, cudaMemcpyHostToDevice, s->stream), "plan upload");
         bs_stage_done(s);
         if (rc) return rc;
+    }
+    if (!plan.sweeps.empty()) {
+        const int dim = 1 << n;
+        const size_t base = (size_t)2 * sizeof(float4) * ((size_t)1 << kSmallTileBits) + (size_t)3 * dim * sizeof(double);
+        const size_t stage = mats.size() * sizeof(float4) + tg.size() * sizeof(TileGate) +
+                             (perms.size() + 3) / 4 * 4 * sizeof(int32_t) + plan.sweeps.size() * sizeof(SmallSweep);
+        constexpr size_t kClusterCap = 216 * 1024;
+        const bool staged = base + stage <= kClusterCap;
+        auto kern = kmax <= 2 ? (staged ? k_small_cluster<2, true> : k_small_cluster<2, false>)
+                              : (staged ? k_small_cluster<4, true> : k_small_cluster<4, false>);
+        static bool attr_set[64] = {false};
+        if (!attr_set[s->device & 63]) {
+            cudaFuncSetAttribute(k_small_cluster<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kClusterCap);
+            cudaFuncSetAttribute(k_small_cluster<2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kClusterCap);
+            cudaFuncSetAttribute(k_small_cluster<4, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kClusterCap);
+            cudaFuncSetAttribute(k_small_cluster<4, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kClusterCap);
+            attr_set[s->device & 63] = true;
+        }
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = 1u << (n - kSmallTileBits);
+        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(1u << (n - kSmallTileBits));
+        cfg.blockDim = dim3(256);
+        cfg.dynamicSmemBytes = staged ? base + stage : base;
+        cfg.stream = s->stream;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, (double2*)s->state, n, (const SmallSweep*)(dev + b_tg + b_m + b_p),
+                                                 (int)plan.sweeps.size(), (const TileGate*)dev, (int)tg.size(),
+                                                 (const float4*)(dev + b_tg), (int)mats.size(), (const int32_t*)(dev + b_tg + b_m),
+                                                 (int)perms.size(), dprobs, shots, seed, dsamples, (volatile int64_t*)done, ticket,
+                                                 io ? io->dtimes : (int64_t*)nullptr);
+        rc = bs_cuda_check(s, e, "small run");
+        if (rc) return rc;
+        s->stats.kernel_launches++;
+        s->stats.sweeps++;
+        s->stats.gates += (int64_t)tg.size();
+        s->stats.bytes_moved += 16.0 * (double)dim;
+        return bs_cuda_check(s, cudaGetLastError(), "small run");
     }
     // the tile (afterwards two arrays of the sampler, whole 32-element chunks), then the probabilities,
     // then (staged) the matrices and permutations
