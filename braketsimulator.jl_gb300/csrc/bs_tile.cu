@@ -153,9 +153,49 @@ __device__ void tile_dense(float4* sm, int T, const TileGate& g, const float4* _
     }
 }
 
+// X on tile bit t under NC in-tile controls (CNOT, CCNOT; TileGate.npar 1 of kind 2): the pairs that meet
+// the controls are enumerated directly and change places.  The general monomial pass walks all pairs,
+// skips half of its lanes at a control and looks up rows and phases (1400 SM cycles a pass of a full
+// tile against 600).
+template <int NC, bool SW>
+__device__ __forceinline__ void tile_cx(float4* sm, int T, const TileGate& g) {
+    int pos[NC + 1];
+    uint32_t m = g.lc_mask;
+    pos[0] = g.tbit[0];
+#pragma unroll
+    for (int q = 1; q <= NC; q++) {
+        pos[q] = __ffs((int)m) - 1;
+        m &= m - 1;
+    }
+#pragma unroll
+    for (int a = 0; a <= NC; a++)
+#pragma unroll
+        for (int b = a + 1; b <= NC; b++)
+            if (pos[b] < pos[a]) { int t = pos[a]; pos[a] = pos[b]; pos[b] = t; }
+    const int bt = 1 << g.tbit[0], on = (int)g.lc_val, n = 1 << (T - 1 - NC);
+#pragma unroll 4
+    for (int gr = threadIdx.x; gr < n; gr += blockDim.x) {
+        int j = gr;
+#pragma unroll
+        for (int q = 0; q <= NC; q++) j = insert0(j, pos[q]);
+        const int ia = sx<SW>(j | on), ib = sx<SW>(j | on | bt);
+        const float4 a = sm[ia], b = sm[ib];
+        sm[ia] = b;
+        sm[ib] = a;
+    }
+}
+
 // monomial gate: column c goes to row perm[2c] with phase i^perm[2c+1]
 template <int K, bool SW = false, bool SM = false>
 __device__ void tile_monomial(float4* sm, int T, const TileGate& g, const int32_t* __restrict__ perms) {
+    if (K == 1 && g.npar == 1) {   // uniform
+        switch (__popc(g.lc_mask)) {
+            case 0: tile_cx<0, SW>(sm, T, g); return;
+            case 1: tile_cx<1, SW>(sm, T, g); return;
+            case 2: tile_cx<2, SW>(sm, T, g); return;
+            default: break;
+        }
+    }
     constexpr int D = 1 << K;
     int pos[K];
 #pragma unroll
@@ -208,36 +248,50 @@ __device__ void tile_diag(float4* sm, int T, int L, const TileGate& g, const flo
     const int nt = 1 << T, lowmask = (1 << L) - 1;
     const float4* m = mats + g.mat_off;
     // pattern bit q: tile bit tbit[q] (32-bit), or a CTA constant for a bit outside the tile;
-    // gates with more than BS_TILE_MAXK bits take the pattern from the 64-bit global index
-    const bool fast = g.k <= BS_TILE_MAXK;
-    int cst = 0, nk = 0;
-    uint32_t enc = 0;   // per in-tile pattern bit: tile position (5 bits) | q << 5, one byte each
-    if (fast)
+    // gates with more than BS_TILE_MAXK bits take the pattern from the 64-bit global index.  The number of
+    // threads is a power of two.
+    auto apply = [&](int js, int di) {
+        const float4 d = ldro<SM>(m + di);
+        if (d.y == 0.f && d.w == 0.f) {
+            if (d.z == 0.f && d.x == 1.f) return;
+            if (d.z == 0.f && d.x == -1.f) { sm[js] = c4f(cmul_ipow(f4c(sm[js]), 2)); return; }
+            if (d.x == 0.f && d.z == 1.f) { sm[js] = c4f(cmul_ipow(f4c(sm[js]), 1)); return; }
+            if (d.x == 0.f && d.z == -1.f) { sm[js] = c4f(cmul_ipow(f4c(sm[js]), 3)); return; }
+        }
+        sm[js] = c4f(cmul(f4m(d), f4c(sm[js])));
+    };
+    const uint32_t lcm = g.lc_mask, lcv = g.lc_val;
+    if (g.k <= BS_TILE_MAXK) {
+        int cst = 0;
+        uint32_t enc = 0;   // per in-tile pattern bit: tile position (5 bits) | q << 5, one byte each
+        int nk = 0;
         for (int q = 0; q < g.k; q++) {
             if (g.tbit[q] >= 0) enc |= (uint32_t)(g.tbit[q] | (q << 5)) << (8 * nk++);
             else cst |= (int)((base >> g.gbit[q]) & 1) << q;
         }
-    for (int j = threadIdx.x; j < nt; j += blockDim.x) {
-        if ((j & (int)g.lc_mask) != (int)g.lc_val) continue;
-        const int js = sx<SW>(j);
-        int di = cst;
-        if (fast) {
+        auto pattern = [&](int j) {
+            int di = 0;
             for (int u = 0; u < nk; u++) {
                 const uint32_t b = (enc >> (8 * u)) & 255u;
                 di |= ((j >> (b & 31u)) & 1) << (b >> 5);
             }
-        } else {
+            return di;
+        };
+        // the pattern of a thread's positions: its own bits once, the bits above them (uniform) each time
+        const int mine = cst | pattern((int)threadIdx.x);
+        for (int j0 = 0; j0 < nt; j0 += blockDim.x) {
+            const int j = j0 | (int)threadIdx.x;
+            if (j >= nt || (j & (int)lcm) != (int)lcv) continue;
+            apply(sx<SW>(j), mine | pattern(j0));
+        }
+    } else {
+        for (int j = threadIdx.x; j < nt; j += blockDim.x) {
+            if ((j & (int)lcm) != (int)lcv) continue;
             const int64_t gi = base | ((int64_t)off_tab[j >> L] << osh) | (int64_t)(j & lowmask);
+            int di = 0;
             for (int q = 0; q < g.k; q++) di |= (int)((gi >> g.gbit[q]) & 1) << q;
+            apply(sx<SW>(j), di);
         }
-        float4 d = ldro<SM>(m + di);
-        if (d.y == 0.f && d.w == 0.f) {
-            if (d.z == 0.f && d.x == 1.f) continue;
-            if (d.z == 0.f && d.x == -1.f) { sm[js] = c4f(cmul_ipow(f4c(sm[js]), 2)); continue; }
-            if (d.x == 0.f && d.z == 1.f) { sm[js] = c4f(cmul_ipow(f4c(sm[js]), 1)); continue; }
-            if (d.x == 0.f && d.z == -1.f) { sm[js] = c4f(cmul_ipow(f4c(sm[js]), 3)); continue; }
-        }
-        sm[js] = c4f(cmul(f4m(d), f4c(sm[js])));
     }
 }
 
@@ -1114,6 +1168,10 @@ inline float4 to_cff(double re, double im) {
 
 namespace {
 
+bool plain_x(const HostGate& h) {
+    return h.kind == 2 && h.k == 1 && h.perm.size() == 4 && h.perm[0] == 1 && h.perm[1] == 0 && h.perm[2] == 0 && h.perm[3] == 0;
+}
+
 bool plain_cz(const HostGate& h) {
     return h.kind == 1 && h.k == 1 && h.mat.size() == 4 && h.mat[0] == 1.0 && h.mat[1] == 0.0 && h.mat[2] == -1.0 &&
            h.mat[3] == 0.0 && __builtin_popcountll(h.cmask) == 1 && h.cval == h.cmask;
@@ -1555,6 +1613,7 @@ int bs_run_sweeps(bs_sim* s, const std::vector<Sweep>& sweeps) {
                 for (int i = 0; i < (1 << hg.k); i++) mats.push_back(to_cff(hg.mat[2 * i], hg.mat[2 * i + 1]));
             } else {
                 perms.insert(perms.end(), hg.perm.begin(), hg.perm.end());
+                if (plain_x(hg)) t.npar = 1;
             }
             if (hg.kind != 1) ln.kmax = std::max(ln.kmax, hg.k);
             if (hg.kind == 0 && hg.k == 1) t.npar = bs_class_2x2(hg);
@@ -2129,6 +2188,7 @@ int bs_small_pack(const bs_sim* s, const std::vector<Sweep>& sweeps, SmallPlan& 
             } else {
                 perms.insert(perms.end(), hg.perm.begin(), hg.perm.end());
                 kmax = std::max(kmax, hg.k);
+                if (plain_x(hg)) t.npar = 1;
             }
             tg.push_back(t);
         }
