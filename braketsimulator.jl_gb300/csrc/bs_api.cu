@@ -74,12 +74,12 @@ struct MapStage {
     char* h = nullptr;
     char* d = nullptr;
     bool tried = false;
-    int64_t ticket = 0;   // bs_run_small calls of this thread: the kernel writes the call's ticket when done
     ~MapStage() {
         if (h) cudaFreeHost(h);
     }
 };
 thread_local MapStage t_map;
+std::atomic<int64_t> g_ticket{0};   // tickets are never used twice
 bool map_stage() {
     if (t_map.h) return true;
     if (t_map.tried) return false;
@@ -88,11 +88,37 @@ bool map_stage() {
     void* d = nullptr;
     if (cudaHostAlloc(&h, kOutStage, cudaHostAllocMapped) != cudaSuccess) { cudaGetLastError(); return false; }
     if (cudaHostGetDevicePointer(&d, h, 0) != cudaSuccess) { cudaGetLastError(); cudaFreeHost(h); return false; }
+    std::memset(h, 0, 256);   // the driver hands out freed blocks again, with an earlier thread's ticket in them
     t_map.h = (char*)h;
     t_map.d = (char*)d;
     return true;
 }
 }  // namespace
+
+MapSlot bs_map_slot(size_t bytes) {
+    MapSlot m;
+    if (256 + bytes > kOutStage || !map_stage()) return m;
+    m.h = t_map.h + 256;
+    m.d = t_map.d + 256;
+    m.word = reinterpret_cast<volatile int64_t*>(t_map.h);
+    m.dword = reinterpret_cast<int64_t*>(t_map.d);
+    m.ticket = ++g_ticket;
+    return m;
+}
+
+int bs_wait_ticket(bs_sim* s, const MapSlot& m, const char* what) {
+    const auto t0 = std::chrono::steady_clock::now();
+    for (uint32_t it = 0;; it++) {
+        if (*m.word == m.ticket) {
+            std::atomic_thread_fence(std::memory_order_acquire);
+            return BS_OK;
+        }
+        if ((it & 1023u) == 1023u && std::chrono::steady_clock::now() - t0 > std::chrono::seconds(2)) break;
+    }
+    const int rc = bs_cuda_check(s, cudaStreamSynchronize(s->stream), what);
+    std::atomic_thread_fence(std::memory_order_acquire);
+    return rc;
+}
 
 int bs_copy_out(bs_sim* s, void* host, const void* dev, size_t bytes, const char* what) {
     if (s->capturing)   // the graph owner's buffer: enqueue only
@@ -631,7 +657,7 @@ int bs_run_small(bs_sim* s, const bs_op* ops, int64_t n_ops, int64_t shots, uint
     SmallIO io{};
     if (mapped) {
         ddone = (int64_t*)t_map.d;
-        ticket = ++t_map.ticket;
+        ticket = ++g_ticket;
         dprobs = (double*)(t_map.d + 256);
         dsamp = (int64_t*)(t_map.d + 256 + pb);
         io.hplan = t_map.h + 256 + pb + sb;
@@ -672,20 +698,12 @@ int bs_run_small(bs_sim* s, const bs_op* ops, int64_t n_ops, int64_t shots, uint
     }
     // Wait for the kernel's completion word rather than synchronising the stream (a round trip through
     // the driver that costs more than the kernel): the kernel writes the ticket after every result is
-    // visible to the host.  A ticket that has not arrived after 2 s (a failed kernel) falls back to the
-    // stream synchronisation, which reports the error.
-    volatile int64_t* word = reinterpret_cast<volatile int64_t*>(t_map.h);
-    const auto t0 = std::chrono::steady_clock::now();
-    bool seen = false;
-    for (uint32_t it = 0;; it++) {
-        if (*word == ticket) { seen = true; break; }
-        if ((it & 1023u) == 1023u && std::chrono::steady_clock::now() - t0 > std::chrono::seconds(2)) break;
-    }
-    std::atomic_thread_fence(std::memory_order_acquire);
-    if (!seen) {
-        rc = bs_cuda_check(s, cudaStreamSynchronize(s->stream), "small run");
-        if (rc) return rc;
-    }
+    // visible to the host.
+    MapSlot slot;
+    slot.word = reinterpret_cast<volatile int64_t*>(t_map.h);
+    slot.ticket = ticket;
+    rc = bs_wait_ticket(s, slot, "small run");
+    if (rc) return rc;
     if (probs_out) std::memcpy(probs_out, t_map.h + 256, (size_t)dim * 8);
     if (shots > 0) std::memcpy(samples_out, t_map.h + 256 + pb, (size_t)shots * 8);
     // device time: the kernel's own start and end stamps (no events on this path)

@@ -325,13 +325,15 @@ void small_image(char* img, const SmallLayout& L, const std::vector<BCirc>& bc, 
 
 uint64_t circuit_seed(uint64_t seed, int c) { return seed ^ ((uint64_t)c * 0x9E3779B97F4A7C15ULL); }
 
-// Handles (one stream each) that run the larger circuits side by side (BS_BATCH_STREAMS, default 4, at
-// most 64).  On the 512-circuit benchmark batch 4, 16 and 32 streams replay in the same 1.30-1.31 s:
-// the largest circuits' sweeps, which fill the GPU on their own, set the time.
+// Handles (one stream each) that run the larger circuits side by side (BS_BATCH_STREAMS, default 8, at
+// most 64).  Replays of a captured batch do not depend on it (4, 16 and 32 took the same time on 512
+// circuits of up to 26 qubits: the largest circuits' sweeps fill the GPU on their own); a batch run at
+// once plans each handle's next circuit on its own thread (48 circuits of 12 to 22 qubits: 18.7 ms on 4,
+// 17.2 on 8, 19.1 on 16).
 int batch_pool_size(size_t n_large) {
     static const int cap = [] {
         const char* v = getenv("BS_BATCH_STREAMS");
-        const int x = v ? atoi(v) : 4;
+        const int x = v ? atoi(v) : 8;
         return std::max(1, std::min(64, x));
     }();
     return (int)std::min<size_t>(n_large, (size_t)cap);

@@ -14,7 +14,7 @@
 //   kind 0: dense 2^k x 2^k on tile-local bits tbit[0..k-1] (matrix bit j <-> tbit[j]); k = 1: npar is
 //           the matrix class (bs_class_2x2)
 //   kind 1: diagonal 2^k entries selected by global bits gbit[0..k-1]
-//   kind 2: monomial (one unit-modulus phase i^p per column) on tile-local bits
+//   kind 2: monomial (one unit-modulus phase i^p per column) on tile-local bits; npar 1: X
 //   kind 3: a run of CZ gates applied as one parity phase (npar, pshift, pmask)
 //   kind 4: fused dense unitary on 5 tile-local bits gbit[0..4] (matrix bit j <-> gbit[j]),
 //           applied on the tensor cores from the bf16 digit slices at tc_off (48 KiB blocks)
@@ -185,6 +185,20 @@ int bs_cuda_check(bs_sim* s, cudaError_t e, const char* what);
 // Device-to-host copy of a result, stream synchronised; small ones land in a pinned per-thread
 // buffer first (a pageable copy takes a staged driver path).  During graph capture: enqueue only.
 int bs_copy_out(bs_sim* s, void* host, const void* dev, size_t bytes, const char* what);
+// This thread's pinned host memory mapped into the device's address space, for a result of up to `bytes`
+// that a kernel writes and a ticket it writes after it (null: not available, or too large).  One result
+// at a time: the call that takes it waits for its ticket (bs_wait_ticket) before it returns.
+struct MapSlot {
+    char* h = nullptr;           // result, host and device address
+    char* d = nullptr;
+    volatile int64_t* word = nullptr;   // ticket word, host address
+    int64_t* dword = nullptr;           // and device address
+    int64_t ticket = 0;
+};
+MapSlot bs_map_slot(size_t bytes);
+// Polls for the slot's ticket; after 2 s (a failed or very long kernel) synchronises the stream, which
+// reports the error.
+int bs_wait_ticket(bs_sim* s, const MapSlot& m, const char* what);
 int bs_ensure_scratch(bs_sim* s, int64_t bytes);
 int bs_ensure_plan(bs_sim* s, int64_t bytes);
 // The counter with which the last block of an expectation is found (zero between calls), allocated on first use.

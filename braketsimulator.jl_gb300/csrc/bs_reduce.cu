@@ -97,16 +97,23 @@ __device__ __forceinline__ void pauli_accumulate(ffsum (&acc)[NT], const TermSet
 // Last block of the call (its launches' blocks add up to last_total in *done): every partial is there,
 // so its warps form the results, one slot each at a time (FP64 sums with compensated leaves), and the
 // counter goes back to zero.  A launch fewer per call than a separate pass over the partials, which
-// took 2.5 to 5 us of device time.
-__device__ void finish_partials(double* partial, int nblocks, int n_slots, unsigned* done, unsigned last_total) {
+// took 2.5 to 5 us of device time; with the results and a ticket in mapped memory the host polls,
+// instead of a copy and a stream synchronisation.
+struct Finish {
+    double* out;            // results (device, or host memory mapped into its address space)
+    unsigned* done;
+    unsigned last_total;
+    volatile int64_t* word; // ticket word of a waiting host (null: none)
+    int64_t ticket;
+};
+__device__ void finish_partials(double* partial, int nblocks, int n_slots, const Finish& f) {
     __shared__ bool s_last;
     __threadfence();
     __syncthreads();
-    if (threadIdx.x == 0) s_last = atomicAdd(done, 1u) + 1u == last_total;
+    if (threadIdx.x == 0) s_last = atomicAdd(f.done, 1u) + 1u == f.last_total;
     __syncthreads();
     if (!s_last) return;
     __threadfence();
-    double* out = partial + (int64_t)nblocks * n_slots;
     const int lane = threadIdx.x & 31;
     for (int slot = threadIdx.x >> 5; slot < n_slots; slot += kRThreads / 32) {
         double s = 0.0, c = 0.0;
@@ -117,9 +124,13 @@ __device__ void finish_partials(double* partial, int nblocks, int n_slots, unsig
             s = t;
         }
         for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-        if (lane == 0) out[slot] = s;
+        if (lane == 0) f.out[slot] = s;
     }
-    if (threadIdx.x == 0) *done = 0;
+    if (threadIdx.x == 0) *f.done = 0;
+    if (!f.word) return;
+    __threadfence_system();
+    __syncthreads();
+    if (threadIdx.x == 0) *f.word = f.ticket;
 }
 
 // SV Pauli terms sharing flip mask xm.  Pairs (i, i^xm) with the top bit of xm clear contribute
@@ -132,7 +143,7 @@ __device__ void finish_partials(double* partial, int nblocks, int n_slots, unsig
 template <bool C64, bool FLIP, bool RE, bool IM, bool ONE>
 __global__ void __launch_bounds__(kRThreads, 4) k_pauli_sv(const typename Elem<C64>::T* __restrict__ psi, int64_t n, uint64_t xm,
                                                            TermSet ts, double* __restrict__ partial, int n_slots,
-                                                           unsigned* __restrict__ done, unsigned last_total) {
+                                                           Finish fin) {
     constexpr int U = (FLIP ? 4 : 8) / (ONE ? 1 : 2);   // positions in flight
     constexpr int NT = ONE ? 1 : kMaxTermsPerPass;
     ffsum acc[NT];
@@ -186,14 +197,14 @@ __global__ void __launch_bounds__(kRThreads, 4) k_pauli_sv(const typename Elem<C
         if (NT > 1 && t >= ts.nt) break;
         block_sum_store((FLIP ? 2.0 : 1.0) * ff2d(acc[t].h, acc[t].l), partial, (int64_t)blockIdx.x * n_slots + ts.slot[t]);
     }
-    finish_partials(partial, gridDim.x, n_slots, done, last_total);
+    finish_partials(partial, gridDim.x, n_slots, fin);
 }
 
 // DM Pauli terms: E = sum_a Re(P[a, a^xm] S[a, a^xm]), S[r, c] at r + c*dim.
 template <bool C64>
 __global__ void __launch_bounds__(kRThreads) k_pauli_dm(const typename Elem<C64>::T* __restrict__ S, int64_t dim,
                                                         uint64_t xm, TermSet ts, double* __restrict__ partial, int n_slots,
-                                                        unsigned* __restrict__ done, unsigned last_total) {
+                                                        Finish fin) {
     ffsum acc[kMaxTermsPerPass];
     for (int t = 0; t < kMaxTermsPerPass; t++) acc[t] = {0.f, 0.f};
     for (int64_t a = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; a < dim; a += (int64_t)gridDim.x * blockDim.x) {
@@ -202,7 +213,7 @@ __global__ void __launch_bounds__(kRThreads) k_pauli_dm(const typename Elem<C64>
     }
     for (int t = 0; t < ts.nt; t++)
         block_sum_store(ff2d(acc[t].h, acc[t].l), partial, (int64_t)blockIdx.x * n_slots + ts.slot[t]);
-    finish_partials(partial, gridDim.x, n_slots, done, last_total);
+    finish_partials(partial, gridDim.x, n_slots, fin);
 }
 
 __global__ void k_sum_partials(const double* __restrict__ partial, int nblocks, int n_slots, double* __restrict__ out) {
@@ -402,11 +413,11 @@ int grid_for(int64_t work) {
 
 template <bool C64>
 void launch_pauli(bs_sim* s, int nb, int64_t dim, uint64_t xm, const TermSet& set, double* partial, int n_terms,
-                  unsigned* done, unsigned last_total) {
+                  const Finish& fin) {
     using T = typename Elem<C64>::T;
     const T* st = (const T*)s->state;
     if (s->kind != BS_KIND_SV) {
-        k_pauli_dm<C64><<<nb, kRThreads, 0, s->stream>>>(st, dim, xm, set, partial, n_terms, done, last_total);
+        k_pauli_dm<C64><<<nb, kRThreads, 0, s->stream>>>(st, dim, xm, set, partial, n_terms, fin);
         return;
     }
     int parts = 0;   // bit 0: a term needs the real part, bit 1: the imaginary part
@@ -415,7 +426,7 @@ void launch_pauli(bs_sim* s, int nb, int64_t dim, uint64_t xm, const TermSet& se
     if (set.nt == 1) kern = !xm ? k_pauli_sv<C64, false, true, false, true>
                           : parts == 1 ? k_pauli_sv<C64, true, true, false, true> : k_pauli_sv<C64, true, false, true, true>;
     else if (!xm) kern = k_pauli_sv<C64, false, true, false, false>;
-    kern<<<nb, kRThreads, 0, s->stream>>>(st, dim, xm, set, partial, n_terms, done, last_total);
+    kern<<<nb, kRThreads, 0, s->stream>>>(st, dim, xm, set, partial, n_terms, fin);
 }
 
 }  // namespace
@@ -509,9 +520,10 @@ int bs_expectation_pauli(bs_sim* s, int n_terms, const uint64_t* xmask, const ui
     if (rc) return rc;
     double* partial = (double*)s->scratch;
     double* res = partial + (int64_t)nb * n_terms;
-    unsigned* done = s->counter;
     unsigned launches = 0;
     for (auto& kv : groups) launches += (unsigned)((kv.second.size() + kMaxTermsPerPass - 1) / kMaxTermsPerPass);
+    const MapSlot slot = s->capturing ? MapSlot{} : bs_map_slot((size_t)n_terms * 8);
+    const Finish fin{slot.h ? (double*)slot.d : res, s->counter, launches * (unsigned)nb, slot.dword, slot.ticket};
     for (auto& kv : groups) {
         const std::vector<int>& ts = kv.second;
         for (size_t c0 = 0; c0 < ts.size(); c0 += kMaxTermsPerPass) {
@@ -523,15 +535,20 @@ int bs_expectation_pauli(bs_sim* s, int n_terms, const uint64_t* xmask, const ui
                 set.ph[j] = ph[t];
                 set.slot[j] = t;
             }
-            if (s->precision == BS_PREC_C64) launch_pauli<true>(s, nb, dim, kv.first, set, partial, n_terms, done, launches * (unsigned)nb);
-            else launch_pauli<false>(s, nb, dim, kv.first, set, partial, n_terms, done, launches * (unsigned)nb);
+            if (s->precision == BS_PREC_C64) launch_pauli<true>(s, nb, dim, kv.first, set, partial, n_terms, fin);
+            else launch_pauli<false>(s, nb, dim, kv.first, set, partial, n_terms, fin);
         }
     }
     rc = bs_cuda_check(s, cudaGetLastError(), "expectation");
     if (rc) return rc;
     if (s->capturing && coeffs) return bs_fail(s, BS_ERR_INVALID_ARG, "coefficients are applied after a captured graph runs");
     // during capture out is the graph owner's pinned buffer, filled on every replay
-    rc = bs_copy_out(s, out, res, (size_t)n_terms * 8, "expectation");
+    if (slot.h) {
+        rc = bs_wait_ticket(s, slot, "expectation");
+        if (!rc) std::memcpy(out, slot.h, (size_t)n_terms * 8);
+    } else {
+        rc = bs_copy_out(s, out, res, (size_t)n_terms * 8, "expectation");
+    }
     if (rc || s->capturing) return rc;
     if (coeffs)
         for (int t = 0; t < n_terms; t++) out[t] *= coeffs[t];
