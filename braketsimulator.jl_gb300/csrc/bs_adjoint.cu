@@ -408,26 +408,17 @@ __global__ void __launch_bounds__(kSweepThreads, C64 ? 2 : 1)
     S* sl = sp + nt;
     float2* vt = reinterpret_cast<float2*>(sl + nt);                        // kSweepPer x kSweepThreads
     int64_t* off_tab = reinterpret_cast<int64_t*>(vt + kSweepPer * kSweepThreads);
-    __shared__ int64_t s_base;
     __shared__ double red[kRotMax][kSweepThreads / 32];
     __shared__ double red_w[kRotMax];
     __shared__ int red_slot[kRotMax];
-    const int64_t tile = tile0 + (int64_t)blockIdx.x;
+    const int64_t base = bs_tile_base(d, tile0 + (int64_t)blockIdx.x);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    if (tid == 0) {
-        int64_t base = 0;
-        int src = 0;
-        for (int bit = 0; bit < d.n_bits; bit++)
-            if (!((d.tile_mask >> bit) & 1ULL)) { base |= ((tile >> src) & 1LL) << bit; src++; }
-        s_base = base;
-    }
     for (int i = tid; i < (1 << H); i += kSweepThreads) {
         int64_t o = 0;
         for (int j = 0; j < H; j++) if ((i >> j) & 1) o |= 1LL << d.hi_bits[j];
         off_tab[i] = o;
     }
     __syncthreads();
-    const int64_t base = s_base;
     const int lowmask = (1 << L) - 1;
     // tile loads: four positions (eight loads) per thread in flight at a time (tiles <= 2^12)
 #pragma unroll
@@ -1105,13 +1096,8 @@ extern "C" int bs_adjoint_gradient(bs_sim* s, const bs_op* ops, int64_t n_ops, c
         if (sweep_restore[sw] >= 0)
             cudaMemcpyAsync(s->state, ckpt(sweep_restore[sw]), state_bytes, cudaMemcpyDeviceToDevice, s->stream);
         SweepDesc d{};
-        d.n_bits = n_bits;
-        d.T = T;
-        d.L = L;
+        bs_tile_geometry(d, n_bits, L, sweeps_hi[sw]);
         d.n_gates = (int)(sweep_first[sw + 1] - sweep_first[sw]);
-        uint64_t tm = (1ULL << L) - 1;
-        for (int i = 0; i < H; i++) { d.hi_bits[i] = sweeps_hi[sw][(size_t)i]; tm |= 1ULL << sweeps_hi[sw][(size_t)i]; }
-        d.tile_mask = tm;
         d.mats = d_m;
         d.perms = d_p;
         for (int64_t t0 = 0; t0 < ntiles; t0 += (1LL << 30)) {

@@ -70,6 +70,7 @@ struct SweepDesc {
     int32_t n_gates;
     int32_t hi_bits[BS_TILE_MAX_BITS];
     uint64_t tile_mask;
+    int8_t out_bits[32];        // the endian bits outside the tile, ascending: the tile number's bits (63: none)
     const TileGate* gates;      // device
     const float4* mats;         // device, complex float-float entries (rh, rl, ih, il)
     const int32_t* perms;       // device
@@ -78,6 +79,18 @@ struct SweepDesc {
     int32_t n_rops;
     int* err;                   // device flag: a bounded tensor-core wait gave up
 };
+
+// Fills hi_bits, tile_mask and out_bits of a sweep over n_bits with L low tile bits and the bits hi above.
+inline void bs_tile_geometry(SweepDesc& d, int n_bits, int L, const std::vector<int>& hi) {
+    d.n_bits = n_bits;
+    d.L = L;
+    d.T = L + (int)hi.size();
+    d.tile_mask = (1ULL << L) - 1;
+    for (size_t i = 0; i < hi.size(); i++) { d.hi_bits[i] = hi[i]; d.tile_mask |= 1ULL << hi[i]; }
+    int k = 0;
+    for (int b = 0; b < n_bits && k < 32; b++) if (!((d.tile_mask >> b) & 1ULL)) d.out_bits[k++] = (int8_t)b;
+    while (k < 32) d.out_bits[k++] = 63;
+}
 
 struct HostGate {                // a gate after lowering to the canonical convention
     int kind;                    // 0 dense, 1 diagonal, 2 monomial, 4 fused 5-bit unitary,
@@ -209,6 +222,17 @@ void bs_stage_done(bs_sim* s);
 // Release the capture arena (the graph that read it is gone).
 void bs_arena_release(bs_sim* s);
 int bs_vec_bits(const bs_sim* s);
+
+#ifdef __CUDACC__
+// Base index of a tile, by a whole warp (the same value in every lane): lane i places the tile number's
+// bit i.  (One thread walking the vector's bits held up the whole CTA for 600 cycles at its start.)
+__device__ __forceinline__ int64_t bs_tile_base(const SweepDesc& d, int64_t tile) {
+    const int lane = threadIdx.x & 31, b = d.out_bits[lane];
+    const uint64_t v = (b < 63 && ((tile >> lane) & 1)) ? 1ULL << b : 0ULL;
+    const uint32_t lo = __reduce_or_sync(0xffffffffu, (uint32_t)v), hi = __reduce_or_sync(0xffffffffu, (uint32_t)(v >> 32));
+    return (int64_t)(((uint64_t)hi << 32) | lo);
+}
+#endif
 
 // ---- lowering (bs_plan.cpp)
 // Convert a gate (reference convention flags) into canonical HostGate(s) on the

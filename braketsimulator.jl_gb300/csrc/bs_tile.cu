@@ -375,40 +375,30 @@ __device__ void tile_kraus_ref_lr(float4* sm, int T, int L, const TileGate& g, c
 // KMAX: widest dense/monomial gate of the sweep (2 or 4); narrow sweeps get a
 // kernel with fewer live registers and therefore more resident warps.
 template <int KMAX, int NT>
-__global__ void __launch_bounds__(NT) k_tile_sweep(double2* __restrict__ psi, SweepDesc d, int64_t tile0) {
+__global__ void __launch_bounds__(NT, NT == 256 && KMAX == 2 ? 3 : 1) k_tile_sweep(double2* __restrict__ psi, SweepDesc d, int64_t tile0) {
     extern __shared__ float4 smem[];
     const int T = d.T, L = d.L, H = T - L;
     const int nt = 1 << T;
     int64_t* off_tab = reinterpret_cast<int64_t*>(smem + nt);
-    __shared__ int64_t s_base;
-    const int64_t tile = tile0 + (int64_t)blockIdx.x;
-    if (threadIdx.x == 0) {
-        int64_t base = 0;
-        int src = 0;
-        for (int bit = 0; bit < d.n_bits; bit++)
-            if (!((d.tile_mask >> bit) & 1ULL)) { base |= ((tile >> src) & 1LL) << bit; src++; }
-        s_base = base;
-    }
+    const int64_t base = bs_tile_base(d, tile0 + (int64_t)blockIdx.x);
     for (int i = threadIdx.x; i < (1 << H); i += blockDim.x) {
         int64_t o = 0;
         for (int j = 0; j < H; j++) if ((i >> j) & 1) o |= 1LL << d.hi_bits[j];
         off_tab[i] = o;
     }
     __syncthreads();
-    const int64_t base = s_base;
     const int lowmask = (1 << L) - 1;
-    // tile load: eight loads per thread in flight at a time (tiles are at most 2^12 amplitudes)
+    // tile load: all of a thread's loads in flight (tiles are at most 2^12 amplitudes)
+    {
+        double2 x[4096 / NT];
 #pragma unroll
-    for (int r = 0; r < 4096 / NT; r += 8) {
-        double2 x[8];
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-            const int j = (r + i) * NT + (int)threadIdx.x;
+        for (int i = 0; i < 4096 / NT; i++) {
+            const int j = i * NT + (int)threadIdx.x;
             if (j < nt) x[i] = __ldcs(psi + (base | off_tab[j >> L] | (int64_t)(j & lowmask)));
         }
 #pragma unroll
-        for (int i = 0; i < 8; i++) {
-            const int j = (r + i) * NT + (int)threadIdx.x;
+        for (int i = 0; i < 4096 / NT; i++) {
+            const int j = i * NT + (int)threadIdx.x;
             if (j < nt) smem[j] = c4f(load_c128(x[i]));
         }
     }
@@ -510,15 +500,6 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_tile_sweep_tc(double2* __rest
         else s_offb[threadIdx.x - 8] = (uint32_t)(o >> L);
     }
     if (warp == 0) tc::tmem_alloc(tc::su32(&s_tmem));
-    // lane i holds the place of the tile number's bit i in the vector index: the i-th bit outside the tile
-    int out_bit = 63;
-    for (int bit = 0, src = 0; bit < d.n_bits; bit++)
-        if (!((d.tile_mask >> bit) & 1ULL)) { if (src == lane) out_bit = bit; src++; }
-    auto base_of = [&](int64_t tile) {
-        const uint64_t v = (out_bit < 63 && ((tile >> lane) & 1)) ? 1ULL << out_bit : 0ULL;
-        const uint32_t lo = __reduce_or_sync(0xffffffffu, (uint32_t)v), hi = __reduce_or_sync(0xffffffffu, (uint32_t)(v >> 32));
-        return (int64_t)(((uint64_t)hi << 32) | lo);
-    };
     tc::fence_before();
     __syncthreads();
     tc::fence_after();
@@ -532,7 +513,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_tile_sweep_tc(double2* __rest
         }
     };
     int64_t tile = tile0 + (int64_t)blockIdx.x;
-    int64_t base = base_of(tile);
+    int64_t base = bs_tile_base(d, tile);
     load(base);
     for (;;) {
         if (warp == kTcThreads / 32 - 1) {
@@ -621,7 +602,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_tile_sweep_tc(double2* __rest
             __stcs(psi + (here | ((int64_t)off32[j >> L] << L) | (int64_t)(j & lowmask)), store_c128(f4c(smem[tc::sw(j)])));
         }
         if (!more) break;
-        base = base_of(tile);
+        base = bs_tile_base(d, tile);
         load(base);
         __syncthreads();   // every thread has read the tile (and s_ntc) before the next one is written
     }
@@ -1028,26 +1009,17 @@ __global__ void __launch_bounds__(kC64Threads, KMAX == 2 ? 4 : 3) k_tile_sweep_c
     const int T = BLK ? 12 : d.T, L = BLK ? 5 : d.L, H = T - L;
     const int nt = 1 << T;
     int64_t* off_tab = reinterpret_cast<int64_t*>(smem + nt);
-    __shared__ int64_t s_base;
     __shared__ TileGate s_gates[kGateChunk];
     __shared__ __align__(16) RegOp s_ops[BLK ? kRegOps : 1];
-    const int64_t tile = tile0 + (int64_t)blockIdx.x;
+    const int64_t base = bs_tile_base(d, tile0 + (int64_t)blockIdx.x);
     const int tid = threadIdx.x;
     const bool staged = BLK && d.n_rops <= kRegOps;
-    if (tid == 0) {
-        int64_t base = 0;
-        int src = 0;
-        for (int bit = 0; bit < d.n_bits; bit++)
-            if (!((d.tile_mask >> bit) & 1ULL)) { base |= ((tile >> src) & 1LL) << bit; src++; }
-        s_base = base;
-    }
     for (int i = tid; i < (1 << H); i += kC64Threads) {
         int64_t o = 0;
         for (int j = 0; j < H; j++) if ((i >> j) & 1) o |= 1LL << d.hi_bits[j];
         off_tab[i] = o;
     }
     __syncthreads();
-    const int64_t base = s_base;
     const int lowmask = (1 << L) - 1;
     // The offset of a tile position is linear over XOR of its bits, so a full tile's 32 accesses of a
     // thread are one pointer plus uniform offsets (rows of 256 bytes), and constant swizzled positions.
@@ -1720,13 +1692,8 @@ int bs_run_sweeps(bs_sim* s, const std::vector<Sweep>& sweeps) {
             continue;
         }
         SweepDesc d{};
-        d.n_bits = n_bits;
-        d.T = T;
-        d.L = L;
+        bs_tile_geometry(d, n_bits, L, ln.hi);
         d.n_gates = ln.n_gates;
-        uint64_t tm = (L >= 64) ? ~0ULL : ((1ULL << L) - 1);
-        for (int i = 0; i < H; i++) { d.hi_bits[i] = ln.hi[(size_t)i]; tm |= 1ULL << ln.hi[(size_t)i]; }
-        d.tile_mask = tm;
         d.gates = d_tg + ln.gate0;
         d.mats = d_m;
         d.perms = d_p;
