@@ -1907,36 +1907,36 @@ __device__ __forceinline__ void small_shots(const double* sprob, int nt, double*
     }
 }
 
-// STAGED: the matrices and permutations are copied into shared memory first (one round trip to the
-// plan, which may live in host-mapped memory) instead of being read from the plan at every gate.
+// STAGED: gates, matrices and permutations are copied into shared memory first, in one go (one round
+// trip to the plan, which may live in host-mapped memory), instead of being read at every gate.
 template <int KMAX, bool STAGED>
-__global__ void __launch_bounds__(512) k_small_run(double2* __restrict__ psi, int n, const TileGate* __restrict__ gates,
-                                                   int ng, const float4* __restrict__ mats, int n_mats,
-                                                   const int32_t* __restrict__ perms, int n_perms,
-                                                   double* __restrict__ probs, int64_t shots, uint64_t seed,
-                                                   int64_t* __restrict__ samples, volatile int64_t* done, int64_t ticket,
-                                                   int64_t* times) {
+__device__ __forceinline__ void small_run(double2* __restrict__ psi, int n, const TileGate* gates, int ng, const float4* mats,
+                                          int n_mats, const int32_t* perms, int n_perms, double* __restrict__ probs,
+                                          int64_t shots, uint64_t seed, int64_t* __restrict__ samples, volatile int64_t* done,
+                                          int64_t ticket, int64_t* times) {
     if (times && threadIdx.x == 0) times[0] = globaltimer_ns();
     extern __shared__ float4 smem[];
-    __shared__ TileGate s_gates[kGateChunk];
+    __shared__ TileGate s_gates[STAGED ? 1 : kGateChunk];
     const int nt = 1 << n, nc32 = (nt + kChunk - 1) / kChunk * kChunk;
     // the probabilities, after the tile (or after the sampler's two arrays, which replace the tile),
-    // then the staged matrices and permutations
+    // then the staged plan
     double* sprob = reinterpret_cast<double*>(reinterpret_cast<char*>(smem) + max(nt * 16, 2 * nc32 * 8));
-    const float4* m_op = mats;
-    const int32_t* p_op = perms;
+    float4* ms = reinterpret_cast<float4*>(sprob + (nt + 1) / 2 * 2);
+    TileGate* gs = reinterpret_cast<TileGate*>(ms + n_mats);
+    int32_t* ps = reinterpret_cast<int32_t*>(gs + ng);
     if (STAGED) {
-        float4* ms = reinterpret_cast<float4*>(sprob + nt);
-        int32_t* ps = reinterpret_cast<int32_t*>(ms + n_mats);
         for (int j = threadIdx.x; j < n_mats; j += blockDim.x) ms[j] = mats[j];
+        const int* gw = reinterpret_cast<const int*>(gates);
+        for (int j = threadIdx.x; j < ng * (int)(sizeof(TileGate) / 4); j += blockDim.x) reinterpret_cast<int*>(gs)[j] = gw[j];
         for (int j = threadIdx.x; j < n_perms; j += blockDim.x) ps[j] = perms[j];
-        m_op = ms;
-        p_op = ps;   // read after the barrier that opens the first chunk of gates
     }
+    const float4* m_op = STAGED ? ms : mats;
+    const int32_t* p_op = STAGED ? ps : perms;
     for (int j = threadIdx.x; j < nt; j += blockDim.x) smem[j] = make_float4(j == 0 ? 1.f : 0.f, 0.f, 0.f, 0.f);
+    __syncthreads();
     for (int gi = 0; gi < ng; gi++) {
-        if (gi % kGateChunk == 0) stage_gates(s_gates, gates + gi, min(kGateChunk, ng - gi));   // one latency per 32 gates
-        const TileGate& g = s_gates[gi % kGateChunk];
+        if (!STAGED && gi % kGateChunk == 0) stage_gates(s_gates, gates + gi, min(kGateChunk, ng - gi));   // one latency per 32 gates
+        const TileGate& g = STAGED ? gs[gi] : s_gates[gi % kGateChunk];
         const int kind = g.kind, k = g.k;
         if (kind == 0) {
             if (k == 1) tile_dense<1, false, STAGED>(smem, n, g, m_op);
@@ -1974,6 +1974,33 @@ __global__ void __launch_bounds__(512) k_small_run(double2* __restrict__ psi, in
     small_shots(sprob, nt, reinterpret_cast<double*>(smem) /* the tile is no longer needed */, s_cdf, threadIdx.x, blockDim.x, shots,
                 seed, samples);
     small_run_done(done, ticket, times);
+}
+
+template <int KMAX, bool STAGED>
+__global__ void __launch_bounds__(512) k_small_run(double2* __restrict__ psi, int n, const TileGate* __restrict__ gates,
+                                                   int ng, const float4* __restrict__ mats, int n_mats,
+                                                   const int32_t* __restrict__ perms, int n_perms,
+                                                   double* __restrict__ probs, int64_t shots, uint64_t seed,
+                                                   int64_t* __restrict__ samples, volatile int64_t* done, int64_t ticket,
+                                                   int64_t* times) {
+    small_run<KMAX, STAGED>(psi, n, gates, ng, mats, n_mats, perms, n_perms, probs, shots, seed, samples, done, ticket, times);
+}
+
+// A short plan (a GHZ circuit on 10 qubits takes 2.6 KB) travels in the kernel's parameters, which saves
+// the round trip to host memory.
+struct alignas(16) SmallInline {
+    char bytes[3584];   // gates, matrices, permutations
+};
+template <int KMAX>
+__global__ void __launch_bounds__(512) k_small_run_inline(double2* __restrict__ psi, int n, const __grid_constant__ SmallInline plan,
+                                                          int ng, int n_mats, int n_perms, double* __restrict__ probs,
+                                                          int64_t shots, uint64_t seed, int64_t* __restrict__ samples,
+                                                          volatile int64_t* done, int64_t ticket, int64_t* times) {
+    const char* p = plan.bytes;
+    const TileGate* gates = reinterpret_cast<const TileGate*>(p);
+    const float4* mats = reinterpret_cast<const float4*>(p + (size_t)ng * sizeof(TileGate));
+    const int32_t* perms = reinterpret_cast<const int32_t*>(mats + n_mats);
+    small_run<KMAX, true>(psi, n, gates, ng, mats, n_mats, perms, n_perms, probs, shots, seed, samples, done, ticket, times);
 }
 
 // The same for states of 2^11 and 2^12: a cluster of 4 or 8 CTAs holds 2^9 amplitudes each, so that the
@@ -2184,15 +2211,19 @@ int bs_small_launch(bs_sim* s, const SmallPlan& plan, double* dprobs, int64_t sh
     const int64_t b_p = al((int64_t)(perms.size() + 1) * (int64_t)sizeof(int32_t));
     const int64_t b_w = al((int64_t)(plan.sweeps.size() + 1) * (int64_t)sizeof(SmallSweep));
     const int64_t b_all = b_tg + b_m + b_p + b_w;
-    char* dev;
+    char* dev = nullptr;
     int rc;
+    const size_t b_inline = tg.size() * sizeof(TileGate) + mats.size() * sizeof(float4) + perms.size() * sizeof(int32_t);
+    const bool inl = plan.sweeps.empty() && b_inline <= sizeof(SmallInline);
     auto write = [&](char* host) {
         if (!tg.empty()) std::memcpy(host, tg.data(), tg.size() * sizeof(TileGate));
         if (!mats.empty()) std::memcpy(host + b_tg, mats.data(), mats.size() * sizeof(float4));
         if (!perms.empty()) std::memcpy(host + b_tg + b_m, perms.data(), perms.size() * sizeof(int32_t));
         if (!plan.sweeps.empty()) std::memcpy(host + b_tg + b_m + b_p, plan.sweeps.data(), plan.sweeps.size() * sizeof(SmallSweep));
     };
-    if (io && b_all <= (int64_t)io->plan_cap) {
+    if (inl) {
+        // in the kernel's parameters
+    } else if (io && b_all <= (int64_t)io->plan_cap) {
         // the plan goes straight into host-mapped memory, which the kernel reads (the previous run on
         // this thread has completed, so nothing reads it any more); the launch orders these writes
         // before the kernel's reads
@@ -2255,7 +2286,7 @@ int bs_small_launch(bs_sim* s, const SmallPlan& plan, double* dprobs, int64_t sh
     // then (staged) the matrices and permutations
     const size_t base = std::max(((size_t)1 << n) * sizeof(float4), (size_t)2 * (((1 << n) + 31) / 32 * 32) * sizeof(double)) +
                         ((size_t)1 << n) * sizeof(double);
-    const size_t stage = mats.size() * sizeof(float4) + perms.size() * sizeof(int32_t);
+    const size_t stage = mats.size() * sizeof(float4) + tg.size() * sizeof(TileGate) + perms.size() * sizeof(int32_t) + 16;
     constexpr size_t kSmemCap = 160 * 1024;
     const bool staged = base + stage <= kSmemCap;
     const size_t smem = staged ? base + stage : base;
@@ -2268,14 +2299,29 @@ int bs_small_launch(bs_sim* s, const SmallPlan& plan, double* dprobs, int64_t sh
         cudaFuncSetAttribute(k_small_run<4, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemCap);
         cudaFuncSetAttribute(k_small_run<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemCap);
         cudaFuncSetAttribute(k_small_run<4, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemCap);
+        cudaFuncSetAttribute(k_small_run_inline<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemCap);
+        cudaFuncSetAttribute(k_small_run_inline<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemCap);
         attr_set[s->device & 63] = true;
     }
     const int threads = std::min(512, std::max(128, (1 << n) / 2));
+    if (inl) {
+        SmallInline blob;
+        char* p = blob.bytes;
+        if (!tg.empty()) std::memcpy(p, tg.data(), tg.size() * sizeof(TileGate));
+        p += tg.size() * sizeof(TileGate);
+        if (!mats.empty()) std::memcpy(p, mats.data(), mats.size() * sizeof(float4));
+        p += mats.size() * sizeof(float4);
+        if (!perms.empty()) std::memcpy(p, perms.data(), perms.size() * sizeof(int32_t));
+        auto k = kmax <= 2 ? k_small_run_inline<2> : k_small_run_inline<4>;
+        k<<<1, threads, base + stage, s->stream>>>((double2*)s->state, n, blob, (int)tg.size(), (int)mats.size(), (int)perms.size(),
+                                                   dprobs, shots, seed, dsamples, done, ticket, io ? io->dtimes : nullptr);
+    } else {
     auto kern = kmax <= 2 ? (staged ? k_small_run<2, true> : k_small_run<2, false>)
                           : (staged ? k_small_run<4, true> : k_small_run<4, false>);
     kern<<<1, threads, smem, s->stream>>>((double2*)s->state, n, d_tg, (int)tg.size(), d_m, (int)mats.size(), d_p,
                                           (int)perms.size(), dprobs, shots, seed, dsamples, done, ticket,
                                           io ? io->dtimes : nullptr);
+    }
     s->stats.kernel_launches++;
     s->stats.sweeps++;
     s->stats.gates += (int64_t)tg.size();
