@@ -334,8 +334,8 @@ __device__ __forceinline__ void apply(float4* sm, const TileGate& g, const TileG
         }
         eb = __reduce_max_sync(0xffffffffu, eb);
         if (lane_id == 0) s_wmax[warp] = eb;
+        __syncthreads();   // otherwise the caller's barrier has ordered s_wmax
     }
-    __syncthreads();
     uint32_t eall = s_wmax[0];
 #pragma unroll
     for (int w = 1; w < NT / 32; w++) eall = max(eall, s_wmax[w]);
