@@ -5,8 +5,8 @@
 // its tile bits fit the block; bits outside the tile (controls, and target bits
 // of diagonal gates) are constant within a CTA, so the block is built once per
 // assignment of those "uniform" bits (at most 3 of them) and each CTA picks its
-// variant.  The products are formed here in FP64; the device applies them to the
-// tile as real 64x64 GEMMs on tcgen05 tensor cores, with both operands split
+// variant.  The products are formed on the device in FP64 (k_tc_build) and applied to
+// the tile as real 64x64 GEMMs on tcgen05 tensor cores, with both operands split
 // into exact 8-bit bf16 digits (an Ozaki-style split) so that the result keeps
 // float-float accuracy.  This replaces, for those gates, the per-gate amplitude
 // loops of the reference (src/gate_kernels.jl:489-775, src/custom_gates.jl:364-416);
@@ -171,28 +171,12 @@ void bs_fuse_tc(const std::vector<HostGate>& in, const int* local, int T, double
             if (e >= 0 && !((bits >> e) & 1ULL)) eb.push_back(e);
         }
         std::sort(eb.begin(), eb.end(), [&](int a, int c) { return local[a] < local[c]; });
-        int pos[64];
-        for (int e = 0; e < 64; e++) pos[e] = -1;
-        for (int q = 0; q < 5; q++) pos[eb[(size_t)q]] = q;
         HostGate f;
         f.kind = 4;
         f.k = 5;
         for (int q = 0; q < 5; q++) f.ebit[q] = eb[(size_t)q];
         for (int e = 0; e < 64; e++) if ((ubits >> e) & 1ULL) f.ubits.push_back(e);
-        const int nvar = 1 << f.ubits.size();
-        f.mat.assign((size_t)nvar * 2 * 32 * 32, 0.0);
-        for (int var = 0; var < nvar; var++) {
-            uint64_t uval = 0;
-            for (size_t i = 0; i < f.ubits.size(); i++) if ((var >> i) & 1) uval |= 1ULL << f.ubits[i];
-            double* m = f.mat.data() + (size_t)var * 2048;
-            std::vector<cd> U(32 * 32, cd(0, 0));
-            for (int r = 0; r < 32; r++) U[(size_t)r * 33] = 1;
-            for (int i : idx) apply_block(in[(size_t)i], pos, uval, U.data());
-            for (int r = 0; r < 32 * 32; r++) {
-                m[2 * r] = U[(size_t)r].real();
-                m[2 * r + 1] = U[(size_t)r].imag();
-            }
-        }
+        f.perm = idx;
         out.push_back(std::move(f));
     };
     std::vector<char> done(G, 0);
@@ -701,15 +685,73 @@ void bs_block_c64(const std::vector<HostGate>& in, const int* local, int T, std:
     }
 }
 
-bool bs_tc_exponent(const double* mat, int n_mat, int& eu) {
-    double mx = 0;
-    for (size_t i = 0; i < (size_t)n_mat * 2048; i++) {
-        if (!std::isfinite(mat[i])) return false;
-        mx = std::max(mx, std::fabs(mat[i]));
+namespace {
+// Upper bound of the largest singular value of a gate's matrix (sqrt(|A^H A|_inf) up to 4x4, which is 1 for a
+// unitary one; else the smaller of the Frobenius norm and sqrt(|A|_1 |A|_inf)); infinite if an entry is not finite.
+double norm_bound(const HostGate& g) {
+    if (g.kind == 2) return 1;
+    for (double v : g.mat) if (!std::isfinite(v)) return INFINITY;
+    const int D = 1 << g.k;
+    const double* m = g.mat.data();
+    if (g.kind == 1) {
+        double mx = 0;
+        for (int i = 0; i < D; i++) mx = std::max(mx, std::hypot(m[2 * i], m[2 * i + 1]));
+        return std::max(mx, 1.0);
     }
-    int e = 0;
-    if (mx > 0) std::frexp(mx, &e);          // mx < 2^e
-    if (e > 12) return false;
-    eu = std::max(e, -60);
+    double b = 0;
+    if (D <= 4) {
+        for (int i = 0; i < D; i++) {
+            double sum = 0;
+            for (int j = 0; j < D; j++) {
+                double re = 0, im = 0;
+                for (int r = 0; r < D; r++) {
+                    const double *x = m + 2 * (r * D + i), *y = m + 2 * (r * D + j);
+                    re += x[0] * y[0] + x[1] * y[1];
+                    im += x[0] * y[1] - x[1] * y[0];
+                }
+                sum += std::fabs(re) + std::fabs(im);
+            }
+            b = std::max(b, sum);
+        }
+    } else {
+        double fro = 0, rmax = 0, cmax = 0, col[32] = {0};
+        for (int r = 0; r < D; r++) {
+            double row = 0;
+            for (int c = 0; c < D; c++) {
+                const double a2 = m[2 * (r * D + c)] * m[2 * (r * D + c)] + m[2 * (r * D + c) + 1] * m[2 * (r * D + c) + 1];
+                const double a = std::sqrt(a2);
+                fro += a2;
+                row += a;
+                col[c] += a;
+            }
+            rmax = std::max(rmax, row);
+        }
+        for (int c = 0; c < D; c++) cmax = std::max(cmax, col[c]);
+        b = std::min(fro, rmax * cmax);
+    }
+    return g.cmask ? std::max(std::sqrt(b), 1.0) : std::sqrt(b);
+}
+}  // namespace
+
+// Whether every entry of a fused unitary (all variants) is below 2^12.  The device forms the products; here a
+// bound from the gates' norms decides, and only where it does not (many gates far from unitary, or entries that
+// are not finite) are the products formed to look at them.
+bool bs_tc_in_range(const HostGate& f, const std::vector<HostGate>& in) {
+    double bound = 1;
+    for (int i : f.perm) bound *= norm_bound(in[(size_t)i]);
+    if (bound < 4000.0) return true;
+    int pos[64];
+    for (int e = 0; e < 64; e++) pos[e] = -1;
+    for (int q = 0; q < 5; q++) pos[f.ebit[q]] = q;
+    std::vector<cd> U(32 * 32);
+    for (int var = 0; var < (1 << f.ubits.size()); var++) {
+        uint64_t uval = 0;
+        for (size_t i = 0; i < f.ubits.size(); i++) if ((var >> i) & 1) uval |= 1ULL << f.ubits[i];
+        std::fill(U.begin(), U.end(), cd(0, 0));
+        for (int r = 0; r < 32; r++) U[(size_t)r * 33] = 1;
+        for (int i : f.perm) apply_block(in[(size_t)i], pos, uval, U.data());
+        for (const cd& u : U)
+            if (!(std::fabs(u.real()) < 4096.0) || !(std::fabs(u.imag()) < 4096.0)) return false;
+    }
     return true;
 }

@@ -44,6 +44,19 @@ struct TileGate {
     int32_t tc_ub[3];
 };
 
+// One gate of a fused unitary, for the kernel that forms its matrices.  Block bit q: 0..4; variant bit i: 8 + i.
+struct TcPart {
+    uint8_t kind, k;            // as TileGate kinds 0..2
+    uint8_t pos[5];             // target j: its block bit, or (diagonal) variant bit
+    uint8_t cmask, cval;        // controls in the block: (row & cmask) == cval
+    uint8_t umask, uval;        // controls among the variant bits
+    int32_t off;                // matrix (complex) or permutation (int pairs) in the pool
+};
+// One fused unitary: its gates, its first matrix variant and its TileGate.
+struct TcBlock {
+    int32_t part0, n_parts, var0, gate;
+};
+
 // One operation of a register block (TileGate kind 8, complex64 sweeps): the block's 5 tile bits index
 // the 32 amplitudes a thread holds in registers.
 //   type 0..2: 2x2 matrix on block bit `bit` (0 complex, 1 all real, 2 real diagonal and imaginary
@@ -100,9 +113,10 @@ struct HostGate {                // a gate after lowering to the canonical conve
     int ebit[BS_MAX_TARGETS];    // endian bit of target j (matrix bit j)
     std::vector<double> mat;     // interleaved complex; dense 4^k*2, diag 2^k*2
     uint64_t cmask = 0, cval = 0;// controls on endian bits
-    std::vector<int> perm;       // monomial: column c -> (row, i-power)
-    std::vector<int> ubits;      // kind 4: out-of-tile bits the fused matrix depends on; mat holds
-                                 // 2^|ubits| matrices, variant v for bit values v_i at ubits[i]
+    std::vector<int> perm;       // monomial: column c -> (row, i-power); kind 4: its gates in order, indices
+                                 // into the list that was fused
+    std::vector<int> ubits;      // kind 4: out-of-tile bits the fused matrix depends on: 2^|ubits|
+                                 // matrices, variant v for bit values v_i at ubits[i]
 };
 
 struct Sweep {
@@ -255,7 +269,7 @@ int bs_tc_min_bits(const bs_sim* s);
 double bs_tc_cost(const bs_sim* s);
 
 // ---- tensor-core fusion (bs_fuse.cpp)
-// Fold runs of in-tile gates into kind-4 HostGates (5 endian bits, 32x32 matrix) where that is cheaper
+// Fold runs of in-tile gates into kind-4 HostGates (5 endian bits and the gates' indices) where that is cheaper
 // (float-float cost above `threshold`).  local[e]: tile position of endian bit e or -1.
 void bs_fuse_tc(const std::vector<HostGate>& in, const int* local, int T, double threshold, std::vector<HostGate>& out);
 void bs_fuse_small(const std::vector<HostGate>& in, const int* local, double pass, int maxk, std::vector<HostGate>& out);
@@ -271,8 +285,8 @@ struct RegItem {
 // drift: relative size error of the one-bit matrices rounded to FP32 so far, carried from sweep to sweep.
 void bs_block_c64(const std::vector<HostGate>& in, const int* local, int T, std::vector<RegItem>& items,
                   std::vector<RegBlock>& blocks, std::vector<float4>& tabs, double& drift);
-// Smallest eu with every entry of the n_mat 32x32 matrices below 2^eu; false if not finite or above 2^12.
-bool bs_tc_exponent(const double* mat, int n_mat, int& eu);
+// Whether every entry of a fused gate's matrices is finite and below 2^12 (in: the list that was fused).
+bool bs_tc_in_range(const HostGate& f, const std::vector<HostGate>& in);
 
 // ---- execution (bs_tile.cu)
 int bs_run_sweeps(bs_sim* s, const std::vector<Sweep>& sweeps);

@@ -14,7 +14,6 @@
 #include <cmath>
 #include <complex>
 #include <cstring>
-#include <thread>
 #include "bs_internal.h"
 #include "bs_ff.cuh"
 #include "bs_tc.cuh"
@@ -454,11 +453,11 @@ constexpr int kTcThreads = BS_TC_THREADS;   // 256 (128 registers) or 512 (64 re
 constexpr int kTcSmem = 49152 + 65536;
 
 // Global offset (>> 5) of the tile's high-bit pattern i (7 bits) from two small tables:
-// a[i & 7] | b[i >> 3].
+// a[i & 15] | b[i >> 4].
 struct HiOff {
     const uint32_t* a;
     const uint32_t* b;
-    __device__ __forceinline__ uint32_t operator[](int i) const { return a[i & 7] | b[i >> 3]; }
+    __device__ __forceinline__ uint32_t operator[](int i) const { return a[i & 15] | b[i >> 4]; }
 };
 
 // Persistent: two CTAs per SM take tiles in turn, so that barriers, offset tables and TMEM are set up once.
@@ -474,13 +473,13 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_tile_sweep_tc(double2* __rest
     __shared__ __align__(8) uint64_t bars[7];   // digit copy, MMAs into D0 / D1, D0 / D1 read, D1 free, D2
     __shared__ uint32_t s_tmem;
     __shared__ int s_fail;
-    __shared__ uint32_t s_offa[8], s_offb[16];
+    __shared__ uint32_t s_offa[16], s_offb[8];
     __shared__ uint32_t s_wmax[kTcThreads / 32];   // per-warp largest high-word exponent field
     __shared__ int s_act[32], s_cnt;                 // kind 5: blocks passing the row/column test
     __shared__ int s_tcq[16], s_ntc;                 // the tile's first 16 fused gates, in order
     __shared__ const uint16_t* s_nsrc;
     const HiOff off32{s_offa, s_offb};
-    constexpr int T = 12, L = 5, H = 7, nt = 1 << T, lowmask = (1 << L) - 1, NL = nt / kTcThreads;
+    constexpr int T = 12, L = 5, H = T - L, nt = 1 << T, lowmask = (1 << L) - 1, NL = nt / kTcThreads;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         s_fail = 0;
@@ -492,12 +491,12 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_tile_sweep_tc(double2* __rest
         tc::mbar_init(tc::su32(&bars[5]));
         tc::mbar_init(tc::su32(&bars[6]));
     }
-    if (threadIdx.x < 24) {
-        const int i = threadIdx.x < 8 ? threadIdx.x : (threadIdx.x - 8) << 3;
+    if (threadIdx.x < 16 + (1 << (H - 4))) {
+        const int i = threadIdx.x < 16 ? threadIdx.x : (threadIdx.x - 16) << 4;
         int64_t o = 0;
         for (int j = 0; j < H; j++) if ((i >> j) & 1) o |= 1LL << d.hi_bits[j];
-        if (threadIdx.x < 8) s_offa[threadIdx.x] = (uint32_t)(o >> L);
-        else s_offb[threadIdx.x - 8] = (uint32_t)(o >> L);
+        if (threadIdx.x < 16) s_offa[threadIdx.x] = (uint32_t)(o >> L);
+        else s_offb[threadIdx.x - 16] = (uint32_t)(o >> L);
     }
     if (warp == 0) tc::tmem_alloc(tc::su32(&s_tmem));
     tc::fence_before();
@@ -618,32 +617,105 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_tile_sweep_tc(double2* __rest
     if (warp == 0) tc::tmem_dealloc(st.tmem);
 }
 
+// The matrices of the fused unitaries, complex 32x32 row-major FP64 per variant, as the product of their gates.
+// A CTA forms 8 columns of one variant (columns are independent), a thread one entry of each product; the
+// entries that are still zero (the product starts from the identity) are skipped.  largest: per fused unitary
+// the bits of its largest |re| or |im|.  Bound by the FP64 units (2 products a clock per SM): 30 to 60 us a list.
+// On the host, in up to 8 threads, the products and their copies kept the GPU waiting: 22 qubits, 30 layers of a
+// gate mix 3.14 -> 1.89 ms, 25 qubits 17.8 -> 16.1, 28-qubit dense circuit 59.7 -> 56.8, 12-qubit density matrix with
+// channels 8.5 -> 7.6.
+__global__ void __launch_bounds__(256) k_tc_build(const TcBlock* __restrict__ blocks, const int32_t* __restrict__ var_block,
+                                                  const TcPart* __restrict__ parts, const double2* __restrict__ pool,
+                                                  const int32_t* __restrict__ perms, double2* __restrict__ mats,
+                                                  unsigned long long* __restrict__ largest) {
+    __shared__ double2 U[2][32][8];
+    const int v = blockIdx.x >> 2, row = threadIdx.x >> 3, col = threadIdx.x & 7, gcol = (blockIdx.x & 3) * 8 + col;
+    const int bi = var_block[v];
+    const TcBlock b = blocks[bi];
+    const int var = v - b.var0;
+    double2 x = make_double2(row == gcol ? 1.0 : 0.0, 0.0);
+    int cur = 0;
+    U[0][row][col] = x;
+    __syncthreads();
+    for (int i = 0; i < b.n_parts; i++) {
+        const TcPart p = parts[b.part0 + i];
+        if ((var & p.umask) != p.uval) continue;   // uniform
+        const int k = p.k;
+        if (p.kind == 1) {
+            int d = 0;
+            for (int q = 0; q < k; q++) d |= (p.pos[q] < 8 ? (row >> p.pos[q]) & 1 : (var >> (p.pos[q] - 8)) & 1) << q;
+            if ((row & p.cmask) == p.cval) {
+                const double2 m = pool[p.off + d];
+                x = make_double2(m.x * x.x - m.y * x.y, m.x * x.y + m.y * x.x);
+            }
+        } else {
+            int t = 0, base = row;
+            for (int q = 0; q < k; q++) {
+                t |= ((row >> p.pos[q]) & 1) << q;
+                base &= ~(1 << p.pos[q]);
+            }
+            if ((row & p.cmask) == p.cval) {
+                double2 y = make_double2(0.0, 0.0);
+                for (int c = 0; c < (1 << k); c++) {
+                    int src = base;
+                    for (int q = 0; q < k; q++) src |= ((c >> q) & 1) << p.pos[q];
+                    if (p.kind == 0) {
+                        const double2 u = U[cur][src][col];
+                        if (u.x == 0.0 && u.y == 0.0) continue;
+                        const double2 m = pool[p.off + (t << k) + c];
+                        y.x += m.x * u.x - m.y * u.y;
+                        y.y += m.x * u.y + m.y * u.x;
+                    } else if (perms[p.off + 2 * c] == t) {
+                        const double2 u = U[cur][src][col];
+                        const int ph = perms[p.off + 2 * c + 1] & 3;
+                        y = ph == 0 ? u : ph == 1 ? make_double2(-u.y, u.x) : ph == 2 ? make_double2(-u.x, -u.y) : make_double2(u.y, -u.x);
+                    }
+                }
+                x = y;
+            }
+        }
+        cur ^= 1;          // the other buffer's readers are behind the previous barrier
+        U[cur][row][col] = x;
+        __syncthreads();
+    }
+    mats[(size_t)v * 1024 + row * 32 + gcol] = x;
+    unsigned long long mx = (unsigned long long)__double_as_longlong(fmax(fabs(x.x), fabs(x.y)));
+    for (int o = 16; o; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    if ((threadIdx.x & 31) == 0) atomicMax(largest + bi, mx);
+}
+
 // Digit slices of the fused matrices for the tensor-core sweep, one CTA per matrix variant.
-// mats: complex 32x32 row-major FP64 per variant; scale[v] = 2^(8 - eu) of the variant's gate.
+// mats: complex 32x32 row-major FP64 per variant; largest: bits of the largest entry of the fused unitary,
+// which gives its tc_eu (entries below 2^tc_eu), written to its TileGate.
 // Entry (n, k) of the real 64x64 embedding (n = 2t'+c' output re/im, k = 2t+c input re/im) is split
-// into six balanced digits d_i in [-256, 256] (u 2^(8-eu) = sum_i d_i 2^(-9i), each digit rounded to
-// nearest even), digit i stored as the bf16 of d_i 2^(-9i) at its place in the K-major no-swizzle
+// into six balanced digits d_i in [-256, 256] (u 2^(8-eu), rounded to a multiple of 2^-45, = sum_i d_i 2^(-9i);
+// taken from the 54-bit integer, the FP64 units would make it 30 us instead of 8), digit i stored as the bf16 of d_i 2^(-9i) at its place in the K-major no-swizzle
 // operand layout (per digit and k-step a 2 KiB block of 8x8 core matrices: row group n/8 at 256 B,
 // K half at 128 B, row n%8 at 16 B).
-__global__ void __launch_bounds__(256) k_tc_digits(const double* __restrict__ mats, const double* __restrict__ scale,
-                                                   uint16_t* __restrict__ pool) {
-    const int v = blockIdx.x;
+__global__ void __launch_bounds__(256) k_tc_digits(const double* __restrict__ mats, const TcBlock* __restrict__ blocks,
+                                                   const int32_t* __restrict__ var_block,
+                                                   const unsigned long long* __restrict__ largest,
+                                                   TileGate* __restrict__ gates, uint16_t* __restrict__ pool) {
+    const int v = blockIdx.x, bi = var_block[v];
     const double* m = mats + (size_t)v * 2048;
     uint16_t* dst = pool + (size_t)v * tc::kPoolBlock;
-    const double sc = scale[v];
+    const unsigned long long lb = largest[bi];
+    const int eu = lb ? max((int)(lb >> 52) - 1022, -60) : 0;
+    if (threadIdx.x == 0 && v == blocks[bi].var0) gates[blocks[bi].gate].tc_eu = eu;
+    const double sc = __longlong_as_double((long long)(1023 + 53 - eu) << 52);   // 2^(53 - eu): the entry as a multiple of 2^(eu-53)
     for (int e = threadIdx.x; e < 64 * 64; e += blockDim.x) {
         const int n = e >> 6, k = e & 63;
         const int tp = n >> 1, cp = n & 1, t = k >> 1, c = k & 1;
         const double re = m[2 * (tp * 32 + t)], im = m[2 * (tp * 32 + t) + 1];
         const double u = (cp == c) ? re : (cp == 0 ? -im : im);
-        double x = u * sc;
         const int s = k >> 4, kc = (k >> 3) & 1, rg = n >> 3, r = n & 7, el = k & 7;
         const int pos = rg * 128 + kc * 64 + r * 8 + el;
+        long long x = __double2ll_rn(u * sc);
 #pragma unroll
-        for (int i = 0; i < 6; i++) {
-            const double d = rint(x);
-            x = (x - d) * 512.0;
-            const float f = __double2float_rn(d) * __int_as_float((127 - 9 * i) << 23);   // exact: |d| <= 256
+        for (int i = 5; i >= 0; i--) {
+            const int d = i ? (int)((x + 256) & 511) - 256 : (int)x;
+            x = (x - d) >> 9;
+            const float f = (float)d * __int_as_float((127 - 9 * i) << 23);   // exact: |d| <= 256
             dst[(size_t)(i * 4 + s) * 1024 + pos] = (uint16_t)(__float_as_uint(f) >> 16);
         }
     }
@@ -1331,47 +1403,27 @@ int bs_run_sweeps(bs_sim* s, const std::vector<Sweep>& sweeps) {
     std::vector<int32_t> big_bits;
     std::vector<RegOp> rops;                 // operations of the register blocks (complex64)
     double reg_drift = 0;
-    std::vector<double> tc_mats, tc_scale;   // fused matrices (complex 32x32 per variant), 2^(8-eu) per variant
+    std::vector<double> tc_pool;             // the fused gates' own matrices (complex), then read by k_tc_build
+    std::vector<TcPart> tc_parts;
+    std::vector<TcBlock> tc_blocks;
+    std::vector<int32_t> tc_var;             // fused unitary of each variant
     int64_t n_var = 0;
     const bool c64 = s->precision == BS_PREC_C64;
     // fused tensor-core sweeps from bs_tc_min_bits vector bits up (22 by default: measured wins at
     // 24, 26, 28 and 30 bits; small states are dominated by host planning)
     const bool use_tc = bs_tc_enabled(s) && !c64 && T == 12 && L == 5 && n_bits >= bs_tc_min_bits(s);
     const double tc_threshold = bs_tc_cost(s);
-    // fusion per sweep (independent, so on a few host threads); a sweep left with unfused 3/4-target
-    // gates or with reference-mode channels keeps its plain gate list, since the tensor-core sweep
+    // a sweep left with unfused 3/4-target gates keeps its plain gate list, since the tensor-core sweep
     // kernel carries float-float paths for 1- and 2-target gates only
-    std::vector<std::vector<HostGate>> fused_all(use_tc ? sweeps.size() : 0);
-    std::vector<char> fused_ok(fused_all.size(), 0);
-    if (use_tc) {
-        auto work = [&](size_t first, size_t step) {
-            for (size_t i = first; i < sweeps.size(); i += step) {
-                const Sweep& sw = sweeps[i];
-                if ((int)sw.hi_bits.size() != T - L) continue;
-                int local[64];
-                for (int b = 0; b < 64; b++) local[b] = -1;
-                for (int b = 0; b < L; b++) local[b] = b;
-                for (size_t q = 0; q < sw.hi_bits.size(); q++) local[sw.hi_bits[q]] = L + (int)q;
-                bs_fuse_tc(sw.gates, local, T, tc_threshold, fused_all[i]);
-                bool ok = true;
-                for (const HostGate& hg : fused_all[i])
-                    if (hg.kind != 1 && hg.kind != 4 && hg.kind != 5 && hg.k >= 3) ok = false;
-                fused_ok[i] = ok;
-            }
-        };
-        const unsigned hw = std::max(1u, std::min(8u, std::thread::hardware_concurrency()));
-        const size_t nth = std::min<size_t>(sweeps.size(), hw);
-        if (nth <= 1) {
-            work(0, 1);
-        } else {
-            std::vector<std::thread> th;
-            for (size_t t = 0; t < nth; t++) th.emplace_back(work, t, nth);
-            for (std::thread& x : th) x.join();
-        }
-    }
-    size_t swi = 0;
+    std::vector<HostGate> fused;
+    auto fuse = [&](const Sweep& sw, const int* local) {
+        if (!use_tc || (int)sw.hi_bits.size() != T - L) return false;
+        bs_fuse_tc(sw.gates, local, T, tc_threshold, fused);
+        for (const HostGate& hg : fused)
+            if (hg.kind != 1 && hg.kind != 4 && hg.kind != 5 && hg.k >= 3) return false;
+        return true;
+    };
     for (const Sweep& sw : sweeps) {
-        const size_t si = swi++;
         Launch ln;
         ln.gate0 = (int64_t)tg.size();
         ln.rop0 = rops.size();
@@ -1387,8 +1439,8 @@ int bs_run_sweeps(bs_sim* s, const std::vector<Sweep>& sweeps) {
         std::vector<HostGate> merged, small;
         std::vector<RegItem> items;        // complex64 sweep by register blocks: the order of its passes
         std::vector<RegBlock> blocks;
-        if (use_tc && fused_ok[si]) {
-            merge_diagonals(fused_all[si], merged);
+        if (fuse(sw, local)) {
+            merge_diagonals(fused, merged);
         } else if (c64) {
             // complex64 sweep: 1- and 2-bit runs fused into dense 2-bit gates where that saves passes (a
             // pass of the complex64 kernel costs about four 1-qubit gates' arithmetic; batch of 512
@@ -1493,13 +1545,34 @@ int bs_run_sweeps(bs_sim* s, const std::vector<Sweep>& sweeps) {
                 t.tc_nu = (int32_t)hg.ubits.size();
                 for (size_t i = 0; i < hg.ubits.size(); i++) t.tc_ub[i] = hg.ubits[i];
                 t.tc_off = (int32_t)n_var;
-                int eu = 0;
-                if (!bs_tc_exponent(hg.mat.data(), nvar, eu))
-                    return bs_fail(s, BS_ERR_INVALID_ARG, "fused gate matrix out of range");
-                tc_mats.insert(tc_mats.end(), hg.mat.begin(), hg.mat.begin() + (size_t)nvar * 2048);
-                for (int v = 0; v < nvar; v++) tc_scale.push_back(std::ldexp(1.0, 8 - eu));
+                if (!bs_tc_in_range(hg, sw.gates)) return bs_fail(s, BS_ERR_INVALID_ARG, "fused gate matrix out of range");
+                int where[64];           // block or variant bit of an endian bit
+                for (int b = 0; b < 64; b++) where[b] = -1;
+                for (int q = 0; q < 5; q++) where[hg.ebit[q]] = q;
+                for (size_t i = 0; i < hg.ubits.size(); i++) where[hg.ubits[i]] = 8 + (int)i;
+                tc_blocks.push_back({(int32_t)tc_parts.size(), (int32_t)hg.perm.size(), (int32_t)n_var, (int32_t)tg.size()});
+                for (int gi : hg.perm) {
+                    const HostGate& g = sw.gates[(size_t)gi];
+                    TcPart p{};
+                    p.kind = (uint8_t)g.kind;
+                    p.k = (uint8_t)g.k;
+                    for (int q = 0; q < g.k; q++) p.pos[q] = (uint8_t)where[g.ebit[q]];
+                    for (uint64_t r = g.cmask; r; r &= r - 1) {
+                        const int e = __builtin_ctzll(r), w = where[e], v = (int)((g.cval >> e) & 1);
+                        if (w < 8) { p.cmask |= (uint8_t)(1 << w); p.cval |= (uint8_t)(v << w); }
+                        else { p.umask |= (uint8_t)(1 << (w - 8)); p.uval |= (uint8_t)(v << (w - 8)); }
+                    }
+                    if (g.kind == 2) {
+                        p.off = (int32_t)perms.size();
+                        perms.insert(perms.end(), g.perm.begin(), g.perm.end());
+                    } else {
+                        p.off = (int32_t)(tc_pool.size() / 2);
+                        tc_pool.insert(tc_pool.end(), g.mat.begin(), g.mat.begin() + ((size_t)2 << (g.kind == 0 ? 2 * g.k : g.k)));
+                    }
+                    tc_parts.push_back(p);
+                }
+                tc_var.insert(tc_var.end(), (size_t)nvar, (int32_t)tc_blocks.size() - 1);
                 n_var += nvar;
-                t.tc_eu = eu;
                 ln.n_tc++;
                 tg.push_back(t);
                 ln.n_gates++;
@@ -1599,19 +1672,24 @@ int bs_run_sweeps(bs_sim* s, const std::vector<Sweep>& sweeps) {
     int64_t b_tg = al((int64_t)tg.size() * (int64_t)sizeof(TileGate));
     int64_t b_m = al((int64_t)mats.size() * (int64_t)sizeof(float4));
     int64_t b_p = al((int64_t)(perms.size() + big_bits.size() + 1) * (int64_t)sizeof(int32_t));
-    int64_t b_tm = al((int64_t)tc_mats.size() * (int64_t)sizeof(double));
-    int64_t b_ts = al((int64_t)tc_scale.size() * (int64_t)sizeof(double));
-    int64_t b_tc = al(n_var * tc::kPoolBlock * (int64_t)sizeof(uint16_t));   // written on the device
     const int64_t b_r = al((int64_t)rops.size() * (int64_t)sizeof(RegOp));
-    const int64_t o_r = b_tg + b_m + b_p, o_tm = o_r + b_r, o_ts = o_tm + b_tm, o_tc = o_ts + b_ts;
+    const int64_t b_fm = al((int64_t)tc_pool.size() * (int64_t)sizeof(double)), b_fp = al((int64_t)tc_parts.size() * (int64_t)sizeof(TcPart));
+    const int64_t b_fb = al((int64_t)tc_blocks.size() * (int64_t)sizeof(TcBlock)), b_fv = al(n_var * (int64_t)sizeof(int32_t));
+    const int64_t b_fx = al((int64_t)tc_blocks.size() * (int64_t)sizeof(unsigned long long));   // largest entries, from 0
+    const int64_t o_r = b_tg + b_m + b_p, o_fm = o_r + b_r, o_fp = o_fm + b_fm, o_fb = o_fp + b_fp, o_fv = o_fb + b_fb;
+    const int64_t o_fx = o_fv + b_fv, o_up = o_fx + b_fx;                       // uploaded up to here
+    const int64_t o_tm = o_up, b_tm = al(n_var * 2048 * (int64_t)sizeof(double));   // written on the device:
+    const int64_t o_tc = o_tm + b_tm, b_tc = al(n_var * tc::kPoolBlock * (int64_t)sizeof(uint16_t));
     int rc = bs_ensure_plan(s, o_tc + b_tc);
     if (rc) return rc;
-    char* host = bs_stage(s, (size_t)o_tc);
+    char* host = bs_stage(s, (size_t)o_up);
     if (!host) return bs_fail(s, BS_ERR_ALLOC, "pinned staging allocation");
-    std::memset(host, 0, (size_t)o_tc);
-    if (!tc_mats.empty()) {
-        std::memcpy(host + o_tm, tc_mats.data(), tc_mats.size() * sizeof(double));
-        std::memcpy(host + o_ts, tc_scale.data(), tc_scale.size() * sizeof(double));
+    std::memset(host, 0, (size_t)o_up);
+    if (n_var) {
+        std::memcpy(host + o_fm, tc_pool.data(), tc_pool.size() * sizeof(double));
+        std::memcpy(host + o_fp, tc_parts.data(), tc_parts.size() * sizeof(TcPart));
+        std::memcpy(host + o_fb, tc_blocks.data(), tc_blocks.size() * sizeof(TcBlock));
+        std::memcpy(host + o_fv, tc_var.data(), tc_var.size() * sizeof(int32_t));
     }
     if (!rops.empty()) std::memcpy(host + o_r, rops.data(), rops.size() * sizeof(RegOp));
     if (!tg.empty()) std::memcpy(host, tg.data(), tg.size() * sizeof(TileGate));
@@ -1620,7 +1698,7 @@ int bs_run_sweeps(bs_sim* s, const std::vector<Sweep>& sweeps) {
     if (!big_bits.empty())
         std::memcpy(host + b_tg + b_m + perms.size() * sizeof(int32_t), big_bits.data(), big_bits.size() * sizeof(int32_t));
     char* dev = (char*)s->plan_buf;
-    rc = bs_cuda_check(s, cudaMemcpyAsync(dev, host, (size_t)o_tc, cudaMemcpyHostToDevice, s->stream), "plan upload");
+    rc = bs_cuda_check(s, cudaMemcpyAsync(dev, host, (size_t)o_up, cudaMemcpyHostToDevice, s->stream), "plan upload");
     bs_stage_done(s);
     if (rc) return rc;
     const TileGate* d_tg = (const TileGate*)dev;
@@ -1654,8 +1732,13 @@ int bs_run_sweeps(bs_sim* s, const std::vector<Sweep>& sweeps) {
     double2* psi = (double2*)s->state;
     uint16_t* d_tc = (uint16_t*)(dev + o_tc);
     if (n_var) {
-        k_tc_digits<<<(unsigned)n_var, 256, 0, s->stream>>>((const double*)(dev + o_tm), (const double*)(dev + o_ts), d_tc);
-        s->stats.kernel_launches++;
+        const TcBlock* d_fb = (const TcBlock*)(dev + o_fb);
+        const int32_t* d_fv = (const int32_t*)(dev + o_fv);
+        unsigned long long* d_fx = (unsigned long long*)(dev + o_fx);
+        k_tc_build<<<(unsigned)(4 * n_var), 256, 0, s->stream>>>(d_fb, d_fv, (const TcPart*)(dev + o_fp), (const double2*)(dev + o_fm),
+                                                                 d_p, (double2*)(dev + o_tm), d_fx);
+        k_tc_digits<<<(unsigned)n_var, 256, 0, s->stream>>>((const double*)(dev + o_tm), d_fb, d_fv, d_fx, (TileGate*)dev, d_tc);
+        s->stats.kernel_launches += 2;
         if (!s->dev_flag) {
             rc = bs_cuda_check(s, cudaMalloc((void**)&s->dev_flag, 256), "flag alloc");
             if (rc) return rc;

@@ -150,3 +150,49 @@ def test_density_matrix_with_noise(n, mode):
             # Kraus kernel runs between sweeps and leaves runs too short to be worth fusing
             assert sim.last_stats()["tc_gates"] > 0
         assert rel_err(sim.density_matrix, ref) < TOL
+
+
+@pytest.mark.parametrize("n", [13, 15])
+@pytest.mark.parametrize("low", [False, True])
+def test_fused_products_of_every_gate_form(n, low):
+    """Blocks of gates of all forms (dense on 1 to 4 targets, real and complex, singular and scaled; diagonal and
+    monomial; controls on either value), with targets and controls inside the block and outside the tile."""
+    rng = np.random.default_rng(77 + n)
+    near = list(range(n - 5, n)) if low else list(range(5))   # 5 bits of one block
+    far = [q for q in range(n) if q not in near]
+    ops = [bs.Instruction(bs.Unitary(haar(rng)), [q]) for q in range(n)]
+    for _ in range(12):
+        p = [int(q) for q in rng.permutation(near)]
+        f = [int(q) for q in rng.choice(far, 2, replace=False)]
+        ops += [bs.Instruction(bs.Unitary(haar(rng, 4)), p[:2]), bs.Instruction(bs.Unitary(haar(rng, 8)), p[1:4]),
+                bs.Instruction(bs.Unitary(haar(rng, 16)), p[:4]), bs.Instruction(bs.Ry(0.3), [p[4]]),
+                bs.Instruction(bs.Control(bs.U(0.4, 0.2, -0.7), (0, 1)), [p[0], f[0], p[1]]),
+                bs.Instruction(bs.Control(bs.PhaseShift(0.9), (1, 0)), [f[0], p[2], p[3]]),
+                bs.Instruction(bs.ZZ(0.7), [p[0], f[1]]), bs.Instruction(bs.CPhaseShift(1.1), [f[1], p[1]]),
+                bs.Instruction(bs.CSwap(), [p[2], p[3], p[4]]), bs.Instruction(bs.Control(bs.Y(), (0,)), [f[1], p[0]]),
+                bs.Instruction(bs.ISwap(), [p[1], p[4]]),
+                bs.Instruction(bs.Unitary(2.0 * haar(rng)), [p[2]]), bs.Instruction(bs.Unitary(0.5 * haar(rng)), [p[3]])]
+    ref = oracle.OracleSV(n).evolve(ops).psi
+    with tc_mode(True):
+        sim = bs.StateVectorSimulator(n, 0).evolve(ops)
+        assert sim.last_stats()["tc_gates"] > 0
+        assert rel_err(sim.state_vector, ref) < TOL
+
+
+@pytest.mark.parametrize("factor,ok", [(15.0, True), (17.0, False)])
+def test_fused_matrix_entries_reach_4096(factor, ok):
+    """Matrices up to 2^12 are applied (15^3 = 3375); above it (17^3 = 4913) the list is refused, whatever the bound
+    from the gates' norms says (a gate between them has norm 4)."""
+    n = 13
+    s = np.array([[factor, 0], [0, 0.25]])
+    g = np.array([[1.0, 0], [0, 4.0]])
+    ops = [bs.Instruction(bs.Unitary(m), [2]) for m in (s, g, s, g, s)] + [bs.Instruction(bs.Ry(0.1), [q]) for q in (3, 4, 5)]
+    with tc_mode(True):
+        sim = bs.StateVectorSimulator(n, 0)
+        if ok:
+            sim.evolve(ops)
+            assert sim.last_stats()["tc_gates"] > 0
+            assert rel_err(sim.state_vector, oracle.OracleSV(n).evolve(ops).psi) < TOL
+        else:
+            with pytest.raises(Exception, match="out of range"):
+                sim.evolve(ops)
