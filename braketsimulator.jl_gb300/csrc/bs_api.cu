@@ -430,7 +430,7 @@ int bs_apply_gate(bs_sim* s, const double* matrix, int k, const int* targets, in
     int rc = bs_lower_gate(s, matrix, k, targets, nc, controls, cvals, flags, s->kind == BS_KIND_DM, hg);
     if (rc) return rc;
     std::vector<Sweep> sw;
-    bs_plan_sweeps(hg, bs_vec_bits(s), bs_sweep_tile_bits(s), sw);
+    bs_plan_sweeps(s, hg, sw);
     s->alias_valid = false;
     return bs_run_sweeps(s, sw);
 }
@@ -443,7 +443,7 @@ int bs_dm_apply_vec_gate(bs_sim* s, const double* matrix, int k, const int* targ
     int rc = bs_lower_gate(s, matrix, k, targets, nc, controls, cvals, flags, false, hg);
     if (rc) return rc;
     std::vector<Sweep> sw;
-    bs_plan_sweeps(hg, bs_vec_bits(s), bs_sweep_tile_bits(s), sw);
+    bs_plan_sweeps(s, hg, sw);
     s->alias_valid = false;
     return bs_run_sweeps(s, sw);
 }
@@ -458,7 +458,7 @@ int bs_apply_kraus(bs_sim* s, const double* kraus, int nk, int k, const int* tar
         int rc = bs_lower_kraus_physical(s, kraus, nk, k, targets, flags, hg);
         if (rc) return rc;
         std::vector<Sweep> sw;
-        bs_plan_sweeps(hg, bs_vec_bits(s), bs_sweep_tile_bits(s), sw);
+        bs_plan_sweeps(s, hg, sw);
         return bs_run_sweeps(s, sw);
     }
     return bs_kraus_reference(s, kraus, nk, k, targets, flags);
@@ -531,7 +531,7 @@ int bs_evolve(bs_sim* s, const bs_op* ops, int64_t n_ops, unsigned noise_mode) {
     auto flush = [&]() -> int {
         if (pending.empty()) return BS_OK;
         std::vector<Sweep> sw;
-        bs_plan_sweeps(pending, bs_vec_bits(s), bs_sweep_tile_bits(s), sw);
+        bs_plan_sweeps(s, pending, sw);
         pending.clear();
         if (s->collect) {   // bs_run_small: plan only
             s->collect->insert(s->collect->end(), std::make_move_iterator(sw.begin()), std::make_move_iterator(sw.end()));

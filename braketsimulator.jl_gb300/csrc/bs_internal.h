@@ -7,7 +7,8 @@
 #include "../../include/braket_gb300.h"
 
 #define BS_TILE_MAX_BITS 12      // 2^12 complex float-float values = 64 KiB of shared memory
-#define BS_TILE_LOW_BITS 5       // low endian bits always in a tile: 32 contiguous amplitudes
+#define BS_TILE_LOW_BITS 5       // low endian bits always in a tile, 32 contiguous amplitudes, but for complex128
+                                 // vectors of 19 bits and more (bs_plan_sweeps)
 #define BS_TILE_MAXK 4           // dense targets per tile gate (16x16 superoperators for 2q noise)
 
 // One gate inside a tile sweep.
@@ -120,7 +121,8 @@ struct HostGate {                // a gate after lowering to the canonical conve
 };
 
 struct Sweep {
-    std::vector<int> hi_bits;    // tile bits above the low contiguous block
+    int low = BS_TILE_LOW_BITS;  // low contiguous bits of the tile
+    std::vector<int> hi_bits;    // tile bits above them
     std::vector<HostGate> gates;
 };
 
@@ -257,7 +259,7 @@ int bs_lower_gate(bs_sim* s, const double* matrix, int k, const int* targets, in
 int bs_lower_kraus_physical(bs_sim* s, const double* kraus, int nk, int k, const int* targets,
                             unsigned flags, std::vector<HostGate>& out);
 // The gates are moved into the sweeps (the input is left with moved-from gates).
-void bs_plan_sweeps(std::vector<HostGate>& gates, int n_bits, int tile_bits, std::vector<Sweep>& out);
+void bs_plan_sweeps(const bs_sim* s, std::vector<HostGate>& gates, std::vector<Sweep>& out);
 // Matrix class of a 2x2 gate: 1 all real, 2 real diagonal and imaginary off-diagonal, else 0 (TileGate.npar).
 int bs_class_2x2(const HostGate& h);
 // Tuned values of a handle (its setting, else the environment, else the default)
@@ -271,7 +273,8 @@ double bs_tc_cost(const bs_sim* s);
 // ---- tensor-core fusion (bs_fuse.cpp)
 // Fold runs of in-tile gates into kind-4 HostGates (5 endian bits and the gates' indices) where that is cheaper
 // (float-float cost above `threshold`).  local[e]: tile position of endian bit e or -1.
-void bs_fuse_tc(const std::vector<HostGate>& in, const int* local, int T, double threshold, std::vector<HostGate>& out);
+double bs_fuse_tc(const std::vector<const HostGate*>& in, const int* local, int T, double threshold,
+                  std::vector<HostGate>* out);   // out null: only the list's cost, in fused unitaries
 void bs_fuse_small(const std::vector<HostGate>& in, const int* local, double pass, int maxk, std::vector<HostGate>& out);
 // Grouping of a complex64 sweep's gates into register blocks: items in order, each a block (index into
 // blocks) or a gate left to its own pass (index into in); tabs collects the diagonal tables.

@@ -229,54 +229,56 @@ double bs_tc_cost(const bs_sim* s) {
     return v ? atof(v) : 2.0;
 }
 
+namespace {
+struct SweepIdx {
+    std::vector<int> hi_bits, gates;   // gates: indices into the list
+};
+
 // Greedy sweep planner.  A gate may move ahead of gates it does not share a bit
 // with; a dense or monomial gate needs its target bits inside the tile, a
 // diagonal gate or a control never does (their bits are read from the index).
-void bs_plan_sweeps(std::vector<HostGate>& gates, int n_bits, int tile_bits, std::vector<Sweep>& out) {
-    const int T = std::min(tile_bits, n_bits);
-    const int L = std::min(BS_TILE_LOW_BITS, T);
+void plan_greedy(const std::vector<HostGate>& gates, int n_bits, int T, int L, std::vector<SweepIdx>& out) {
     const int cap = T - L;
     const size_t G = gates.size();
+    out.clear();
+    // what a gate touches, and the bits above L it needs in the tile.  kind 5 (reference-rule channel) acts on
+    // the elements whose row and column agree on every other bit: it commutes with nothing, so it touches
+    // every bit, and it needs its row and column bits
+    std::vector<uint64_t> touch(G), need(G);
+    for (size_t i = 0; i < G; i++) {
+        const HostGate& g = gates[i];
+        uint64_t m = g.cmask, nd = 0;
+        for (int q = 0; q < g.k; q++) m |= 1ULL << g.ebit[q];
+        if (g.kind != 1)
+            for (int q = 0; q < (g.kind == 5 ? 2 * g.k : g.k); q++) if (g.ebit[q] >= L) nd |= 1ULL << g.ebit[q];
+        touch[i] = g.kind == 5 ? ~(uint64_t)0 : m;
+        need[i] = nd;
+    }
     std::vector<char> done(G, 0);
     size_t remaining = G, first = 0;
-    // kind 5 (reference-rule channel) acts on the elements whose row and column agree on every other
-    // bit: it commutes with nothing, so it touches every bit, and it needs its row and column bits
-    auto touch = [&](const HostGate& g) {
-        if (g.kind == 5) return ~(uint64_t)0;
-        uint64_t m = g.cmask;
-        for (int q = 0; q < g.k; q++) m |= 1ULL << g.ebit[q];
-        return m;
-    };
-    auto need = [&](const HostGate& g) {
-        uint64_t m = 0;
-        if (g.kind == 1) return m;
-        const int nb = g.kind == 5 ? 2 * g.k : g.k;
-        for (int q = 0; q < nb; q++) if (g.ebit[q] >= L) m |= 1ULL << g.ebit[q];
-        return m;
-    };
     while (remaining) {
-        Sweep sw;
+        SweepIdx sw;
         uint64_t chosen = 0, blocked = 0;
         int nchosen = 0;
         bool big_alone = false;
         for (size_t i = first; i < G; i++) {
             if (done[i]) continue;
             const HostGate& g = gates[i];
-            uint64_t t = touch(g);
+            const uint64_t t = touch[i];
             if (t & blocked) { blocked |= t; continue; }
-            uint64_t nb = need(g) & ~chosen;
-            int add = __builtin_popcountll(nb);
-            bool too_big = (g.kind != 1) && (g.k > BS_TILE_MAXK || __builtin_popcountll(need(g)) > cap);
+            const uint64_t nb = need[i] & ~chosen;
+            const int add = __builtin_popcountll(nb);
+            const bool too_big = (g.kind != 1) && (g.k > BS_TILE_MAXK || __builtin_popcountll(need[i]) > cap);
             if (too_big) {
                 // a gate no tile can hold runs in a sweep of its own
-                if (sw.gates.empty()) { sw.gates.push_back(std::move(gates[i])); done[i] = 1; remaining--; big_alone = true; }
+                if (sw.gates.empty()) { sw.gates.push_back((int)i); done[i] = 1; remaining--; big_alone = true; }
                 blocked |= t;
                 break;
             }
             if (nchosen + add <= cap) {
                 chosen |= nb;
                 nchosen += add;
-                sw.gates.push_back(std::move(gates[i]));
+                sw.gates.push_back((int)i);
                 done[i] = 1;
                 remaining--;
             } else {
@@ -290,6 +292,57 @@ void bs_plan_sweeps(std::vector<HostGate>& gates, int n_bits, int tile_bits, std
                 if (!((chosen >> b) & 1ULL)) sw.hi_bits.push_back(b);
             std::sort(sw.hi_bits.begin(), sw.hi_bits.end());
         }
+        out.push_back(std::move(sw));
+    }
+}
+
+// Time of a plan with tensor-core sweeps, in fused unitaries (1.45 ms of 2^28 amplitudes; a sweep's read and
+// write is 1.3 of them, with rows of 128 bytes 1.4).  Given up once it is above `most`.
+double tc_plan_cost(const bs_sim* s, const std::vector<HostGate>& gates, int T, int L, const std::vector<SweepIdx>& sweeps,
+                    double most) {
+    double cost = (L == 3 ? 1.4 : 1.3) * (double)sweeps.size();
+    std::vector<const HostGate*> in;
+    for (const SweepIdx& sw : sweeps) {
+        if (cost > most) break;
+        int local[64];
+        for (int b = 0; b < 64; b++) local[b] = b < L ? b : -1;
+        for (size_t q = 0; q < sw.hi_bits.size(); q++) local[sw.hi_bits[q]] = L + (int)q;
+        in.clear();
+        for (int i : sw.gates) in.push_back(&gates[(size_t)i]);
+        cost += bs_fuse_tc(in, local, T, bs_tc_cost(s), nullptr);
+    }
+    return cost;
+}
+}  // namespace
+
+// Low contiguous bits of the tiles.  Fewer of them leave more bits to choose, which saves sweeps (each reads and
+// writes the state once), for shorter rows of memory: 512, 256 or 128 bytes of complex128.  At 26 bits the sweeps
+// of a 13-qubit density matrix cost the same with rows of 256 bytes and 5% more with 128 (24 sweeps 24.0 ms, 19
+// sweeps 21.7 and 22.2).  Complex128 vectors of 19 bits and more take 4 low bits (20 bits 0.85 -> 0.82 ms);
+// from 24 bits the tensor-core sweeps take the best of 3, 4 and 5, since how the sweeps' gates group into fused
+// unitaries differs (28-qubit dense circuit: 24 unitaries in 9 sweeps 56.9 ms with 5, 22 in 7 48.4 with 4; 25
+// qubits: 11 in 5 3.67 with 5, 14 in 5 4.12 with 4).  Planning one costs 0.1 ms, too much below.
+// The gates are moved into the sweeps.
+void bs_plan_sweeps(const bs_sim* s, std::vector<HostGate>& gates, std::vector<Sweep>& out) {
+    const int n_bits = bs_vec_bits(s), T = std::min(bs_sweep_tile_bits(s), n_bits);
+    std::vector<SweepIdx> best, other;
+    int low = std::min(BS_TILE_LOW_BITS, T);
+    if (s->precision == BS_PREC_C128 && T == BS_TILE_MAX_BITS && n_bits >= 19) low = 4;
+    plan_greedy(gates, n_bits, T, low, best);
+    if (low == 4 && n_bits >= 24 && bs_tc_enabled(s) && n_bits >= bs_tc_min_bits(s)) {
+        double cost = tc_plan_cost(s, gates, T, low, best, 1e300);
+        for (int L : {5, 3}) {
+            plan_greedy(gates, n_bits, T, L, other);
+            if (L == 3 && other.size() >= best.size()) continue;
+            const double c = tc_plan_cost(s, gates, T, L, other, cost);
+            if (c < cost) { cost = c; low = L; best.swap(other); }
+        }
+    }
+    for (SweepIdx& b : best) {
+        Sweep sw;
+        sw.low = low;
+        sw.hi_bits = std::move(b.hi_bits);
+        for (int i : b.gates) sw.gates.push_back(std::move(gates[(size_t)i]));
         out.push_back(std::move(sw));
     }
 }

@@ -441,7 +441,7 @@ __global__ void __launch_bounds__(NT, NT == 256 && KMAX == 2 ? 3 : 1) k_tile_swe
     }
 }
 
-// Sweep with fused 5-bit unitaries on the tensor cores (gate kind 4), T = 12, L = 5.
+// Sweep with fused 5-bit unitaries on the tensor cores (gate kind 4), T = 12, L = 3 to 5.
 // Dynamic shared memory: 48 KiB matrix digit slices | 64 KiB tile (static: split offset tables, the
 // per-warp exponents, kind-5 scratch), so that two CTAs fit on an SM; each holds 256 of the SM's 512
 // TMEM columns, so one CTA's MMAs overlap the other's CUDA-core work.  The tile is stored with the
@@ -452,7 +452,7 @@ __global__ void __launch_bounds__(NT, NT == 256 && KMAX == 2 ? 3 : 1) k_tile_swe
 constexpr int kTcThreads = BS_TC_THREADS;   // 256 (128 registers) or 512 (64 registers, spills; measured slower)
 constexpr int kTcSmem = 49152 + 65536;
 
-// Global offset (>> 5) of the tile's high-bit pattern i (7 bits) from two small tables:
+// Global offset (>> L) of the tile's high-bit pattern i (12 - L bits) from two small tables:
 // a[i & 15] | b[i >> 4].
 struct HiOff {
     const uint32_t* a;
@@ -464,6 +464,7 @@ struct HiOff {
 // Without any gate a sweep of 28 qubits takes 1.8 ms (2.4 with a CTA per tile; HBM allows 1.26), with the
 // gates of the 12-qubit density matrix 7.3 ms instead of 7.7.  The next tile's loads issued before this
 // one's stores (64 registers of them) were slower, 62 against 59 ms at 28 qubits.
+template <int L>
 __global__ void __launch_bounds__(kTcThreads, 2) k_tile_sweep_tc(double2* __restrict__ psi, SweepDesc d, int64_t tile0,
                                                                  int64_t tile_end) {
     // 128-byte alignment: each 128-byte core matrix of the matrix operand sits in one shared-memory line
@@ -473,13 +474,13 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_tile_sweep_tc(double2* __rest
     __shared__ __align__(8) uint64_t bars[7];   // digit copy, MMAs into D0 / D1, D0 / D1 read, D1 free, D2
     __shared__ uint32_t s_tmem;
     __shared__ int s_fail;
-    __shared__ uint32_t s_offa[16], s_offb[8];
+    __shared__ uint32_t s_offa[16], s_offb[1 << (8 - L)];
     __shared__ uint32_t s_wmax[kTcThreads / 32];   // per-warp largest high-word exponent field
     __shared__ int s_act[32], s_cnt;                 // kind 5: blocks passing the row/column test
     __shared__ int s_tcq[16], s_ntc;                 // the tile's first 16 fused gates, in order
     __shared__ const uint16_t* s_nsrc;
     const HiOff off32{s_offa, s_offb};
-    constexpr int T = 12, L = 5, H = T - L, nt = 1 << T, lowmask = (1 << L) - 1, NL = nt / kTcThreads;
+    constexpr int T = 12, H = T - L, nt = 1 << T, lowmask = (1 << L) - 1, NL = nt / kTcThreads;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         s_fail = 0;
@@ -1387,13 +1388,12 @@ int bs_run_sweeps(bs_sim* s, const std::vector<Sweep>& sweeps) {
     if (sweeps.empty()) return BS_OK;
     const int n_bits = bs_vec_bits(s);
     const int T = std::min(bs_sweep_tile_bits(s), n_bits);
-    const int L = std::min(BS_TILE_LOW_BITS, T);
     // pack: per sweep [TileGate...], then one float4 pool, then one int pool
     std::vector<TileGate> tg;
     std::vector<float4> mats;
     std::vector<int32_t> perms;
     struct Launch {
-        int64_t gate0; int n_gates; std::vector<int> hi; bool big; int big_gate; int kmax = 1;
+        int64_t gate0; int n_gates; std::vector<int> hi; int low; bool big; int big_gate; int kmax = 1;
         int n_tc = 0;
         bool blk = false;          // has register blocks, with operations rop0 .. rop0 + n_rops
         size_t rop0 = 0;
@@ -1411,14 +1411,16 @@ int bs_run_sweeps(bs_sim* s, const std::vector<Sweep>& sweeps) {
     const bool c64 = s->precision == BS_PREC_C64;
     // fused tensor-core sweeps from bs_tc_min_bits vector bits up (22 by default: measured wins at
     // 24, 26, 28 and 30 bits; small states are dominated by host planning)
-    const bool use_tc = bs_tc_enabled(s) && !c64 && T == 12 && L == 5 && n_bits >= bs_tc_min_bits(s);
+    const bool use_tc = bs_tc_enabled(s) && !c64 && T == 12 && n_bits >= bs_tc_min_bits(s);
     const double tc_threshold = bs_tc_cost(s);
     // a sweep left with unfused 3/4-target gates keeps its plain gate list, since the tensor-core sweep
     // kernel carries float-float paths for 1- and 2-target gates only
     std::vector<HostGate> fused;
     auto fuse = [&](const Sweep& sw, const int* local) {
-        if (!use_tc || (int)sw.hi_bits.size() != T - L) return false;
-        bs_fuse_tc(sw.gates, local, T, tc_threshold, fused);
+        if (!use_tc || (int)sw.hi_bits.size() != T - sw.low) return false;
+        std::vector<const HostGate*> in;
+        for (const HostGate& g : sw.gates) in.push_back(&g);
+        bs_fuse_tc(in, local, T, tc_threshold, &fused);
         for (const HostGate& hg : fused)
             if (hg.kind != 1 && hg.kind != 4 && hg.kind != 5 && hg.k >= 3) return false;
         return true;
@@ -1429,6 +1431,8 @@ int bs_run_sweeps(bs_sim* s, const std::vector<Sweep>& sweeps) {
         ln.rop0 = rops.size();
         ln.n_gates = 0;
         ln.hi = sw.hi_bits;
+        const int L = sw.low;
+        ln.low = L;
         ln.big = false;
         ln.big_gate = -1;
         // tile-local position of each endian bit
@@ -1706,8 +1710,6 @@ int bs_run_sweeps(bs_sim* s, const std::vector<Sweep>& sweeps) {
     const int32_t* d_p = (const int32_t*)(dev + b_tg + b_m);
     const int32_t* d_big = d_p + perms.size();
 
-    const int H = T - L;
-    const size_t smem = ((size_t)1 << T) * sizeof(float4) + ((size_t)1 << H) * sizeof(int64_t);
     static bool attr_set[64] = {false};
     if (!attr_set[s->device & 63]) {
         // largest carveout: three 65 KiB tiles per SM instead of two
@@ -1725,8 +1727,10 @@ int bs_run_sweeps(bs_sim* s, const std::vector<Sweep>& sweeps) {
         attrs((const void*)k_tile_sweep_c64<4, true>);
         cudaFuncSetAttribute(k_dense_big_c64, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
         cudaFuncSetAttribute(k_dense_big, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
-        cudaFuncSetAttribute(k_tile_sweep_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem);
-        cudaFuncSetAttribute(k_tile_sweep_tc, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+        for (auto f : {k_tile_sweep_tc<3>, k_tile_sweep_tc<4>, k_tile_sweep_tc<5>}) {
+            cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem);
+            cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+        }
         attr_set[s->device & 63] = true;
     }
     double2* psi = (double2*)s->state;
@@ -1775,6 +1779,9 @@ int bs_run_sweeps(bs_sim* s, const std::vector<Sweep>& sweeps) {
             continue;
         }
         SweepDesc d{};
+        const int L = ln.low, H = T - L;
+        const size_t smem = ((size_t)1 << T) * sizeof(float4) + ((size_t)1 << H) * sizeof(int64_t);
+        auto ktc = L == 5 ? k_tile_sweep_tc<5> : L == 4 ? k_tile_sweep_tc<4> : k_tile_sweep_tc<3>;
         bs_tile_geometry(d, n_bits, L, ln.hi);
         d.n_gates = ln.n_gates;
         d.gates = d_tg + ln.gate0;
@@ -1787,7 +1794,7 @@ int bs_run_sweeps(bs_sim* s, const std::vector<Sweep>& sweeps) {
         for (int64_t t0 = 0; t0 < ntiles; t0 += (1LL << 30)) {
             int64_t nb = std::min<int64_t>(ntiles - t0, 1LL << 30);
             if (ln.n_tc > 0 && s->capturing) {
-                k_tile_sweep_tc<<<(unsigned)std::min<int64_t>(nb, 2 * 152), kTcThreads, kTcSmem, s->stream>>>(psi, d, t0, t0 + nb);
+                ktc<<<(unsigned)std::min<int64_t>(nb, 2 * 152), kTcThreads, kTcSmem, s->stream>>>(psi, d, t0, t0 + nb);
                 s->stats.tc_launches++;
             } else if (ln.n_tc > 0) {
                 const size_t pe = 2 * s->tc_events_used;
@@ -1798,7 +1805,7 @@ int bs_run_sweeps(bs_sim* s, const std::vector<Sweep>& sweeps) {
                     s->tc_events.push_back(e);
                 }
                 cudaEventRecord(s->tc_events[pe], s->stream);
-                k_tile_sweep_tc<<<(unsigned)std::min<int64_t>(nb, 2 * 152), kTcThreads, kTcSmem, s->stream>>>(psi, d, t0, t0 + nb);
+                ktc<<<(unsigned)std::min<int64_t>(nb, 2 * 152), kTcThreads, kTcSmem, s->stream>>>(psi, d, t0, t0 + nb);
                 cudaEventRecord(s->tc_events[pe + 1], s->stream);
                 s->tc_events_used++;
                 s->stats.tc_launches++;

@@ -196,3 +196,22 @@ def test_fused_matrix_entries_reach_4096(factor, ok):
         else:
             with pytest.raises(Exception, match="out of range"):
                 sim.evolve(ops)
+
+
+@pytest.mark.parametrize("n", [18, 19, 21, 22, 23, 24, 25])
+@pytest.mark.parametrize("ring", [False, True])
+def test_rows_of_a_tile_by_size(n, ring):
+    """Tiles take 5, 4 or 3 low bits by the vector's size and the plan's cost: the state against tiles of 2^11 with 5
+    low bits on the float-float path (double-double sums of about 300 gates: 1e-12 relative)."""
+    rng = np.random.default_rng(300 + n)
+    ops = brick(n, 3, rng)
+    for layer in range(3):
+        for q in range(n):
+            ops.append(bs.Instruction(bs.Ry(float(rng.uniform(-3, 3))), [q]))
+            ops.append(bs.Instruction(bs.CNot() if ring else bs.CPhaseShift(0.4), [q, (q + (1 if ring else 7)) % n]))
+    sim = bs.StateVectorSimulator(n, 0).evolve(ops)
+    assert (sim.last_stats()["tc_gates"] > 0) == (n >= 22)
+    ref = bs.StateVectorSimulator(n, 0)
+    bs.set_tuning(ref, tile_bits=11, tc=0)
+    ref.evolve(ops)
+    assert rel_err(sim.state_vector, ref.state_vector) < TOL
