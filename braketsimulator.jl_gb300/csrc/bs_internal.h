@@ -121,7 +121,9 @@ struct HostGate {                // a gate after lowering to the canonical conve
 };
 
 struct Sweep {
-    int low = BS_TILE_LOW_BITS;  // low contiguous bits of the tile
+    int tile = 0;                // bits of the tile
+    int low = BS_TILE_LOW_BITS;  // the low contiguous ones
+    bool tc = false;             // gates may be fused for the tensor cores
     std::vector<int> hi_bits;    // tile bits above them
     std::vector<HostGate> gates;
 };

@@ -190,15 +190,15 @@ int bs_tile_bits(const bs_sim* s) {
     return (b >= 10 && b <= BS_TILE_MAX_BITS) ? b : BS_TILE_MAX_BITS;
 }
 
-// Complex128 vectors of 11 to 18 bits take smaller tiles where nothing sets the tile bits (and no
-// tensor-core sweeps, which have tiles of 2^12, are asked for): 128 tiles at 16 to 18 bits, 4 to 64 of
+// Complex128 vectors of 11 to 18 bits take smaller tiles where nothing sets the tile bits (the
+// tensor-core sweeps have tiles of 2^12): 128 tiles at 16 to 18 bits, 4 to 64 of
 // 2^9 below, for 152 SMs.  A gate's pass over a tile takes its time per amplitude, which outweighs the
 // launches of the extra sweeps: 17 qubits, 8 ansatz layers, 15 sweeps of 32 tiles (2^12) 0.90 ms, 22 of
 // 128 (2^10) 0.33 ms, with 16 warps a tile and half the products of the real rotations.
 int bs_sweep_tile_bits(const bs_sim* s) {
     const int n = bs_vec_bits(s), b = bs_tile_bits(s);
     if (s->tune.tile_bits >= 0 || getenv("BS_TILE_BITS") || s->precision != BS_PREC_C128) return b;
-    if (n <= 10 || n >= 19 || (bs_tc_enabled(s) && n >= bs_tc_min_bits(s))) return b;
+    if (n <= 10 || n >= 19) return b;
     return std::max(kSmallTileBits, n - 7);
 }
 
@@ -220,7 +220,7 @@ bool bs_tc_enabled(const bs_sim* s) {
 int bs_tc_min_bits(const bs_sim* s) {
     if (s && s->tune.tc_min_bits >= 0) return s->tune.tc_min_bits;
     const char* v = getenv("BS_TC_MIN_BITS");
-    return v ? atoi(v) : 22;   // measured wins from 24 bits up; small states are bound by host planning
+    return v ? atoi(v) : 22;   // some lists from 16 (use_tc)
 }
 
 double bs_tc_cost(const bs_sim* s) {
@@ -313,23 +313,48 @@ double tc_plan_cost(const bs_sim* s, const std::vector<HostGate>& gates, int T, 
     }
     return cost;
 }
+
+// Whether a list runs in tensor-core sweeps: from bs_tc_min_bits vector bits; and, where nothing sets those, below
+// the default of 22 for the lists the float-float path is slowest at, counted in its time for a dense 1-qubit gate.
+// Wide gates (3 and 4 targets, the two-qubit channels of a density matrix among them) from 16 bits: 8-qubit density
+// matrix with channels, 1 layer 0.42 -> 0.21 ms, 10 qubits, 4 layers 5.05 -> 0.87.  Generic complex matrices from 20
+// bits: 6 dense layers of 20 qubits 0.64 -> 0.29 ms, 2 layers 0.23 -> 0.15; at 19 bits with 2 layers they lose what
+// the matrices' forming takes (0.14 both).  Of those lists the error against FP64 is lower too (1.7e-14 of the norm
+// for 3.3e-14 at 20 qubits).  Real rotations and H, which cost the float-float path half, stay there: 21 qubits of
+// them would gain time, but the error grows by up to a fifth.
+bool use_tc(const bs_sim* s, const std::vector<HostGate>& gates, int n_bits) {
+    if (!bs_tc_enabled(s) || s->precision != BS_PREC_C128 || bs_tile_bits(s) != BS_TILE_MAX_BITS || n_bits < BS_TILE_MAX_BITS)
+        return false;
+    if (n_bits >= bs_tc_min_bits(s)) return true;
+    if (n_bits < 16 || s->tune.tc_min_bits >= 0 || getenv("BS_TC_MIN_BITS")) return false;
+    double generic = 0, wide = 0;
+    for (const HostGate& g : gates) {
+        if (g.kind != 0 || (g.k == 1 && bs_class_2x2(g))) continue;
+        const double cost = (double)(1 << g.k) / 2.0;
+        generic += cost;
+        if (g.k >= 3) wide += cost;
+    }
+    return wide >= 24 || (n_bits >= 20 && generic >= 40);
+}
 }  // namespace
 
 // Low contiguous bits of the tiles.  Fewer of them leave more bits to choose, which saves sweeps (each reads and
 // writes the state once), for shorter rows of memory: 512, 256 or 128 bytes of complex128.  At 26 bits the sweeps
 // of a 13-qubit density matrix cost the same with rows of 256 bytes and 5% more with 128 (24 sweeps 24.0 ms, 19
-// sweeps 21.7 and 22.2).  Complex128 vectors of 19 bits and more take 4 low bits (20 bits 0.85 -> 0.82 ms);
-// from 24 bits the tensor-core sweeps take the best of 3, 4 and 5, since how the sweeps' gates group into fused
-// unitaries differs (28-qubit dense circuit: 24 unitaries in 9 sweeps 56.9 ms with 5, 22 in 7 48.4 with 4; 25
-// qubits: 11 in 5 3.67 with 5, 14 in 5 4.12 with 4).  Planning one costs 0.1 ms, too much below.
+// sweeps 21.7 and 22.2).  Complex128 vectors of 19 bits and more take 4 low bits (20 bits 0.85 -> 0.82 ms), as do
+// the tensor-core sweeps; from 24 bits these take the best of 3, 4 and 5, since how the sweeps' gates group into
+// fused unitaries differs (28-qubit dense circuit: 24 unitaries in 9 sweeps 56.9 ms with 5, 22 in 7 48.4 with 4; 25
+// qubits: 11 in 5 3.67 with 5, 14 in 5 4.12 with 4).  The other two plans cost 0.05 to 0.1 ms, too much below.
 // The gates are moved into the sweeps.
 void bs_plan_sweeps(const bs_sim* s, std::vector<HostGate>& gates, std::vector<Sweep>& out) {
-    const int n_bits = bs_vec_bits(s), T = std::min(bs_sweep_tile_bits(s), n_bits);
+    const int n_bits = bs_vec_bits(s);
+    const bool tc = !s->collect && use_tc(s, gates, n_bits);   // not where the plan is for a small run
+    const int T = std::min(tc ? BS_TILE_MAX_BITS : bs_sweep_tile_bits(s), n_bits);
     std::vector<SweepIdx> best, other;
     int low = std::min(BS_TILE_LOW_BITS, T);
-    if (s->precision == BS_PREC_C128 && T == BS_TILE_MAX_BITS && n_bits >= 19) low = 4;
+    if (s->precision == BS_PREC_C128 && T == BS_TILE_MAX_BITS && (tc || n_bits >= 19)) low = 4;
     plan_greedy(gates, n_bits, T, low, best);
-    if (low == 4 && n_bits >= 24 && bs_tc_enabled(s) && n_bits >= bs_tc_min_bits(s)) {
+    if (tc && n_bits >= 24) {
         double cost = tc_plan_cost(s, gates, T, low, best, 1e300);
         for (int L : {5, 3}) {
             plan_greedy(gates, n_bits, T, L, other);
@@ -340,7 +365,9 @@ void bs_plan_sweeps(const bs_sim* s, std::vector<HostGate>& gates, std::vector<S
     }
     for (SweepIdx& b : best) {
         Sweep sw;
+        sw.tile = T;
         sw.low = low;
+        sw.tc = tc;
         sw.hi_bits = std::move(b.hi_bits);
         for (int i : b.gates) sw.gates.push_back(std::move(gates[(size_t)i]));
         out.push_back(std::move(sw));

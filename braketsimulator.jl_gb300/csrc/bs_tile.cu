@@ -1387,7 +1387,7 @@ uint32_t reg_thread_order(const int* bits) {
 int bs_run_sweeps(bs_sim* s, const std::vector<Sweep>& sweeps) {
     if (sweeps.empty()) return BS_OK;
     const int n_bits = bs_vec_bits(s);
-    const int T = std::min(bs_sweep_tile_bits(s), n_bits);
+    const int T = sweeps.front().tile;   // of one plan: all sweeps the same
     // pack: per sweep [TileGate...], then one float4 pool, then one int pool
     std::vector<TileGate> tg;
     std::vector<float4> mats;
@@ -1409,9 +1409,7 @@ int bs_run_sweeps(bs_sim* s, const std::vector<Sweep>& sweeps) {
     std::vector<int32_t> tc_var;             // fused unitary of each variant
     int64_t n_var = 0;
     const bool c64 = s->precision == BS_PREC_C64;
-    // fused tensor-core sweeps from bs_tc_min_bits vector bits up (22 by default: measured wins at
-    // 24, 26, 28 and 30 bits; small states are dominated by host planning)
-    const bool use_tc = bs_tc_enabled(s) && !c64 && T == 12 && n_bits >= bs_tc_min_bits(s);
+    const bool use_tc = sweeps.front().tc;
     const double tc_threshold = bs_tc_cost(s);
     // a sweep left with unfused 3/4-target gates keeps its plain gate list, since the tensor-core sweep
     // kernel carries float-float paths for 1- and 2-target gates only

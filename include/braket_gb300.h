@@ -251,7 +251,7 @@ int bs_batch_destroy(bs_batch* batch);
  *   BS_TUNE_TILE_BITS     10..12  amplitude bits per tile of the sweep kernels (BS_TILE_BITS)
  *   BS_TUNE_TILE_THREADS  256|512 threads per CTA of the float-float sweep (BS_TILE_THREADS)
  *   BS_TUNE_TC            0|1     fused tensor-core sweeps (BS_TC)
- *   BS_TUNE_TC_MIN_BITS   n       vector bits from which they are used (BS_TC_MIN_BITS, 22)
+ *   BS_TUNE_TC_MIN_BITS   n       vector bits from which they are used (BS_TC_MIN_BITS, 22; unset: some lists from 16)
  *   BS_TUNE_TC_COST       x       fuse a block when its float-float cost (dense 1-qubit gates)
  *                                 exceeds x (BS_TC_COST, 2)
  *   BS_TUNE_ADJ_SEGMENTS  S >= 1  bs_adjoint_gradient: forward segments, psi kept after each of the

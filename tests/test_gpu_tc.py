@@ -210,8 +210,33 @@ def test_rows_of_a_tile_by_size(n, ring):
             ops.append(bs.Instruction(bs.Ry(float(rng.uniform(-3, 3))), [q]))
             ops.append(bs.Instruction(bs.CNot() if ring else bs.CPhaseShift(0.4), [q, (q + (1 if ring else 7)) % n]))
     sim = bs.StateVectorSimulator(n, 0).evolve(ops)
-    assert (sim.last_stats()["tc_gates"] > 0) == (n >= 22)
+    assert (sim.last_stats()["tc_gates"] > 0) == (n >= 20)   # 3 layers of generic matrices
     ref = bs.StateVectorSimulator(n, 0)
     bs.set_tuning(ref, tile_bits=11, tc=0)
     ref.evolve(ops)
     assert rel_err(sim.state_vector, ref.state_vector) < TOL
+
+
+@pytest.mark.parametrize("n,kind,wide,layers,tc", [(19, "sv", 0, 3, False), (20, "sv", 0, 2, True), (20, "sv", 0, 1, False),
+                                                   (16, "sv", 2, 0, False), (16, "sv", 3, 0, True), (15, "sv", 3, 0, False),
+                                                   (20, "real", 0, 3, False), (8, "dm", 3, 0, True), (8, "dm", 2, 0, False)])
+def test_lists_below_22_bits(n, kind, wide, layers, tc):
+    """Which lists run on the tensor cores below 22 bits: generic one-qubit matrices from 20 bits, gates on 4 targets
+    (and two-qubit channels) from 16, real rotations not; the states against the oracle."""
+    rng = np.random.default_rng(60 + n)
+    ops = [bs.Instruction(bs.H(), [q]) for q in range(n)]
+    for _ in range(layers):
+        ops += [bs.Instruction(bs.Ry(float(rng.uniform(-3, 3))) if kind == "real" else bs.Unitary(haar(rng)), [q]) for q in range(n)]
+        ops += [bs.Instruction(bs.CZ(), [q, q + 1]) for q in range(n - 1)]
+    for i in range(wide):
+        q = [int(x) for x in rng.permutation(n)[:4]]
+        ops.append(bs.Instruction(bs.TwoQubitDepolarizing(0.02), q[:2]) if kind == "dm" else bs.Instruction(bs.Unitary(haar(rng, 16)), q))
+        ops.append(bs.Instruction(bs.CNot(), q[2:]))
+    if kind == "dm":
+        sim = bs.DensityMatrixSimulator(n, 0, noise_mode="physical").evolve(ops)
+        got, ref = sim.density_matrix, oracle.OracleDM(n, physical=True).evolve(ops).matrix
+    else:
+        sim = bs.StateVectorSimulator(n, 0).evolve(ops)
+        got, ref = sim.state_vector, oracle.OracleSV(n).evolve(ops).psi
+    assert (sim.last_stats()["tc_gates"] > 0) == tc
+    assert rel_err(got, ref) < TOL
