@@ -62,7 +62,7 @@ struct TcBlock {
 // the 32 amplitudes a thread holds in registers.
 //   type 0..2: 2x2 matrix on block bit `bit` (0 complex, 1 all real, 2 real diagonal and imaginary
 //              off-diagonal), 3: X on it, 4: complex 2x2 on the pairs of `mask` only, 5: diagonal, 32
-//              float4 (re, re, -im, im) per variant at `tab`, 6: sign of the patterns in `mask`, 7:
+//              pairs of float4, (re, re, -im, im) in high and in low words, per variant at `tab`, 6: sign of the patterns in `mask`, 7:
 //              diagonal 2x2 on block bit `bit`.
 //   Types 3 and 4 act on the pairs p of `mask` (pair p: block pattern p with a zero put in at `bit`).
 //   Controls outside the block: (thread's tile position & lc_mask) == lc_val and (base & gc_mask) == gc_val.

@@ -7,16 +7,17 @@
 // the gate is D[128 x 64] = A[128 x 64] * U_real^T, one tcgen05 GEMM per tile.
 //
 // Exactness (Ozaki-style split): the tile is scaled by a power of two (from the
-// largest exponent over the tile) so that |x| < 2^8, and both x and U_real (on
-// the device, from the FP64 matrix) are split into six balanced 9-bit digits, digit j carried as bf16 d_j * 2^(-9j) with
-// |d_j| <= 256, which 8 significant bits hold exactly.
+// largest exponent over the tile) so that |x| < 2^8, and both x and U_real (by
+// k_tc_digits, from the FP64 matrix) are split into six balanced 9-bit digits,
+// digit j carried as bf16 d_j * 2^(-9j) with |d_j| <= 256, which 8 significant
+// bits hold exactly.
 // The 21 digit pairs with i + j <= 5 are accumulated in five rounds by digit
 // weight: i+j = 0, 1, 2, 3 each alone (every product a multiple of the same
 // power of two and every partial sum at most 4 * 64 * 2^16 = 2^24 of it, so
 // these FP32 sums are exact) and i+j = 4, 5 together (rounding at 2^-59 of the
 // result).  8-bit digits left two of those 24 bits unused and took 26 pairs
-// for less precision (TODO).  After
-// each round the CUDA cores fold the FP32 accumulator into a running
+// for less precision (28-qubit dense circuit: sweeps 80.1 -> 78.3 ms, error of
+// its expectation values 7.9e-14 -> 8e-15).  After each round the CUDA cores fold the FP32 accumulator into a running
 // float-float sum, while the tensor cores run other rounds in the other of two
 // accumulators; two threads issue, one per accumulator, so that neither chain
 // of issue, fold and re-issue waits for the other.  What remains is the 48-bit

@@ -1013,11 +1013,12 @@ __device__ __forceinline__ void reg_ops(f2 (&v)[32], const RegOp* op, int n, con
                 const int b = op->ub[u];
                 var |= (b < 64 ? (jt >> b) & 1 : (int)((base >> (b - 64)) & 1)) << u;
             }
-            const float4* t = tabs + op->tab + 32 * var;
+            const float4* t = tabs + op->tab + 64 * var;
 #pragma unroll
             for (int c = 0; c < 32; c++) {
-                const float4 d = __ldg(t + c);
-                v[c] = fma2(pk(d.z, d.w), swap2(v[c]), mul2(pk(d.x, d.y), v[c]));
+                const float4 d = __ldg(t + 2 * c), e = __ldg(t + 2 * c + 1);   // high words, low words
+                const f2 w = swap2(v[c]);
+                v[c] = fma2(pk(d.z, d.w), w, fma2(pk(d.x, d.y), v[c], fma2(pk(e.z, e.w), w, mul2(pk(e.x, e.y), v[c]))));
             }
         } else {
             const uint32_t mask = op->mask;
@@ -1457,7 +1458,8 @@ int bs_run_sweeps(bs_sim* s, const std::vector<Sweep>& sweeps) {
                 // type.  Blocks without folded diagonals always win (their operations are cheaper than a
                 // pass); sweeps of many diagonals on scattered bits (16 of them a ring layer, where the
                 // blocks took 62 us a sweep at 22 qubits against 47) or of 2- to 4-target dense gates may
-                // not, and keep the pass per (fused) gate.
+                // not, and keep the pass per (fused) gate.  The tables' low words (6% of a 22-qubit gradient) are
+                // not counted: without the blocks these gates would be rounded to single precision.
                 static const double op_cost[8] = {480, 230, 320, 260, 550, 480, 250, 320};
                 bs_block_c64(sw.gates, local, T, items, blocks, tabs, drift);
                 double with = 0;
