@@ -79,6 +79,7 @@ struct MapStage {
     }
 };
 thread_local MapStage t_map;
+thread_local bool t_no_map = false;
 std::atomic<int64_t> g_ticket{0};   // tickets are never used twice
 bool map_stage() {
     if (t_map.h) return true;
@@ -95,9 +96,11 @@ bool map_stage() {
 }
 }  // namespace
 
+void bs_thread_without_map() { t_no_map = true; }
+
 MapSlot bs_map_slot(size_t bytes) {
     MapSlot m;
-    if (256 + bytes > kOutStage || !map_stage()) return m;
+    if (t_no_map || 256 + bytes > kOutStage || !map_stage()) return m;
     m.h = t_map.h + 256;
     m.d = t_map.d + 256;
     m.word = reinterpret_cast<volatile int64_t*>(t_map.h);
@@ -144,11 +147,15 @@ int bs_ensure_scratch(bs_sim* s, int64_t bytes) {
     if (s->scratch) cudaFree(s->scratch);
     s->scratch = nullptr;
     s->scratch_bytes = 0;
-    int rc = bs_cuda_check(s, cudaMalloc(&s->scratch, (size_t)bytes), "scratch allocation");
+    // the counter of bs_scratch_counter lies behind it: an allocation of its own was 0.1 ms of every handle
+    bytes = (bytes + 255) & ~(int64_t)255;
+    int rc = bs_cuda_check(s, cudaMalloc(&s->scratch, (size_t)bytes + 256), "scratch allocation");
     if (rc) return rc;
     s->scratch_bytes = bytes;
-    return BS_OK;
+    return bs_cuda_check(s, cudaMemsetAsync((char*)s->scratch + bytes, 0, 256, s->stream), "counter reset");
 }
+
+unsigned* bs_scratch_counter(const bs_sim* s) { return (unsigned*)((char*)s->scratch + s->scratch_bytes); }
 int bs_ensure_plan(bs_sim* s, int64_t bytes) {
     if (s->plan_bytes >= bytes) return BS_OK;
     if (s->capturing) return bs_fail(s, BS_ERR_STATE, "plan buffer growth during graph capture");
@@ -162,14 +169,6 @@ int bs_ensure_plan(bs_sim* s, int64_t bytes) {
     if (rc) return rc;
     s->plan_bytes = b;
     return BS_OK;
-}
-
-int bs_ensure_counter(bs_sim* s) {
-    if (s->counter) return BS_OK;
-    if (s->capturing) return bs_fail(s, BS_ERR_STATE, "counter allocation during graph capture");
-    int rc = bs_cuda_check(s, cudaMalloc((void**)&s->counter, 256), "counter allocation");
-    if (rc) return rc;
-    return bs_cuda_check(s, cudaMemsetAsync(s->counter, 0, 256, s->stream), "counter reset");
 }
 
 namespace {
@@ -282,7 +281,6 @@ int bs_destroy(bs_sim* s) {
     if (s->plan_buf) cudaFree(s->plan_buf);
     if (s->adj_work) cudaFree(s->adj_work);
     if (s->dev_flag) cudaFree(s->dev_flag);
-    if (s->counter) cudaFree(s->counter);
     if (s->alias_ap) cudaFree(s->alias_ap);
     if (s->alias_ix) cudaFree(s->alias_ix);
     if (s->ev0) cudaEventDestroy(s->ev0);

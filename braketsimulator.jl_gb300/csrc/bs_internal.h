@@ -181,7 +181,6 @@ struct bs_sim {
     int64_t plan_bytes = 0;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     int* dev_flag = nullptr;      // device error flag of the tensor-core sweeps
-    unsigned* counter = nullptr;  // bs_ensure_counter
     bool flag_armed = false;
     std::vector<cudaEvent_t> tc_events;   // pool: an event pair around each tensor-core launch
     size_t tc_events_used = 0;            // pairs recorded since the last bs_collect_tc_time
@@ -227,13 +226,16 @@ struct MapSlot {
     int64_t ticket = 0;
 };
 MapSlot bs_map_slot(size_t bytes);
+// Called by a thread that lives for one call: its results take the copy, since mapping memory for it costs more.
+void bs_thread_without_map();
 // Polls for the slot's ticket; after 2 s (a failed or very long kernel) synchronises the stream, which
 // reports the error.
 int bs_wait_ticket(bs_sim* s, const MapSlot& m, const char* what);
 int bs_ensure_scratch(bs_sim* s, int64_t bytes);
 int bs_ensure_plan(bs_sim* s, int64_t bytes);
-// The counter with which the last block of an expectation is found (zero between calls), allocated on first use.
-int bs_ensure_counter(bs_sim* s);
+// The counter with which the last block of an expectation is found (zero between calls), behind the scratch buffer
+// (after bs_ensure_scratch).
+unsigned* bs_scratch_counter(const bs_sim* s);
 // Pinned host region for one upload of `bytes`; call bs_stage_done after queuing the copy.
 char* bs_stage(bs_sim* s, size_t bytes);
 void bs_stage_done(bs_sim* s);

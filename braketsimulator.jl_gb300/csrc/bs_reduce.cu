@@ -516,14 +516,12 @@ int bs_expectation_pauli(bs_sim* s, int n_terms, const uint64_t* xmask, const ui
     const int nb = (int)std::max<int64_t>(1, std::min<int64_t>((dim + 4 * kRThreads - 1) / (4 * kRThreads), 152 * 4));
     int rc = bs_ensure_scratch(s, ((int64_t)nb * n_terms + n_terms) * 8);
     if (rc) return rc;
-    rc = bs_ensure_counter(s);
-    if (rc) return rc;
     double* partial = (double*)s->scratch;
     double* res = partial + (int64_t)nb * n_terms;
     unsigned launches = 0;
     for (auto& kv : groups) launches += (unsigned)((kv.second.size() + kMaxTermsPerPass - 1) / kMaxTermsPerPass);
     const MapSlot slot = s->capturing ? MapSlot{} : bs_map_slot((size_t)n_terms * 8);
-    const Finish fin{slot.h ? (double*)slot.d : res, s->counter, launches * (unsigned)nb, slot.dword, slot.ticket};
+    const Finish fin{slot.h ? (double*)slot.d : res, bs_scratch_counter(s), launches * (unsigned)nb, slot.dword, slot.ticket};
     for (auto& kv : groups) {
         const std::vector<int>& ts = kv.second;
         for (size_t c0 = 0; c0 < ts.size(); c0 += kMaxTermsPerPass) {
