@@ -143,3 +143,19 @@ def test_captured_batch_autotune_keeps_results():
         # every tuning computes the same state to 1e-12; shots may differ only at exact CDF ties
         assert np.max(np.abs(exp - ref)) < 1e-11
         assert np.mean(smp == smp_ref) > 0.99
+
+
+@pytest.mark.parametrize("per,precision,tol", [(682, "c128", 1e-12), (683, "c128", 1e-12), (683, "c64", 2e-5)])
+def test_batch_on_four_and_eight_handles(per, precision, tol):
+    """12 circuits of 13 qubits with 8184 instructions in all run on 4 handles, with 8196 on 8."""
+    rng = np.random.default_rng(per)
+    n = 13
+    circuits, obs = [], []
+    for _ in range(12):
+        ins = [bs.Instruction([bs.Rx, bs.Ry, bs.Rz][int(rng.integers(3))](float(rng.uniform(-3, 3))), [int(rng.integers(n))])
+               if i % 3 else bs.Instruction(bs.CNot(), [int(x) for x in rng.choice(n, 2, replace=False)]) for i in range(per)]
+        circuits.append(ins)
+        obs.append([{int(q): "XYZ"[rng.integers(3)] for q in rng.choice(n, 2, replace=False)} for _ in range(3)])
+    exp, _, _ = bs.batch_simulate(circuits, [n] * 12, obs, shots=10, seed=2, precision=precision)
+    for c in range(12):
+        assert np.max(np.abs(exp[c] - exact(circuits[c], n, obs[c])[0])) < tol
