@@ -154,11 +154,6 @@ __device__ __forceinline__ f2 mul2(f2 a, f2 b) {
     asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
     return d;
 }
-__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
-    f2 d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
 // complex MAC into two accumulators: (ar, ai) += m * x, m = (mrh+mrl) + i(mih+mil)
 __device__ __forceinline__ void cmac_first(ffacc& ar, ffacc& ai, const cff& m, const cff& x) {
     acc_first(ar, m.rh, m.rl, x.rh, x.rl);

@@ -357,349 +357,6 @@ void bs_fuse_small(const std::vector<HostGate>& in, const int* local, double pas
 }
 
 namespace {
-
-// What a register block needs to know of a gate.
-struct RegGate {
-    enum Kind { kOneBit, kSwap, kDiag, kOther } kind = kOther;
-    uint64_t hard = 0;    // bits it moves amplitudes along: must be block bits
-    uint64_t soft = 0;    // controls and diagonal bits: read from the index anywhere
-};
-
-bool plain_swap(const HostGate& g) {
-    return g.kind == 2 && g.k == 2 && g.cmask == 0 && g.perm.size() == 8 && g.perm[0] == 0 && g.perm[1] == 0 &&
-           g.perm[2] == 2 && g.perm[3] == 0 && g.perm[4] == 1 && g.perm[5] == 0 && g.perm[6] == 3 && g.perm[7] == 0;
-}
-bool sign_only(const HostGate& g) {   // Z on one bit, any controls
-    return g.kind == 1 && g.k == 1 && g.mat[0] == 1.0 && g.mat[1] == 0.0 && g.mat[2] == -1.0 && g.mat[3] == 0.0;
-}
-
-RegGate reg_gate(const HostGate& g) {
-    RegGate r;
-    uint64_t t = 0;
-    for (int q = 0; q < g.k; q++) t |= 1ULL << g.ebit[q];
-    if (g.kind == 1) {
-        const int nb = __builtin_popcountll(t | g.cmask);
-        if (nb <= 2 || sign_only(g)) {
-            r.kind = RegGate::kDiag;
-            r.soft = t | g.cmask;
-        } else {
-            r.soft = t | g.cmask;
-        }
-    } else {
-        r.hard = t;
-        r.soft = g.cmask;
-        if (g.kind <= 2 && g.k == 1) r.kind = RegGate::kOneBit;
-        else if (plain_swap(g)) r.kind = RegGate::kSwap;
-    }
-    return r;
-}
-
-void matrix_2x2(const HostGate& g, cd* m) {
-    for (int i = 0; i < 4; i++) m[i] = 0;
-    if (g.kind == 0) {
-        for (int i = 0; i < 4; i++) m[i] = cd(g.mat[2 * i], g.mat[2 * i + 1]);
-    } else if (g.kind == 1) {
-        m[0] = cd(g.mat[0], g.mat[1]);
-        m[3] = cd(g.mat[2], g.mat[3]);
-    } else {
-        static const cd ipow[4] = {cd(1, 0), cd(0, 1), cd(-1, 0), cd(0, -1)};
-        for (int c = 0; c < 2; c++) m[g.perm[2 * c] * 2 + c] = ipow[g.perm[2 * c + 1] & 3];
-    }
-}
-
-bool complex_2x2(const cd* m) {
-    const bool dr = m[0].imag() == 0.0 && m[3].imag() == 0.0;
-    return !(dr && m[1].imag() == 0.0 && m[2].imag() == 0.0) && !(dr && m[1].real() == 0.0 && m[2].real() == 0.0) &&
-           !(m[1] == 0.0 && m[2] == 0.0);
-}
-
-// The gates of one block in order, turned into operations.  One-bit gates without controls that meet on
-// the same bit are multiplied out in FP64 where that saves work; diagonal gates fold into one table while they commute back
-// to it; signs with the same outside controls fold into one mask.
-struct BlockBuilder {
-    int pos[64];                      // block bit of an endian bit, or -1
-    const int* local;
-    std::vector<RegOp> ops;
-    std::vector<std::vector<cd>> tab; // per op (type 5): its table, variant-major
-    std::vector<cd> mats;             // per op (types 0..4): 2x2 in FP64
-    std::vector<uint64_t> hard, soft; // per op, endian bits
-
-    void push(const RegOp& o, const cd* m, std::vector<cd> t, uint64_t h, uint64_t s) {
-        ops.push_back(o);
-        for (int i = 0; i < 4; i++) mats.push_back(m ? m[i] : cd(0, 0));
-        tab.push_back(std::move(t));
-        hard.push_back(h);
-        soft.push_back(s);
-    }
-    void outside_controls(RegOp& o, uint64_t cmask, uint64_t cval) const {
-        for (uint64_t r = cmask; r; r &= r - 1) {
-            const int e = __builtin_ctzll(r);
-            if (pos[e] >= 0) continue;
-            const uint32_t v = (uint32_t)((cval >> e) & 1ULL);
-            if (local[e] >= 0) { o.lc_mask |= (uint16_t)(1u << local[e]); o.lc_val |= (uint16_t)(v << local[e]); }
-            else { o.gc_mask |= 1ULL << e; o.gc_val |= (uint64_t)v << e; }
-        }
-    }
-    // pairs of block bit b whose pattern meets the controls inside the block
-    uint32_t pair_mask(int b, uint64_t cmask, uint64_t cval) const {
-        uint32_t m = 0;
-        for (uint32_t p = 0; p < 16; p++) {
-            const uint32_t c = ((p >> b) << (b + 1)) | (p & ((1u << b) - 1u));
-            bool ok = true;
-            for (uint64_t r = cmask; r; r &= r - 1) {
-                const int e = __builtin_ctzll(r);
-                if (pos[e] >= 0 && ((c >> pos[e]) & 1u) != (uint32_t)((cval >> e) & 1ULL)) ok = false;
-            }
-            if (ok) m |= 1u << p;
-        }
-        return m;
-    }
-    void one_bit(const HostGate& g) {
-        const int e = g.ebit[0], b = pos[e];
-        const uint64_t h = 1ULL << e;
-        cd m[4];
-        matrix_2x2(g, m);
-        if (!g.cmask) {
-            // the last operation on this bit, if it is a one-bit gate without controls
-            for (int i = (int)ops.size() - 1; i >= 0; i--) {
-                if (!((hard[(size_t)i] | soft[(size_t)i]) & h)) continue;
-                if (hard[(size_t)i] == h && soft[(size_t)i] == 0 && ops[(size_t)i].type <= 3) {
-                    cd* a = &mats[4 * (size_t)i];
-                    const cd r[4] = {m[0] * a[0] + m[1] * a[2], m[0] * a[1] + m[1] * a[3], m[2] * a[0] + m[3] * a[2],
-                                     m[2] * a[1] + m[3] * a[3]};
-                    // two gates of the cheap classes stay two where their product is a full complex matrix
-                    // (as many instructions, and their shape can be kept)
-                    if (complex_2x2(r) && !complex_2x2(a) && !complex_2x2(m)) break;
-                    for (int q = 0; q < 4; q++) a[q] = r[q];
-                    return;
-                }
-                break;
-            }
-        }
-        RegOp o{};
-        o.bit = (uint8_t)b;
-        o.mask = pair_mask(b, g.cmask, g.cval);
-        outside_controls(o, g.cmask, g.cval);
-        push(o, m, {}, h, g.cmask);
-    }
-    void diag(const HostGate& g) {
-        uint64_t bits = g.cmask;
-        for (int q = 0; q < g.k; q++) bits |= 1ULL << g.ebit[q];
-        if (sign_only(g)) {
-            uint32_t mask = 0;
-            for (uint32_t c = 0; c < 32; c++) {
-                bool ok = true;
-                for (uint64_t r = bits; r; r &= r - 1) {
-                    const int e = __builtin_ctzll(r);
-                    const uint32_t want = ((g.cmask >> e) & 1ULL) ? (uint32_t)((g.cval >> e) & 1ULL) : 1u;
-                    if (pos[e] >= 0 && ((c >> pos[e]) & 1u) != want) ok = false;
-                }
-                if (ok) mask |= 1u << c;
-            }
-            RegOp o{};
-            o.type = 6;
-            o.mask = mask;
-            outside_controls(o, bits, g.cval | (bits & ~g.cmask));
-            for (int i = (int)ops.size() - 1; i >= 0 && !(hard[(size_t)i] & bits); i--) {
-                RegOp& p = ops[(size_t)i];
-                if (p.type == 6 && p.lc_mask == o.lc_mask && p.lc_val == o.lc_val && p.gc_mask == o.gc_mask && p.gc_val == o.gc_val) {
-                    p.mask ^= mask;
-                    soft[(size_t)i] |= bits;
-                    return;
-                }
-            }
-            push(o, nullptr, {}, 0, bits);
-            return;
-        }
-        uint64_t out = 0;
-        for (uint64_t r = bits; r; r &= r - 1) if (pos[__builtin_ctzll(r)] < 0) out |= r & (0 - r);
-        // back to a table this gate commutes with, if the bits outside the block stay at most two
-        int at = -1;
-        for (int i = (int)ops.size() - 1; i >= 0 && !(hard[(size_t)i] & bits); i--)
-            if (ops[(size_t)i].type == 5 && __builtin_popcountll(outside(i) | out) <= 2) { at = i; break; }
-        if (at < 0 && g.k == 1 && !g.cmask && pos[g.ebit[0]] >= 0) {   // Rz, S, T, ... on a block bit
-            one_bit(g);
-            return;
-        }
-        if (at < 0) {
-            RegOp o{};
-            o.type = 5;
-            push(o, nullptr, std::vector<cd>(32, cd(1, 0)), 0, 0);
-            at = (int)ops.size() - 1;
-        }
-        widen(at, out);
-        RegOp& o = ops[(size_t)at];
-        soft[(size_t)at] |= bits;
-        for (int v = 0; v < (1 << o.nu); v++)
-            for (uint32_t c = 0; c < 32; c++) {
-                auto bit_of = [&](int e) -> int {
-                    if (pos[e] >= 0) return (int)((c >> pos[e]) & 1u);
-                    for (int u = 0; u < o.nu; u++) if (o.ub[u] == code(e)) return (v >> u) & 1;
-                    return 0;
-                };
-                bool ok = true;
-                for (uint64_t r = g.cmask; r; r &= r - 1) {
-                    const int e = __builtin_ctzll(r);
-                    if (bit_of(e) != (int)((g.cval >> e) & 1ULL)) ok = false;
-                }
-                if (!ok) continue;
-                int di = 0;
-                for (int q = 0; q < g.k; q++) di |= bit_of(g.ebit[q]) << q;
-                tab[(size_t)at][(size_t)v * 32 + c] *= cd(g.mat[2 * di], g.mat[2 * di + 1]);
-            }
-    }
-    int code(int e) const { return local[e] >= 0 ? local[e] : 64 + e; }
-    uint64_t outside(int i) const {
-        uint64_t m = 0;
-        for (int e = 0; e < 64; e++)
-            for (int u = 0; u < ops[(size_t)i].nu; u++) if (pos[e] < 0 && code(e) == ops[(size_t)i].ub[u]) m |= 1ULL << e;
-        return m;
-    }
-    void widen(int i, uint64_t out) {
-        for (uint64_t r = out & ~outside(i); r; r &= r - 1) {
-            RegOp& o = ops[(size_t)i];
-            o.ub[o.nu] = (int16_t)code(__builtin_ctzll(r));
-            std::vector<cd>& t = tab[(size_t)i];
-            t.insert(t.end(), t.begin(), t.begin() + (long)(32 << o.nu));
-            o.nu++;
-        }
-    }
-    // FP32 matrix entries are off by up to 2^-25, equal gates (every H) by the same amount, and after a few
-    // hundred gates that is the larger part of a complex64 state's error (18 qubits, 30 layers: 1e-6 of
-    // the expectation values from rounded matrices, 2e-7 from rounded states).  So a common factor near
-    // 1 is chosen whose rounded entries keep the matrix's shape, which works where few entries differ
-    // (real, real/imaginary and diagonal matrices); the size error that leaves (`drift`) goes into the
-    // next factor, so it does not add up.  A table's 32 entries have no such factor and carry low words
-    // (22-qubit gradient, 30 inputs: error of the energy 7.0e-8 -> 5.5e-8 of the Hamiltonian's norm, of the
-    // gradient 4.7e-7 -> 4.0e-7, before register blocks 6.7e-8 and 5.7e-7; 6.84 -> 7.29 ms).
-    void finish(RegBlock& b, std::vector<float4>& tabs, double& drift) {
-        for (size_t i = 0; i < ops.size(); i++) {
-            RegOp o = ops[i];
-            const cd* m = &mats[4 * i];
-            const bool whole = !o.lc_mask && !o.gc_mask && o.mask == 0xffffu;
-            if (o.type == 5) {
-                o.tab = (int32_t)tabs.size();
-                for (const cd& e : tab[i]) {
-                    const float re = (float)e.real(), im = (float)e.imag();
-                    tabs.push_back(make_float4(re, re, -im, im));
-                    const float rl = (float)(e.real() - (double)re), il = (float)(e.imag() - (double)im);
-                    tabs.push_back(make_float4(rl, rl, -il, il));
-                }
-            } else if (o.type != 6) {
-                double e[8], n2 = 0;
-                for (int q = 0; q < 4; q++) { e[2 * q] = m[q].real(); e[2 * q + 1] = m[q].imag(); }
-                for (double x : e) n2 += x * x;
-                const bool x = m[0] == 0.0 && m[3] == 0.0 && m[1] == 1.0 && m[2] == 1.0;
-                const bool dr = e[1] == 0.0 && e[7] == 0.0;
-                if (x) o.type = 3;
-                else if (o.mask != 0xffffu) o.type = 4;
-                else if (dr && e[3] == 0.0 && e[5] == 0.0) o.type = 1;
-                else if (dr && e[2] == 0.0 && e[4] == 0.0) o.type = 2;
-                else if (e[2] == 0.0 && e[3] == 0.0 && e[4] == 0.0 && e[5] == 0.0) o.type = 7;
-                else o.type = 0;
-                double fix = 1.0;
-                if (whole && !x && n2 > 0) {
-                    double best = 0, best_fix = 1.0, best_drift = drift;
-                    const double f0 = 1.0 / (1.0 + drift);
-                    for (int k = -8; k <= 8; k++) {
-                        const double f = f0 * (1.0 + k * 0x1p-26);
-                        // R = rounded entries; its size against e, and its distance from e at that size
-                        double r2 = 0, re = 0;
-                        for (double v : e) { const double d = (double)(float)(v * f) - v; r2 += d * d; re += d * v; }
-                        const double rel = re / n2;                          // size error, to first order
-                        const double dn = drift + rel;
-                        const double cost = r2 / n2 - rel * rel + dn * dn / 16.0;   // shape, and the size error carried on
-                        if (k == -8 || cost < best) { best = cost; best_fix = f; best_drift = dn; }
-                    }
-                    fix = best_fix;
-                    drift = best_drift;
-                }
-                for (int q = 0; q < 8; q++) o.m[q] = (float)(e[q] * fix);
-            }
-            b.ops.push_back(o);
-        }
-    }
-};
-
-}  // namespace
-
-// Greedy, as the sweep planner: a block takes every gate, in order, that commutes with all the gates it
-// leaves behind and whose moved bits fit into 5 block bits; diagonal gates and controls need no block bit.
-void bs_block_c64(const std::vector<HostGate>& in, const int* local, int T, std::vector<RegItem>& items,
-                  std::vector<RegBlock>& blocks, std::vector<float4>& tabs, double& drift) {
-    const size_t G = in.size();
-    std::vector<RegGate> info(G);
-    for (size_t i = 0; i < G; i++) info[i] = reg_gate(in[i]);
-    std::vector<char> done(G, 0);
-    int tile_e[16];
-    for (int p = 0; p < 16; p++) tile_e[p] = -1;
-    for (int e = 0; e < 64; e++) if (local[e] >= 0 && local[e] < T) tile_e[local[e]] = e;
-    for (size_t first = 0; first < G;) {
-        if (done[first]) { first++; continue; }
-        if (info[first].kind == RegGate::kOther) {
-            RegItem it;
-            it.gate = (int)first;
-            items.push_back(it);
-            done[first] = 1;
-            continue;
-        }
-        uint64_t bits = 0, left_hard = 0, left_any = 0, wish = 0;
-        std::vector<size_t> take;
-        for (size_t i = first; i < G; i++) {
-            if (done[i]) continue;
-            const RegGate& r = info[i];
-            const bool ok = r.kind != RegGate::kOther && !(r.hard & left_any) && !(r.soft & left_hard) &&
-                            __builtin_popcountll(bits | r.hard) <= 5;
-            if (!ok) {
-                left_hard |= r.hard;
-                left_any |= r.hard | r.soft;
-                continue;
-            }
-            bits |= r.hard;
-            wish |= r.soft;
-            take.push_back(i);
-            done[i] = 1;
-        }
-        // fill up with tile bits the gates read (as block bits they need no outside control), then others
-        for (int e = 0; e < 64 && __builtin_popcountll(bits) < 5; e++)
-            if (((wish >> e) & 1ULL) && local[e] >= 0) bits |= 1ULL << e;
-        for (int p = T - 1; p >= 0 && __builtin_popcountll(bits) < 5; p--)
-            if (tile_e[p] >= 0) bits |= 1ULL << tile_e[p];
-        RegBlock b;
-        BlockBuilder bb;
-        bb.local = local;
-        for (int e = 0; e < 64; e++) bb.pos[e] = -1;
-        int nb = 0;
-        for (int p = 0; p < T && nb < 5; p++)
-            if (tile_e[p] >= 0 && ((bits >> tile_e[p]) & 1ULL)) { bb.pos[tile_e[p]] = nb; b.bits[nb++] = p; }
-        for (size_t i : take) {
-            const HostGate& g = in[i];
-            if (info[i].kind == RegGate::kDiag) {
-                bb.diag(g);
-            } else if (info[i].kind == RegGate::kSwap) {
-                // three controlled X
-                for (int s = 0; s < 3; s++) {
-                    HostGate x;
-                    x.kind = 2;
-                    x.k = 1;
-                    x.perm = {1, 0, 0, 0};
-                    x.ebit[0] = g.ebit[s & 1];
-                    x.cmask = x.cval = 1ULL << g.ebit[1 - (s & 1)];
-                    bb.one_bit(x);
-                }
-            } else {
-                bb.one_bit(g);
-            }
-        }
-        bb.finish(b, tabs, drift);
-        RegItem it;
-        it.block = (int)blocks.size();
-        blocks.push_back(std::move(b));
-        items.push_back(it);
-    }
-}
-
-namespace {
 // Upper bound of the largest singular value of a gate's matrix (sqrt(|A^H A|_inf) up to 4x4, which is 1 for a
 // unitary one; else the smaller of the Frobenius norm and sqrt(|A|_1 |A|_inf)); infinite if an entry is not finite.
 double norm_bound(const HostGate& g) {

@@ -19,8 +19,6 @@
 //   kind 3: a run of CZ gates applied as one parity phase (npar, pshift, pmask)
 //   kind 4: fused dense unitary on 5 tile-local bits gbit[0..4] (matrix bit j <-> gbit[j]),
 //           applied on the tensor cores from the bf16 digit slices at tc_off (48 KiB blocks)
-//   kind 8: register block (complex64): tile bits gbit[0..4] are held in registers, perm_off: the 7 other
-//           tile bits in thread-index order, 4 bits each; the sweep's rops[mat_off .. mat_off + k) are applied
 //   kind 5: Kraus channel on k <= 2 targets in the reference's block-diagonal update rule
 //           (density matrix): tbit[0..2k-1] row then column target bits, pmask[0..1], its superoperator
 //           at mat_off
@@ -58,25 +56,6 @@ struct TcBlock {
     int32_t part0, n_parts, var0, gate;
 };
 
-// One operation of a register block (TileGate kind 8, complex64 sweeps): the block's 5 tile bits index
-// the 32 amplitudes a thread holds in registers.
-//   type 0..2: 2x2 matrix on block bit `bit` (0 complex, 1 all real, 2 real diagonal and imaginary
-//              off-diagonal), 3: X on it, 4: complex 2x2 on the pairs of `mask` only, 5: diagonal, 32
-//              pairs of float4, (re, re, -im, im) in high and in low words, per variant at `tab`, 6: sign of the patterns in `mask`, 7:
-//              diagonal 2x2 on block bit `bit`.
-//   Types 3 and 4 act on the pairs p of `mask` (pair p: block pattern p with a zero put in at `bit`).
-//   Controls outside the block: (thread's tile position & lc_mask) == lc_val and (base & gc_mask) == gc_val.
-struct RegOp {
-    uint8_t type, bit, nu, pad;  // nu (type 5): bits outside the block that select the variant
-    uint32_t mask;
-    uint16_t lc_mask, lc_val;
-    int16_t ub[2];               // tile position, or 64 + endian bit of the base
-    int32_t tab;
-    int32_t pad2;
-    uint64_t gc_mask, gc_val;
-    float m[8];                  // m00, m01, m10, m11 as (re, im)
-};
-
 struct SweepDesc {
     int32_t n_bits;             // endian bits of the vector (n for SV, 2n for DM)
     int32_t T;                  // tile bits
@@ -89,8 +68,6 @@ struct SweepDesc {
     const float4* mats;         // device, complex float-float entries (rh, rl, ih, il)
     const int32_t* perms;       // device
     const uint16_t* tc_pool;    // device, kind-4 digit slices (24576 bf16 per gate)
-    const RegOp* rops;          // device, operations of the sweep's register blocks (kind 8)
-    int32_t n_rops;
     int* err;                   // device flag: a bounded tensor-core wait gave up
 };
 
@@ -280,18 +257,6 @@ double bs_tc_cost(const bs_sim* s);
 double bs_fuse_tc(const std::vector<const HostGate*>& in, const int* local, int T, double threshold,
                   std::vector<HostGate>* out);   // out null: only the list's cost, in fused unitaries
 void bs_fuse_small(const std::vector<HostGate>& in, const int* local, double pass, int maxk, std::vector<HostGate>& out);
-// Grouping of a complex64 sweep's gates into register blocks: items in order, each a block (index into
-// blocks) or a gate left to its own pass (index into in); tabs collects the diagonal tables.
-struct RegBlock {
-    int bits[5];                 // tile positions, ascending; block bit q <-> bits[q]
-    std::vector<RegOp> ops;
-};
-struct RegItem {
-    int block = -1, gate = -1;
-};
-// drift: relative size error of the one-bit matrices rounded to FP32 so far, carried from sweep to sweep.
-void bs_block_c64(const std::vector<HostGate>& in, const int* local, int T, std::vector<RegItem>& items,
-                  std::vector<RegBlock>& blocks, std::vector<float4>& tabs, double& drift);
 // Whether every entry of a fused gate's matrices is finite and below 2^12 (in: the list that was fused).
 bool bs_tc_in_range(const HostGate& f, const std::vector<HostGate>& in);
 

@@ -778,9 +778,6 @@ inline void split_d(double x, float& h, float& l) {
 // ---------------------------------------------------------------------------
 // complex64 states: the same tiles and gate tables, FP32 complex arithmetic
 // (the matrix entries are the FP32-rounded hi parts of the float-float table).
-// The tile is stored with bits 4..11 folded into bits 0..3 (linear over XOR, a bijection), so that 16
-// lanes of a half-warp that differ in 4 tile bits of distinct residues mod 4 hit 16 distinct banks.
-__device__ __forceinline__ int sw64(int j) { return j ^ (((j >> 4) ^ (j >> 8)) & 15); }
 __device__ __forceinline__ float2 c64_mul(float4 m, float2 x) {
     return make_float2(fmaf(m.x, x.x, -m.z * x.y), fmaf(m.x, x.y, m.z * x.x));
 }
@@ -831,7 +828,7 @@ __device__ void tile_dense_c64(float2* sm, int T, const TileGate& g, const float
 #pragma unroll
             for (int q = 0; q < K; q++) if ((c >> q) & 1) j |= 1 << tb[q];
             idx[c] = j;
-            x[c] = sm[sw64(j)];
+            x[c] = sm[j];
         }
 #pragma unroll
         for (int r = 0; r < D; r++) {
@@ -844,7 +841,7 @@ __device__ void tile_dense_c64(float2* sm, int T, const TileGate& g, const float
                 re = fmaf(ar, x[c].x, fmaf(-ai, x[c].y, re));
                 im = fmaf(ar, x[c].y, fmaf(ai, x[c].x, im));
             }
-            sm[sw64(idx[r])] = make_float2(re, im);
+            sm[idx[r]] = make_float2(re, im);
         }
     }
 }
@@ -874,7 +871,7 @@ __device__ void tile_mono_c64(float2* sm, int T, const TileGate& g, const int32_
 #pragma unroll
             for (int q = 0; q < K; q++) if ((c >> q) & 1) j |= 1 << tb[q];
             idx[c] = j;
-            x[c] = sm[sw64(j)];
+            x[c] = sm[j];
         }
 #pragma unroll
         for (int c = 0; c < D; c++) {
@@ -882,7 +879,7 @@ __device__ void tile_mono_c64(float2* sm, int T, const TileGate& g, const int32_
             int j = jb;
 #pragma unroll
             for (int q = 0; q < K; q++) if ((r >> q) & 1) j |= 1 << tb[q];
-            sm[sw64(j)] = c64_ipow(x[c], __ldg(p + 2 * c + 1));
+            sm[j] = c64_ipow(x[c], __ldg(p + 2 * c + 1));
         }
     }
 }
@@ -908,7 +905,7 @@ __device__ void tile_diag_c64(float2* sm, int T, int L, const TileGate& g, const
             }
             const float4 d = __ldg(m + di);
             if (d.z == 0.f && d.x == 1.f && d.y == 0.f) continue;
-            sm[sw64(j)] = c64_mul(d, sm[sw64(j)]);
+            sm[j] = c64_mul(d, sm[j]);
         }
         return;
     }
@@ -919,201 +916,56 @@ __device__ void tile_diag_c64(float2* sm, int T, int L, const TileGate& g, const
         for (int q = 0; q < g.k; q++) di |= (int)((gi >> g.gbit[q]) & 1) << q;
         const float4 d = __ldg(m + di);
         if (d.z == 0.f && d.x == 1.f && d.y == 0.f) continue;
-        sm[sw64(j)] = c64_mul(d, sm[sw64(j)]);
+        sm[j] = c64_mul(d, sm[j]);
     }
 }
 
 
-// ---- register blocks (kind 8): 5 tile bits of the block index the 32 amplitudes a thread holds in
-// registers (f32x2 pairs re, im), the other 7 tile bits are its thread index; every operation of the
-// block is applied there, and the tile is read and written once per block instead of once per gate.
-// What bounds a pass of the tile is shared memory (64 KiB moved at 128 B per clock: 512 cycles per SM,
-// measured ~1200 with the index arithmetic and the barrier), not the arithmetic of its few gates, and a
-// block takes about 9 gates of a mixed circuit.  Packed f32x2 arithmetic halves the issue slots.
-// Measured: 25 qubits, 415 gates {H, Rx, Ry, Rz, CNOT, CZ, Swap, CCNot} in 18 sweeps: 250 passes 7.9 ms,
-// 42 blocks 4.4 ms (issue 44%: 4.9 k instructions a thread and sweep; HBM would allow 1.4 ms).
-__device__ __forceinline__ f2 swap2(f2 v) {
-    const float2 u = up(v);
-    return pk(u.y, u.x);
-}
-// 2x2 on block bit B of all pairs, or (MASKED) of the pairs in pm.  CLS 0 complex, 1 real, 2 real
-// diagonal with imaginary off-diagonal entries, 3 diagonal.
-template <int B, int CLS, bool MASKED>
-__device__ __forceinline__ void reg_1q(f2 (&v)[32], const RegOp& o, uint32_t pm) {
-    const f2 ar = pk(o.m[0], o.m[0]), dr = pk(o.m[6], o.m[6]);
-    const f2 br = pk(o.m[2], o.m[2]), cr = pk(o.m[4], o.m[4]);
-    const f2 ai = pk(-o.m[1], o.m[1]), di = pk(-o.m[7], o.m[7]);
-    const f2 bi = pk(-o.m[3], o.m[3]), ci = pk(-o.m[5], o.m[5]);
-#pragma unroll
-    for (int p = 0; p < 16; p++) {
-        if (MASKED && !((pm >> p) & 1u)) continue;   // uniform
-        const int c0 = ((p >> B) << (B + 1)) | (p & ((1 << B) - 1)), c1 = c0 | (1 << B);
-        const f2 x = v[c0], y = v[c1];
-        if (CLS == 1) {
-            v[c0] = fma2(br, y, mul2(ar, x));
-            v[c1] = fma2(dr, y, mul2(cr, x));
-        } else if (CLS == 2) {
-            v[c0] = fma2(bi, swap2(y), mul2(ar, x));
-            v[c1] = fma2(ci, swap2(x), mul2(dr, y));
-        } else if (CLS == 3) {
-            v[c0] = fma2(ai, swap2(x), mul2(ar, x));
-            v[c1] = fma2(di, swap2(y), mul2(dr, y));
-        } else {
-            const f2 sx2 = swap2(x), sy2 = swap2(y);
-            v[c0] = fma2(bi, sy2, fma2(br, y, fma2(ai, sx2, mul2(ar, x))));
-            v[c1] = fma2(di, sy2, fma2(dr, y, fma2(ci, sx2, mul2(cr, x))));
-        }
-    }
-}
-template <int B>
-__device__ __forceinline__ void reg_x(f2 (&v)[32], uint32_t pm) {
-#pragma unroll
-    for (int p = 0; p < 16; p++) {
-        const int c0 = ((p >> B) << (B + 1)) | (p & ((1 << B) - 1)), c1 = c0 | (1 << B);
-        const bool s = (pm >> p) & 1u;
-        const f2 x = v[c0], y = v[c1];
-        v[c0] = s ? y : x;
-        v[c1] = s ? x : y;
-    }
-}
-template <int B>
-__device__ __forceinline__ void reg_bit(f2 (&v)[32], const RegOp& o, int type) {
-    switch (type) {
-        case 0: reg_1q<B, 0, false>(v, o, 0xffffu); break;
-        case 1: reg_1q<B, 1, false>(v, o, 0xffffu); break;
-        case 2: reg_1q<B, 2, false>(v, o, 0xffffu); break;
-        case 3: reg_x<B>(v, o.mask); break;
-        case 7: reg_1q<B, 3, false>(v, o, 0xffffu); break;
-        default: reg_1q<B, 0, true>(v, o, o.mask); break;
-    }
-}
-
-constexpr int kC64Threads = 128;   // 2^12 amplitudes, 32 per thread
-
-constexpr int kRegOps = 64;        // operations staged in shared memory at a time
-
-// The operations op[0 .. n) on the thread's registers; jt: its tile position with the block bits zero.
-__device__ __forceinline__ void reg_ops(f2 (&v)[32], const RegOp* op, int n, const float4* __restrict__ tabs,
-                                        int64_t base, int jt) {
-    for (; n > 0; n--, op++) {
-        if ((base & (int64_t)op->gc_mask) != (int64_t)op->gc_val) continue;   // uniform in the CTA
-        const int type = op->type;
-        if ((jt & (int)op->lc_mask) != (int)op->lc_val) continue;
-        if (type < 5 || type == 7) {
-            switch (op->bit) {
-                case 0: reg_bit<0>(v, *op, type); break;
-                case 1: reg_bit<1>(v, *op, type); break;
-                case 2: reg_bit<2>(v, *op, type); break;
-                case 3: reg_bit<3>(v, *op, type); break;
-                default: reg_bit<4>(v, *op, type); break;
-            }
-        } else if (type == 5) {
-            int var = 0;
-            for (int u = 0; u < op->nu; u++) {
-                const int b = op->ub[u];
-                var |= (b < 64 ? (jt >> b) & 1 : (int)((base >> (b - 64)) & 1)) << u;
-            }
-            const float4* t = tabs + op->tab + 64 * var;
-#pragma unroll
-            for (int c = 0; c < 32; c++) {
-                const float4 d = __ldg(t + 2 * c), e = __ldg(t + 2 * c + 1);   // high words, low words
-                const f2 w = swap2(v[c]);
-                v[c] = fma2(pk(d.z, d.w), w, fma2(pk(d.x, d.y), v[c], fma2(pk(e.z, e.w), w, mul2(pk(e.x, e.y), v[c]))));
-            }
-        } else {
-            const uint32_t mask = op->mask;
-#pragma unroll
-            for (int c = 0; c < 32; c++) {
-                const uint32_t s = (mask << (31 - c)) & 0x80000000u;
-                const float2 u = up(v[c]);
-                v[c] = pk(__uint_as_float(__float_as_uint(u.x) ^ s), __uint_as_float(__float_as_uint(u.y) ^ s));
-            }
-        }
-    }
-}
-
-// staged: s_ops holds all the sweep's operations (else they are staged here, kRegOps at a time: the
-// latency of reading them one by one from global memory was the kernel's largest stall)
-__device__ __forceinline__ void reg_block(float2* sm, const TileGate& g, RegOp* s_ops, bool staged,
-                                          const RegOp* __restrict__ rops, const float4* __restrict__ tabs, int64_t base) {
-    const int tid = threadIdx.x;
-    int jt = 0;
-    const uint32_t order = (uint32_t)g.perm_off;
-#pragma unroll
-    for (int i = 0; i < 7; i++) jt |= ((tid >> i) & 1) << ((order >> (4 * i)) & 15u);
-    const int sj = 8 * sw64(jt);   // byte offsets in the tile
-    int off[5];
-#pragma unroll
-    for (int q = 0; q < 5; q++) off[q] = 8 * sw64(1 << g.gbit[q]);
-    char* smv = reinterpret_cast<char*>(sm);
-    f2 v[32];
-#pragma unroll
-    for (int c = 0; c < 32; c++) {
-        int j = sj;
-#pragma unroll
-        for (int q = 0; q < 5; q++) if ((c >> q) & 1) j ^= off[q];
-        v[c] = *reinterpret_cast<f2*>(smv + j);
-    }
-    if (staged) {
-        reg_ops(v, s_ops + g.mat_off, g.k, tabs, base, jt);
-    } else {
-        for (int n0 = 0; n0 < g.k; n0 += kRegOps) {
-            const int n = min(kRegOps, g.k - n0);
-            __syncthreads();
-            stage_words(s_ops, rops + g.mat_off + n0, n * (int)(sizeof(RegOp) / 4));
-            __syncthreads();
-            reg_ops(v, s_ops, n, tabs, base, jt);
-        }
-    }
-#pragma unroll
-    for (int c = 0; c < 32; c++) {
-        int j = sj;
-#pragma unroll
-        for (int q = 0; q < 5; q++) if ((c >> q) & 1) j ^= off[q];
-        *reinterpret_cast<f2*>(smv + j) = v[c];
-    }
-}
-
-// BLK: the sweep has register blocks (tiles of 2^12 with 5 low bits).  128 threads of 32 amplitudes;
-// four CTAs fill the register file.
-template <int KMAX, bool BLK>
-__global__ void __launch_bounds__(kC64Threads, KMAX == 2 ? 4 : 3) k_tile_sweep_c64(float2* __restrict__ psi, SweepDesc d, int64_t tile0) {
+// FULL: tiles of 2^12 with 5 low bits (vectors of 12 bits and more): a thread's 16 loads are all in flight, at
+// one pointer plus uniform offsets; smaller tiles take eight at a time.
+template <int KMAX, bool FULL>
+__global__ void __launch_bounds__(kThreads, KMAX == 2 ? 4 : 3) k_tile_sweep_c64(float2* __restrict__ psi, SweepDesc d, int64_t tile0) {
     extern __shared__ float4 smem4[];
     float2* smem = reinterpret_cast<float2*>(smem4);
-    const int T = BLK ? 12 : d.T, L = BLK ? 5 : d.L, H = T - L;
+    const int T = FULL ? 12 : d.T, L = FULL ? 5 : d.L, H = T - L;
     const int nt = 1 << T;
     int64_t* off_tab = reinterpret_cast<int64_t*>(smem + nt);
-    __shared__ TileGate s_gates[kGateChunk];
-    __shared__ __align__(16) RegOp s_ops[BLK ? kRegOps : 1];
     const int64_t base = bs_tile_base(d, tile0 + (int64_t)blockIdx.x);
     const int tid = threadIdx.x;
-    const bool staged = BLK && d.n_rops <= kRegOps;
-    for (int i = tid; i < (1 << H); i += kC64Threads) {
+    for (int i = tid; i < (1 << H); i += kThreads) {
         int64_t o = 0;
         for (int j = 0; j < H; j++) if ((i >> j) & 1) o |= 1LL << d.hi_bits[j];
         off_tab[i] = o;
     }
     __syncthreads();
     const int lowmask = (1 << L) - 1;
-    // The offset of a tile position is linear over XOR of its bits, so a full tile's 32 accesses of a
-    // thread are one pointer plus uniform offsets (rows of 256 bytes), and constant swizzled positions.
-    float2* rows = psi + (base | off_tab[tid >> 5] | (int64_t)(tid & 31));
-    const int st = sw64(tid);
-    if (BLK) {
+    // the offset of a tile position is linear over XOR of its bits: position i * kThreads + tid of a full tile
+    // lies at rows + off_tab[8 i]
+    float2* rows = FULL ? psi + (base | off_tab[tid >> 5] | (int64_t)(tid & 31)) : psi;
+    if (FULL) {
+        float2 x[4096 / kThreads];
 #pragma unroll
-        for (int r = 0; r < 32; r += 16) {
-            float2 x[16];
+        for (int i = 0; i < 4096 / kThreads; i++) x[i] = __ldcs(rows + off_tab[(kThreads >> 5) * i]);
 #pragma unroll
-            for (int i = 0; i < 16; i++) x[i] = __ldcs(rows + off_tab[4 * (r + i)]);
-            if (r == 0 && staged) stage_words(s_ops, d.rops, d.n_rops * (int)(sizeof(RegOp) / 4));
-#pragma unroll
-            for (int i = 0; i < 16; i++) smem[st ^ sw64((r + i) << 7)] = x[i];
-        }
+        for (int i = 0; i < 4096 / kThreads; i++) smem[i * kThreads + tid] = x[i];
     } else {
-        for (int j = tid; j < nt; j += kC64Threads)
-            smem[sw64(j)] = __ldcs(psi + (base | off_tab[j >> L] | (int64_t)(j & lowmask)));
+#pragma unroll
+        for (int r = 0; r < 4096 / kThreads; r += 8) {
+            float2 x[8];
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                const int j = (r + i) * kThreads + tid;
+                if (j < nt) x[i] = __ldcs(psi + (base | off_tab[j >> L] | (int64_t)(j & lowmask)));
+            }
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                const int j = (r + i) * kThreads + tid;
+                if (j < nt) smem[j] = x[i];
+            }
+        }
     }
     __syncthreads();
+    __shared__ TileGate s_gates[kGateChunk];
     for (int g0 = 0; g0 < d.n_gates; g0 += kGateChunk) {
     const int ng = min(kGateChunk, d.n_gates - g0);
     stage_gates(s_gates, d.gates + g0, ng);
@@ -1121,12 +973,10 @@ __global__ void __launch_bounds__(kC64Threads, KMAX == 2 ? 4 : 3) k_tile_sweep_c
         const TileGate& g = s_gates[gl];
         if ((base & (int64_t)g.gc_mask) != (int64_t)g.gc_val) continue;
         const int kind = g.kind, k = g.k;
-        if (BLK && kind == 8) {
-            reg_block(smem, g, s_ops, staged, d.rops, d.mats, base);
-        } else if (kind == 3) {
-            for (int j = tid; j < nt; j += kC64Threads) {
+        if (kind == 3) {
+            for (int j = tid; j < nt; j += kThreads) {
                 const int64_t gi = base | off_tab[j >> L] | (int64_t)(j & lowmask);
-                if (parity_odd(g, gi)) { float2 v = smem[sw64(j)]; smem[sw64(j)] = make_float2(-v.x, -v.y); }
+                if (parity_odd(g, gi)) { float2 v = smem[j]; smem[j] = make_float2(-v.x, -v.y); }
             }
         } else if (kind == 1) {
             tile_diag_c64(smem, T, L, g, d.mats, base, off_tab);
@@ -1144,12 +994,12 @@ __global__ void __launch_bounds__(kC64Threads, KMAX == 2 ? 4 : 3) k_tile_sweep_c
         __syncthreads();
     }
     }
-    if (BLK) {
-#pragma unroll 16
-        for (int i = 0; i < 32; i++) __stcs(rows + off_tab[4 * i], smem[st ^ sw64(i << 7)]);
+    if (FULL) {
+#pragma unroll
+        for (int i = 0; i < 4096 / kThreads; i++) __stcs(rows + off_tab[(kThreads >> 5) * i], smem[i * kThreads + tid]);
     } else {
-        for (int j = tid; j < nt; j += kC64Threads)
-            __stcs(psi + (base | off_tab[j >> L] | (int64_t)(j & lowmask)), smem[sw64(j)]);
+        for (int j = tid; j < nt; j += kThreads)
+            __stcs(psi + (base | off_tab[j >> L] | (int64_t)(j & lowmask)), smem[j]);
     }
 }
 
@@ -1366,25 +1216,6 @@ void tc_offset_tables(const int32_t* tb, std::vector<int32_t>& out) {
 }
 }  // namespace
 
-namespace {
-// The 7 tile bits outside a register block in thread-index order, 4 bits each: the first four of
-// distinct residues mod 4 where there are such (a half-warp's accesses then touch every bank once).
-uint32_t reg_thread_order(const int* bits) {
-    uint32_t used = 0, order = 0, res = 0;
-    int n = 0;
-    for (int q = 0; q < 5; q++) used |= 1u << bits[q];
-    for (int p = 0; p < 12 && n < 4; p++)
-        if (!((used >> p) & 1u) && !((res >> (p & 3)) & 1u)) {
-            res |= 1u << (p & 3);
-            used |= 1u << p;
-            order |= (uint32_t)p << (4 * n++);
-        }
-    for (int p = 0; p < 12; p++)
-        if (!((used >> p) & 1u)) order |= (uint32_t)p << (4 * n++);
-    return order;
-}
-}  // namespace
-
 int bs_run_sweeps(bs_sim* s, const std::vector<Sweep>& sweeps) {
     if (sweeps.empty()) return BS_OK;
     const int n_bits = bs_vec_bits(s);
@@ -1396,14 +1227,9 @@ int bs_run_sweeps(bs_sim* s, const std::vector<Sweep>& sweeps) {
     struct Launch {
         int64_t gate0; int n_gates; std::vector<int> hi; int low; bool big; int big_gate; int kmax = 1;
         int n_tc = 0;
-        bool blk = false;          // has register blocks, with operations rop0 .. rop0 + n_rops
-        size_t rop0 = 0;
-        int n_rops = 0;
     };
     std::vector<Launch> launches;
     std::vector<int32_t> big_bits;
-    std::vector<RegOp> rops;                 // operations of the register blocks (complex64)
-    double reg_drift = 0;
     std::vector<double> tc_pool;             // the fused gates' own matrices (complex), then read by k_tc_build
     std::vector<TcPart> tc_parts;
     std::vector<TcBlock> tc_blocks;
@@ -1427,7 +1253,6 @@ int bs_run_sweeps(bs_sim* s, const std::vector<Sweep>& sweeps) {
     for (const Sweep& sw : sweeps) {
         Launch ln;
         ln.gate0 = (int64_t)tg.size();
-        ln.rop0 = rops.size();
         ln.n_gates = 0;
         ln.hi = sw.hi_bits;
         const int L = sw.low;
@@ -1440,83 +1265,23 @@ int bs_run_sweeps(bs_sim* s, const std::vector<Sweep>& sweeps) {
         for (int b = 0; b < L; b++) local[b] = b;
         for (size_t i = 0; i < sw.hi_bits.size(); i++) local[sw.hi_bits[i]] = L + (int)i;
         std::vector<HostGate> merged, small;
-        std::vector<RegItem> items;        // complex64 sweep by register blocks: the order of its passes
-        std::vector<RegBlock> blocks;
         if (fuse(sw, local)) {
             merge_diagonals(fused, merged);
         } else if (c64) {
             // complex64 sweep: 1- and 2-bit runs fused into dense 2-bit gates where that saves passes (a
             // pass of the complex64 kernel costs about four 1-qubit gates' arithmetic; batch of 512
             // circuits 1.79 -> 1.48 s on the device).  The float-float kernel is bound by its
-            // arithmetic: fusing there measured slower (18 qubits: 7.7 -> 9.2 ms)
-            bool use_blocks = false;
-            std::vector<float4> tabs;
-            double drift = reg_drift;
-            if (T == 12 && L == 5) {
-                // Register blocks where they cost less.  In SM cycles per tile, measured at 25 qubits: a pass
-                // of the tile for one gate 1200; a block 600 for its read and write, and its operations by
-                // type.  Blocks without folded diagonals always win (their operations are cheaper than a
-                // pass); sweeps of many diagonals on scattered bits (16 of them a ring layer, where the
-                // blocks took 62 us a sweep at 22 qubits against 47) or of 2- to 4-target dense gates may
-                // not, and keep the pass per (fused) gate.  The tables' low words (6% of a 22-qubit gradient) are
-                // not counted: without the blocks these gates would be rounded to single precision.
-                static const double op_cost[8] = {480, 230, 320, 260, 550, 480, 250, 320};
-                bs_block_c64(sw.gates, local, T, items, blocks, tabs, drift);
-                double with = 0;
-                bool all = !items.empty();
-                for (const RegItem& it : items) {
-                    all = all && it.block >= 0;
-                    with += it.block < 0 ? 1200.0 : 600.0;
-                    if (it.block >= 0)
-                        for (const RegOp& o : blocks[(size_t)it.block].ops) {
-                            with += op_cost[o.type];
-                            all = all && o.type != 5;
-                        }
-                }
-                use_blocks = all;
-                if (!use_blocks) {
-                    bs_fuse_small(sw.gates, local, 4.0, 2, small);
-                    merge_diagonals(small, merged);
-                    use_blocks = with < 1200.0 * (double)merged.size();
-                }
-            } else {
-                bs_fuse_small(sw.gates, local, 4.0, 2, small);
-                merge_diagonals(small, merged);
-            }
-            if (use_blocks) {
-                reg_drift = drift;
-                const int32_t tab0 = (int32_t)mats.size();
-                mats.insert(mats.end(), tabs.begin(), tabs.end());
-                for (RegBlock& b : blocks) for (RegOp& o : b.ops) o.tab += tab0;
-                merged.clear();
-                for (const RegItem& it : items) {
-                    if (it.block < 0) { merged.push_back(sw.gates[(size_t)it.gate]); continue; }
-                    HostGate h;          // placeholder, packed below
-                    h.kind = 8;
-                    h.k = it.block;
-                    merged.push_back(std::move(h));
-                }
-            }
+            // arithmetic: fusing there measured slower (18 qubits: 7.7 -> 9.2 ms).  The products are formed in
+            // FP64, so matrix and state are rounded once per run; 32 amplitudes in a thread's registers and
+            // an operation per gate (25 qubits, 415 gates 9.9 -> 6.0 ms) rounded the state once per gate, up
+            // to 1.6 times the error on lists of generic matrices, and is not used
+            bs_fuse_small(sw.gates, local, 4.0, 2, small);
+            merge_diagonals(small, merged);
         } else {
             merge_diagonals(sw.gates, merged);
         }
         const std::vector<HostGate>* glist = &merged;
         for (const HostGate& hg : *glist) {
-            if (hg.kind == 8) {
-                const RegBlock& b = blocks[(size_t)hg.k];
-                TileGate t{};
-                t.kind = 8;
-                t.k = (int32_t)b.ops.size();
-                t.mat_off = (int32_t)(rops.size() - ln.rop0);
-                for (int q = 0; q < 5; q++) t.gbit[q] = b.bits[q];
-                t.perm_off = (int32_t)reg_thread_order(b.bits);
-                rops.insert(rops.end(), b.ops.begin(), b.ops.end());
-                ln.n_rops += (int)b.ops.size();
-                ln.blk = true;
-                tg.push_back(t);
-                ln.n_gates++;
-                continue;
-            }
             if (hg.kind == 5) {
                 // reference-rule channel: its row and column target bits are tile bits (the planner needs them)
                 TileGate t{};
@@ -1676,11 +1441,10 @@ int bs_run_sweeps(bs_sim* s, const std::vector<Sweep>& sweeps) {
     int64_t b_tg = al((int64_t)tg.size() * (int64_t)sizeof(TileGate));
     int64_t b_m = al((int64_t)mats.size() * (int64_t)sizeof(float4));
     int64_t b_p = al((int64_t)(perms.size() + big_bits.size() + 1) * (int64_t)sizeof(int32_t));
-    const int64_t b_r = al((int64_t)rops.size() * (int64_t)sizeof(RegOp));
     const int64_t b_fm = al((int64_t)tc_pool.size() * (int64_t)sizeof(double)), b_fp = al((int64_t)tc_parts.size() * (int64_t)sizeof(TcPart));
     const int64_t b_fb = al((int64_t)tc_blocks.size() * (int64_t)sizeof(TcBlock)), b_fv = al(n_var * (int64_t)sizeof(int32_t));
     const int64_t b_fx = al((int64_t)tc_blocks.size() * (int64_t)sizeof(unsigned long long));   // largest entries, from 0
-    const int64_t o_r = b_tg + b_m + b_p, o_fm = o_r + b_r, o_fp = o_fm + b_fm, o_fb = o_fp + b_fp, o_fv = o_fb + b_fb;
+    const int64_t o_fm = b_tg + b_m + b_p, o_fp = o_fm + b_fm, o_fb = o_fp + b_fp, o_fv = o_fb + b_fb;
     const int64_t o_fx = o_fv + b_fv, o_up = o_fx + b_fx;                       // uploaded up to here
     const int64_t o_tm = o_up, b_tm = al(n_var * 2048 * (int64_t)sizeof(double));   // written on the device:
     const int64_t o_tc = o_tm + b_tm, b_tc = al(n_var * tc::kPoolBlock * (int64_t)sizeof(uint16_t));
@@ -1695,7 +1459,6 @@ int bs_run_sweeps(bs_sim* s, const std::vector<Sweep>& sweeps) {
         std::memcpy(host + o_fb, tc_blocks.data(), tc_blocks.size() * sizeof(TcBlock));
         std::memcpy(host + o_fv, tc_var.data(), tc_var.size() * sizeof(int32_t));
     }
-    if (!rops.empty()) std::memcpy(host + o_r, rops.data(), rops.size() * sizeof(RegOp));
     if (!tg.empty()) std::memcpy(host, tg.data(), tg.size() * sizeof(TileGate));
     if (!mats.empty()) std::memcpy(host + b_tg, mats.data(), mats.size() * sizeof(float4));
     if (!perms.empty()) std::memcpy(host + b_tg + b_m, perms.data(), perms.size() * sizeof(int32_t));
@@ -1788,8 +1551,6 @@ int bs_run_sweeps(bs_sim* s, const std::vector<Sweep>& sweeps) {
         d.mats = d_m;
         d.perms = d_p;
         d.tc_pool = d_tc;
-        d.rops = (const RegOp*)(dev + o_r) + ln.rop0;
-        d.n_rops = ln.n_rops;
         d.err = s->dev_flag;
         for (int64_t t0 = 0; t0 < ntiles; t0 += (1LL << 30)) {
             int64_t nb = std::min<int64_t>(ntiles - t0, 1LL << 30);
@@ -1811,9 +1572,10 @@ int bs_run_sweeps(bs_sim* s, const std::vector<Sweep>& sweeps) {
                 s->stats.tc_launches++;
             } else if (c64) {
                 const size_t sm64 = ((size_t)1 << T) * sizeof(float2) + ((size_t)1 << H) * sizeof(int64_t);
-                auto kern = ln.kmax <= 2 ? (ln.blk ? k_tile_sweep_c64<2, true> : k_tile_sweep_c64<2, false>)
-                                         : (ln.blk ? k_tile_sweep_c64<4, true> : k_tile_sweep_c64<4, false>);
-                kern<<<(unsigned)nb, kC64Threads, sm64, s->stream>>>((float2*)s->state, d, t0);
+                const bool full = T == 12 && L == 5;
+                auto kern = ln.kmax <= 2 ? (full ? k_tile_sweep_c64<2, true> : k_tile_sweep_c64<2, false>)
+                                         : (full ? k_tile_sweep_c64<4, true> : k_tile_sweep_c64<4, false>);
+                kern<<<(unsigned)nb, kThreads, sm64, s->stream>>>((float2*)s->state, d, t0);
             } else if (bs_tile_threads(s) == 512 || (s->tune.tile_threads < 0 && ntiles <= 152)) {
                 // one tile per SM at most: 16 warps on it instead of 8
                 if (ln.kmax <= 2) k_tile_sweep<2, 512><<<(unsigned)nb, 512, smem, s->stream>>>(psi, d, t0);
