@@ -1238,16 +1238,26 @@ int bs_run_sweeps(bs_sim* s, const std::vector<Sweep>& sweeps) {
     const bool c64 = s->precision == BS_PREC_C64;
     const bool use_tc = sweeps.front().tc;
     const double tc_threshold = bs_tc_cost(s);
-    // a sweep left with unfused 3/4-target gates keeps its plain gate list, since the tensor-core sweep
-    // kernel carries float-float paths for 1- and 2-target gates only
+    // A sweep keeps its plain gate list, on the float-float kernel, where it is left with unfused 3/4-target gates
+    // (the tensor-core sweep carries float-float paths for 1- and 2-target gates only) and where a fused matrix would
+    // reach 2^12, beyond its digits' range (gates far from unitary; the float-float values have FP32's exponents).
+    // Below 16 bits only the environment or a handle's tuning brings a list here; asked by BS_TC_MIN_BITS for
+    // tensor-core sweeps of such a size, one that has no digits is refused, not run elsewhere.
+    const bool refuse = n_bits < 16 && s->tune.tc_min_bits < 0;
     std::vector<HostGate> fused;
+    bool out_of_range = false;
     auto fuse = [&](const Sweep& sw, const int* local) {
         if (!use_tc || (int)sw.hi_bits.size() != T - sw.low) return false;
         std::vector<const HostGate*> in;
         for (const HostGate& g : sw.gates) in.push_back(&g);
         bs_fuse_tc(in, local, T, tc_threshold, &fused);
-        for (const HostGate& hg : fused)
+        for (const HostGate& hg : fused) {
             if (hg.kind != 1 && hg.kind != 4 && hg.kind != 5 && hg.k >= 3) return false;
+            if (hg.kind == 4 && !bs_tc_in_range(hg, sw.gates)) {
+                out_of_range = true;
+                return false;
+            }
+        }
         return true;
     };
     for (const Sweep& sw : sweeps) {
@@ -1265,7 +1275,9 @@ int bs_run_sweeps(bs_sim* s, const std::vector<Sweep>& sweeps) {
         for (int b = 0; b < L; b++) local[b] = b;
         for (size_t i = 0; i < sw.hi_bits.size(); i++) local[sw.hi_bits[i]] = L + (int)i;
         std::vector<HostGate> merged, small;
-        if (fuse(sw, local)) {
+        const bool tc = fuse(sw, local);
+        if (out_of_range && refuse) return bs_fail(s, BS_ERR_INVALID_ARG, "fused gate matrix out of range");
+        if (tc) {
             merge_diagonals(fused, merged);
         } else if (c64) {
             // complex64 sweep: 1- and 2-bit runs fused into dense 2-bit gates where that saves passes (a
@@ -1314,7 +1326,6 @@ int bs_run_sweeps(bs_sim* s, const std::vector<Sweep>& sweeps) {
                 t.tc_nu = (int32_t)hg.ubits.size();
                 for (size_t i = 0; i < hg.ubits.size(); i++) t.tc_ub[i] = hg.ubits[i];
                 t.tc_off = (int32_t)n_var;
-                if (!bs_tc_in_range(hg, sw.gates)) return bs_fail(s, BS_ERR_INVALID_ARG, "fused gate matrix out of range");
                 int where[64];           // block or variant bit of an endian bit
                 for (int b = 0; b < 64; b++) where[b] = -1;
                 for (int q = 0; q < 5; q++) where[hg.ebit[q]] = q;

@@ -240,3 +240,32 @@ def test_lists_below_22_bits(n, kind, wide, layers, tc):
         got, ref = sim.state_vector, oracle.OracleSV(n).evolve(ops).psi
     assert (sim.last_stats()["tc_gates"] > 0) == tc
     assert rel_err(got, ref) < TOL
+
+
+@pytest.mark.parametrize("n,kind,tune", [(13, "sv", True), (16, "sv", False), (20, "sv", False), (22, "sv", False), (8, "dm", False)])
+@pytest.mark.parametrize("same", [True, False])
+def test_products_out_of_range_run_on_the_float_float_sweeps(n, kind, tune, same):
+    """Lists that take the tensor cores by their size, gates or tuning and whose fused product has entries of 2^12 and
+    more: matrices of norm 17 six times on one qubit, or twice on each of five.  The sweep that holds them runs
+    float-float, the others stay fused; the state against the oracle."""
+    rng = np.random.default_rng(800 + n)
+    big = np.array([[17.0, 0.3], [0.2, 0.25]])
+    ops = [bs.Instruction(bs.Unitary(haar(rng)), [q]) for q in range(n) for _ in range(1 + 2 * (n >= 20))]
+    for layer in range(2):
+        ops += [bs.Instruction(bs.CZ(), [q, q + 1]) for q in range(n - 1)]
+        ops += [bs.Instruction(bs.Unitary(haar(rng)), [q]) for q in range(n)]
+        for _ in range(2 if n < 20 and kind == "sv" else 0):
+            ops.append(bs.Instruction(bs.Unitary(haar(rng, 16)), [int(q) for q in rng.permutation(n)[:4]]))
+    if kind == "dm":
+        ops += [bs.Instruction(bs.TwoQubitDepolarizing(0.02), [int(q) for q in rng.permutation(n)[:2]]) for _ in range(4)]
+    ops += [bs.Instruction(bs.Unitary(big), [2])] * 6 if same else [bs.Instruction(bs.Unitary(big), [q]) for q in range(5)] * 2
+    ops += [bs.Instruction(bs.Ry(0.1), [q]) for q in (3, 4, 5)]
+    if kind == "dm":
+        sim = bs.DensityMatrixSimulator(n, 0, noise_mode="physical").evolve(ops)
+        got, ref = sim.density_matrix, oracle.OracleDM(n, physical=True).evolve(ops).matrix
+    else:
+        sim = bs.StateVectorSimulator(n, 0)
+        if tune:
+            bs.set_tuning(sim, tc_min_bits=12)
+        got, ref = sim.evolve(ops).state_vector, oracle.OracleSV(n).evolve(ops).psi
+    assert rel_err(got, ref) < TOL
