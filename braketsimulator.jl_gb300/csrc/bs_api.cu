@@ -1,11 +1,11 @@
 // C ABI entry points: handle lifecycle, state transfer, gate / channel / evolve.
 #include <algorithm>
 #include <atomic>
-#include <chrono>
 #include <iterator>
 #include <cstring>
 #include <new>
 #include "bs_internal.h"
+#include "bs_ticket.h"
 
 int bs_fail(bs_sim* s, int code, const std::string& msg) {
     if (s) s->err = msg;
@@ -110,16 +110,8 @@ MapSlot bs_map_slot(size_t bytes) {
 }
 
 int bs_wait_ticket(bs_sim* s, const MapSlot& m, const char* what) {
-    const auto t0 = std::chrono::steady_clock::now();
-    for (uint32_t it = 0;; it++) {
-        if (*m.word == m.ticket) {
-            std::atomic_thread_fence(std::memory_order_acquire);
-            return BS_OK;
-        }
-        if ((it & 1023u) == 1023u && std::chrono::steady_clock::now() - t0 > std::chrono::seconds(2)) break;
-    }
-    const int rc = bs_cuda_check(s, cudaStreamSynchronize(s->stream), what);
-    std::atomic_thread_fence(std::memory_order_acquire);
+    const int rc = bs_poll_ticket(m.word, m.ticket, 2.0, [&] { return bs_cuda_check(s, cudaStreamSynchronize(s->stream), what); });
+    if (rc == BS_ERR_TIMEOUT) return bs_fail(s, rc, std::string(what) + ": the stream ended without the result");
     return rc;
 }
 

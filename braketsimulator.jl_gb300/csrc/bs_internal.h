@@ -206,7 +206,7 @@ MapSlot bs_map_slot(size_t bytes);
 // Called by a thread that lives for one call: its results take the copy, since mapping memory for it costs more.
 void bs_thread_without_map();
 // Polls for the slot's ticket; after 2 s (a failed or very long kernel) synchronises the stream, which
-// reports the error.
+// reports the error.  A stream that ended without the ticket is an error too.
 int bs_wait_ticket(bs_sim* s, const MapSlot& m, const char* what);
 int bs_ensure_scratch(bs_sim* s, int64_t bytes);
 int bs_ensure_plan(bs_sim* s, int64_t bytes);

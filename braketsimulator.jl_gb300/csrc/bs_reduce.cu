@@ -491,6 +491,7 @@ int bs_expectation_pauli(bs_sim* s, int n_terms, const uint64_t* xmask, const ui
     if (!s) return BS_ERR_INVALID_ARG;
     if (n_terms < 0 || (n_terms > 0 && (!xmask || !zmask || !out))) return bs_fail(s, BS_ERR_INVALID_ARG, "bad term arrays");
     if (n_terms == 0) return BS_OK;
+    if (s->capturing && coeffs) return bs_fail(s, BS_ERR_INVALID_ARG, "coefficients are applied after a captured graph runs");
     const int n = s->n;
     const uint64_t qmask = (n >= 64) ? ~0ULL : ((1ULL << n) - 1);
     // group by flip mask on endian bits
@@ -538,16 +539,18 @@ int bs_expectation_pauli(bs_sim* s, int n_terms, const uint64_t* xmask, const ui
         }
     }
     rc = bs_cuda_check(s, cudaGetLastError(), "expectation");
-    if (rc) return rc;
-    if (s->capturing && coeffs) return bs_fail(s, BS_ERR_INVALID_ARG, "coefficients are applied after a captured graph runs");
     // during capture out is the graph owner's pinned buffer, filled on every replay
-    if (slot.h) {
+    if (!rc && slot.h) {
         rc = bs_wait_ticket(s, slot, "expectation");
         if (!rc) std::memcpy(out, slot.h, (size_t)n_terms * 8);
-    } else {
+    } else if (!rc) {
         rc = bs_copy_out(s, out, res, (size_t)n_terms * 8, "expectation");
     }
-    if (rc || s->capturing) return rc;
+    if (s->capturing) return rc;
+    if (rc) {   // launches that ran without the others leave the counter short of its total: the next call starts at zero
+        cudaMemsetAsync(fin.done, 0, sizeof(unsigned), s->stream);
+        return rc;
+    }
     if (coeffs)
         for (int t = 0; t < n_terms; t++) out[t] *= coeffs[t];
     return BS_OK;
