@@ -292,6 +292,11 @@ __device__ __forceinline__ bool wait_bar1(const State& st, int k) {
     return ok;
 }
 
+// The status of a warp one of whose lanes waited on its own: false in every lane if that wait gave up, so that the
+// warp leaves as a whole.  (With the one lane gone ahead to the caller's barrier, the others would stop for good at
+// the next wait's shuffle.)
+__device__ __forceinline__ bool warp_ok(bool ok) { return __all_sync(0xffffffffu, ok); }
+
 // Applies fused gate g to the (swizzled) 2^12 tile sm of float4 (re hi, im hi, re lo, im lo).
 // Called by all NT threads of the CTA (NT/128 threads per tile column, 32*128/NT amplitudes each),
 // which then synchronise.  base: the CTA's global base index (selects the matrix variant).  s_wmax: NT/32 per-warp maxima of the high words' exponent fields.
@@ -422,6 +427,7 @@ __device__ __forceinline__ void apply(float4* sm, const TileGate& g, const TileG
             if (wait_bar1(st, 4)) issue_round<2>(st.tmem, kD1, b0, st.bar + 16u);
             else ok = false;
         }
+        ok = warp_ok(ok);
     }
     st.ph ^= (1u << 3) | (1u << 4);
     // round 2 (D1); once it has completed, round 0 goes into D2

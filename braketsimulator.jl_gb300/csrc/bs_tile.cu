@@ -1615,14 +1615,19 @@ void bs_collect_tc_time(bs_sim* s) {
 }
 
 namespace {
-// A wait that nothing completes: one thread waits on a fresh mbarrier (no arrival, no copy and no MMA
-// in flight) with the tensor-core sweep's bounded wait, gives up after `limit` cycles and raises the
-// device flag, as a sweep whose copy or MMA never landed would.
-__global__ void k_wait_selftest(int* __restrict__ err, long long limit) {
+// Waits that nothing completes, in the form of the tensor-core sweep: two issuing threads wait on a fresh mbarrier (no
+// arrival, no copy and no MMA in flight) with its bounded wait, give up after `limit` cycles, their warps take no
+// further warp-wide step, and all threads meet at a barrier.  Raises the device flag, as a sweep whose copy or MMA
+// never landed would, where exactly those two warps left, each as a whole.
+__global__ void __launch_bounds__(kTcThreads) k_wait_selftest(int* __restrict__ err, long long limit) {
     __shared__ __align__(8) uint64_t bar;
     if (threadIdx.x == 0) tc::mbar_init(tc::su32(&bar));
     __syncthreads();
-    if (threadIdx.x == 0 && !tc::mbar_wait_for(tc::su32(&bar), 0u, limit)) atomicExch(err, 1);
+    bool ok = true;
+    if (threadIdx.x == 0 || threadIdx.x == 128) ok = tc::mbar_wait_for(tc::su32(&bar), 0u, limit);
+    ok = tc::warp_ok(ok);
+    if (ok) ok = __shfl_sync(0xffffffffu, 1, 0) != 0;
+    if (__syncthreads_count(!ok) == 64 && threadIdx.x == 0) atomicExch(err, 1);
 }
 }  // namespace
 
@@ -1638,7 +1643,7 @@ extern "C" int bs_selftest_wait_timeout(bs_sim* s, double seconds) {
     rc = bs_cuda_check(s, cudaMemsetAsync(s->dev_flag, 0, sizeof(int), s->stream), "flag reset");
     if (rc) return rc;
     s->flag_armed = true;
-    k_wait_selftest<<<1, 32, 0, s->stream>>>(s->dev_flag, (long long)(seconds * 2.0e9));
+    k_wait_selftest<<<1, kTcThreads, 0, s->stream>>>(s->dev_flag, (long long)(seconds * 2.0e9));
     rc = bs_cuda_check(s, cudaGetLastError(), "self-test launch");
     if (rc) return rc;
     rc = bs_check_device_flag(s);

@@ -265,3 +265,24 @@ def test_small_tiles_and_matrix_classes(n):
             ops.append(bs.Instruction(g, [int(q), r]))
     sim = bs.StateVectorSimulator(n, 0).evolve(ops)
     assert rel_err(sim.state_vector, oracle.OracleSV(n).evolve(ops).psi) < 1e-12
+
+
+def test_warps_whose_issuing_thread_gives_up_leave_as_a_whole():
+    """The tensor-core sweep's issuing threads wait alone.  Where such a wait gives up, the warp takes no further
+    warp-wide step and all threads reach the barrier behind: the self-test counts them there (it reports the timeout
+    only for exactly the two issuers' warps), ends within its limit, and fused sweeps run afterwards."""
+    import time
+    import oracle
+    n, rng = 13, np.random.default_rng(6)
+    sim = bs.StateVectorSimulator(n, 0)
+    for _ in range(3):
+        t0 = time.perf_counter()
+        with pytest.raises(bs._abi.BraketGB300Error) as e:
+            sim._h.call("bs_selftest_wait_timeout", 0.01)
+        assert e.value.code == bs._abi.BS_ERR_TIMEOUT and time.perf_counter() - t0 < 1.0
+    ops = [bs.Instruction(bs.U(*(float(a) for a in rng.uniform(-3, 3, 3))), [q]) for _ in range(3) for q in range(n)]
+    bs.set_tuning(sim, tc=1, tc_min_bits=12)
+    sim.evolve(ops)
+    assert sim.last_stats()["tc_gates"] > 0
+    ref = oracle.OracleSV(n).evolve(ops).psi
+    assert np.linalg.norm(sim.state_vector - ref) <= 1e-12 * np.linalg.norm(ref)
