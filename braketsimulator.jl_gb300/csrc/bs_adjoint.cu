@@ -726,6 +726,7 @@ extern "C" int bs_adjoint_gradient(bs_sim* s, const bs_op* ops, int64_t n_ops, c
     if (S < 0) {
         size_t fr = 0, tot = 0;
         cudaMemGetInfo(&fr, &tot);
+        fr += bs_kept_bytes();   // freed where they are in the way
         const int by_mem = (int)std::min<size_t>(64, fr / 4 / std::max<size_t>(state_bytes, 1));
         S = std::min(std::min(16, 1 + n_param_gates / 16), by_mem + 1);
     }
@@ -733,36 +734,22 @@ extern "C" int bs_adjoint_gradient(bs_sim* s, const bs_op* ops, int64_t n_ops, c
     // One allocation for the checkpoints and lambda.  Up to kKeepBytes it stays with the handle for the next
     // gradient (15 allocations and frees a call were 1.2 ms, a fifth of a 20-qubit gradient); larger ones
     // are given back at the end of the call.
-    constexpr size_t kKeepBytes = (size_t)1 << 30;
     const size_t slot = (state_bytes + 255) & ~(size_t)255;
-    void* once = nullptr;      // an allocation of this call only
+    size_t work_bytes = 0;
     char* work = nullptr;
     for (;;) {
         const size_t need = slot * (size_t)S;   // S - 1 checkpoints, lambda
-        if (need <= s->adj_work_bytes) { work = (char*)s->adj_work; break; }
-        void* p = nullptr;
-        if (need <= kKeepBytes) {
-            if (s->adj_work) cudaFree(s->adj_work);
-            s->adj_work = nullptr;
-            s->adj_work_bytes = 0;
-        }
-        if (cudaMalloc(&p, need) == cudaSuccess) {
-            work = (char*)p;
-            if (need <= kKeepBytes) { s->adj_work = p; s->adj_work_bytes = need; }
-            else once = p;
-            break;
-        }
-        cudaGetLastError();
-        if (s->adj_work) {        // the kept workspace goes first
-            cudaFree(s->adj_work);
-            s->adj_work = nullptr;
-            s->adj_work_bytes = 0;
-            continue;
-        }
+        work = (char*)bs_keep_take(s, need, &work_bytes);
+        if (work) break;
+        work_bytes = need;
+        if (bs_malloc((void**)&work, need) == cudaSuccess) break;
         if (S == 1) return bs_fail(s, BS_ERR_ALLOC, "lambda allocation: out of memory");
         S = std::max(1, S / 2);   // memory binds: fewer checkpoints, more uncomputation
     }
-    auto free_ckpt = [&]() { if (once) cudaFree(once); once = nullptr; };   // synchronises with the stream's work
+    auto free_ckpt = [&]() {
+        if (work_bytes <= kKeepBytes) bs_keep(s, work, work_bytes);
+        else cudaFree(work);   // synchronises with the stream's work
+    };
     // segment j covers ops [seg[j], seg[j+1]), split evenly by gate count
     std::vector<int64_t> seg(1, 0);
     {

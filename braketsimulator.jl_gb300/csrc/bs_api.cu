@@ -5,6 +5,7 @@
 #include <cstring>
 #include <new>
 #include "bs_internal.h"
+#include "bs_keep.h"
 #include "bs_ticket.h"
 
 int bs_fail(bs_sim* s, int code, const std::string& msg) {
@@ -133,6 +134,29 @@ int bs_copy_out(bs_sim* s, void* host, const void* dev, size_t bytes, const char
     return rc;
 }
 
+namespace {
+thread_local cudaError_t t_alloc = cudaSuccess;
+struct DeviceMem {
+    static void* get(size_t bytes) {
+        void* p = nullptr;
+        t_alloc = cudaMalloc(&p, bytes);
+        if (t_alloc != cudaSuccess) cudaGetLastError();
+        return p;
+    }
+    static void put(void* p) { cudaFree(p); }
+};
+KeepPool<DeviceMem> g_keep(kKeepAll);
+}  // namespace
+
+cudaError_t bs_malloc(void** p, size_t bytes) {
+    *p = g_keep.get(bytes);
+    return t_alloc;
+}
+void* bs_keep_take(const bs_sim* s, size_t bytes, size_t* got) { return g_keep.take(s, bytes, got); }
+void bs_keep(const bs_sim* s, void* p, size_t bytes) { g_keep.keep(s, p, bytes); }
+size_t bs_kept_bytes() { return g_keep.idle_bytes(); }
+void bs_free_kept() { g_keep.drop_all(); }
+
 int bs_ensure_scratch(bs_sim* s, int64_t bytes) {
     if (s->scratch_bytes >= bytes) return BS_OK;
     if (s->capturing) return bs_fail(s, BS_ERR_STATE, "scratch growth during graph capture");
@@ -141,7 +165,7 @@ int bs_ensure_scratch(bs_sim* s, int64_t bytes) {
     s->scratch_bytes = 0;
     // the counter of bs_scratch_counter lies behind it: an allocation of its own was 0.1 ms of every handle
     bytes = (bytes + 255) & ~(int64_t)255;
-    int rc = bs_cuda_check(s, cudaMalloc(&s->scratch, (size_t)bytes + 256), "scratch allocation");
+    int rc = bs_cuda_check(s, bs_malloc(&s->scratch, (size_t)bytes + 256), "scratch allocation");
     if (rc) return rc;
     s->scratch_bytes = bytes;
     return bs_cuda_check(s, cudaMemsetAsync((char*)s->scratch + bytes, 0, 256, s->stream), "counter reset");
@@ -157,7 +181,7 @@ int bs_ensure_plan(bs_sim* s, int64_t bytes) {
     s->plan_buf = nullptr;
     s->plan_bytes = 0;
     int64_t b = std::max<int64_t>(bytes, 1 << 16);
-    int rc = bs_cuda_check(s, cudaMalloc(&s->plan_buf, (size_t)b), "plan allocation");
+    int rc = bs_cuda_check(s, bs_malloc(&s->plan_buf, (size_t)b), "plan allocation");
     if (rc) return rc;
     s->plan_bytes = b;
     return BS_OK;
@@ -215,15 +239,7 @@ int alloc_state(bs_sim* s, int n) {
         if (s->state) cudaFree(s->state);
         s->state = nullptr;
         s->cap_bytes = 0;
-        cudaError_t e = cudaMalloc(&s->state, (size_t)bytes);
-        if (e != cudaSuccess && s->adj_work) {   // the kept workspace goes before a state does not fit
-            cudaGetLastError();
-            cudaFree(s->adj_work);
-            s->adj_work = nullptr;
-            s->adj_work_bytes = 0;
-            e = cudaMalloc(&s->state, (size_t)bytes);
-        }
-        int rc = bs_cuda_check(s, e, "state allocation");
+        int rc = bs_cuda_check(s, bs_malloc(&s->state, (size_t)bytes), "state allocation");
         if (rc) return rc;
         s->cap_bytes = bytes;
     }
@@ -271,7 +287,7 @@ int bs_destroy(bs_sim* s) {
     if (s->state) cudaFree(s->state);
     if (s->scratch) cudaFree(s->scratch);
     if (s->plan_buf) cudaFree(s->plan_buf);
-    if (s->adj_work) cudaFree(s->adj_work);
+    g_keep.drop(s);
     if (s->dev_flag) cudaFree(s->dev_flag);
     if (s->alias_ap) cudaFree(s->alias_ap);
     if (s->alias_ix) cudaFree(s->alias_ix);

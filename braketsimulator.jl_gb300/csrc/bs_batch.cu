@@ -394,7 +394,7 @@ extern "C" int bs_run_batch(int n_circuits, const int* n_qubits, const bs_op* co
         rc = pack_small(small, n_qubits, ops, n_ops, bc, bg);
         if (!rc) {
             const SmallLayout L = small_layout(bc.size(), bg.size(), n_circuits, n_terms, shots);
-            if (cudaMalloc(&dbuf, L.total) != cudaSuccess) rc = BS_ERR_ALLOC;
+            if (bs_malloc((void**)&dbuf, L.total) != cudaSuccess) rc = BS_ERR_ALLOC;
             if (!rc) {
                 img.resize(L.o_e);
                 small_image(img.data(), L, bc, bg, xme, zme, phs);
@@ -532,7 +532,7 @@ int batch_pack_small(bs_batch* b, const bs_op* const* ops, const int64_t* n_ops)
         if (b->dsmall) cudaFree(b->dsmall);
         b->dsmall = nullptr;
         b->dsmall_bytes = 0;
-        if (cudaMalloc(&b->dsmall, b->L.total) != cudaSuccess) return BS_ERR_ALLOC;
+        if (bs_malloc((void**)&b->dsmall, b->L.total) != cudaSuccess) return BS_ERR_ALLOC;
         b->dsmall_bytes = b->L.total;
     }
     free_pinned(b->img_old);

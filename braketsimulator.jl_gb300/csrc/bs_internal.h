@@ -150,9 +150,6 @@ struct bs_sim {
     int64_t* alias_ix = nullptr;
     int64_t alias_len = 0;
     bool alias_valid = false;
-    // adjoint gradients: checkpoints and lambda, kept between calls up to 1 GiB (bs_adjoint_gradient)
-    void* adj_work = nullptr;
-    size_t adj_work_bytes = 0;
     // plan upload buffer
     void* plan_buf = nullptr;
     int64_t plan_bytes = 0;
@@ -208,6 +205,14 @@ void bs_thread_without_map();
 // Polls for the slot's ticket; after 2 s (a failed or very long kernel) synchronises the stream, which
 // reports the error.  A stream that ended without the ticket is an error too.
 int bs_wait_ticket(bs_sim* s, const MapSlot& m, const char* what);
+// Device allocation (cudaMalloc's status).  The blocks that handles keep between calls (bs_keep.h: the checkpoints and
+// lambda of adjoint gradients, up to 1 GiB a handle and 4 GiB over all) are freed before it fails.
+cudaError_t bs_malloc(void** p, size_t bytes);
+constexpr size_t kKeepBytes = (size_t)1 << 30, kKeepAll = 4 * kKeepBytes;
+void* bs_keep_take(const bs_sim* s, size_t bytes, size_t* got);   // the handle's kept block, if it is large enough
+void bs_keep(const bs_sim* s, void* p, size_t bytes);              // for its next call
+size_t bs_kept_bytes();
+void bs_free_kept();
 int bs_ensure_scratch(bs_sim* s, int64_t bytes);
 int bs_ensure_plan(bs_sim* s, int64_t bytes);
 // The counter with which the last block of an expectation is found (zero between calls), behind the scratch buffer

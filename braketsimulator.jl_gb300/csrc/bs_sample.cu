@@ -298,9 +298,9 @@ int alias_alloc(bs_sim* s, int64_t n) {
     s->alias_ap = nullptr;
     s->alias_ix = nullptr;
     s->alias_len = 0;
-    int rc = bs_cuda_check(s, cudaMalloc(&s->alias_ap, (size_t)n * 8), "alias allocation");
+    int rc = bs_cuda_check(s, bs_malloc((void**)&s->alias_ap, (size_t)n * 8), "alias allocation");
     if (rc) return rc;
-    rc = bs_cuda_check(s, cudaMalloc(&s->alias_ix, (size_t)n * 8), "alias allocation");
+    rc = bs_cuda_check(s, bs_malloc((void**)&s->alias_ix, (size_t)n * 8), "alias allocation");
     if (rc) return rc;
     s->alias_len = n;
     return BS_OK;
@@ -393,7 +393,13 @@ int bs_sample_alias(bs_sim* s, const int64_t* j, const double* u, int64_t shots,
     // stream buffers after the alias scratch use: j, u, out, flag
     const int64_t bytes = shots * 24 + 64;
     void* buf = nullptr;
-    int rc = bs_cuda_check(s, cudaMallocAsync(&buf, (size_t)bytes, s->stream), "sample buffers");
+    cudaError_t e = cudaMallocAsync(&buf, (size_t)bytes, s->stream);
+    if (e != cudaSuccess && bs_kept_bytes()) {
+        cudaGetLastError();
+        bs_free_kept();
+        e = cudaMallocAsync(&buf, (size_t)bytes, s->stream);
+    }
+    int rc = bs_cuda_check(s, e, "sample buffers");
     if (rc) return rc;
     int64_t* dj = (int64_t*)buf;
     double* du = (double*)(dj + shots);

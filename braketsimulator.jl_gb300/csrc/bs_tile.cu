@@ -1518,7 +1518,7 @@ int bs_run_sweeps(bs_sim* s, const std::vector<Sweep>& sweeps) {
         k_tc_digits<<<(unsigned)n_var, 256, 0, s->stream>>>((const double*)(dev + o_tm), d_fb, d_fv, d_fx, (TileGate*)dev, d_tc);
         s->stats.kernel_launches += 2;
         if (!s->dev_flag) {
-            rc = bs_cuda_check(s, cudaMalloc((void**)&s->dev_flag, 256), "flag alloc");
+            rc = bs_cuda_check(s, bs_malloc((void**)&s->dev_flag, 256), "flag alloc");
             if (rc) return rc;
         }
         if (!s->flag_armed) {
@@ -1637,7 +1637,7 @@ extern "C" int bs_selftest_wait_timeout(bs_sim* s, double seconds) {
     if (s->capturing) return bs_fail(s, BS_ERR_STATE, "not during graph capture");
     int rc = BS_OK;
     if (!s->dev_flag) {
-        rc = bs_cuda_check(s, cudaMalloc((void**)&s->dev_flag, 256), "flag alloc");
+        rc = bs_cuda_check(s, bs_malloc((void**)&s->dev_flag, 256), "flag alloc");
         if (rc) return rc;
     }
     rc = bs_cuda_check(s, cudaMemsetAsync(s->dev_flag, 0, sizeof(int), s->stream), "flag reset");

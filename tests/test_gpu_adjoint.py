@@ -204,3 +204,26 @@ def test_diagonal_gate_that_is_not_unitary_keeps_its_place():
         ops += [bs.Instruction(bs.Unitary(m), [0]), bs.Instruction(bs.ZZ(0.9), [0, 2]), bs.Instruction(bs.Rx(-0.8), [0])]
         grads.append(adj.adjoint_gradient(bs.StateVectorSimulator(4, 0), ops, h)[1])
     assert np.max(np.abs(grads[0] - grads[1])) < 1e-12
+
+
+def test_gradients_keep_at_most_4_gib_between_calls():
+    """Checkpoints stay for a handle's next gradient, 4 GiB over all handles: ten simulators of 21 qubits (512 MiB of
+    checkpoints each) leave no more than that behind beside their states, plans and scratch, and nothing once closed."""
+    import gc
+    import torch
+    n, rng = 21, np.random.default_rng(4)
+    ops = [bs.Instruction([bs.Rx, bs.Ry][(q + k) % 2](float(rng.uniform(-3, 3))), [q]) for k in range(12) for q in range(n)]
+    h = hamiltonian(n, 3, rng)
+    adj.adjoint_gradient(bs.StateVectorSimulator(n, 0), ops, h)   # the library's own set-up
+    gc.collect()
+    free0 = torch.cuda.mem_get_info()[0]
+    sims = [bs.StateVectorSimulator(n, 0) for _ in range(10)]
+    first = [adj.adjoint_gradient(s, ops, h) for s in sims]
+    left = free0 - torch.cuda.mem_get_info()[0]
+    assert left < (4 << 30) + 10 * (64 << 20), left >> 20
+    again = [adj.adjoint_gradient(s, ops, h) for s in sims]
+    for (e, g), (e2, g2) in zip(first, again):
+        assert abs(e - e2) < 1e-12 and np.max(np.abs(g - g2)) < 1e-12
+    del sims
+    gc.collect()
+    assert free0 - torch.cuda.mem_get_info()[0] < 64 << 20

@@ -43,3 +43,71 @@ int main() {
     return 0;
 }
 """)
+
+
+def test_blocks_kept_between_calls_are_given_back(tmp_path):
+    """The pool of kept device blocks on a fake of the allocator with room for 100 bytes: at most its cap is kept, the
+    oldest block goes first, a block goes with its owner, and an allocation that does not fit frees the pool and is
+    tried again, also from another thread."""
+    run_cpp(tmp_path, r"""
+#include "bs_keep.h"
+#include <cstdio>
+#include <map>
+#include <thread>
+#define CHECK(x) do { if (!(x)) { std::printf("line %d: %s\n", __LINE__, #x); return 1; } } while (0)
+struct Fake {
+    static std::mutex m;
+    static std::map<void*, size_t> live;
+    static size_t used() { size_t n = 0; for (auto& k : live) n += k.second; return n; }
+    static void* get(size_t n) {
+        std::lock_guard<std::mutex> lock(m);
+        if (used() + n > 100) return nullptr;
+        void* p = new char[n];
+        live[p] = n;
+        return p;
+    }
+    static void put(void* p) {
+        std::lock_guard<std::mutex> lock(m);
+        if (!live.erase(p)) std::abort();   // freed twice
+        delete[] (char*)p;
+    }
+};
+std::mutex Fake::m;
+std::map<void*, size_t> Fake::live;
+int main() {
+    KeepPool<Fake> pool(60);
+    int a, b, c;
+    size_t got = 0;
+    CHECK(!pool.take(&a, 10, &got));
+    void* p = pool.get(40);
+    pool.keep(&a, p, 40);
+    CHECK(!pool.take(&b, 10, &got));                        // another handle's
+    CHECK(pool.take(&a, 30, &got) == p && got == 40 && pool.idle_bytes() == 0);
+    pool.keep(&a, p, 40);
+    CHECK(!pool.take(&a, 50, &got) && Fake::used() == 0);   // too small: freed
+    pool.keep(&a, pool.get(30), 30);
+    pool.keep(&b, pool.get(30), 30);
+    pool.keep(&c, pool.get(20), 20);                        // above the cap: the oldest goes
+    CHECK(pool.idle_bytes() == 50 && !pool.take(&a, 1, &got));
+    pool.drop(&b);
+    CHECK(Fake::used() == 20);
+    pool.keep(&b, pool.get(40), 40);
+    void* big = pool.get(90);                               // does not fit beside the kept blocks
+    CHECK(big && pool.idle_bytes() == 0 && Fake::used() == 90);
+    CHECK(!pool.get(20));
+    Fake::put(big);
+    auto work = [&](void* me) {
+        for (int i = 0; i < 2000; i++) {
+            size_t n = 0;
+            void* q = pool.take(me, 10, &n);
+            if (!q) { n = 10 + i % 7; q = pool.get(n); }
+            if (q) pool.keep(me, q, n);
+        }
+        pool.drop(me);
+    };
+    std::thread t1(work, &a), t2(work, &b), t3(work, &c);
+    t1.join(); t2.join(); t3.join();
+    CHECK(pool.idle_bytes() == 0 && Fake::used() == 0);
+    return 0;
+}
+""")
