@@ -290,7 +290,7 @@ __global__ void __launch_bounds__(kRThreads) k_matrix_expect(const typename Elem
 // index are the thread's, and the chunk's other bits run with the target bits outermost, so a thread
 // adds up all indices of one output in float-float and touches the shared histogram once for them (an
 // FP64 shared-memory atomic per probability held the pass to 1.5 TB/s; 26 qubits, 8 targets: 0.69 ->
-// 0.32 ms).
+// 0.32 ms).  The diagonal of a density matrix is summed in FP64 as it is stored: 2^n elements only.
 struct Marg {
     int nbits, k, cb;
     int bit[12];               // target endian bits, ascending
@@ -318,6 +318,7 @@ __global__ void __launch_bounds__(kRThreads) k_marginal(const typename Elem<C64>
         for (uint32_t t = 0; t < nt; t++) {
             const int64_t i0 = (c << d.cb) | deposit(t, d.tmask) | threadIdx.x;
             ffsum acc{0.f, 0.f};
+            double diag = 0.0;
             uint32_t r = 0;          // runs over the submasks of rmask
             for (uint32_t n = 0; n < nr; n += 8) {
                 typename Elem<C64>::T v[8];
@@ -330,10 +331,10 @@ __global__ void __launch_bounds__(kRThreads) k_marginal(const typename Elem<C64>
 #pragma unroll
                 for (int u = 0; u < 8; u++)
                     if (n + u < nr && (int64_t)threadIdx.x < dim) {
-                        const cff a = Elem<C64>::load(v[u]);
                         if (dm) {
-                            fsum_add(acc, a.rh, a.rl);
+                            diag += (double)v[u].x;
                         } else {
+                            const cff a = Elem<C64>::load(v[u]);
                             ffacc q;
                             acc_first(q, a.rh, a.rl, a.rh, a.rl);
                             acc_add(q, a.ih, a.il, a.ih, a.il);
@@ -344,7 +345,7 @@ __global__ void __launch_bounds__(kRThreads) k_marginal(const typename Elem<C64>
             if ((int64_t)threadIdx.x < dim) {
                 int o = 0;
                 for (int q = 0; q < d.k; q++) o |= (int)((i0 >> d.bit[q]) & 1) << q;
-                atomicAdd(&hist[o], ff2d(acc.h, acc.l));
+                atomicAdd(&hist[o], dm ? diag : ff2d(acc.h, acc.l));
             }
         }
     __syncthreads();

@@ -509,3 +509,21 @@ def test_readouts_at_the_kernels_edges(n, precision):
     want = np.searchsorted(cdf, u * cdf[-1])
     # the host's running sum is off by about 1e-16 * sqrt(2^n): a shot that close to a boundary may differ
     assert np.count_nonzero(got != want) <= 2
+
+
+@pytest.mark.parametrize("n", [1, 5, 9])
+def test_marginals_of_a_density_matrix_hold_every_bit(n):
+    """The diagonal is summed in FP64: multiples of 2^-52 whose sum stays below 1 add up exactly in any order, and an
+    element of 2^-130, below FP32's range, stays what it is."""
+    rng = np.random.default_rng(n)
+    d = (rng.integers(1, 1 << (52 - n), 1 << n) | 1) * 2.0 ** -52
+    sim = bs.DensityMatrixSimulator(n, 0)
+    sim.density_matrix = np.diag(d).astype(np.complex128)
+    for t in sorted({1, (n + 1) // 2, n}):
+        q = sorted(int(x) for x in rng.choice(n, t, replace=False))
+        want = d.reshape([2] * n).sum(axis=tuple(x for x in range(n) if x not in q)).ravel()
+        assert np.array_equal(sim.marginal_probabilities(q), want)
+    tiny = np.zeros(1 << n)
+    tiny[0], tiny[-1] = 2.0 ** -130, 0.75
+    sim.density_matrix = np.diag(tiny).astype(np.complex128)
+    assert np.array_equal(sim.marginal_probabilities([0]), [2.0 ** -130, 0.75])
