@@ -211,6 +211,12 @@ int bs_tile_threads(const bs_sim* s) {
     return (t == 512) ? 512 : 256;
 }
 
+// With one tile per SM at most, 16 warps on it instead of 8, where nothing sets the threads.
+int bs_sweep_threads(const bs_sim* s, int64_t ntiles) {
+    if (s->tune.tile_threads < 0 && !getenv("BS_TILE_THREADS") && ntiles <= 152) return 512;
+    return bs_tile_threads(s);
+}
+
 bool bs_tc_enabled(const bs_sim* s) {
     if (s && s->tune.tc >= 0) return s->tune.tc != 0;
     const char* v = getenv("BS_TC");   // read on every call, so a process can compare both paths

@@ -1587,8 +1587,7 @@ int bs_run_sweeps(bs_sim* s, const std::vector<Sweep>& sweeps) {
                 auto kern = ln.kmax <= 2 ? (full ? k_tile_sweep_c64<2, true> : k_tile_sweep_c64<2, false>)
                                          : (full ? k_tile_sweep_c64<4, true> : k_tile_sweep_c64<4, false>);
                 kern<<<(unsigned)nb, kThreads, sm64, s->stream>>>((float2*)s->state, d, t0);
-            } else if (bs_tile_threads(s) == 512 || (s->tune.tile_threads < 0 && ntiles <= 152)) {
-                // one tile per SM at most: 16 warps on it instead of 8
+            } else if (bs_sweep_threads(s, ntiles) == 512) {
                 if (ln.kmax <= 2) k_tile_sweep<2, 512><<<(unsigned)nb, 512, smem, s->stream>>>(psi, d, t0);
                 else k_tile_sweep<4, 512><<<(unsigned)nb, 512, smem, s->stream>>>(psi, d, t0);
             } else {

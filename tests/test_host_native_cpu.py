@@ -111,3 +111,34 @@ int main() {
     return 0;
 }
 """)
+
+
+def test_threads_of_a_sweep_follow_what_is_set(tmp_path):
+    """512 threads for sweeps of up to 152 tiles is the choice where nothing is set: BS_TILE_THREADS and a handle's tuning
+    hold for every size."""
+    cuda = next((p for p in (os.environ.get("CUDA_HOME"), "/usr/local/cuda") if p and os.path.exists(os.path.join(p, "include"))), None)
+    if not cuda:
+        pytest.skip("no CUDA headers")
+    run_cpp(tmp_path, r"""
+#include <cstdio>
+#include <cstdlib>
+#include "bs_internal.h"
+int bs_fail(bs_sim*, int code, const std::string&) { return code; }
+int bs_vec_bits(const bs_sim* s) { return s->n; }
+double bs_fuse_tc(const std::vector<const HostGate*>&, const int*, int, double, std::vector<HostGate>*) { return 0; }
+#define CHECK(x) do { if (!(x)) { std::printf("line %d: %s\n", __LINE__, #x); return 1; } } while (0)
+int main() {
+    bs_sim s;
+    unsetenv("BS_TILE_THREADS");
+    CHECK(bs_sweep_threads(&s, 152) == 512 && bs_sweep_threads(&s, 153) == 256);
+    setenv("BS_TILE_THREADS", "256", 1);
+    CHECK(bs_sweep_threads(&s, 1) == 256 && bs_sweep_threads(&s, 4096) == 256);
+    setenv("BS_TILE_THREADS", "512", 1);
+    CHECK(bs_sweep_threads(&s, 4096) == 512);
+    s.tune.tile_threads = 256;
+    CHECK(bs_sweep_threads(&s, 1) == 256);
+    unsetenv("BS_TILE_THREADS");
+    CHECK(bs_sweep_threads(&s, 1) == 256);
+    return 0;
+}
+""", "-I", os.path.join(cuda, "include"), os.path.join(CSRC, "bs_plan.cpp"))
