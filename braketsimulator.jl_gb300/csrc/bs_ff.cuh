@@ -113,14 +113,6 @@ __device__ __forceinline__ void acc_add(ffacc& a, float ch, float cl, float xh, 
     a.s = t;
     a.c = __fadd_rn(a.c, __fadd_rn(e, err));
 }
-// add a float-float value (no product)
-__device__ __forceinline__ void acc_add_ff(ffacc& a, float xh, float xl) {
-    float t = __fadd_rn(a.s, xh);
-    float bb = __fsub_rn(t, a.s);
-    float err = __fadd_rn(__fsub_rn(a.s, __fsub_rn(t, bb)), __fsub_rn(xh, bb));
-    a.s = t;
-    a.c = __fadd_rn(a.c, __fadd_rn(xl, err));
-}
 __device__ __forceinline__ ff acc_done(const ffacc& a) {
     float s = __fadd_rn(a.s, a.c);
     return {s, __fsub_rn(a.c, __fsub_rn(s, a.s))};
@@ -177,7 +169,6 @@ __device__ __forceinline__ cff cmul(const cff& m, const cff& x) {
     cmac_first(ar, ai, m, x);
     return cdone(ar, ai);
 }
-__device__ __forceinline__ cff cneg(const cff& x) { return {-x.rh, -x.rl, -x.ih, -x.il}; }
 // multiply by i^p (p = 0..3): exact component permutation
 __device__ __forceinline__ cff cmul_ipow(const cff& x, int p) {
     switch (p & 3) {

@@ -7,7 +7,7 @@
 // assignment of those "uniform" bits (at most 3 of them) and each CTA picks its
 // variant.  The products are formed on the device in FP64 (k_tc_build) and applied to
 // the tile as real 64x64 GEMMs on tcgen05 tensor cores, with both operands split
-// into exact 8-bit bf16 digits (an Ozaki-style split) so that the result keeps
+// into exact 9-bit digits carried in bf16 (an Ozaki-style split) so that the result keeps
 // float-float accuracy.  This replaces, for those gates, the per-gate amplitude
 // loops of the reference (src/gate_kernels.jl:489-775, src/custom_gates.jl:364-416);
 // the fused product itself has no counterpart there.
