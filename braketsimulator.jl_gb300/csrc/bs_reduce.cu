@@ -304,8 +304,8 @@ __device__ __forceinline__ uint32_t deposit(uint32_t v, uint32_t mask) {   // th
     }
     return out;
 }
-template <bool C64>
-__global__ void __launch_bounds__(kRThreads) k_marginal(const typename Elem<C64>::T* __restrict__ st, int dm, Marg d,
+template <bool C64, bool DM>
+__global__ void __launch_bounds__(kRThreads) k_marginal(const typename Elem<C64>::T* __restrict__ st, Marg d,
                                                         double* __restrict__ partial) {
     extern __shared__ double hist[];
     const int D = 1 << d.k;
@@ -325,13 +325,13 @@ __global__ void __launch_bounds__(kRThreads) k_marginal(const typename Elem<C64>
 #pragma unroll
                 for (int u = 0; u < 8; u++) {
                     const int64_t i = i0 | r;
-                    if (n + u < nr && (int64_t)threadIdx.x < dim) v[u] = st[dm ? i * (dim + 1) : i];
+                    if (n + u < nr && (int64_t)threadIdx.x < dim) v[u] = st[DM ? i * (dim + 1) : i];
                     r = (r - rmask) & rmask;
                 }
 #pragma unroll
                 for (int u = 0; u < 8; u++)
                     if (n + u < nr && (int64_t)threadIdx.x < dim) {
-                        if (dm) {
+                        if (DM) {
                             diag += (double)v[u].x;
                         } else {
                             const cff a = Elem<C64>::load(v[u]);
@@ -345,7 +345,7 @@ __global__ void __launch_bounds__(kRThreads) k_marginal(const typename Elem<C64>
             if ((int64_t)threadIdx.x < dim) {
                 int o = 0;
                 for (int q = 0; q < d.k; q++) o |= (int)((i0 >> d.bit[q]) & 1) << q;
-                atomicAdd(&hist[o], dm ? diag : ff2d(acc.h, acc.l));
+                atomicAdd(&hist[o], DM ? diag : ff2d(acc.h, acc.l));
             }
         }
     __syncthreads();
@@ -623,11 +623,14 @@ int bs_marginal_probabilities(bs_sim* s, int k, const int* targets, double* host
     int rc = bs_ensure_scratch(s, ((int64_t)nb * D + D) * 8);
     if (rc) return rc;
     double* partial = (double*)s->scratch;
-    const int dm = s->kind == BS_KIND_DM;
-    if (s->precision == BS_PREC_C64)
-        k_marginal<true><<<nb, kRThreads, (size_t)D * 8, s->stream>>>((const float2*)s->state, dm, d, partial);
-    else
-        k_marginal<false><<<nb, kRThreads, (size_t)D * 8, s->stream>>>((const double2*)s->state, dm, d, partial);
+    const bool dm = s->kind == BS_KIND_DM;
+    if (s->precision == BS_PREC_C64) {
+        auto kern = dm ? k_marginal<true, true> : k_marginal<true, false>;
+        kern<<<nb, kRThreads, (size_t)D * 8, s->stream>>>((const float2*)s->state, d, partial);
+    } else {
+        auto kern = dm ? k_marginal<false, true> : k_marginal<false, false>;
+        kern<<<nb, kRThreads, (size_t)D * 8, s->stream>>>((const double2*)s->state, d, partial);
+    }
     k_sum_partials<<<D, 256, 0, s->stream>>>(partial, nb, D, partial + (int64_t)nb * D);
     return bs_copy_out(s, host_out, partial + (int64_t)nb * D, (size_t)D * 8, "marginal");
 }
