@@ -372,9 +372,11 @@ __device__ void tile_kraus_ref_lr(float4* sm, int T, int L, const TileGate& g, c
 }
 
 // KMAX: widest dense/monomial gate of the sweep (2 or 4); narrow sweeps get a
-// kernel with fewer live registers and therefore more resident warps.
+// kernel with fewer live registers and therefore more resident warps.  At 256 threads three or (wide) two
+// CTAs share an SM; without the bound the wide kernel took 186 registers and an SM to itself (one 4-target
+// gate at 21 qubits 140 -> 222 us).
 template <int KMAX, int NT>
-__global__ void __launch_bounds__(NT, NT == 256 && KMAX == 2 ? 3 : 1) k_tile_sweep(double2* __restrict__ psi, SweepDesc d, int64_t tile0) {
+__global__ void __launch_bounds__(NT, NT == 256 ? (KMAX == 2 ? 3 : 2) : 1) k_tile_sweep(double2* __restrict__ psi, SweepDesc d, int64_t tile0) {
     extern __shared__ float4 smem[];
     const int T = d.T, L = d.L, H = T - L;
     const int nt = 1 << T;
