@@ -94,23 +94,23 @@ __device__ __forceinline__ void pauli_accumulate(ffsum (&acc)[NT], const TermSet
     }
 }
 
-// Last block of the call (its launches' blocks add up to last_total in *done): every partial is there,
-// so its warps form the results, one slot each at a time (FP64 sums with compensated leaves), and the
-// counter goes back to zero.  A launch fewer per call than a separate pass over the partials, which
-// took 2.5 to 5 us of device time; with the results and a ticket in mapped memory the host polls,
-// instead of a copy and a stream synchronisation.
+// Last block of the call's last launch (the others pass a null `done`: they have ended when it starts): every
+// partial is there, so its warps form the results, one slot each at a time (FP64 sums with compensated
+// leaves), and the counter goes back to zero.  A launch fewer per call than a separate pass over the
+// partials, which took 2.5 to 5 us of device time; with the results and a ticket in mapped memory the host
+// polls, instead of a copy and a stream synchronisation.
 struct Finish {
     double* out;            // results (device, or host memory mapped into its address space)
-    unsigned* done;
-    unsigned last_total;
+    unsigned* done;         // counts the launch's blocks
     volatile int64_t* word; // ticket word of a waiting host (null: none)
     int64_t ticket;
 };
 __device__ void finish_partials(double* partial, int nblocks, int n_slots, const Finish& f) {
     __shared__ bool s_last;
+    if (!f.done) return;    // uniform
     __threadfence();
     __syncthreads();
-    if (threadIdx.x == 0) s_last = atomicAdd(f.done, 1u) + 1u == f.last_total;
+    if (threadIdx.x == 0) s_last = atomicAdd(f.done, 1u) + 1u == gridDim.x;
     __syncthreads();
     if (!s_last) return;
     __threadfence();
@@ -523,7 +523,7 @@ int bs_expectation_pauli(bs_sim* s, int n_terms, const uint64_t* xmask, const ui
     unsigned launches = 0;
     for (auto& kv : groups) launches += (unsigned)((kv.second.size() + kMaxTermsPerPass - 1) / kMaxTermsPerPass);
     const MapSlot slot = s->capturing ? MapSlot{} : bs_map_slot((size_t)n_terms * 8);
-    const Finish fin{slot.h ? (double*)slot.d : res, bs_scratch_counter(s), launches * (unsigned)nb, slot.dword, slot.ticket};
+    Finish fin{slot.h ? (double*)slot.d : res, nullptr, slot.dword, slot.ticket};
     for (auto& kv : groups) {
         const std::vector<int>& ts = kv.second;
         for (size_t c0 = 0; c0 < ts.size(); c0 += kMaxTermsPerPass) {
@@ -535,6 +535,7 @@ int bs_expectation_pauli(bs_sim* s, int n_terms, const uint64_t* xmask, const ui
                 set.ph[j] = ph[t];
                 set.slot[j] = t;
             }
+            if (--launches == 0) fin.done = bs_scratch_counter(s);
             if (s->precision == BS_PREC_C64) launch_pauli<true>(s, nb, dim, kv.first, set, partial, n_terms, fin);
             else launch_pauli<false>(s, nb, dim, kv.first, set, partial, n_terms, fin);
         }
@@ -548,8 +549,8 @@ int bs_expectation_pauli(bs_sim* s, int n_terms, const uint64_t* xmask, const ui
         rc = bs_copy_out(s, out, res, (size_t)n_terms * 8, "expectation");
     }
     if (s->capturing) return rc;
-    if (rc) {   // launches that ran without the others leave the counter short of its total: the next call starts at zero
-        cudaMemsetAsync(fin.done, 0, sizeof(unsigned), s->stream);
+    if (rc) {   // a launch that did not end leaves the counter where it was: the next call starts at zero
+        cudaMemsetAsync(bs_scratch_counter(s), 0, sizeof(unsigned), s->stream);
         return rc;
     }
     if (coeffs)
