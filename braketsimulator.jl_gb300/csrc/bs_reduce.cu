@@ -17,6 +17,7 @@
 #include <vector>
 #include "bs_internal.h"
 #include "bs_ff.cuh"
+#include "bs_cdf.cuh"
 
 namespace {
 
@@ -290,7 +291,11 @@ __global__ void __launch_bounds__(kRThreads) k_matrix_expect(const typename Elem
 // index are the thread's, and the chunk's other bits run with the target bits outermost, so a thread
 // adds up all indices of one output in float-float and touches the shared histogram once for them (an
 // FP64 shared-memory atomic per probability held the pass to 1.5 TB/s; 26 qubits, 8 targets: 0.69 ->
-// 0.32 ms).  The diagonal of a density matrix is summed in FP64 as it is stored: 2^n elements only.
+// 0.32 ms).  U positions are in flight at a time, as many as a thread has of one output (up to 8; at 8 for every
+// size the steps left out were still issued, and 19 qubits took 12.6 us in the kernel for 6.4 before).  The diagonal
+// of a density matrix is summed in FP64 as it is stored: 2^n elements only.  Where no target is among the low 5
+// bits a warp adds to one place: its sums are added up first (32 additions to one address in turn held such target
+// sets to 2.2 ms at 26 qubits).
 struct Marg {
     int nbits, k, cb;
     int bit[12];               // target endian bits, ascending
@@ -304,7 +309,7 @@ __device__ __forceinline__ uint32_t deposit(uint32_t v, uint32_t mask) {   // th
     }
     return out;
 }
-template <bool C64, bool DM>
+template <bool C64, bool DM, int U>
 __global__ void __launch_bounds__(kRThreads) k_marginal(const typename Elem<C64>::T* __restrict__ st, Marg d,
                                                         double* __restrict__ partial) {
     extern __shared__ double hist[];
@@ -320,17 +325,17 @@ __global__ void __launch_bounds__(kRThreads) k_marginal(const typename Elem<C64>
             ffsum acc{0.f, 0.f};
             double diag = 0.0;
             uint32_t r = 0;          // runs over the submasks of rmask
-            for (uint32_t n = 0; n < nr; n += 8) {
-                typename Elem<C64>::T v[8];
+            for (uint32_t n = 0; n < nr; n += U) {   // nr, a power of two, is a multiple of U
+                typename Elem<C64>::T v[U];
 #pragma unroll
-                for (int u = 0; u < 8; u++) {
+                for (int u = 0; u < U; u++) {
                     const int64_t i = i0 | r;
-                    if (n + u < nr && (int64_t)threadIdx.x < dim) v[u] = st[DM ? i * (dim + 1) : i];
+                    if ((int64_t)threadIdx.x < dim) v[u] = st[DM ? i * (dim + 1) : i];
                     r = (r - rmask) & rmask;
                 }
 #pragma unroll
-                for (int u = 0; u < 8; u++)
-                    if (n + u < nr && (int64_t)threadIdx.x < dim) {
+                for (int u = 0; u < U; u++)
+                    if ((int64_t)threadIdx.x < dim) {
                         if (DM) {
                             diag += (double)v[u].x;
                         } else {
@@ -342,7 +347,12 @@ __global__ void __launch_bounds__(kRThreads) k_marginal(const typename Elem<C64>
                         }
                     }
             }
-            if ((int64_t)threadIdx.x < dim) {
+            const bool one = d.bit[0] >= 5;   // a warp's indices (all below dim, or none) have one output: one addition for them
+            if (one) {
+                if (DM) for (int s = 16; s > 0; s >>= 1) diag += __shfl_down_sync(0xffffffffu, diag, s);
+                else ff_warp_sum(acc);
+            }
+            if ((int64_t)threadIdx.x < dim && (!one || (threadIdx.x & 31) == 0)) {
                 int o = 0;
                 for (int q = 0; q < d.k; q++) o |= (int)((i0 >> d.bit[q]) & 1) << q;
                 atomicAdd(&hist[o], DM ? diag : ff2d(acc.h, acc.l));
@@ -625,13 +635,17 @@ int bs_marginal_probabilities(bs_sim* s, int k, const int* targets, double* host
     if (rc) return rc;
     double* partial = (double*)s->scratch;
     const bool dm = s->kind == BS_KIND_DM;
+    const int traced = d.cb - 8 - __builtin_popcount(d.tmask);   // 2^traced positions of an output per thread and chunk
     if (s->precision == BS_PREC_C64) {
-        auto kern = dm ? k_marginal<true, true> : k_marginal<true, false>;
+        auto kern = dm ? k_marginal<true, true, 1> : traced >= 3 ? k_marginal<true, false, 8> : traced == 2 ? k_marginal<true, false, 4>
+                  : traced == 1 ? k_marginal<true, false, 2> : k_marginal<true, false, 1>;
         kern<<<nb, kRThreads, (size_t)D * 8, s->stream>>>((const float2*)s->state, d, partial);
     } else {
-        auto kern = dm ? k_marginal<false, true> : k_marginal<false, false>;
+        auto kern = dm ? k_marginal<false, true, 1> : traced >= 3 ? k_marginal<false, false, 8> : traced == 2 ? k_marginal<false, false, 4>
+                  : traced == 1 ? k_marginal<false, false, 2> : k_marginal<false, false, 1>;
         kern<<<nb, kRThreads, (size_t)D * 8, s->stream>>>((const double2*)s->state, d, partial);
     }
+    if (nb == 1) return bs_copy_out(s, host_out, partial, (size_t)D * 8, "marginal");   // one block's sums are the result
     k_sum_partials<<<D, 256, 0, s->stream>>>(partial, nb, D, partial + (int64_t)nb * D);
     return bs_copy_out(s, host_out, partial + (int64_t)nb * D, (size_t)D * 8, "marginal");
 }

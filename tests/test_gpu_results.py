@@ -527,3 +527,15 @@ def test_marginals_of_a_density_matrix_hold_every_bit(n):
     tiny[0], tiny[-1] = 2.0 ** -130, 0.75
     sim.density_matrix = np.diag(tiny).astype(np.complex128)
     assert np.array_equal(sim.marginal_probabilities([0]), [2.0 ** -130, 0.75])
+
+
+@pytest.mark.parametrize("targets", [[0], [11, 12, 13], [12, 13], [13], [3, 11], [11, 12, 13, 21], [14, 16, 21], [0, 5, 12, 20]])
+@pytest.mark.parametrize("precision", ["c128", "c64"])
+def test_marginals_by_traced_positions(targets, precision):
+    """22 qubits: chunks of 2^11 indices, in which a thread adds up 8, 4, 2 or 1 positions of an output by the targets
+    among the index bits 8 to 10 (qubits 11 to 13); FP64-grade sums of the stored state's probabilities."""
+    n = 22
+    sim = _dense_state(n, 5, precision=precision)
+    p = (np.abs(sim.state_vector) ** 2).reshape([2] * n)
+    ref = p.sum(axis=tuple(q for q in range(n) if q not in targets)).ravel()
+    assert np.max(np.abs(sim.marginal_probabilities(targets) - ref)) < 1e-13
