@@ -322,11 +322,13 @@ double tc_plan_cost(const bs_sim* s, const std::vector<HostGate>& gates, int T, 
 
 // Whether a list runs in tensor-core sweeps: from bs_tc_min_bits vector bits; and, where nothing sets those, below
 // the default of 22 for the lists the float-float path is slowest at, counted in its time for a dense 1-qubit gate.
-// Wide gates (3 and 4 targets, the two-qubit channels of a density matrix among them) from 16 bits: 8-qubit density
-// matrix with channels, 1 layer 0.42 -> 0.21 ms, 10 qubits, 4 layers 5.05 -> 0.87.  Generic complex matrices from 20
-// bits: 6 dense layers of 20 qubits 0.64 -> 0.29 ms, 2 layers 0.23 -> 0.15; at 19 bits with 2 layers they lose what
-// the matrices' forming takes (0.14 both).  Of those lists the error against FP64 is lower too (1.7e-14 of the norm
-// for 3.3e-14 at 20 qubits).  Real rotations and H, which cost the float-float path half, stay there: 21 qubits of
+// Gates on 4 targets (the two-qubit channels of a density matrix among them) from 16 bits: 8-qubit density
+// matrix with channels, 1 layer 0.42 -> 0.21 ms, 10 qubits, 4 layers 5.05 -> 0.87; three gates 0.18 -> 0.15 at 17
+// qubits.  Gates on 3 targets lose there (17 qubits, 6 of them 0.13 -> 0.19, 40 even) and count as generic ones.
+// Generic complex matrices from 20 bits: 6 dense layers of 20 qubits 0.64 -> 0.29 ms, 2 layers 0.23 -> 0.15; at 19
+// bits with 2 layers they lose what the matrices' forming takes (0.14 both).  Of those lists the norm-wise error
+// against FP64 is lower too (1.6e-14 for 2.7e-14 at 20 qubits; 0.7e-14 for 2.0e-14 of an 8-qubit density matrix); single
+// elements far below a tile's largest lose a digit or two (there, relative, 7e-12 for 2e-13).  Real rotations and H, which cost the float-float path half, stay there: 21 qubits of
 // them would gain time, but the error grows by up to a fifth.
 bool use_tc(const bs_sim* s, const std::vector<HostGate>& gates, int n_bits) {
     if (!bs_tc_enabled(s) || s->precision != BS_PREC_C128 || bs_tile_bits(s) != BS_TILE_MAX_BITS || n_bits < BS_TILE_MAX_BITS)
@@ -338,7 +340,7 @@ bool use_tc(const bs_sim* s, const std::vector<HostGate>& gates, int n_bits) {
         if (g.kind != 0 || (g.k == 1 && bs_class_2x2(g))) continue;
         const double cost = (double)(1 << g.k) / 2.0;
         generic += cost;
-        if (g.k >= 3) wide += cost;
+        if (g.k >= 4) wide += cost;
     }
     return wide >= 24 || (n_bits >= 20 && generic >= 40);
 }

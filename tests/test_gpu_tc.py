@@ -269,3 +269,15 @@ def test_products_out_of_range_run_on_the_float_float_sweeps(n, kind, tune, same
             bs.set_tuning(sim, tc_min_bits=12)
         got, ref = sim.evolve(ops).state_vector, oracle.OracleSV(n).evolve(ops).psi
     assert rel_err(got, ref) < TOL
+
+
+@pytest.mark.parametrize("n,gates,tc", [(16, 6, False), (17, 12, False), (19, 24, False), (20, 12, True), (21, 3, False)])
+def test_gates_on_three_targets_below_22_bits(n, gates, tc):
+    """Lists of 3-target gates stay on the float-float sweeps below 20 bits, which are faster for them, and count as
+    generic matrices from there (at least 40 units of a dense 1-qubit gate, 4 each); the states against the oracle."""
+    rng = np.random.default_rng(90 + n)
+    ops = [bs.Instruction(bs.H(), [q]) for q in range(n)]
+    ops += [bs.Instruction(bs.Unitary(haar(rng, 8)), [int(x) for x in rng.permutation(n)[:3]]) for _ in range(gates)]
+    sim = bs.StateVectorSimulator(n, 0).evolve(ops)
+    assert (sim.last_stats()["tc_gates"] > 0) == tc
+    assert rel_err(sim.state_vector, oracle.OracleSV(n).evolve(ops).psi) < TOL
