@@ -1996,7 +1996,10 @@ int bs_small_pack(const bs_sim* s, const std::vector<Sweep>& sweeps, SmallPlan& 
     const int n = s->n;
     if (s->kind != BS_KIND_SV || s->precision != BS_PREC_C128 || n > 12) return BS_ERR_UNSUPPORTED;
     const int T = std::min(bs_sweep_tile_bits(s), n), L = BS_TILE_LOW_BITS;
-    const bool cluster = T == kSmallTileBits && n > T;   // else the whole state is the tile, whatever the sweeps
+    // One CTA has the whole state as its tile, whatever the sweeps.  Its launch is 3 to 4 us cheaper than a cluster's, which
+    // takes 0.5 to 1 us less for a gate (11 qubits, a call of 1 gate 26 and 31 us, of 5 gates 35 both); only lists of one
+    // sweep may take it, since a value is rounded to complex128 between two.
+    const bool cluster = T == kSmallTileBits && n > T && (sweeps.size() > 1 || (!sweeps.empty() && sweeps[0].gates.size() > 4));
     std::vector<TileGate>& tg = out.tg;
     std::vector<float4>& mats = out.mats;
     std::vector<int32_t>& perms = out.perms;
@@ -2056,12 +2059,6 @@ int bs_small_pack(const bs_sim* s, const std::vector<Sweep>& sweeps, SmallPlan& 
             tg.push_back(t);
         }
         if (cluster) out.sweeps.back().ng = (int32_t)tg.size() - out.sweeps.back().g0;
-    }
-    if (cluster && out.sweeps.empty()) {   // no gate: |0...0> still has to be written
-        SmallSweep w{};
-        for (int q = 0; q < T - L; q++) w.hi[q] = (int8_t)(L + q);
-        for (int b = T, r = 0; b < n; b++) w.out[r++] = (int8_t)b;
-        out.sweeps.push_back(w);
     }
     out.kmax = kmax;
     return BS_OK;

@@ -141,3 +141,19 @@ def test_simulate_uses_the_small_path_with_the_same_measurements():
     m = r["measurements"]
     assert m.shape == (400, 5)
     assert np.all((m == 0).all(axis=1) | (m == 1).all(axis=1))
+
+
+@pytest.mark.parametrize("n", [11, 12])
+@pytest.mark.parametrize("gates", [0, 1, 3, 4, 5, 8])
+@pytest.mark.parametrize("spread", [False, True])
+def test_run_of_short_lists_in_one_cta_or_a_cluster(n, gates, spread):
+    """11 and 12 qubits: lists of one sweep and up to 4 gates run in one CTA, others in a cluster; the probabilities are
+    evolve's bit by bit and the shots samples(seed)'s on either side of the line."""
+    rng = np.random.default_rng(10 * n + gates)
+    qs = range(n) if spread else range(n - 5, n)   # the low index bits are in every tile
+    ops = [bs.Instruction(bs.U(*(float(a) for a in rng.uniform(-3, 3, 3))), [qs[(3 * i) % len(qs)]]) for i in range(gates)]
+    sim, ref = bs.StateVectorSimulator(n, 200), bs.StateVectorSimulator(n, 200)
+    p, shots = sim.run(ops, 200, seed=7)
+    ref.evolve(ops)
+    assert np.array_equal(p, ref.probabilities()) and np.array_equal(sim.state_vector, ref.state_vector)
+    assert np.array_equal(shots, ref.samples(seed=7))
