@@ -325,20 +325,6 @@ void small_image(char* img, const SmallLayout& L, const std::vector<BCirc>& bc, 
 
 uint64_t circuit_seed(uint64_t seed, int c) { return seed ^ ((uint64_t)c * 0x9E3779B97F4A7C15ULL); }
 
-// Handles (one stream each) that run the larger circuits side by side (BS_BATCH_STREAMS, at most 64; else 4, or
-// 8 for a batch run at once whose lists have 8192 instructions or more).  Replays of a captured batch do not depend
-// on it (4, 16 and 32 took the same time on 512 circuits of up to 26 qubits: the largest circuits' sweeps fill the
-// GPU on their own).  A batch run at once plans each handle's next circuit on its own thread, but a handle takes
-// 0.25 ms to set up and give back: 48 circuits of 12 to 22 qubits, 14 thousand instructions, 18.7 ms on 4, 17.2 on
-// 8, 19.1 on 16; 14 circuits of 12 to 16 qubits, 4 thousand, 5.2 on 4 and 6.1 on 8.
-int batch_pool_size(size_t n_large, int64_t n_ops) {
-    static const int set = [] {
-        const char* v = getenv("BS_BATCH_STREAMS");
-        return v ? std::max(1, std::min(64, atoi(v))) : 0;
-    }();
-    return (int)std::min<size_t>(n_large, (size_t)(set ? set : n_ops >= 8192 ? 8 : 4));
-}
-
 void add_stats(bs_stats& a, const bs_stats& b) {
     a.sweeps += b.sweeps;
     a.kernel_launches += b.kernel_launches;
@@ -408,8 +394,12 @@ extern "C" int bs_run_batch(int n_circuits, const int* n_qubits, const bs_op* co
     std::atomic<int> err{0};
     std::sort(large.begin(), large.end(), [&](int a, int b) { return n_qubits[a] > n_qubits[b]; });
     int64_t large_ops = 0;
-    for (int c : large) large_ops += n_ops[c];
-    const int workers = batch_pool_size(large.size(), large_ops);
+    double eight = 0;   // bytes of the states that eight handles would hold at once
+    for (size_t i = 0; i < large.size(); i++) {
+        large_ops += n_ops[large[i]];
+        if (i < 8) eight += std::ldexp(precision == BS_PREC_C64 ? 8.0 : 16.0, n_qubits[large[i]]);
+    }
+    const int workers = bs_batch_handles(large.size(), large_ops, eight);
     std::vector<bs_stats> wst((size_t)std::max(workers, 1));
     int dev = 0;
     cudaGetDevice(&dev);
@@ -717,7 +707,7 @@ int bs_batch_create(int n_circuits, const int* n_qubits, const bs_op* const* ops
     for (int c = 0; c < n_circuits; c++) (small_ok(precision, n_qubits[c], ops[c], n_ops[c]) ? b->small : b->large).push_back(c);
     // largest first onto the handle with the least work so far (work ~ 2^n)
     std::sort(b->large.begin(), b->large.end(), [&](int x, int y) { return n_qubits[x] > n_qubits[y] || (n_qubits[x] == n_qubits[y] && x < y); });
-    const int workers = batch_pool_size(b->large.size(), 0);
+    const int workers = bs_batch_handles(b->large.size(), 0, 0.0);
     std::vector<double> load((size_t)workers, 0.0);
     std::vector<int> wmax((size_t)workers, 1);
     b->owner.assign((size_t)n_circuits, -1);

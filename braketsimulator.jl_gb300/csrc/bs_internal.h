@@ -252,6 +252,7 @@ int bs_class_2x2(const HostGate& h);
 int bs_tile_bits(const bs_sim* s);
 int bs_sweep_tile_bits(const bs_sim* s);   // tile bits the sweeps use for the handle's size
 int bs_tile_threads(const bs_sim* s);
+int bs_batch_handles(size_t n_large, int64_t n_ops, double eight_bytes);   // handles of a batch
 int bs_sweep_threads(const bs_sim* s, int64_t ntiles);   // threads of a float-float sweep over that many tiles
 bool bs_tc_enabled(const bs_sim* s);
 int bs_tc_min_bits(const bs_sim* s);

@@ -217,6 +217,19 @@ int bs_sweep_threads(const bs_sim* s, int64_t ntiles) {
     return bs_tile_threads(s);
 }
 
+// Handles (one stream each) that run the larger circuits of a batch side by side (BS_BATCH_STREAMS, at most 64; else 4,
+// or 8 for a batch run at once whose lists have 8192 instructions or more).  Replays of a captured batch do not depend
+// on it (4, 16 and 32 took the same time on 512 circuits of up to 26 qubits: the largest circuits' sweeps fill the
+// GPU on their own).  A batch run at once plans each handle's next circuit on its own thread, but a handle takes
+// 0.25 ms to set up and give back: 48 circuits of 12 to 22 qubits, 14 thousand instructions, 18.7 ms on 4, 17.2 on
+// 8, 19.1 on 16; 14 circuits of 12 to 16 qubits, 4 thousand, 5.2 on 4 and 6.1 on 8.  Each handle holds a state, so
+// eight are taken only where theirs are 8 GiB together: larger ones fill the GPU from four.
+int bs_batch_handles(size_t n_large, int64_t n_ops, double eight_bytes) {
+    const char* v = getenv("BS_BATCH_STREAMS");
+    const int set = v ? std::max(1, std::min(64, atoi(v))) : 0;
+    return (int)std::min<size_t>(n_large, (size_t)(set ? set : n_ops >= 8192 && eight_bytes <= 8.0 * (1 << 30) ? 8 : 4));
+}
+
 bool bs_tc_enabled(const bs_sim* s) {
     if (s && s->tune.tc >= 0) return s->tune.tc != 0;
     const char* v = getenv("BS_TC");   // read on every call, so a process can compare both paths

@@ -113,13 +113,7 @@ int main() {
 """)
 
 
-def test_threads_of_a_sweep_follow_what_is_set(tmp_path):
-    """512 threads for sweeps of up to 152 tiles is the choice where nothing is set: BS_TILE_THREADS and a handle's tuning
-    hold for every size."""
-    cuda = next((p for p in (os.environ.get("CUDA_HOME"), "/usr/local/cuda") if p and os.path.exists(os.path.join(p, "include"))), None)
-    if not cuda:
-        pytest.skip("no CUDA headers")
-    run_cpp(tmp_path, r"""
+PLAN = r"""
 #include <cstdio>
 #include <cstdlib>
 #include "bs_internal.h"
@@ -127,6 +121,20 @@ int bs_fail(bs_sim*, int code, const std::string&) { return code; }
 int bs_vec_bits(const bs_sim* s) { return s->n; }
 double bs_fuse_tc(const std::vector<const HostGate*>&, const int*, int, double, std::vector<HostGate>*) { return 0; }
 #define CHECK(x) do { if (!(x)) { std::printf("line %d: %s\n", __LINE__, #x); return 1; } } while (0)
+"""
+
+
+def run_plan(tmp_path, main):
+    cuda = next((p for p in (os.environ.get("CUDA_HOME"), "/usr/local/cuda") if p and os.path.exists(os.path.join(p, "include"))), None)
+    if not cuda:
+        pytest.skip("no CUDA headers")
+    run_cpp(tmp_path, PLAN + main, "-I", os.path.join(cuda, "include"), os.path.join(CSRC, "bs_plan.cpp"))
+
+
+def test_threads_of_a_sweep_follow_what_is_set(tmp_path):
+    """512 threads for sweeps of up to 152 tiles is the choice where nothing is set: BS_TILE_THREADS and a handle's tuning
+    hold for every size."""
+    run_plan(tmp_path, r"""
 int main() {
     bs_sim s;
     unsetenv("BS_TILE_THREADS");
@@ -141,4 +149,21 @@ int main() {
     CHECK(bs_sweep_threads(&s, 1) == 256);
     return 0;
 }
-""", "-I", os.path.join(cuda, "include"), os.path.join(CSRC, "bs_plan.cpp"))
+""")
+
+
+def test_eight_handles_of_a_batch_hold_at_most_8_gib(tmp_path):
+    """Eight handles for lists of 8192 instructions and more, unless their states take more than 8 GiB together; four
+    otherwise; never more than circuits; BS_BATCH_STREAMS as set."""
+    run_plan(tmp_path, r"""
+int main() {
+    const double gib = 1 << 30;
+    unsetenv("BS_BATCH_STREAMS");
+    CHECK(bs_batch_handles(48, 8191, gib) == 4 && bs_batch_handles(48, 8192, gib) == 8);
+    CHECK(bs_batch_handles(48, 100000, 8 * gib) == 8 && bs_batch_handles(48, 100000, 8.5 * gib) == 4);
+    CHECK(bs_batch_handles(3, 100000, gib) == 3 && bs_batch_handles(0, 0, 0) == 0);
+    setenv("BS_BATCH_STREAMS", "6", 1);
+    CHECK(bs_batch_handles(48, 100000, 128 * gib) == 6 && bs_batch_handles(48, 1, gib) == 6);
+    return 0;
+}
+""")
