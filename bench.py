@@ -147,9 +147,10 @@ def peaks():
 
 # Tensor-core sweep (k_tile_sweep_tc): executed bf16 MMA work per fused gate per 2^12-amplitude tile
 # (21 digit pairs x 4 k-steps, each M=128 N=64 K=16), and the DRAM bytes per amplitude per launch that
-# ncu measured for it on the 27-qubit dense circuit (2.1488e9 read + 2.0865e9 written per launch).
+# ncu measured for it on a 27-qubit dense circuit (3 low bits, persistent CTAs: 2.1489e9 read + 2.0872e9 written
+# per launch, profiles/k_tile_sweep_tc_dense27q.md).
 TC_FLOP_PER_TILE_GATE = 84 * 2 * 128 * 64 * 16
-TC_DRAM_BYTES_PER_AMP = (2.148804e9 + 2.086545e9) / 2 ** 27
+TC_DRAM_BYTES_PER_AMP = (2.148857e9 + 2.087174e9) / 2 ** 27
 
 
 def workload_name():
