@@ -145,7 +145,7 @@ struct DeviceMem {
     }
     static void put(void* p) { cudaFree(p); }
 };
-KeepPool<DeviceMem> g_keep(kKeepAll);
+KeepPool<DeviceMem>& g_keep = *new KeepPool<DeviceMem>(kKeepAll);   // outlives handles that are destroyed at exit
 }  // namespace
 
 cudaError_t bs_malloc(void** p, size_t bytes) {
